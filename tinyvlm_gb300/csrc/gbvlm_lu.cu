@@ -225,13 +225,21 @@ __device__ __forceinline__ void static_for(F&& f) {
 // Shared state of the register panel (dynamic shared memory, so the
 // out-of-line pivot exchange below addresses the same buffers).
 template <class T, int NT, bool CLUSTER>
-struct PanelSmem {
+struct PanelSmem {  // rows are read and written as 16-byte vectors
     static constexpr int NW = NT / 32;
     static constexpr int CM = CLUSTER ? PR_MAX_CLUSTER : 1;
     T s_row[2][NW][GK];  // each warp's candidate row
     T c_row[2][CM][GK];  // candidate rows pushed by the CTAs of the cluster
     PivKey<T> s_key[2][NW];
     PivKey<T> c_key[2][CM];
+    // the attempt without interchanges: per slice the diagonal block's rows of
+    // U (row-major) and the reciprocals of its pivots; in a cluster the CTAs'
+    // verdicts
+    static constexpr int MS = CLUSTER || NT < 2 * PACK_MIN_SLICE ? 1 : NT / PACK_MIN_SLICE;
+    alignas(16) T f_u[MS][GK][GK];
+    T f_rd[MS][GK];
+    int f_bad[MS];
+    int f_cta[CM];
 };
 
 template <class T>
@@ -313,6 +321,69 @@ __device__ __noinline__ PivotOut<T> panel_exchange(int buf, int csize, int rank,
     return o;
 }
 
+// Barrier of the panel's threads: the whole CTA in a cluster, the slice's
+// remaining warps otherwise (barrier 1 + slice, as in panel_exchange).
+template <int NT, bool CLUSTER>
+__device__ __forceinline__ void panel_barrier(int nwa, int bar) {
+    if constexpr (CLUSTER) {
+        __syncthreads();
+    } else {
+        constexpr int MS = NT >= 2 * PACK_MIN_SLICE ? NT / PACK_MIN_SLICE : 1;
+        static_for<1, MS + 1>([&](auto BI) {
+            constexpr int id = decltype(BI)::value;
+            if (bar == id) asm volatile("bar.sync %0, %1;" ::"n"(id), "r"(nwa * 32) : "memory");
+        });
+    }
+}
+
+// The diagonal block without interchanges, one warp, lane r holding row r:
+// the rows of U and the pivots' reciprocals go to shared memory.  Returns
+// false (in every lane) where partial pivoting would have left the diagonal,
+// or where a pivot is zero, subnormal or not a number.  Each row sees the
+// operations of the pivoting loop in their order.
+template <class T>
+__device__ __forceinline__ bool panel_diag(T (&x)[GK], int nb, T (*u)[GK], T* rds, int lane) {
+    using V2 = typename Vec4<T>::type;
+    bool good = true;
+    static_for<0, GK>([&](auto JJ) {
+        constexpr int jj = decltype(JJ)::value;
+        if (jj < nb) {
+            const T d = __shfl_sync(0xffffffffu, x[jj], jj);
+            if (lane == jj) {  // row jj of U is final
+#pragma unroll
+                for (int t = jj & ~3; t < GK; t += 4) {
+                    V2 v;
+                    v.x = x[t];
+                    v.y = x[t + 1];
+                    v.z = x[t + 2];
+                    v.w = x[t + 3];
+                    *reinterpret_cast<V2*>(&u[jj][t]) = v;
+                }
+            }
+            const T rd = rcp_rn(d);
+            if (lane == jj) rds[jj] = rd;
+            __syncwarp();
+            const bool below = lane > jj && lane < nb;
+            good = good && tabs(d) >= (sizeof(T) == 4 ? (T)FLT_MIN : (T)DBL_MIN) &&
+                   (!below || tabs(x[jj]) <= tabs(d));
+            if (below) {
+                const T lm = x[jj] * rd;
+                x[jj] = lm;
+                const uint32_t ua = (uint32_t)__cvta_generic_to_shared(&u[jj][0]);
+#pragma unroll
+                for (int tg = (jj + 1) & ~3; tg < GK; tg += 4) {
+                    T v[4];
+                    lds4(ua + tg * (uint32_t)sizeof(T), v);
+#pragma unroll
+                    for (int e = 0; e < 4; e++)
+                        if (tg + e > jj) x[tg + e] -= lm * v[e];
+                }
+            }
+        }
+    });
+    return __all_sync(0xffffffffu, good);
+}
+
 template <class T, int NT, bool CLUSTER, int RPT>
 __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const int32_t* act, int slab, int trim,
                                                    const int32_t* pack, int count) {
@@ -369,12 +440,83 @@ __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const
 #pragma unroll
         for (int t = 0; t < GK; t++) x[i][t] = (lid[i] >= 0 && t < nb) ? src[t * ld] : (T)0;
     }
+
+    // Attempt without interchanges.  The pivot search is the panel's serial
+    // chain (a barrier, two reductions and a broadcast per column); if every
+    // pivot is the diagonal, as it is throughout an AIC, none of it is needed.
+    // So one warp factors the 32 x 32 diagonal block, the other rows are
+    // eliminated against it, each on its own, and every row checks on the way
+    // that |a| <= |pivot| held in each column: exactly then partial pivoting
+    // would have kept the diagonal (it comes first on ties).  The operations
+    // of a row and their order are those of the pivoting loop, so the factors
+    // are the same bits; nothing is written before the verdict.  A panel that
+    // fails is read again and takes the pivoting loop, and so, without an
+    // attempt, does one whose predecessor moved rows.
+    bool fast = false;
+    if constexpr (RPT == 1) {
+        const bool tried =
+            k < GK || __all_sync(0xffffffffu, ipiv[k - GK + lane] == (int32_t)(k - GK + lane));
+        if (tried) {
+            T(*fu)[GK] = sm.f_u[slice];
+            T* frd = sm.f_rd[slice];
+            auto load_row = [&](int r, bool have) {
+                const T* src = A + (k + r) + k * ld;
+#pragma unroll
+                for (int t = 0; t < GK; t++) x[0][t] = (have && t < nb) ? src[t * ld] : (T)0;
+            };
+            bool good = true;
+            const bool first = tid < 32;  // the slice's first warp factors the diagonal block
+            if (first) {
+                if (rank != 0) load_row(lane, lane < nb);  // rank 0's first warp holds those rows
+                good = panel_diag<T>(x[0], nb, fu, frd, lane);
+                if (rank != 0) load_row(lid[0], lid[0] >= 0);
+                if (lane == 0) sm.f_bad[slice] = good ? 0 : 1;
+            }
+            panel_barrier<NT, CLUSTER>(nwa, bar);
+            if (good && sm.f_bad[slice] == 0 && !(first && rank == 0)) {
+                static_for<0, GK>([&](auto JJ) {
+                    constexpr int jj = decltype(JJ)::value;
+                    if (jj < nb) {
+                        const uint32_t ua = (uint32_t)__cvta_generic_to_shared(&fu[jj][0]);
+                        const T d = lds1(ua + jj * (uint32_t)sizeof(T), T(0));
+                        good = good && tabs(x[0][jj]) <= tabs(d);
+                        const T lm = x[0][jj] * frd[jj];
+                        x[0][jj] = lm;
+#pragma unroll
+                        for (int tg = (jj + 1) & ~3; tg < GK; tg += 4) {
+                            T v[4];
+                            lds4(ua + tg * (uint32_t)sizeof(T), v);
+#pragma unroll
+                            for (int e = 0; e < 4; e++)
+                                if (tg + e > jj) x[0][tg + e] -= lm * v[e];
+                        }
+                    }
+                });
+                if (lid[0] < 0) good = true;  // no row
+            }
+            // the verdict of the slice, or of every CTA of the cluster
+            if (!__all_sync(0xffffffffu, good) && lane == 0) sm.f_bad[slice] = 1;
+            panel_barrier<NT, CLUSTER>(nwa, bar);
+            fast = *(volatile int*)&sm.f_bad[slice] == 0;
+            if constexpr (CLUSTER) {
+                cg::cluster_group cl = cg::this_cluster();
+                if (tid < csize) *cl.map_shared_rank(&sm.f_cta[rank], tid) = fast ? 0 : 1;
+                cl.sync();
+                fast = __all_sync(0xffffffffu, lane >= csize || *(volatile int*)&sm.f_cta[lane < csize ? lane : 0] == 0);
+            }
+            if (fast) {
+                if (rank == 0 && tid < nb) ipiv[k + tid] = (int32_t)(k + tid);
+            } else {
+                load_row(lid[0], lid[0] >= 0);
+            }
+        }
+    }
     Key cand = Key::none();  // best candidate of the own rows for the current column
 #pragma unroll
     for (int i = 0; i < RPT; i++)
         if (lid[i] >= 0) cand = Key::kmax(cand, Key::make(x[i][0], lid[i]));
 
-    static_for<0, GK>([&](auto JJ) {
+    if (!fast) static_for<0, GK>([&](auto JJ) {
         constexpr int jj = decltype(JJ)::value;
         if (jj < nb) {
             const int buf = jj & 1;
@@ -446,7 +588,8 @@ __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const
             }
         }
     });
-    if constexpr (CLUSTER) cg::this_cluster().sync();  // no CTA leaves while its rows may still be read
+    if constexpr (CLUSTER)
+        if (!fast) cg::this_cluster().sync();  // no CTA leaves while its rows may still be read
     // panels of a system run in order, so the first zero pivot recorded is the first of the factorisation
     if (zero_col >= 0) atomicCAS(&B.info[sid], 0, (int32_t)(k + zero_col + 1));
     if (B.mv) {  // the panel's row moves, for the other columns of the outer block
