@@ -160,8 +160,8 @@ int gbvlm_device_info(int32_t* sm_count, int64_t* free_bytes, int64_t* total_byt
  * keeps the choices in a committed table.  Defaults are the hand-measured
  * shapes.  A batch plan copies the values when it is created; the other
  * calls read them at each launch.
- *   wake.waves           1..16   split-K slices of the wake sums: about
- *                                waves x SMs CTAs (default 4)
+ *   wake.waves           1..16   split-K slices of the wake sums and the roll-up:
+ *                                about 4 x waves x SMs CTAs (default 4)
  *   hbvlm.waves          1..16   slices of the HBVLM wake operator (4)
  *   hbvlm.min_rows       8..512  wake rows per operator slice at least (32)
  *   batch.group_hi/lo            batch LU size groups: n > hi, lo < n <= hi,

@@ -34,7 +34,7 @@ inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 // Launch-shape parameters (gbvlm_tune_set); defaults are the hand-measured
 // shapes, the autotuner's table overrides them per workload shape.
 struct TuneParams {
-    int64_t wake_waves = 4;            // split-K slices of the wake sums: about waves x SMs CTAs
+    int64_t wake_waves = 4;            // split-K slices of the lattice sums: about 4 x waves x SMs CTAs
     int64_t hbvlm_waves = 4;           // slices of the HBVLM wake operator, likewise
     int64_t hbvlm_min_rows = 32;       // wake rows per operator slice at least
     int64_t batch_group_hi = 1024;     // batch LU size groups: n > hi, lo < n <= hi, n <= lo

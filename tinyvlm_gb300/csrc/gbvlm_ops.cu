@@ -331,137 +331,253 @@ static int rhs_velocities(T* rhs, int32_t nsurf, const gbvlm_dims* dims, const T
 }
 
 // ---------------------------------------------------------------------------
-// a3: wake influence on the RHS (vlm_backend_cpu.cpp:181-224), N-body tiled.
-// Grid x: blocks of 128 target panels (all surfaces packed); grid y: slices
-// of the active wake ring rows (split-K).  Each block stages WK_ROWS ring rows
-// (vertex lines + gammas) of one lifting wake in shared memory and every
-// thread walks them span-wise with the shared vertex/segment chain, keeping
-// a scalar sum of gamma_r (v_r . n) for its point and its mirror.  Partial
-// sums go to a scratch buffer [slice][target] and a second kernel reduces
-// them in a fixed order into rhs, so results do not depend on scheduling.
+// Lattice sums: a3, the wake influence on the RHS (vlm_backend_cpu.cpp:181-224),
+// and a17, the free-wake roll-up (ispc:215-271).
+//
+// Grid x: blocks of LT_THREADS evaluation points, one per thread; grid y:
+// slices of the sources (split-K).  The sources are cut into pieces of at most
+// LT_ROWS ring rows x LT_SPAN rings; a slice takes a run of consecutive
+// pieces.  A piece is staged in shared memory as vertices, segment vectors and
+// net segment strengths (lattice_walk), so each segment is evaluated once for
+// the two rings it bounds.  Each slice writes its sums to a scratch table and
+// a second kernel adds them in a fixed order, so results do not depend on
+// scheduling.
+//
+// Bound: the fp32 (fp64) pipe.  Per point and ring two segments and 1.25
+// vertices, each with its image: about 100 fp32 operations on the FMA pipe,
+// where the ring-by-ring walk spent 220.
+// LT_ROWS: a piece's last vertex line is formed again by the next piece, so
+// (LT_ROWS + 1) / LT_ROWS vertices per ring; five lines' relative vectors are
+// 30 registers (float).  LT_SPAN: short, so that a wake of a few rows still
+// gives every SM work; each piece repeats one vertex column.
+// Measured (before -> after): 1600 points x 40,000 rings 595 -> 370 us in
+// float; 576 points, wakes of 1 to 159 x 48 rings in double, 731 -> 317 ms
+// per 160-step run; roll-up of 12,150 vertices (whose 95 blocks, one per 128
+// points, had left SMs idle) 3417 -> 952 us.
 // ---------------------------------------------------------------------------
-constexpr int WK_THREADS = 128;
-constexpr int WK_ROWS = 8;
-constexpr int WK_MAXSPAN = 512;  // spanwise vertices staged per row chunk
+constexpr int LT_THREADS = 128;
+constexpr int LT_ROWS = 4;
+constexpr int LT_SPAN = 32;
+constexpr int LT_MIN_BLOCKS_F32 = 5;
 
 template <class T>
-struct WakeArgs {
-    Surfs<T> s;          // a=colloc, b=normals (targets); c=verts_wake, d=gamma_wake, flag=lifting
+struct LatticeArgs {
+    // RHS: a = colloc, b = normals; roll-up: a = verts_wing, b = gamma_wing;
+    // c = verts_wake, d = gamma_wake, flag = lifting; o0 = verts_wake (roll-up, written by the reduction)
+    Surfs<T> s;
     int32_t iteration;
-    int32_t window;      // 0 = no window
+    int32_t window;  // 0 = no window
     T sigma2;
-    int64_t total_rows;  // sum over lifting surfaces of active ring rows
-    int64_t rows_per_slice;
-    T* partial;          // [slices][n_targets]
-    int32_t sc;          // spanwise rings staged per chunk (<= WK_MAXSPAN)
+    T* partial;             // [slices][n_points], roll-up: [slices][3][n_points]
     const int64_t* it_dev;  // if set: the iteration, read on the device (the grid covers up to `iteration`)
+    int64_t voff[GBVLM_MAX_SURFACES + 1];  // roll-up: packed moving-vertex offsets
+    int64_t npts;
 };
 
-// number of active ring rows of surface m and the first one
+// one source lattice: vertex lines of n vertices, ring rows [first, first + rows)
 template <class T>
-__device__ __forceinline__ void wake_rows(const WakeArgs<T>& w, int m, int64_t& first, int64_t& count) {
-    const int64_t v_m = w.s.nwv[m];
-    const int64_t it = w.it_dev ? *w.it_dev : w.iteration;
-    first = v_m - it - 1;
-    int64_t end = v_m - 1;
-    if (w.window > 0 && it > w.window) end = v_m - 1 - it + w.window;
-    count = end - first;
-    if (count < 0) count = 0;
+struct Lattice {
+    const T* v;
+    const T* g;
+    int64_t n, vld, first, rows, groups, chunks;
+};
+
+template <class T, bool ROLL>
+__device__ __forceinline__ Lattice<T> lattice_of(const LatticeArgs<T>& w, int l, int64_t it) {
+    const int m = ROLL ? l >> 1 : l;
+    Lattice<T> L;
+    L.n = w.s.ns[m] + 1;
+    if (ROLL && !(l & 1)) {
+        L.v = w.s.a[m];
+        L.g = w.s.b[m];
+        L.vld = L.n * (w.s.nc[m] + 1);
+        L.first = 0;
+        L.rows = w.s.nc[m];
+    } else {
+        L.v = w.s.c[m];
+        L.g = w.s.d[m];
+        L.vld = L.n * w.s.nwv[m];
+        L.first = w.s.nwv[m] - it - 1;
+        int64_t end = w.s.nwv[m] - 1;
+        if (!ROLL && w.window > 0 && it > w.window) end = L.first + w.window;
+        L.rows = w.s.flag[m] ? max(end - L.first, (int64_t)0) : 0;
+    }
+    L.groups = (L.rows + LT_ROWS - 1) / LT_ROWS;
+    L.chunks = (L.n - 1 + LT_SPAN - 1) / LT_SPAN;
+    return L;
 }
 
-template <class T, bool SIGMA>
-__global__ void __launch_bounds__(WK_THREADS) k_wake_influence(WakeArgs<T> w) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    const int SC = w.sc, W = SC + 1;
-    T* sv = reinterpret_cast<T*>(smem_raw);  // [(WK_ROWS+1) rows][3][W]
-    T* sg = sv + (WK_ROWS + 1) * 3 * W;      // [WK_ROWS][SC]
-    const int64_t ntg = w.s.poff[w.s.n];
-    const int64_t g = (int64_t)blockIdx.x * WK_THREADS + threadIdx.x;
-    const bool active = g < ntg;
+template <class T, bool SIGMA, bool ROLL>
+__global__ void __launch_bounds__(LT_THREADS, sizeof(T) == 4 ? LT_MIN_BLOCKS_F32 : 1) k_lattice_sum(LatticeArgs<T> w) {
+    constexpr int LR = LT_ROWS + 1, W = LT_SPAN + 1;
+    __shared__ Quad<T> sv[LR * W], ss[LR * W], sc[LR * W];
+    const int64_t g = (int64_t)blockIdx.x * LT_THREADS + threadIdx.x;
+    const bool active = g < w.npts;
     T px = 0, py = 0, pz = 0, nx = 0, ny = 0, nz = 0;
     if (active) {
-        int m = find_surf(w.s, g);
-        int64_t p = g - w.s.poff[m], np = w.s.ns[m] * w.s.nc[m];
-        px = w.s.a[m][p]; py = w.s.a[m][np + p]; pz = w.s.a[m][2 * np + p];
-        nx = w.s.b[m][p]; ny = w.s.b[m][np + p]; nz = w.s.b[m][2 * np + p];
-    }
-    // this block's global row range [R0, R1) over the concatenation of lifting wakes
-    int64_t total_rows = w.total_rows;
-    if (w.it_dev) {  // rows of the current iteration; slices past them contribute zero
-        total_rows = 0;
-        for (int m = 0; m < w.s.n; m++)
-            if (w.s.flag[m]) {
-                int64_t f_, c_;
-                wake_rows(w, m, f_, c_);
-                total_rows += c_;
-            }
-    }
-    // the device-iteration form spreads the current rows over all its slices
-    // (its grid is sized for the largest row count, at capture)
-    const int64_t rps = w.it_dev ? max((total_rows + gridDim.y - 1) / gridDim.y, (int64_t)WK_ROWS) : w.rows_per_slice;
-    const int64_t R0 = (int64_t)blockIdx.y * rps;
-    const int64_t R1 = min(R0 + rps, total_rows);
-    T acc = 0;
-    int64_t base = 0;
-    for (int m = 0; m < w.s.n && base < R1; m++) {
-        if (!w.s.flag[m]) continue;
-        int64_t first, count;
-        wake_rows(w, m, first, count);
-        const int64_t lo = max(R0, base), hi = min(R1, base + count);
-        if (lo < hi) {
-            const int64_t n = w.s.ns[m] + 1;  // spanwise vertices
-            const int64_t vld = n * w.s.nwv[m];
-            const T* vk = w.s.c[m];
-            const T* gk = w.s.d[m];
-            for (int64_t sc0 = 0; sc0 < n - 1; sc0 += SC) {
-                const int64_t sc1 = min(sc0 + (int64_t)SC, n - 1);  // rings [sc0, sc1)
-                const int nvs = (int)(sc1 - sc0 + 1);
-                for (int64_t r0 = lo; r0 < hi; r0 += WK_ROWS) {
-                    const int nr = (int)min((int64_t)WK_ROWS, hi - r0);
-                    const int64_t row0 = first + (r0 - base);  // first ring row of this chunk
-                    __syncthreads();
-                    for (int t = threadIdx.x; t < (nr + 1) * nvs; t += blockDim.x) {
-                        int r = t / nvs, sl = t - r * nvs;
-                        int64_t vi = (sc0 + sl) + (row0 + r) * n;
-                        sv[(r * 3 + 0) * W + sl] = vk[vi];
-                        sv[(r * 3 + 1) * W + sl] = vk[vld + vi];
-                        sv[(r * 3 + 2) * W + sl] = vk[2 * vld + vi];
-                    }
-                    for (int t = threadIdx.x; t < nr * (nvs - 1); t += blockDim.x) {
-                        int r = t / (nvs - 1), sl = t - r * (nvs - 1);
-                        sg[r * SC + sl] = gk[(row0 + r) * (n - 1) + sc0 + sl];
-                    }
-                    __syncthreads();
-                    if (active) {
-                        for (int r = 0; r < nr; r++) {
-                            const T* gr = sg + r * SC;
-                            strip_normal<T, SIGMA>(sv + r * 3 * W, sv + (r + 1) * 3 * W, W, nvs, px, py, pz, nx, ny, nz,
-                                                   w.sigma2, [&](int kk, T val) { acc += gr[kk] * val; });
-                        }
-                    }
-                }
-            }
+        if constexpr (ROLL) {
+            int m = 0;
+            while (m + 1 < w.s.n && g >= w.voff[m + 1]) m++;
+            const int64_t n = w.s.ns[m] + 1, vld = n * w.s.nwv[m];
+            const int64_t vi = (w.s.nwv[m] - w.iteration) * n + (g - w.voff[m]);
+            px = w.s.c[m][vi]; py = w.s.c[m][vld + vi]; pz = w.s.c[m][2 * vld + vi];
+        } else {
+            const int m = find_surf(w.s, g);
+            const int64_t p = g - w.s.poff[m], np = w.s.ns[m] * w.s.nc[m];
+            px = w.s.a[m][p]; py = w.s.a[m][np + p]; pz = w.s.a[m][2 * np + p];
+            nx = w.s.b[m][p]; ny = w.s.b[m][np + p]; nz = w.s.b[m][2 * np + p];
         }
-        base += count;
     }
-    if (active) w.partial[(int64_t)blockIdx.y * ntg + g] = acc;
+    const int64_t it = w.it_dev ? *w.it_dev : (int64_t)w.iteration;
+    const int nlat = ROLL ? 2 * w.s.n : w.s.n;
+    int64_t pieces = 0;
+    for (int l = 0; l < nlat; l++) {
+        const Lattice<T> L = lattice_of<T, ROLL>(w, l, it);
+        pieces += L.groups * L.chunks;
+    }
+    // slices past the pieces of the current iteration contribute zero
+    const int64_t per = (pieces + gridDim.y - 1) / gridDim.y;
+    const int64_t u0 = (int64_t)blockIdx.y * per, u1 = min(u0 + per, pieces);
+    T ax = 0, ay = 0, az = 0;  // RHS: the sum in ax
+    int64_t base = 0;
+    for (int l = 0; l < nlat && base < u1; l++) {
+        const Lattice<T> L = lattice_of<T, ROLL>(w, l, it);
+        const int64_t cnt = L.groups * L.chunks;
+        for (int64_t u = max(u0, base); u < min(u1, base + cnt); u++) {
+            const int64_t grp = (u - base) / L.chunks, ch = (u - base) - grp * L.chunks;
+            const int64_t r0 = L.first + grp * LT_ROWS, rend = L.first + L.rows;
+            const int nr = (int)min((int64_t)LT_ROWS, rend - r0);
+            const int64_t k0 = ch * (L.n - 1) / L.chunks, k1 = (ch + 1) * (L.n - 1) / L.chunks;
+            const int nk = (int)(k1 - k0), nl = nr + 1;
+            __syncthreads();  // the previous piece has been read
+            for (int e = threadIdx.x; e < nl * (nk + 1); e += LT_THREADS) {
+                const int li = e / (nk + 1), k = e - li * (nk + 1);
+                const int64_t row = r0 + li, col = k0 + k, vi = col + row * L.n;
+                // strengths of the four rings around the vertex that the two segments bound; none outside the lattice
+                const int64_t gi = row * (L.n - 1) + col;
+                const bool here = row < rend, left = col > 0, right = col < L.n - 1, above = row > L.first;
+                const T g_l = here && left ? L.g[gi - 1] : (T)0;
+                const T g_r = here && right ? L.g[gi] : (T)0;
+                const T g_al = above && left ? L.g[gi - 1 - (L.n - 1)] : (T)0;
+                const T x = L.v[vi], y = L.v[L.vld + vi], z = L.v[2 * L.vld + vi];
+                Quad<T> q{x, y, z, g_l - g_al};
+                sv[li * W + k] = q;
+                q = Quad<T>{0, 0, 0, g_l - g_r};
+                if (k > 0) {
+                    q.x = x - L.v[vi - 1];
+                    q.y = y - L.v[L.vld + vi - 1];
+                    q.z = z - L.v[2 * L.vld + vi - 1];
+                }
+                ss[li * W + k] = q;
+                if (li < nr) sc[li * W + k] = Quad<T>{L.v[vi + L.n] - x, L.v[L.vld + vi + L.n] - y,
+                                                      L.v[2 * L.vld + vi + L.n] - z, 0};
+            }
+            __syncthreads();
+            T bx = 0, by = 0, bz = 0;  // the piece's own sums: fewer roundings of the running ones
+            lattice_walk<T, SIGMA, LR>(sv, ss, sc, W, nl, nk, k0 == 0, r0 + nr == rend, px, py, pz, w.sigma2,
+                                       [&](T gm, T q0, T q1, T cy, T cx0, T cx1, T cz0, T cz1) {
+                                           if constexpr (ROLL) {
+                                               q0 *= gm;
+                                               q1 *= gm;
+                                               bx += q0 * cx0 + q1 * cx1;
+                                               by += (q0 - q1) * cy;
+                                               bz += q0 * cz0 + q1 * cz1;
+                                           } else {
+                                               const T tn = cy * ny;
+                                               bx += gm * (q0 * (cx0 * nx + tn + cz0 * nz) + q1 * (cx1 * nx - tn + cz1 * nz));
+                                           }
+                                       });
+            ax += bx;
+            ay += by;
+            az += bz;
+        }
+        base += cnt;
+    }
+    if (active) {
+        const int64_t np = w.npts;
+        if constexpr (ROLL) {
+            T* o = w.partial + (int64_t)blockIdx.y * 3 * np + g;
+            o[0] = ax;
+            o[np] = ay;
+            o[2 * np] = az;
+        } else {
+            w.partial[(int64_t)blockIdx.y * np + g] = ax;
+        }
+    }
+}
+
+// The slices' sums of a point, in order: LT_RED threads per point take every
+// LT_RED-th slice, then the point's partial sums are added.
+constexpr int LT_RED = 8;
+
+template <class T>
+__device__ __forceinline__ T slice_sum(const T* partial, int64_t slices, int64_t stride, int64_t at, bool active,
+                                       T (*sh)[32]) {
+    const int p = threadIdx.x & 31, q = threadIdx.x >> 5;
+    T s = 0;
+    if (active)
+#pragma unroll 4
+        for (int64_t k = q; k < slices; k += LT_RED) s += partial[k * stride + at];
+    __syncthreads();  // the previous sum's use of sh
+    sh[q][p] = s;
+    __syncthreads();
+    s = sh[0][p];
+#pragma unroll
+    for (int j = 1; j < LT_RED; j++) s += sh[j][p];
+    return s;
 }
 
 template <class T>
-__global__ void k_wake_reduce(const T* partial, int64_t slices, int64_t ntg, T* rhs) {
-    int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (g >= ntg) return;
-    T s = 0;
-    for (int64_t k = 0; k < slices; k++) s += partial[k * ntg + g];
-    rhs[g] -= s * inv_four_pi<T>();
+__global__ void __launch_bounds__(32 * LT_RED) k_wake_reduce(const T* partial, int64_t slices, int64_t ntg, T* rhs) {
+    __shared__ T sh[LT_RED][32];
+    const int64_t g = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
+    const T s = slice_sum<T>(partial, slices, ntg, g, g < ntg, sh);
+    if (g < ntg && threadIdx.x < 32) rhs[g] -= s * inv_four_pi<T>();
 }
+
+// moves the wake's vertices in place: every old position has been read
+template <class T>
+__global__ void __launch_bounds__(32 * LT_RED) k_roll_reduce(LatticeArgs<T> w, int64_t slices, T dt) {
+    __shared__ T sh[LT_RED][32];
+    const int64_t g = (int64_t)blockIdx.x * 32 + (threadIdx.x & 31);
+    const bool on = g < w.npts;
+    T v[3];
+#pragma unroll
+    for (int k = 0; k < 3; k++) v[k] = slice_sum<T>(w.partial, slices, 3 * w.npts, k * w.npts + g, on, sh);
+    if (!on || threadIdx.x >= 32) return;
+    int m = 0;
+    while (m + 1 < w.s.n && g >= w.voff[m + 1]) m++;
+    const int64_t n = w.s.ns[m] + 1, vld = n * w.s.nwv[m];
+    const int64_t vi = (w.s.nwv[m] - w.iteration) * n + (g - w.voff[m]);
+    const T sc = dt * inv_four_pi<T>();
+#pragma unroll
+    for (int k = 0; k < 3; k++) w.s.o0[m][k * vld + vi] += v[k] * sc;
+}
+
+static int64_t lattice_pieces(int64_t rows, int64_t ns) { return cdiv(rows, LT_ROWS) * cdiv(ns, LT_SPAN); }
+
+// Slices of `pieces` pieces for `npts` points: about 4 x `wake.waves` x SMs
+// CTAs (tuned per shape; a CTA of one or two pieces is short, so the last
+// wave's idle part is too), one piece each at least.  `cap`: values that the
+// scratch holds, `vals` per point and slice.
+static int64_t lattice_slices(int64_t pieces, int64_t npts, int64_t vals, int64_t cap) {
+    int64_t want = cdiv(4 * tune().wake_waves * sm_count(), cdiv(npts, LT_THREADS));
+    want = std::min<int64_t>(want, cap / (npts * vals));
+    if (want < 1) want = 1;
+    return cdiv(pieces, cdiv(pieces, want));
+}
+
+// partial sums of a launch are at most this many values (4 MiB of floats: the
+// allocation-free entry point's array, so that it and the regular one cut the
+// sums alike)
+constexpr int64_t LT_SCRATCH = 1 << 20;
 
 template <class T>
 static int wake_influence(T* rhs, int32_t nsurf, const gbvlm_dims* dims, const T* const* gamma_wake,
                           const T* const* colloc, const T* const* normals, const T* const* verts_wake,
                           const int32_t* lifting, int32_t iteration, T sigma, int32_t window, T* scratch,
                           size_t scratch_elems, cudaStream_t st, const int64_t* it_dev = nullptr) {
-    WakeArgs<T> w;
+    LatticeArgs<T> w;
     int rc = make_surfs(w.s, nsurf, dims);
     if (rc) return rc;
     GB_REQUIRE(rhs != nullptr, "rhs is null");
@@ -471,7 +587,7 @@ static int wake_influence(T* rhs, int32_t nsurf, const gbvlm_dims* dims, const T
     w.iteration = iteration;
     w.window = window;
     w.sigma2 = sigma * sigma;
-    int64_t total = 0;
+    int64_t pieces = 0;
     for (int m = 0; m < nsurf; m++) {
         GB_REQUIRE(colloc[m] && normals[m], "null pointer for surface %d", m);
         w.s.a[m] = colloc[m];
@@ -482,25 +598,16 @@ static int wake_influence(T* rhs, int32_t nsurf, const gbvlm_dims* dims, const T
             GB_REQUIRE(dims[m].nwv >= iteration + 1, "surface %d: nwv=%lld < iteration+1", m, (long long)dims[m].nwv);
             w.s.c[m] = verts_wake[m];
             w.s.d[m] = gamma_wake[m];
-            int64_t end = dims[m].nwv - 1;
-            if (window > 0 && iteration > window) end = dims[m].nwv - 1 - iteration + window;
-            total += end - (dims[m].nwv - iteration - 1);
+            pieces += lattice_pieces(window > 0 && iteration > window ? window : iteration, dims[m].ns);
         } else {
             w.s.flag[m] = 0;
         }
     }
-    if (total == 0) return GBVLM_OK;
+    if (pieces == 0) return GBVLM_OK;
     const int64_t ntg = w.s.poff[nsurf];
-    const int64_t xblocks = cdiv(ntg, WK_THREADS);
-    // enough slices to cover about `wake.waves` waves of the device's SMs
-    // (tuned per shape), at least WK_ROWS rows each; a caller-owned scratch
-    // caps the slice count at what it holds
-    int64_t want = cdiv(tune().wake_waves * sm_count(), xblocks);
-    if (scratch != nullptr) want = std::min<int64_t>(want, (int64_t)(scratch_elems / (size_t)ntg));
-    int64_t slices = want < 1 ? 1 : want;
-    int64_t rps = cdiv(total, slices);
-    if (rps < WK_ROWS) rps = WK_ROWS;
-    slices = cdiv(total, rps);
+    w.npts = ntg;
+    const int64_t cap = scratch ? std::min<int64_t>((int64_t)scratch_elems, LT_SCRATCH) : LT_SCRATCH;
+    const int64_t slices = lattice_slices(pieces, ntg, 1, cap);
     if (scratch == nullptr) {
         GB_REQUIRE(it_dev == nullptr, "the device-iteration form needs its own scratch");
         void* p = nullptr;
@@ -511,172 +618,61 @@ static int wake_influence(T* rhs, int32_t nsurf, const gbvlm_dims* dims, const T
         GB_REQUIRE((size_t)(slices * ntg) <= scratch_elems, "scratch too small: need %lld elements",
                    (long long)(slices * ntg));
     }
-    w.total_rows = total;
-    w.rows_per_slice = rps;
     w.partial = scratch;
-    int64_t maxs = 1;
-    for (int m = 0; m < nsurf; m++)
-        if (w.s.flag[m] && dims[m].ns > maxs) maxs = dims[m].ns;
-    w.sc = (int32_t)(maxs < WK_MAXSPAN ? maxs : WK_MAXSPAN);
-    const size_t smem = ((WK_ROWS + 1) * 3 * (w.sc + 1) + WK_ROWS * w.sc) * sizeof(T);
-    dim3 grid((unsigned)xblocks, (unsigned)slices);
-    if (sigma != (T)0) {
-        GB_CUDA(cudaFuncSetAttribute(k_wake_influence<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_wake_influence<T, true><<<grid, WK_THREADS, smem, st>>>(w);
-    } else {
-        GB_CUDA(cudaFuncSetAttribute(k_wake_influence<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_wake_influence<T, false><<<grid, WK_THREADS, smem, st>>>(w);
-    }
+    dim3 grid((unsigned)cdiv(ntg, LT_THREADS), (unsigned)slices);
+    if (sigma != (T)0)
+        k_lattice_sum<T, true, false><<<grid, LT_THREADS, 0, st>>>(w);
+    else
+        k_lattice_sum<T, false, false><<<grid, LT_THREADS, 0, st>>>(w);
     GB_LAUNCH_CHECK();
-    k_wake_reduce<T><<<(unsigned)cdiv(ntg, 256), 256, 0, st>>>(scratch, slices, ntg, rhs);
+    k_wake_reduce<T><<<(unsigned)cdiv(ntg, 32), 32 * LT_RED, 0, st>>>(scratch, slices, ntg, rhs);
     GB_LAUNCH_CHECK();
     return GBVLM_OK;
-}
-
-// ---------------------------------------------------------------------------
-// a17: free-wake roll-up (ispc:215-271).  One thread per moving wake vertex;
-// block-stages chunks of source ring rows.  Sources: every wing lattice
-// (all ring rows) and every lifting wake (its active ring rows).  New
-// positions go to `out` (a copy of the wake) so that all reads see the old
-// positions; the host then swaps/copies.
-// ---------------------------------------------------------------------------
-constexpr int RU_THREADS = 128;
-
-template <class T>
-struct RollArgs {
-    Surfs<T> s;  // a=verts_wing, b=gamma_wing, c=verts_wake(old), d=gamma_wake, flag=lifting; o0=out wake
-    int32_t iteration;
-    T sigma2, dt;
-    int64_t voff[GBVLM_MAX_SURFACES + 1];  // packed moving-vertex offsets
-    int32_t sc;                             // spanwise rings staged per chunk
-};
-
-template <class T, bool SIGMA>
-__device__ __forceinline__ void lattice_vel(T px, T py, T pz, const T* v, int64_t vld, int64_t n, int64_t r0, int64_t r1,
-                                            const T* gam, T sigma2, T* sv, T* sgm, int SC, V3<T>& vel) {
-    const int W = SC + 1;
-    for (int64_t sc0 = 0; sc0 < n - 1; sc0 += SC) {
-        const int64_t sc1 = min(sc0 + (int64_t)SC, n - 1);
-        const int nvs = (int)(sc1 - sc0 + 1);
-        for (int64_t rr = r0; rr < r1; rr += WK_ROWS) {
-            const int nr = (int)min((int64_t)WK_ROWS, r1 - rr);
-            __syncthreads();
-            for (int t = threadIdx.x; t < (nr + 1) * nvs; t += blockDim.x) {
-                int r = t / nvs, sl = t - r * nvs;
-                int64_t vi = (sc0 + sl) + (rr + r) * n;
-                sv[(r * 3 + 0) * W + sl] = v[vi];
-                sv[(r * 3 + 1) * W + sl] = v[vld + vi];
-                sv[(r * 3 + 2) * W + sl] = v[2 * vld + vi];
-            }
-            for (int t = threadIdx.x; t < nr * (nvs - 1); t += blockDim.x) {
-                int r = t / (nvs - 1), sl = t - r * (nvs - 1);
-                sgm[r * SC + sl] = gam[(rr + r) * (n - 1) + sc0 + sl];
-            }
-            __syncthreads();
-            for (int r = 0; r < nr; r++) {
-                const T* gr = sgm + r * SC;
-                strip_vec<T, SIGMA>(sv + r * 3 * W, sv + (r + 1) * 3 * W, W, nvs, px, py, pz, sigma2,
-                                    [&](int kk, V3<T> v) {
-                                        const T gm = gr[kk];
-                                        vel.x += gm * v.x;
-                                        vel.y += gm * v.y;
-                                        vel.z += gm * v.z;
-                                    });
-            }
-        }
-    }
-}
-
-template <class T, bool SIGMA>
-__global__ void __launch_bounds__(RU_THREADS) k_rollup(RollArgs<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* sv = reinterpret_cast<T*>(smem_raw);
-    T* sgm = sv + (WK_ROWS + 1) * 3 * (a.sc + 1);
-    const int64_t total = a.voff[a.s.n];
-    const int64_t g = (int64_t)blockIdx.x * RU_THREADS + threadIdx.x;
-    const bool active = g < total;
-    int m = 0;
-    int64_t vi = 0, vld = 0;
-    T px = 0, py = 0, pz = 0;
-    if (active) {
-        while (m + 1 < a.s.n && g >= a.voff[m + 1]) m++;
-        const int64_t n = a.s.ns[m] + 1;
-        vld = n * a.s.nwv[m];
-        vi = (a.s.nwv[m] - a.iteration) * n + (g - a.voff[m]);
-        px = a.s.c[m][vi]; py = a.s.c[m][vld + vi]; pz = a.s.c[m][2 * vld + vi];
-    }
-    V3<T> vel{0, 0, 0};
-    for (int k = 0; k < a.s.n; k++) {
-        const int64_t n = a.s.ns[k] + 1;
-        lattice_vel<T, SIGMA>(px, py, pz, a.s.a[k], n * (a.s.nc[k] + 1), n, 0, a.s.nc[k], a.s.b[k], a.sigma2, sv, sgm, a.sc, vel);
-        if (!a.s.flag[k]) continue;
-        const int64_t nw = a.s.nwv[k];
-        lattice_vel<T, SIGMA>(px, py, pz, a.s.c[k], n * nw, n, nw - a.iteration - 1, nw - 1, a.s.d[k], a.sigma2, sv, sgm, a.sc, vel);
-    }
-    if (active) {
-        const T sc = a.dt * inv_four_pi<T>();
-        a.s.o0[m][vi] = px + vel.x * sc;
-        a.s.o0[m][vld + vi] = py + vel.y * sc;
-        a.s.o0[m][2 * vld + vi] = pz + vel.z * sc;
-    }
 }
 
 template <class T>
 static int wake_rollup(int32_t nsurf, const gbvlm_dims* dims, T* const* verts_wake, const T* const* verts_wing,
                        const T* const* gamma_wing, const T* const* gamma_wake, const int32_t* lifting, T sigma, T dt,
                        int32_t iteration, cudaStream_t st) {
-    RollArgs<T> a;
-    int rc = make_surfs(a.s, nsurf, dims);
+    LatticeArgs<T> w;
+    int rc = make_surfs(w.s, nsurf, dims);
     if (rc) return rc;
     GB_REQUIRE(lifting != nullptr, "lifting is null");
     GB_REQUIRE(iteration >= 0, "iteration < 0");
     if (iteration == 0) return GBVLM_OK;
-    size_t wake_bytes = 0;
-    a.voff[0] = 0;
+    w.voff[0] = 0;
+    int64_t pieces = 0;
     for (int m = 0; m < nsurf; m++) {
         GB_REQUIRE(verts_wake[m] && verts_wing[m] && gamma_wing[m], "null pointer for surface %d", m);
         GB_REQUIRE(dims[m].nwv >= iteration + 1, "surface %d: nwv=%lld < iteration+1", m, (long long)dims[m].nwv);
-        a.s.a[m] = verts_wing[m];
-        a.s.b[m] = gamma_wing[m];
-        a.s.c[m] = verts_wake[m];
-        a.s.d[m] = gamma_wake ? gamma_wake[m] : nullptr;
-        a.s.flag[m] = lifting[m] ? 1 : 0;
+        w.s.a[m] = verts_wing[m];
+        w.s.b[m] = gamma_wing[m];
+        w.s.c[m] = verts_wake[m];
+        w.s.d[m] = gamma_wake ? gamma_wake[m] : nullptr;
+        w.s.o0[m] = verts_wake[m];
+        w.s.flag[m] = lifting[m] ? 1 : 0;
         if (lifting[m]) GB_REQUIRE(gamma_wake && gamma_wake[m], "gamma_wake of surface %d is null", m);
-        a.voff[m + 1] = a.voff[m] + (int64_t)iteration * (dims[m].ns + 1);
-        wake_bytes += sizeof(T) * 3 * (dims[m].ns + 1) * dims[m].nwv;
+        w.voff[m + 1] = w.voff[m] + (int64_t)iteration * (dims[m].ns + 1);
+        pieces += lattice_pieces(dims[m].nc, dims[m].ns) + (lifting[m] ? lattice_pieces(iteration, dims[m].ns) : 0);
     }
+    w.npts = w.voff[nsurf];
+    w.iteration = iteration;
+    w.window = 0;
+    w.it_dev = nullptr;
+    w.sigma2 = sigma * sigma;
+    const int64_t slices = lattice_slices(pieces, w.npts, 3, LT_SCRATCH);
     void* scratch = nullptr;
-    rc = device_scratch(wake_bytes, &scratch, st);
+    rc = device_scratch(sizeof(T) * 3 * slices * w.npts, &scratch, st);
     if (rc) return rc;
-    size_t off = 0;
-    for (int m = 0; m < nsurf; m++) {
-        a.s.o0[m] = (T*)((char*)scratch + off);
-        off += sizeof(T) * 3 * (dims[m].ns + 1) * dims[m].nwv;
-    }
-    a.iteration = iteration;
-    a.sigma2 = sigma * sigma;
-    a.dt = dt;
-    int64_t maxs = 1;
-    for (int m = 0; m < nsurf; m++)
-        if (dims[m].ns > maxs) maxs = dims[m].ns;
-    a.sc = (int32_t)(maxs < WK_MAXSPAN ? maxs : WK_MAXSPAN);
-    const size_t smem = ((WK_ROWS + 1) * 3 * (a.sc + 1) + WK_ROWS * a.sc) * sizeof(T);
-    const int64_t total = a.voff[nsurf];
-    if (sigma != (T)0) {
-        GB_CUDA(cudaFuncSetAttribute(k_rollup<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_rollup<T, true><<<(unsigned)cdiv(total, RU_THREADS), RU_THREADS, smem, st>>>(a);
-    } else {
-        GB_CUDA(cudaFuncSetAttribute(k_rollup<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_rollup<T, false><<<(unsigned)cdiv(total, RU_THREADS), RU_THREADS, smem, st>>>(a);
-    }
+    w.partial = (T*)scratch;
+    dim3 grid((unsigned)cdiv(w.npts, LT_THREADS), (unsigned)slices);
+    if (sigma != (T)0)
+        k_lattice_sum<T, true, true><<<grid, LT_THREADS, 0, st>>>(w);
+    else
+        k_lattice_sum<T, false, true><<<grid, LT_THREADS, 0, st>>>(w);
     GB_LAUNCH_CHECK();
-    for (int m = 0; m < nsurf; m++) {
-        const int64_t n = dims[m].ns + 1, vld = n * dims[m].nwv, begin = (dims[m].nwv - iteration) * n;
-        for (int k = 0; k < 3; k++) {
-            GB_CUDA(cudaMemcpyAsync(verts_wake[m] + k * vld + begin, a.s.o0[m] + k * vld + begin,
-                                    sizeof(T) * iteration * n, cudaMemcpyDeviceToDevice, st));
-        }
-    }
+    k_roll_reduce<T><<<(unsigned)cdiv(w.npts, 32), 32 * LT_RED, 0, st>>>(w, slices, dt);
+    GB_LAUNCH_CHECK();
     return GBVLM_OK;
 }
 

@@ -72,27 +72,141 @@ __device__ __forceinline__ void strip_normal(const T* top, const T* bot, int W, 
     }
 }
 
-// Same walk returning 4*pi times the full velocity of each ring (direct + mirror).
-template <class T, bool SIGMA, class F>
-__device__ __forceinline__ void strip_vec(const T* top, const T* bot, int W, int nvs, T px, T py, T pz, T sg, F&& f) {
-    auto V = [&](const T* line, int sl) { return V3<T>{line[sl], line[W + sl], line[2 * W + sl]}; };
-    V3<T> v0 = V(top, 0), v3 = V(bot, 0);
-    Rel<T> A0 = make_rel<T>(px - v0.x, py - v0.y, pz - v0.z), A3 = make_rel<T>(px - v3.x, py - v3.y, pz - v3.z);
-    Rel<T> B0 = make_rel<T>(px - v0.x, -py - v0.y, pz - v0.z), B3 = make_rel<T>(px - v3.x, -py - v3.y, pz - v3.z);
-    V3<T> Ca = seg_vec<T, SIGMA>(A0, A3, v3.x - v0.x, v3.y - v0.y, v3.z - v0.z, sg);
-    V3<T> Cb = seg_vec<T, SIGMA>(B0, B3, v3.x - v0.x, v3.y - v0.y, v3.z - v0.z, sg);
-    for (int k = 1; k < nvs; k++) {
-        const V3<T> v1 = V(top, k), v2 = V(bot, k);
-        const Rel<T> A1 = make_rel<T>(px - v1.x, py - v1.y, pz - v1.z), A2 = make_rel<T>(px - v2.x, py - v2.y, pz - v2.z);
-        const Rel<T> B1 = make_rel<T>(px - v1.x, -py - v1.y, pz - v1.z), B2 = make_rel<T>(px - v2.x, -py - v2.y, pz - v2.z);
-        const T cx = v2.x - v1.x, cy = v2.y - v1.y, cz = v2.z - v1.z;
-        const T tx = v1.x - v0.x, ty = v1.y - v0.y, tz = v1.z - v0.z;
-        const T bx = v3.x - v2.x, by = v3.y - v2.y, bz = v3.z - v2.z;
-        const V3<T> Cra = seg_vec<T, SIGMA>(A1, A2, cx, cy, cz, sg), Crb = seg_vec<T, SIGMA>(B1, B2, cx, cy, cz, sg);
-        const V3<T> ra = seg_vec<T, SIGMA>(A0, A1, tx, ty, tz, sg) + Cra + seg_vec<T, SIGMA>(A2, A3, bx, by, bz, sg) - Ca;
-        const V3<T> rb = seg_vec<T, SIGMA>(B0, B1, tx, ty, tz, sg) + Crb + seg_vec<T, SIGMA>(B2, B3, bx, by, bz, sg) - Cb;
-        f(k - 1, V3<T>{ra.x + rb.x, ra.y - rb.y, ra.z + rb.z});
-        A0 = A1; A3 = A2; B0 = B1; B3 = B2; Ca = Cra; Cb = Crb; v0 = v1; v3 = v2;
+// ---------------------------------------------------------------------------
+// Sums over a whole lattice with given ring strengths.  A segment belongs to
+// two rings, so the sum needs each segment once, with the difference of their
+// strengths: per ring one spanwise and one chordwise segment and one vertex,
+// where the ring-by-ring walk evaluates three segments and two vertices.  A
+// point and its image in y = 0 share every product without a y in it.
+// ---------------------------------------------------------------------------
+
+// a vertex seen from the point (y0, n0) and from its image (y1, n1)
+template <class T> struct RelPair { T x, z, y0, y1, n0, n1; };
+
+template <class T>
+__device__ __forceinline__ RelPair<T> make_rel_pair(T px, T py, T pz, T vx, T vy, T vz) {
+    RelPair<T> r;
+    r.x = px - vx;
+    r.z = pz - vz;
+    r.y0 = py - vy;
+    r.y1 = -py - vy;
+    const T s = r.x * r.x + r.z * r.z;
+    r.n0 = fast_len<T>(r.y0 * r.y0 + s);
+    r.n1 = fast_len<T>(r.y1 * r.y1 + s);
+    return r;
+}
+
+// x < c for x a sum of squares or a length (not negative, possibly NaN) and
+// c > 0: in double by the bits, which order like the values, since the fp64
+// pipe is the bound there (a NaN is not below, whatever its sign)
+__device__ __forceinline__ bool below(float x, float c) { return x < c; }
+__device__ __forceinline__ bool below(double x, double c) {
+    return (unsigned long long)__double_as_longlong(x) < (unsigned long long)__double_as_longlong(c);
+}
+__device__ __forceinline__ bool not_negative(float x) { return x >= 0.f; }
+__device__ __forceinline__ bool not_negative(double x) { return __double2hiint(x) >= 0; }
+
+// the quotients n0 / d0 and n1 / d1; in double with one division (a cut
+// quotient is zero whatever its operands)
+__device__ __forceinline__ void two_quotients(float n0, float d0, bool cut0, float n1, float d1, bool cut1, float& q0,
+                                              float& q1) {
+    q0 = fast_div<float>(n0, d0);
+    q1 = fast_div<float>(n1, d1);
+    if (cut0) q0 = 0.f;
+    if (cut1) q1 = 0.f;
+}
+__device__ __forceinline__ void two_quotients(double n0, double d0, bool cut0, double n1, double d1, bool cut1,
+                                              double& q0, double& q1) {
+    if (cut0) d0 = 1.0;
+    if (cut1) d1 = 1.0;
+    const double inv = 1.0 / (d0 * d1);
+    q0 = cut0 ? 0.0 : n0 * (d1 * inv);
+    q1 = cut1 ? 0.0 : n1 * (d0 * inv);
+}
+
+// seg_coeff for a point and its image: k and r0 x a of both (the y component
+// of the cross product is common)
+template <class T, bool SIGMA>
+__device__ __forceinline__ void seg_pair(const RelPair<T>& a, const RelPair<T>& b, T rx, T ry, T rz, T sigma2, T& k0,
+                                         T& k1, T& cy, T& cx0, T& cx1, T& cz0, T& cz1) {
+    const T px = ry * a.z, pz = ry * a.x;
+    cy = rz * a.x - rx * a.z;
+    cx0 = px - rz * a.y0;
+    cx1 = px - rz * a.y1;
+    cz0 = rx * a.y0 - pz;
+    cz1 = rx * a.y1 - pz;
+    const T cyy = cy * cy;
+    const T sq0 = cz0 * cz0 + (cx0 * cx0 + cyy), sq1 = cz1 * cz1 + (cx1 * cx1 + cyy);
+    const T abxz = a.x * b.x + a.z * b.z;
+    const T ab0 = a.y0 * b.y0 + abxz, ab1 = a.y1 * b.y1 + abxz;
+    const T nab0 = a.n0 * b.n0, nab1 = a.n1 * b.n1;
+    const T s0 = a.n0 + b.n0, s1 = a.n1 + b.n1;
+    constexpr T rcut = Prec<T>::rcut_norm;
+    const bool cut0 = below(sq0, (T)RCUT_SQ) | below(a.n0, rcut) | below(b.n0, rcut);
+    const bool cut1 = below(sq1, (T)RCUT_SQ) | below(a.n1, rcut) | below(b.n1, rcut);
+    const bool pos0 = not_negative(ab0), pos1 = not_negative(ab1);
+    T num0 = pos0 ? s0 : s0 * (nab0 - ab0), num1 = pos1 ? s1 : s1 * (nab1 - ab1);
+    T den0 = nab0 * (pos0 ? nab0 + ab0 : sq0), den1 = nab1 * (pos1 ? nab1 + ab1 : sq1);
+    if (SIGMA) {
+        const T sm = sigma2 * (rx * rx + ry * ry + rz * rz);
+        num0 *= sq0;
+        num1 *= sq1;
+        den0 *= dsqrt<T>(sq0 * sq0 + sm * sm);
+        den1 *= dsqrt<T>(sq1 * sq1 + sm * sm);
+    }
+    two_quotients(num0, den0, cut0, num1, den1, cut1, k0, k1);
+}
+
+// four consecutive values in one or two 16-byte loads
+template <class T> struct alignas(16) Quad { T x, y, z, w; };
+
+// A piece of a lattice in shared memory: nl <= LR vertex lines of nk + 1
+// vertices, line l's vertex k at [l * W + k].
+//   v: position, and the net strength of the spanwise segment k-1 -> k
+//   s: that segment's vector, and the net strength of the chordwise segment
+//      from this line to the next at k
+//   c: the chordwise segment's vector
+// Calls add(g, k0, k1, cy, cx0, cx1, cz0, cz1) for every segment of strength
+// g.  The spanwise segments of the last line belong to the next piece unless
+// `last`, the chordwise ones of vertex 0 to the piece before unless `first`.
+template <class T, bool SIGMA, int LR, class F>
+__device__ __forceinline__ void lattice_walk(const Quad<T>* v, const Quad<T>* s, const Quad<T>* c, int W, int nl, int nk,
+                                             bool first, bool last, T px, T py, T pz, T sg, F&& add) {
+    RelPair<T> prev[LR];
+    T k0, k1, cy, cx0, cx1, cz0, cz1;
+#pragma unroll
+    for (int l = 0; l < LR; l++)
+        if (l < nl) {
+            const Quad<T> q = v[l * W];
+            prev[l] = make_rel_pair<T>(px, py, pz, q.x, q.y, q.z);
+            if (l > 0 && first) {
+                const Quad<T> e = c[(l - 1) * W];
+                seg_pair<T, SIGMA>(prev[l > 0 ? l - 1 : 0], prev[l], e.x, e.y, e.z, sg, k0, k1, cy, cx0, cx1, cz0, cz1);
+                add(s[(l - 1) * W].w, k0, k1, cy, cx0, cx1, cz0, cz1);
+            }
+        }
+#pragma unroll 1
+    for (int k = 1; k <= nk; k++) {
+        RelPair<T> up = prev[0];
+        T gup = 0;
+#pragma unroll
+        for (int l = 0; l < LR; l++)
+            if (l < nl) {
+                const Quad<T> q = v[l * W + k], e = s[l * W + k];
+                const RelPair<T> cur = make_rel_pair<T>(px, py, pz, q.x, q.y, q.z);
+                if (l + 1 < nl || last) {
+                    seg_pair<T, SIGMA>(prev[l], cur, e.x, e.y, e.z, sg, k0, k1, cy, cx0, cx1, cz0, cz1);
+                    add(q.w, k0, k1, cy, cx0, cx1, cz0, cz1);
+                }
+                if (l > 0) {
+                    const Quad<T> d = c[(l - 1) * W + k];
+                    seg_pair<T, SIGMA>(up, cur, d.x, d.y, d.z, sg, k0, k1, cy, cx0, cx1, cz0, cz1);
+                    add(gup, k0, k1, cy, cx0, cx1, cz0, cz1);
+                }
+                up = cur;
+                gup = e.w;
+                prev[l] = cur;
+            }
     }
 }
 
