@@ -13,6 +13,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 #include <vector>
 
 #include "gbvlm_internal.h"
@@ -336,27 +337,35 @@ static int rhs_velocities(T* rhs, int32_t nsurf, const gbvlm_dims* dims, const T
 //
 // Grid x: blocks of LT_THREADS evaluation points, one per thread; grid y:
 // slices of the sources (split-K).  The sources are cut into pieces of at most
-// LT_ROWS ring rows x LT_SPAN rings; a slice takes a run of consecutive
+// LatticeRows ring rows x LT_SPAN rings; a slice takes a run of consecutive
 // pieces.  A piece is staged in shared memory as vertices, segment vectors and
 // net segment strengths (lattice_walk), so each segment is evaluated once for
 // the two rings it bounds.  Each slice writes its sums to a scratch table and
 // a second kernel adds them in a fixed order, so results do not depend on
 // scheduling.
 //
-// Bound: the fp32 (fp64) pipe.  Per point and ring two segments and 1.25
-// vertices, each with its image: about 100 fp32 operations on the FMA pipe,
-// where the ring-by-ring walk spent 220.
-// LT_ROWS: a piece's last vertex line is formed again by the next piece, so
-// (LT_ROWS + 1) / LT_ROWS vertices per ring; five lines' relative vectors are
-// 30 registers (float).  LT_SPAN: short, so that a wake of a few rows still
-// gives every SM work; each piece repeats one vertex column.
-// Measured (before -> after): 1600 points x 40,000 rings 595 -> 370 us in
-// float; 576 points, wakes of 1 to 159 x 48 rings in double, 731 -> 317 ms
-// per 160-step run; roll-up of 12,150 vertices (whose 95 blocks, one per 128
-// points, had left SMs idle) 3417 -> 952 us.
+// Bound: issue slots and the fp32 pipe (float), the fp64 pipe (double, 89 % busy).
+// Per point and ring two segments and 1.25 vertices, each with its image: 190
+// instructions, where the ring-by-ring walk spent 370.
+// LatticeRows: a piece's last vertex line is formed again by the next piece, so
+// (rows + 1) / rows vertices per ring; a line's relative vectors are 6
+// registers in float, 12 in double, where three rows leave room for a third
+// block per SM (1600 points x 8000 rings 3.81 ms with four rows, 3.01 with
+// three).  LT_SPAN: short, so that a wake of a few rows still gives every SM
+// work; each piece repeats one vertex column.  Full pieces of float are
+// straight code without tests of the line count (370 -> 308 us below); the same
+// in double costs registers (3.01 -> 3.31 ms).
+// Measured (before -> after): 1600 points x 40,000 rings in float 595 -> 308 us,
+// 8000 rings in double 7.0 -> 2.90 ms; roll-up of 12,150 vertices (95 blocks
+// before, one per 128 points, which left SMs idle) 3417 -> 763 us.
+// Not kept: the point and its image as the two halves of packed fp32
+// instructions (issue slots per ring 190 -> 150, but 128 registers: 320 us),
+// and the cut-offs left out of a first walk that a second one repeats where a
+// lane met one (298 us, but the roll-up 763 -> 819).
 // ---------------------------------------------------------------------------
 constexpr int LT_THREADS = 128;
-constexpr int LT_ROWS = 4;
+template <class T> struct LatticeRows { static constexpr int value = 4; };
+template <> struct LatticeRows<double> { static constexpr int value = 3; };
 constexpr int LT_SPAN = 32;
 constexpr int LT_MIN_BLOCKS_F32 = 5;
 
@@ -402,14 +411,15 @@ __device__ __forceinline__ Lattice<T> lattice_of(const LatticeArgs<T>& w, int l,
         if (!ROLL && w.window > 0 && it > w.window) end = L.first + w.window;
         L.rows = w.s.flag[m] ? max(end - L.first, (int64_t)0) : 0;
     }
-    L.groups = (L.rows + LT_ROWS - 1) / LT_ROWS;
+    L.groups = (L.rows + LatticeRows<T>::value - 1) / LatticeRows<T>::value;
     L.chunks = (L.n - 1 + LT_SPAN - 1) / LT_SPAN;
     return L;
 }
 
 template <class T, bool SIGMA, bool ROLL>
 __global__ void __launch_bounds__(LT_THREADS, sizeof(T) == 4 ? LT_MIN_BLOCKS_F32 : 1) k_lattice_sum(LatticeArgs<T> w) {
-    constexpr int LR = LT_ROWS + 1, W = LT_SPAN + 1;
+    constexpr int ROWS = LatticeRows<T>::value, LR = ROWS + 1, W = LT_SPAN + 1;
+    constexpr bool FAST = sizeof(T) == 4 && !SIGMA;  // full pieces as straight code
     __shared__ Quad<T> sv[LR * W], ss[LR * W], sc[LR * W];
     const int64_t g = (int64_t)blockIdx.x * LT_THREADS + threadIdx.x;
     const bool active = g < w.npts;
@@ -445,8 +455,8 @@ __global__ void __launch_bounds__(LT_THREADS, sizeof(T) == 4 ? LT_MIN_BLOCKS_F32
         const int64_t cnt = L.groups * L.chunks;
         for (int64_t u = max(u0, base); u < min(u1, base + cnt); u++) {
             const int64_t grp = (u - base) / L.chunks, ch = (u - base) - grp * L.chunks;
-            const int64_t r0 = L.first + grp * LT_ROWS, rend = L.first + L.rows;
-            const int nr = (int)min((int64_t)LT_ROWS, rend - r0);
+            const int64_t r0 = L.first + grp * ROWS, rend = L.first + L.rows;
+            const int nr = (int)min((int64_t)ROWS, rend - r0);
             const int64_t k0 = ch * (L.n - 1) / L.chunks, k1 = (ch + 1) * (L.n - 1) / L.chunks;
             const int nk = (int)(k1 - k0), nl = nr + 1;
             __syncthreads();  // the previous piece has been read
@@ -474,19 +484,24 @@ __global__ void __launch_bounds__(LT_THREADS, sizeof(T) == 4 ? LT_MIN_BLOCKS_F32
             }
             __syncthreads();
             T bx = 0, by = 0, bz = 0;  // the piece's own sums: fewer roundings of the running ones
-            lattice_walk<T, SIGMA, LR>(sv, ss, sc, W, nl, nk, k0 == 0, r0 + nr == rend, px, py, pz, w.sigma2,
-                                       [&](T gm, T q0, T q1, T cy, T cx0, T cx1, T cz0, T cz1) {
-                                           if constexpr (ROLL) {
-                                               q0 *= gm;
-                                               q1 *= gm;
-                                               bx += q0 * cx0 + q1 * cx1;
-                                               by += (q0 - q1) * cy;
-                                               bz += q0 * cz0 + q1 * cz1;
-                                           } else {
-                                               const T tn = cy * ny;
-                                               bx += gm * (q0 * (cx0 * nx + tn + cz0 * nz) + q1 * (cx1 * nx - tn + cz1 * nz));
-                                           }
-                                       });
+            auto walk = [&](auto FULL) {
+                lattice_walk<T, SIGMA, LR, decltype(FULL)::value>(
+                    sv, ss, sc, W, nl, nk, k0 == 0, r0 + nr == rend, px, py, pz, w.sigma2,
+                    [&](T gm, T q0, T q1, T cy, T cx0, T cx1, T cz0, T cz1) {
+                        if constexpr (ROLL) {
+                            q0 *= gm;
+                            q1 *= gm;
+                            bx += q0 * cx0 + q1 * cx1;
+                            by += (q0 - q1) * cy;
+                            bz += q0 * cz0 + q1 * cz1;
+                        } else {
+                            const T tn = cy * ny;
+                            bx += gm * (q0 * (cx0 * nx + tn + cz0 * nz) + q1 * (cx1 * nx - tn + cz1 * nz));
+                        }
+                    });
+            };
+            if (FAST && nl == LR) walk(std::integral_constant<bool, FAST>{});
+            else walk(std::false_type{});
             ax += bx;
             ay += by;
             az += bz;
@@ -554,7 +569,10 @@ __global__ void __launch_bounds__(32 * LT_RED) k_roll_reduce(LatticeArgs<T> w, i
     for (int k = 0; k < 3; k++) w.s.o0[m][k * vld + vi] += v[k] * sc;
 }
 
-static int64_t lattice_pieces(int64_t rows, int64_t ns) { return cdiv(rows, LT_ROWS) * cdiv(ns, LT_SPAN); }
+template <class T>
+static int64_t lattice_pieces(int64_t rows, int64_t ns) {
+    return cdiv(rows, (int64_t)LatticeRows<T>::value) * cdiv(ns, (int64_t)LT_SPAN);
+}
 
 // Slices of `pieces` pieces for `npts` points: about 4 x `wake.waves` x SMs
 // CTAs (tuned per shape; a CTA of one or two pieces is short, so the last
@@ -598,7 +616,7 @@ static int wake_influence(T* rhs, int32_t nsurf, const gbvlm_dims* dims, const T
             GB_REQUIRE(dims[m].nwv >= iteration + 1, "surface %d: nwv=%lld < iteration+1", m, (long long)dims[m].nwv);
             w.s.c[m] = verts_wake[m];
             w.s.d[m] = gamma_wake[m];
-            pieces += lattice_pieces(window > 0 && iteration > window ? window : iteration, dims[m].ns);
+            pieces += lattice_pieces<T>(window > 0 && iteration > window ? window : iteration, dims[m].ns);
         } else {
             w.s.flag[m] = 0;
         }
@@ -653,7 +671,7 @@ static int wake_rollup(int32_t nsurf, const gbvlm_dims* dims, T* const* verts_wa
         w.s.flag[m] = lifting[m] ? 1 : 0;
         if (lifting[m]) GB_REQUIRE(gamma_wake && gamma_wake[m], "gamma_wake of surface %d is null", m);
         w.voff[m + 1] = w.voff[m] + (int64_t)iteration * (dims[m].ns + 1);
-        pieces += lattice_pieces(dims[m].nc, dims[m].ns) + (lifting[m] ? lattice_pieces(iteration, dims[m].ns) : 0);
+        pieces += lattice_pieces<T>(dims[m].nc, dims[m].ns) + (lifting[m] ? lattice_pieces<T>(iteration, dims[m].ns) : 0);
     }
     w.npts = w.voff[nsurf];
     w.iteration = iteration;

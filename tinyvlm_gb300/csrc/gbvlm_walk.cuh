@@ -80,6 +80,26 @@ __device__ __forceinline__ void strip_normal(const T* top, const T* bot, int W, 
 // point and its image in y = 0 share every product without a y in it.
 // ---------------------------------------------------------------------------
 
+// Square root and reciprocal of the double walk: the hardware's 20-bit
+// approximation and one step of Householder's third-order iteration (its
+// relative error e becomes about e^3), to within two units in the last place.
+// Five and three fp64 instructions where sqrt() and 1 / x take about twice
+// that, on the pipe that bounds the walk.
+__device__ __forceinline__ float length_of(float n2) { return fast_len<float>(n2); }
+__device__ __forceinline__ double length_of(double n2) {
+    double y;
+    const double m = n2 + 1e-290;  // a zero length stays (almost) zero
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(m));
+    const double t = m * y, e = fma(-t, y, 1.0);
+    return fma(t * e, fma(e, 0.375, 0.5), t);
+}
+__device__ __forceinline__ double reciprocal(double d) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+
 // a vertex seen from the point (y0, n0) and from its image (y1, n1)
 template <class T> struct RelPair { T x, z, y0, y1, n0, n1; };
 
@@ -91,8 +111,8 @@ __device__ __forceinline__ RelPair<T> make_rel_pair(T px, T py, T pz, T vx, T vy
     r.y0 = py - vy;
     r.y1 = -py - vy;
     const T s = r.x * r.x + r.z * r.z;
-    r.n0 = fast_len<T>(r.y0 * r.y0 + s);
-    r.n1 = fast_len<T>(r.y1 * r.y1 + s);
+    r.n0 = length_of(r.y0 * r.y0 + s);
+    r.n1 = length_of(r.y1 * r.y1 + s);
     return r;
 }
 
@@ -119,7 +139,7 @@ __device__ __forceinline__ void two_quotients(double n0, double d0, bool cut0, d
                                               double& q0, double& q1) {
     if (cut0) d0 = 1.0;
     if (cut1) d1 = 1.0;
-    const double inv = 1.0 / (d0 * d1);
+    const double inv = reciprocal(d0 * d1);
     q0 = cut0 ? 0.0 : n0 * (d1 * inv);
     q1 = cut1 ? 0.0 : n1 * (d0 * inv);
 }
@@ -145,8 +165,16 @@ __device__ __forceinline__ void seg_pair(const RelPair<T>& a, const RelPair<T>& 
     const bool cut0 = below(sq0, (T)RCUT_SQ) | below(a.n0, rcut) | below(b.n0, rcut);
     const bool cut1 = below(sq1, (T)RCUT_SQ) | below(a.n1, rcut) | below(b.n1, rcut);
     const bool pos0 = not_negative(ab0), pos1 = not_negative(ab1);
-    T num0 = pos0 ? s0 : s0 * (nab0 - ab0), num1 = pos1 ? s1 : s1 * (nab1 - ab1);
-    T den0 = nab0 * (pos0 ? nab0 + ab0 : sq0), den1 = nab1 * (pos1 ? nab1 + ab1 : sq1);
+    T num0, num1, den0, den1;
+    if constexpr (sizeof(T) == 8) {
+        // nab + |ab| serves both signs of ab: two fp64 additions less
+        const T e0 = nab0 + fabs(ab0), e1 = nab1 + fabs(ab1);
+        num0 = s0 * (pos0 ? (T)1 : e0), num1 = s1 * (pos1 ? (T)1 : e1);
+        den0 = nab0 * (pos0 ? e0 : sq0), den1 = nab1 * (pos1 ? e1 : sq1);
+    } else {
+        num0 = pos0 ? s0 : s0 * (nab0 - ab0), num1 = pos1 ? s1 : s1 * (nab1 - ab1);
+        den0 = nab0 * (pos0 ? nab0 + ab0 : sq0), den1 = nab1 * (pos1 ? nab1 + ab1 : sq1);
+    }
     if (SIGMA) {
         const T sm = sigma2 * (rx * rx + ry * ry + rz * rz);
         num0 *= sq0;
@@ -169,14 +197,15 @@ template <class T> struct alignas(16) Quad { T x, y, z, w; };
 // Calls add(g, k0, k1, cy, cx0, cx1, cz0, cz1) for every segment of strength
 // g.  The spanwise segments of the last line belong to the next piece unless
 // `last`, the chordwise ones of vertex 0 to the piece before unless `first`.
-template <class T, bool SIGMA, int LR, class F>
+// FULL: nl == LR, known to the compiler, so a vertex column is straight code.
+template <class T, bool SIGMA, int LR, bool FULL, class F>
 __device__ __forceinline__ void lattice_walk(const Quad<T>* v, const Quad<T>* s, const Quad<T>* c, int W, int nl, int nk,
                                              bool first, bool last, T px, T py, T pz, T sg, F&& add) {
     RelPair<T> prev[LR];
     T k0, k1, cy, cx0, cx1, cz0, cz1;
 #pragma unroll
     for (int l = 0; l < LR; l++)
-        if (l < nl) {
+        if (FULL || l < nl) {
             const Quad<T> q = v[l * W];
             prev[l] = make_rel_pair<T>(px, py, pz, q.x, q.y, q.z);
             if (l > 0 && first) {
@@ -191,10 +220,10 @@ __device__ __forceinline__ void lattice_walk(const Quad<T>* v, const Quad<T>* s,
         T gup = 0;
 #pragma unroll
         for (int l = 0; l < LR; l++)
-            if (l < nl) {
+            if (FULL || l < nl) {
                 const Quad<T> q = v[l * W + k], e = s[l * W + k];
                 const RelPair<T> cur = make_rel_pair<T>(px, py, pz, q.x, q.y, q.z);
-                if (l + 1 < nl || last) {
+                if ((FULL ? l + 1 < LR : l + 1 < nl) || last) {
                     seg_pair<T, SIGMA>(prev[l], cur, e.x, e.y, e.z, sg, k0, k1, cy, cx0, cx1, cz0, cz1);
                     add(q.w, k0, k1, cy, cx0, cx1, cz0, cz1);
                 }
