@@ -80,6 +80,8 @@ struct BatchArgs {
     const int64_t* goff;
     const int32_t* uidx;    // batch solve -> the caller's solve index
     int32_t* bad;           // per system: 1 if its case's vertices hold a non-finite coordinate
+    int32_t* fail;          // per system: 1 if its factorisation needs row interchanges (LuBatch::fail)
+    int32_t only_failed;    // the run repeats those systems with interchanges: the others' outputs stay
 };
 
 __device__ __forceinline__ void split_hl(double x, float& h, float& l) {
@@ -94,6 +96,7 @@ __global__ void __launch_bounds__(256) k_batch_geom(BatchArgs a) {
     SysDesc& S = a.sys[blockIdx.x];
     const int64_t ns = S.ns, nc = S.nc, nv = (ns + 1) * (nc + 1), np = ns * nc;
     const double al = S.alpha_geom;
+    if (threadIdx.x == 0 && !a.only_failed) a.fail[blockIdx.x] = 0;
     int bad = 0;
     for (int64_t v = threadIdx.x; v < nv; v += blockDim.x) {
         for (int k = 0; k < 3; k++) {
@@ -731,6 +734,7 @@ template <int LD_THREADS>
 __global__ void __launch_bounds__(LD_THREADS) k_batch_loads(BatchArgs a, const int32_t* solve_sys, int32_t want_gamma) {
     const int32_t sol = blockIdx.x;
     const int32_t si = solve_sys[sol];
+    if (a.only_failed && !a.fail[si]) return;
     const SysDesc& S = a.sys[si];
     const int q = sol - S.rhs_off;
     const int64_t ns = S.ns, nc = S.nc, n = S.n, nv = (ns + 1) * (nc + 1);
@@ -844,6 +848,11 @@ struct gbvlm_batch_s {
     int64_t* d_goff = nullptr;
     int32_t* d_uidx = nullptr;   // batch solve -> the caller's solve
     int32_t* d_bad = nullptr;    // per system: non-finite input vertices
+    int32_t* d_fail = nullptr;   // per system: its factorisation needs row interchanges
+    // a run factors without interchanges; whether a system needed them is
+    // looked up, and its solves repeated, before the run's results are handed
+    // out or its inputs replaced
+    bool unchecked = false;
     void* status = nullptr;      // pinned: error words and pivot flags read back with the results
     SysDesc* d_sys = nullptr;
     int32_t* d_solve_sys = nullptr;
@@ -959,10 +968,21 @@ static cudaError_t launch_assemble_lo(gbvlm_batch h, unsigned tiles, int64_t til
     return cudaGetLastError();
 }
 
-static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullptr, bool serial_lu = false) {
+// one size group's factorisation: without interchanges, or (pivot) with them
+static int batch_factor(gbvlm_batch h, int g, cudaStream_t st, bool lookahead, bool pivot) {
+    if (pivot || !h->plans[g].fast) return lu_batch_factor<float>(h->lub, h->plans[g], st, lookahead);
+    LuBatch<float> B = h->lub;
+    B.fail = h->d_fail;
+    return lu_batch_factor_fast<float>(B, h->plans[g], st, lookahead);
+}
+
+// pivot: repeat the systems that d_fail marks, with interchanges
+static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullptr, bool serial_lu = false,
+                         bool pivot = false) {
     auto mark = [&](int k) { if (ev) cudaEventRecord(ev[k], st); };
     int64_t nlaunch = 0;
-    for (int g = 0; g < h->ngroups; g++) nlaunch += lu_plan_launches(h->plans[g], 4);
+    for (int g = 0; g < h->ngroups; g++)
+        nlaunch += h->plans[g].fast ? lu_plan_launches_fast(h->plans[g], 4) : lu_plan_launches(h->plans[g], 4);
     int32_t mr = 0;
     for (auto& s : h->sys) mr = std::max(mr, s.nrhs);
     const int64_t solves = h->use_flow ? trs_flow_launches(mr, h->flow.groups) : (mr + 7) / 8;
@@ -983,6 +1003,8 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
     a.goff = h->d_goff;
     a.uidx = h->d_uidx;
     a.bad = h->d_bad;
+    a.fail = h->d_fail;
+    a.only_failed = pivot ? 1 : 0;
     // staged: every phase after the previous one on `st` (stage timing, or
     // kernel timing without the groups' launches overlapping); otherwise each
     // size group's assembly and factorisation run on its own branch, group 0
@@ -1014,7 +1036,7 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
     mark(3);
     if (staged) {
         for (int g = 0; g < h->ngroups; g++) {
-            int rc = lu_batch_factor<float>(h->lub, h->plans[g], st, !serial_lu);
+            int rc = batch_factor(h, g, st, !serial_lu, pivot);
             if (rc) return rc;
         }
     } else {
@@ -1030,7 +1052,7 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
                     GB_CUDA(launch_assemble_lo(h, (unsigned)h->gtile[g][1], h->gtile[g][0], a, h->lo_side));
                 }
             }
-            int rc = lu_batch_factor<float>(h->lub, h->plans[g], h->side[g], true);
+            int rc = batch_factor(h, g, h->side[g], true, pivot);
             if (rc) return rc;
             GB_CUDA(cudaEventRecord(h->join[g], h->side[g]));
         }
@@ -1085,6 +1107,22 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
         GB_LAUNCH_CHECK();
     }
     mark(6);
+    return GBVLM_OK;
+}
+
+// After a run: repeats, with row interchanges, the solves of the systems whose
+// factorisation needed them (synchronises st).  The others' outputs stay.
+static int batch_settle(gbvlm_batch h, cudaStream_t st) {
+    if (!h->unchecked) return GBVLM_OK;
+    GB_CUDA(cudaStreamWaitEvent(st, h->done, 0));
+    std::vector<int32_t> f(h->nsys);
+    GB_CUDA(cudaMemcpyAsync(f.data(), h->d_fail, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
+    GB_CUDA(cudaStreamSynchronize(st));
+    h->unchecked = false;
+    if (std::none_of(f.begin(), f.end(), [](int32_t x) { return x != 0; })) return GBVLM_OK;
+    const int rc = batch_enqueue(h, st, nullptr, false, true);
+    if (rc) return rc;
+    GB_CUDA(cudaEventRecord(h->done, st));
     return GBVLM_OK;
 }
 
@@ -1208,6 +1246,7 @@ int gbvlm_batch_create_ex(gbvlm_batch* out, int32_t ncases, const gbvlm_dims* di
     const size_t o_ssys = reserve(sizeof(int32_t) * solve_sys.size());
     const size_t o_uidx = reserve(sizeof(int32_t) * solve_sys.size());
     const size_t o_bad = reserve(sizeof(int32_t) * h->nsys);
+    const size_t o_fail = reserve(sizeof(int32_t) * h->nsys);
     // tile prefix tables
     // ring rows per float assembly tile: at most 4, at most 2 with 256-ring span chunks (shared memory)
     h->asm_rows = (int)std::min<int64_t>(h->tp.batch_assembly_rows, h->tp.batch_assembly_span > 128 ? 2 : 4);
@@ -1255,6 +1294,7 @@ int gbvlm_batch_create_ex(gbvlm_batch* out, int32_t ncases, const gbvlm_dims* di
     h->d_solve_sys = (int32_t*)(base + o_ssys);
     h->d_uidx = (int32_t*)(base + o_uidx);
     h->d_bad = (int32_t*)(base + o_bad);
+    h->d_fail = (int32_t*)(base + o_fail);
     h->d_tpfx = (int64_t*)(base + o_tpfx);
     h->d_tpfx_rows = (int64_t*)(base + o_tpfx_rows);
     h->d_rpfx = (int64_t*)(base + o_rpfx);
@@ -1455,6 +1495,10 @@ int gbvlm_batch_set_inputs(gbvlm_batch h, const float* verts, const double* alph
     for (int32_t u = 0; u < h->nsolve; u++)
         GB_REQUIRE(isfinite(alphas[u]), "alpha %d is not finite", u);
     cudaStream_t st = to_cuda(stream);
+    {
+        const int rc = batch_settle(h, st);  // the last run still needs its inputs
+        if (rc) return rc;
+    }
     // conditions baked into the graph: rebuild it if they change
     const double r[3] = {ref_pt ? ref_pt[0] : 0, ref_pt ? ref_pt[1] : 0, ref_pt ? ref_pt[2] : 0};
     if (u_inf != h->u_inf || rho != h->rho || r[0] != h->ref[0] || r[1] != h->ref[1] || r[2] != h->ref[2]) {
@@ -1494,6 +1538,7 @@ int gbvlm_batch_run_eager(gbvlm_batch h, int32_t want_gamma, gbvlm_stream stream
         cudaGraphExecDestroy(h->exec);
         h->exec = nullptr;
     }
+    h->unchecked = true;
     int rc = batch_enqueue(h, to_cuda(stream));
     if (rc == GBVLM_OK) GB_CUDA(cudaEventRecord(h->done, to_cuda(stream)));
     return rc;
@@ -1525,6 +1570,7 @@ int gbvlm_batch_run(gbvlm_batch h, int32_t want_gamma, gbvlm_stream stream) {
         h->graph = g;
         GB_CUDA(cudaGraphInstantiate(&h->exec, h->graph, cudaGraphInstantiateFlagUseNodePriority));
     }
+    h->unchecked = true;
     GB_CUDA(cudaGraphLaunch(h->exec, st));
     GB_CUDA(cudaEventRecord(h->done, st));
     return GBVLM_OK;
@@ -1535,6 +1581,7 @@ int gbvlm_batch_profile(gbvlm_batch h, float* stage_ms, gbvlm_stream stream) {
     cudaStream_t st = to_cuda(stream);
     cudaEvent_t ev[7];
     for (int k = 0; k < 7; k++) GB_CUDA(cudaEventCreate(&ev[k]));
+    h->unchecked = true;
     int rc = batch_enqueue(h, st, ev);
     if (rc == GBVLM_OK) {
         cudaEventRecord(h->done, st);
@@ -1554,6 +1601,7 @@ int gbvlm_batch_update_profile(gbvlm_batch h, double* out, gbvlm_stream stream) 
     cudaStream_t st = to_cuda(stream);
     std::vector<cudaEvent_t> ev;
     for (int g = 0; g < h->ngroups; g++) h->plans[g].tc_events = &ev;
+    h->unchecked = true;
     int rc = batch_enqueue(h, st, nullptr, true);
     for (int g = 0; g < h->ngroups; g++) h->plans[g].tc_events = nullptr;
     double ms = 0;
@@ -1585,13 +1633,9 @@ int gbvlm_batch_results(gbvlm_batch h, double* coeffs, float* gamma, gbvlm_strea
     GB_REQUIRE(!gamma || h->want_gamma, "gamma requested but the last run did not store it");
     cudaStream_t st = to_cuda(stream);
     constexpr int G = gbvlm_batch_s::MAX_GROUPS;
-    // outputs are already in the caller's order: straight into the caller's buffers
-    GB_CUDA(cudaMemcpyAsync(coeffs, h->d_out, sizeof(double) * 5 * h->nsolve, cudaMemcpyDeviceToHost, st));
-    if (gamma)
-        GB_CUDA(cudaMemcpyAsync(gamma, h->d_gamma, sizeof(float) * h->gamma_floats, cudaMemcpyDeviceToHost, st));
     // status words (bounded-wait errors of the LU plans and the triangular
-    // solve, pivot flags) with the same synchronisation
-    const size_t sbytes = sizeof(int32_t) * (G + 1 + 2 * (size_t)h->nsys);
+    // solve, pivot flags, systems that need interchanges) with the same synchronisation
+    const size_t sbytes = sizeof(int32_t) * (G + 1 + 3 * (size_t)h->nsys);
     if (!h->status) {
         h->status = pinned_take(sbytes);
         if (!h->status) {
@@ -1601,15 +1645,29 @@ int gbvlm_batch_results(gbvlm_batch h, double* coeffs, float* gamma, gbvlm_strea
         h->status_bytes = sbytes;
     }
     int32_t* hs = (int32_t*)h->status;
-    memset(hs, 0, sizeof(int32_t) * (G + 1));
-    for (int g = 0; g < h->ngroups; g++)
-        if (h->plans[g].d_err)
-            GB_CUDA(cudaMemcpyAsync(hs + g, h->plans[g].d_err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    if (h->use_flow && h->flow.d_ctl)
-        GB_CUDA(cudaMemcpyAsync(hs + G, h->flow.d_ctl + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaMemcpyAsync(hs + G + 1, h->lub.info, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaMemcpyAsync(hs + G + 1 + h->nsys, h->d_bad, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaStreamSynchronize(st));
+    const int32_t* fail = hs + G + 1 + 2 * h->nsys;
+    while (true) {
+        // outputs are already in the caller's order: straight into the caller's buffers
+        GB_CUDA(cudaMemcpyAsync(coeffs, h->d_out, sizeof(double) * 5 * h->nsolve, cudaMemcpyDeviceToHost, st));
+        if (gamma)
+            GB_CUDA(cudaMemcpyAsync(gamma, h->d_gamma, sizeof(float) * h->gamma_floats, cudaMemcpyDeviceToHost, st));
+        memset(hs, 0, sizeof(int32_t) * (G + 1));
+        for (int g = 0; g < h->ngroups; g++)
+            if (h->plans[g].d_err)
+                GB_CUDA(cudaMemcpyAsync(hs + g, h->plans[g].d_err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        if (h->use_flow && h->flow.d_ctl)
+            GB_CUDA(cudaMemcpyAsync(hs + G, h->flow.d_ctl + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaMemcpyAsync(hs + G + 1, h->lub.info, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaMemcpyAsync(hs + G + 1 + h->nsys, h->d_bad, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaMemcpyAsync(hs + G + 1 + 2 * h->nsys, h->d_fail, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost,
+                                st));
+        GB_CUDA(cudaStreamSynchronize(st));
+        const bool again = h->unchecked && std::any_of(fail, fail + h->nsys, [](int32_t x) { return x != 0; });
+        h->unchecked = h->unchecked && again;
+        if (!again) break;
+        const int rc = batch_settle(h, st);  // repeats them, with interchanges
+        if (rc) return rc;
+    }
     for (int g = 0; g < h->ngroups; g++)
         if (hs[g]) {
             set_error("LU: a tensor-core update tile timed out waiting for its MMAs");

@@ -39,7 +39,8 @@ constexpr int PR_MAX_CLUSTER = 16;   // largest cluster of the register panel
 constexpr int SW2_THREADS = 256;     // k_swap2: columns per CTA
 constexpr int PACK_MIN_SLICE = 128;  // narrowest slice of a packed one-CTA panel (at most 8 systems per CTA)
 constexpr int TRSM_COLS = 128;
-constexpr int GT = 64;  // update tile edge
+constexpr int GT = 64;      // update tile edge
+constexpr int GT_F64 = 32;  // ... in double, without interchanges: more CTAs for the fp64 units
 constexpr int GK = LU_NB;
 constexpr int PERM_SMEM = 12 * 1024;  // systems up to this size build the permutation in shared memory
 constexpr int TS_SMEM_BYTES = 200 * 1024;
@@ -341,8 +342,8 @@ __device__ __forceinline__ void panel_barrier(int nwa, int bar) {
 // false (in every lane) where partial pivoting would have left the diagonal,
 // or where a pivot is zero, subnormal or not a number.  Each row sees the
 // operations of the pivoting loop in their order.
-template <class T>
-__device__ __forceinline__ bool panel_diag(T (&x)[GK], int nb, T (*u)[GK], T* rds, int lane) {
+template <class T, int LDU>
+__device__ __forceinline__ bool panel_diag(T (&x)[GK], int nb, T* u, T* rds, int lane) {
     using V2 = typename Vec4<T>::type;
     bool good = true;
     static_for<0, GK>([&](auto JJ) {
@@ -357,7 +358,7 @@ __device__ __forceinline__ bool panel_diag(T (&x)[GK], int nb, T (*u)[GK], T* rd
                     v.y = x[t + 1];
                     v.z = x[t + 2];
                     v.w = x[t + 3];
-                    *reinterpret_cast<V2*>(&u[jj][t]) = v;
+                    *reinterpret_cast<V2*>(u + jj * LDU + t) = v;
                 }
             }
             const T rd = rcp_rn(d);
@@ -369,7 +370,7 @@ __device__ __forceinline__ bool panel_diag(T (&x)[GK], int nb, T (*u)[GK], T* rd
             if (below) {
                 const T lm = x[jj] * rd;
                 x[jj] = lm;
-                const uint32_t ua = (uint32_t)__cvta_generic_to_shared(&u[jj][0]);
+                const uint32_t ua = (uint32_t)__cvta_generic_to_shared(u + jj * LDU);
 #pragma unroll
                 for (int tg = (jj + 1) & ~3; tg < GK; tg += 4) {
                     T v[4];
@@ -468,7 +469,7 @@ __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const
             const bool first = tid < 32;  // the slice's first warp factors the diagonal block
             if (first) {
                 if (rank != 0) load_row(lane, lane < nb);  // rank 0's first warp holds those rows
-                good = panel_diag<T>(x[0], nb, fu, frd, lane);
+                good = panel_diag<T, GK>(x[0], nb, &fu[0][0], frd, lane);
                 if (rank != 0) load_row(lid[0], lid[0] >= 0);
                 if (lane == 0) sm.f_bad[slice] = good ? 0 : 1;
             }
@@ -623,6 +624,344 @@ __device__ __forceinline__ int find_block(const int64_t* pfx, int cnt, int64_t b
         if (pfx[mid] <= b) lo = mid; else hi = mid - 1;
     }
     return lo;
+}
+
+// one value by cp.async; !load fills the destination with zero and reads nothing
+template <class T>
+__device__ __forceinline__ void cp_async_zfill(uint32_t dst, const T* src, bool load) {
+    if constexpr (sizeof(T) == 4)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(load ? 4 : 0) : "memory");
+    else
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(load ? 8 : 0) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Factorisation without interchanges.  AICs are dominated by their diagonal:
+// partial pivoting keeps every row in place.  So a factorisation first runs
+// without the pivot search, in two launches per block of W columns and the
+// trailing update, and checks on the way that the search would have found the
+// diagonal every time: |a| <= |pivot| for every entry below every pivot (the
+// diagonal comes first on ties), no pivot zero, subnormal or not a number.  A
+// system that fails (LuBatch::fail) is left alone from there on, and the
+// caller factors it again with the pivoting launches from the original matrix.
+//
+//   k_lu_diag : one CTA per system factors the W x W diagonal block in shared
+//               memory (W = 128 in float, 32 in double)
+//   k_lu_rows : L21 = A21 U11^-1 a thread per row and U12 = L11^-1 A12 a
+//               thread per column, by substitution in fp32 (fp64) arithmetic;
+//               no thread needs another's values
+//
+// Against the pivoting launches (per 128 columns four register panels, their
+// row moves and inner updates, and the explicit inverse of L11 with its
+// product: 14 dependent launches) this is the block's serial chain cut to
+// three launches; the substitution is at least as accurate as the tensor
+// cores' three TF32 passes that it replaces there.
+// Measured, whole calls (pivoting launches -> these): 512 wings x 8 angles
+// 13.35 -> 11.47 ms, 64 x 4 exact 7.38 -> 5.73 ms, 16,384 unknowns x 64 angles
+// 69.8 -> 62.2 ms, 1000 unknowns 1.61 -> 1.04 ms, 256 unknowns 483 -> 375 us; in
+// double 900 unknowns 6.40 -> 4.80 ms.
+// ---------------------------------------------------------------------------
+template <class T> struct Fast {
+    static constexpr int W = sizeof(T) == 4 ? LU_OUTER : GK;
+    static constexpr int NB = W / GK;
+    static constexpr int LD = W + 16 / (int)sizeof(T);            // diagonal block's row stride: 16-byte aligned rows
+    static constexpr int DT = sizeof(T) == 4 ? 256 : 32;          // threads of k_lu_diag
+    static constexpr int RT = sizeof(T) == 4 ? 128 : 32;          // rows or columns per CTA of k_lu_rows: in double
+                                                                  // few, to reach the fp64 units of many SMs
+    static constexpr int LDX = RT + 1;
+    static constexpr int MSIZE = NB * (NB + 1) / 2 * GK * GK;     // the blocks on and above the diagonal
+    static constexpr int WORK = W * W + W;                        // per system: the factored block by rows, reciprocal pivots
+    static constexpr size_t diag_smem = sizeof(T) * (size_t)(W * LD + GK * GK + W);
+    static constexpr size_t rows_smem = sizeof(T) * (size_t)(MSIZE + W + W * LDX);
+};
+
+// x against 32 rows of a triangle, u its address and `stride` bytes per row:
+// ROWS (x a row of A21, u the rows of U): l_j = x_j / u_jj, x_t -= l_j u_jt, and
+// whether |x_j| <= |u_jj| throughout; else (x a column of A12, u the columns of
+// the unit lower triangle): x_t -= x_j l_tj
+template <class T, bool ROWS>
+__device__ __forceinline__ bool eliminate32(T (&x)[GK], uint32_t u, uint32_t stride, const T* rd) {
+    bool good = true;
+    static_for<0, GK>([&](auto JJ) {
+        constexpr int jj = decltype(JJ)::value;
+        const uint32_t ua = u + jj * stride;
+        T lm = x[jj];
+        if constexpr (ROWS) {
+            good = good && tabs(lm) <= tabs(lds1(ua + jj * (uint32_t)sizeof(T), T(0)));
+            lm = lm * rd[jj];
+            x[jj] = lm;
+        }
+#pragma unroll
+        for (int tg = (jj + 1) & ~3; tg < GK; tg += 4) {
+            T v[4];
+            lds4(ua + tg * (uint32_t)sizeof(T), v);
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+                if (tg + e > jj) x[tg + e] -= lm * v[e];
+        }
+    });
+    return good;
+}
+
+// the block's trailing part after its 32-column step c: rows and columns past
+// it, NC x 32 of each; warp w holds 4 NC rows, a lane NC columns
+template <int NC, int LD>
+__device__ __forceinline__ void diag_update(float* S, int c, int wid, int lane) {
+    const int lo = GK * (c + 1), r0 = lo + 4 * NC * wid;
+    float acc[4 * NC][NC];
+#pragma unroll
+    for (int i = 0; i < 4 * NC; i++)
+#pragma unroll
+        for (int j = 0; j < NC; j++) acc[i][j] = 0.f;
+#pragma unroll 1
+    for (int k = 0; k < GK; k += 4) {
+        float b[4][NC];
+#pragma unroll
+        for (int e = 0; e < 4; e++)
+#pragma unroll
+            for (int j = 0; j < NC; j++) b[e][j] = S[(GK * c + k + e) * LD + lo + 32 * j + lane];
+#pragma unroll
+        for (int i = 0; i < 4 * NC; i++) {
+            const float4 a = *reinterpret_cast<const float4*>(S + (r0 + i) * LD + GK * c + k);
+#pragma unroll
+            for (int j = 0; j < NC; j++) {
+                acc[i][j] += a.x * b[0][j];
+                acc[i][j] += a.y * b[1][j];
+                acc[i][j] += a.z * b[2][j];
+                acc[i][j] += a.w * b[3][j];
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < 4 * NC; i++)
+#pragma unroll
+        for (int j = 0; j < NC; j++) S[(r0 + i) * LD + lo + 32 * j + lane] -= acc[i][j];
+}
+
+template <class T>
+__global__ void __launch_bounds__(Fast<T>::DT) k_lu_diag(LuBatch<T> B, int64_t k0, const int32_t* act, T* work,
+                                                         int32_t base) {
+    using F = Fast<T>;
+    constexpr int W = F::W, LD = F::LD, DT = F::DT;
+    extern __shared__ __align__(16) unsigned char fast_smem[];
+    T* S = reinterpret_cast<T*>(fast_smem);  // the block by rows
+    T* LT = S + W * LD;                      // the current 32 x 32 triangle's L by columns
+    T* rds = LT + GK * GK;                   // reciprocal pivots
+    __shared__ int s_bad;
+    const int32_t sid = act[blockIdx.x];
+    const int64_t n = B.n[sid], ld = B.ld[sid];
+    T* A = B.A[sid] + k0 + k0 * ld;
+    const int w = (int)min((int64_t)W, n - k0);
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    // the identity permutation, for a system that fails too: a batch's solves
+    // run on its factors, whatever they hold, before it is factored again
+    for (int e = tid; e < w; e += DT) {
+        B.ipiv[sid][k0 + e] = (int32_t)(k0 + e);
+        B.perm[sid][k0 + e] = (int32_t)(k0 + e);
+    }
+    if (B.fail[sid]) return;
+    if (tid == 0) s_bad = 0;
+    for (int e = tid; e < W * W; e += DT) {
+        const int r = e & (W - 1), c = e / W;
+        const bool in = r < w && c < w;
+        cp_async_zfill<T>((uint32_t)__cvta_generic_to_shared(S + r * LD + c), in ? A + r + c * ld : A, in);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    if (w < W) {  // past the system's end: an identity, which changes nothing
+        for (int r = w + tid; r < W; r += DT) S[r * LD + r] = (T)1;
+        __syncthreads();
+    }
+#pragma unroll 1
+    for (int c = 0; c < F::NB; c++) {
+        T* D = S + GK * c * LD + GK * c;
+        if (wid == 0) {
+            T x[GK];
+#pragma unroll
+            for (int t = 0; t < GK; t++) x[t] = D[lane * LD + t];
+            __syncwarp();
+            const bool good = panel_diag<T, LD>(x, GK, D, rds + GK * c, lane);
+            if (!good && lane == 0) s_bad = 1;
+#pragma unroll
+            for (int t = 0; t < GK; t++) {
+                if (t < lane) D[lane * LD + t] = x[t];
+                LT[t * GK + lane] = x[t];
+            }
+        }
+        if constexpr (F::NB > 1) {
+            __syncthreads();
+            const int lo = GK * (c + 1);
+            const int i = lo + (tid & (DT / 2 - 1));
+            T x[GK];
+            if (i < W) {
+                if (tid < DT / 2) {  // a row below
+                    T* row = S + i * LD + GK * c;
+#pragma unroll
+                    for (int t = 0; t < GK; t += 4) {
+                        T v[4];
+                        lds4((uint32_t)__cvta_generic_to_shared(row + t), v);
+#pragma unroll
+                        for (int e = 0; e < 4; e++) x[t + e] = v[e];
+                    }
+                    const bool good = eliminate32<T, true>(x, (uint32_t)__cvta_generic_to_shared(D),
+                                                           LD * (uint32_t)sizeof(T), rds + GK * c);
+                    if (!good) s_bad = 1;
+                    using V2 = typename Vec4<T>::type;
+#pragma unroll
+                    for (int t = 0; t < GK; t += 4) {
+                        V2 v;
+                        v.x = x[t];
+                        v.y = x[t + 1];
+                        v.z = x[t + 2];
+                        v.w = x[t + 3];
+                        *reinterpret_cast<V2*>(row + t) = v;
+                    }
+                } else {  // a column to the right
+#pragma unroll
+                    for (int t = 0; t < GK; t++) x[t] = S[(GK * c + t) * LD + i];
+                    eliminate32<T, false>(x, (uint32_t)__cvta_generic_to_shared(LT), GK * (uint32_t)sizeof(T), nullptr);
+#pragma unroll
+                    for (int t = 0; t < GK; t++) S[(GK * c + t) * LD + i] = x[t];
+                }
+            }
+            __syncthreads();
+            if (c == 0) diag_update<3, LD>(S, 0, wid, lane);
+            if (c == 1) diag_update<2, LD>(S, 1, wid, lane);
+            if (c == 2) diag_update<1, LD>(S, 2, wid, lane);
+            __syncthreads();
+        }
+    }
+    __syncthreads();
+    if (s_bad) {
+        if (tid == 0) B.fail[sid] = 1;
+        return;
+    }
+    for (int e = tid; e < W * W; e += DT) {
+        const int r = e & (W - 1), c = e / W;
+        if (r < w && c < w) A[r + c * ld] = S[r * LD + c];
+    }
+    T* wk = work + (int64_t)(sid - base) * F::WORK;
+    for (int e = tid; e < W * W; e += DT) wk[e] = S[(e / W) * LD + (e & (W - 1))];
+    for (int e = tid; e < W; e += DT) wk[W * W + e] = rds[e];
+}
+
+template <class T>
+__global__ void __launch_bounds__(Fast<T>::RT) k_lu_rows(LuBatch<T> B, int64_t k0, const int32_t* act,
+                                                         const int64_t* pfx, int cnt, const T* work, int32_t base) {
+    using F = Fast<T>;
+    constexpr int W = F::W, NB = F::NB, RT = F::RT, LDX = F::LDX;
+    extern __shared__ __align__(16) unsigned char fast_smem[];
+    T* M = reinterpret_cast<T*>(fast_smem);  // block row p: 32 rows of (NB - p) x 32
+    T* rds = M + F::MSIZE;
+    T* Xs = rds + W;                         // solved values, [W][LDX]: a thread's own column
+    const int a = find_block(pfx, cnt, blockIdx.x);
+    const int32_t sid = act[a];
+    // another CTA of the system may set it meanwhile: one thread's reading for all
+    if (__syncthreads_or(threadIdx.x == 0 && *(volatile int32_t*)&B.fail[sid])) return;
+    const int64_t n = B.n[sid], ld = B.ld[sid];
+    T* A = B.A[sid];
+    const int64_t kend = k0 + W;  // systems here have n > kend
+    const int64_t nr = (n - kend + RT - 1) / RT, idx = blockIdx.x - pfx[a];
+    const bool rows = idx < nr;
+    const int64_t i0 = kend + (rows ? idx : idx - nr) * RT;
+    const int tid = threadIdx.x, lane = tid & 31, w0 = tid & ~31;
+    const bool have = i0 + tid < n;
+    const T* wk = work + (int64_t)(sid - base) * F::WORK;
+    auto moff = [](int p) { return GK * GK * (p * NB - p * (p - 1) / 2); };
+#pragma unroll
+    for (int p = 0; p < NB; p++)
+#pragma unroll
+        for (int c = p; c < NB; c++) {  // one 32 x 32 block, a warp per row
+            const T* src = rows ? wk + (GK * p) * W + GK * c : A + (k0 + GK * c) + (k0 + GK * p) * ld;
+            const int64_t sld = rows ? (int64_t)W : ld;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(M + moff(p) + GK * (c - p) + lane);
+#pragma unroll
+            for (int j = tid >> 5; j < GK; j += RT / 32)
+                cp_async_zfill<T>(dst + (uint32_t)(j * (NB - p) * GK) * (uint32_t)sizeof(T), src + j * sld + lane, true);
+        }
+    if (rows) {
+        for (int e = tid; e < W; e += RT)
+            cp_async_zfill<T>((uint32_t)__cvta_generic_to_shared(rds + e), wk + W * W + e, true);
+    } else {
+        // columns are read by warps, 32 rows at a time, and turned in shared memory
+        for (int q = 0; q < 32; q++) {
+            const bool ok = i0 + w0 + q < n;
+            const T* col = ok ? A + k0 + lane + (i0 + w0 + q) * ld : A;
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Xs + lane * LDX + w0 + q);
+#pragma unroll
+            for (int c = 0; c < NB; c++)
+                cp_async_zfill<T>(dst + (uint32_t)(GK * c * LDX) * (uint32_t)sizeof(T), col + (ok ? GK * c : 0), ok);
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    // a row's entries are read a 32-column step ahead of their use
+    T nx[GK];
+    const T* rsrc = A + i0 + tid + k0 * ld;
+#pragma unroll
+    for (int t = 0; t < GK; t++) nx[t] = rows && have ? rsrc[t * ld] : (T)0;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    bool good = true;
+    const uint32_t Ma = (uint32_t)__cvta_generic_to_shared(M);
+#pragma unroll 1
+    for (int c = 0; c < NB; c++) {
+        T x[GK];
+        if (rows) {
+#pragma unroll
+            for (int t = 0; t < GK; t++) x[t] = nx[t];
+            if (c + 1 < NB) {
+                rsrc += GK * ld;
+#pragma unroll
+                for (int t = 0; t < GK; t++) nx[t] = have ? rsrc[t * ld] : (T)0;
+            }
+        } else {
+#pragma unroll
+            for (int t = 0; t < GK; t++) x[t] = Xs[(GK * c + t) * LDX + tid];
+        }
+#pragma unroll 1
+        for (int p = 0; p < c; p++) {
+            const uint32_t wb = (uint32_t)((NB - p) * GK) * (uint32_t)sizeof(T);
+            uint32_t ua = Ma + (uint32_t)(moff(p) + GK * (c - p)) * (uint32_t)sizeof(T);
+#pragma unroll 4
+            for (int jj = 0; jj < GK; jj++, ua += wb) {
+                const T l = Xs[(GK * p + jj) * LDX + tid];
+#pragma unroll
+                for (int tg = 0; tg < GK; tg += 4) {
+                    T v[4];
+                    lds4(ua + tg * (uint32_t)sizeof(T), v);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) x[tg + e] -= l * v[e];
+                }
+            }
+        }
+        const uint32_t ud = Ma + (uint32_t)moff(c) * (uint32_t)sizeof(T);
+        const uint32_t ub = (uint32_t)((NB - c) * GK) * (uint32_t)sizeof(T);
+        if (rows) {
+            good = eliminate32<T, true>(x, ud, ub, rds + GK * c) && good;
+            T* dst = A + i0 + tid + (k0 + GK * c) * ld;
+            if (have)
+#pragma unroll
+                for (int t = 0; t < GK; t++) dst[t * ld] = x[t];
+        } else {
+            eliminate32<T, false>(x, ud, ub, nullptr);
+        }
+        if (!rows || c + 1 < NB)
+#pragma unroll
+            for (int t = 0; t < GK; t++) Xs[(GK * c + t) * LDX + tid] = x[t];
+    }
+    if (rows) {
+        if (have && !good) B.fail[sid] = 1;
+        return;
+    }
+    __syncwarp();  // a warp's 32 columns are its own
+#pragma unroll 4
+    for (int q = 0; q < 32; q++) {
+        if (i0 + w0 + q >= n) break;
+        T* col = A + k0 + (i0 + w0 + q) * ld;
+#pragma unroll
+        for (int c = 0; c < NB; c++) col[GK * c + lane] = Xs[(GK * c + lane) * LDX + w0 + q];
+    }
 }
 
 template <class T>
@@ -977,14 +1316,16 @@ __global__ void __launch_bounds__(IN_THREADS) k_inner(LuBatch<float> B, int64_t 
 // outer panel's columns [k+GK, min(n, kend)) over rows [k+GK, n); the columns
 // right of the block wait for the block's swaps, U12 solve and tensor-core
 // update.
-template <class T>
-__global__ void __launch_bounds__(256) k_update(LuBatch<T> B, int64_t k, const int32_t* act, const int64_t* pfx,
-                                               int cnt, int64_t kend, int mode) {
+template <class T, int GT = 64>
+__global__ void __launch_bounds__(GT * GT / 16) k_update(LuBatch<T> B, int64_t k, const int32_t* act,
+                                                        const int64_t* pfx, int cnt, int64_t kend, int mode) {
+    constexpr int NT = GT * GT / 16;  // threads
     constexpr int SW = GT + 4;  // row stride keeps 16-byte alignment of every 4-run
     __shared__ __align__(16) T sA[GK][SW];  // L21 tile: [kk][row]
     __shared__ __align__(16) T sB[GK][SW];  // U12 tile: [kk][col]
     const int a = find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
+    if (B.fail && B.fail[sid]) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     T* A = B.A[sid];
     const int64_t lo = k + GK;  // systems here have n > k + GK
@@ -1003,24 +1344,24 @@ __global__ void __launch_bounds__(256) k_update(LuBatch<T> B, int64_t k, const i
     }
     const int tid = threadIdx.x;
     {
-        constexpr int PER = GK * GT / 256;  // elements of each tile per thread
+        constexpr int PER = GK * GT / NT;  // elements of each tile per thread
         T va[PER], vb[PER];
 #pragma unroll
         for (int u = 0; u < PER; u++) {
-            const int e = tid + u * 256;
+            const int e = tid + u * NT;
             const int64_t r = r0 + e % GT, c = c0 + e / GK;
             va[u] = r < row_hi ? A[r + (k + e / GT) * ld] : (T)0;
             vb[u] = c < col_hi ? A[(k + e % GK) + c * ld] : (T)0;
         }
 #pragma unroll
         for (int u = 0; u < PER; u++) {
-            const int e = tid + u * 256;
+            const int e = tid + u * NT;
             sA[e / GT][e % GT] = va[u];
             sB[e % GK][e / GK] = vb[u];
         }
     }
     __syncthreads();
-    const int tx = tid & 15, ty = tid >> 4;
+    const int tx = tid % (GT / 4), ty = tid / (GT / 4);
     T acc[4][4];
 #pragma unroll
     for (int i = 0; i < 4; i++)
@@ -1075,6 +1416,9 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_update_tc(LuBatch<float> B, 
     __shared__ uint32_t tslot;
     const int a = find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
+    // without interchanges: nothing to do for a system that needs them (the next
+    // diagonal block may set it meanwhile: one thread's reading for all)
+    if (part != 1 && B.fail && __syncthreads_or(threadIdx.x == 0 && *(volatile int32_t*)&B.fail[sid])) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     float* A = B.A[sid];
     const int64_t lo = k0 + w;  // systems here have n > k0 + w
@@ -1654,14 +1998,6 @@ template <class T> struct One {
     static constexpr size_t smem = sizeof(T) * (size_t)(FB * LD + 3 * FB + Q * FB);
 };
 constexpr int64_t ONE_MIN = 64;  // up to here k_trsolve: a chain of one or two 32-row blocks needs no hand-over
-
-template <class T>
-__device__ __forceinline__ void cp_async_zfill(uint32_t dst, const T* src, bool load) {
-    if constexpr (sizeof(T) == 4)
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(load ? 4 : 0) : "memory");
-    else
-        asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(dst), "l"(src), "r"(load ? 8 : 0) : "memory");
-}
 
 // sum of a row of 32 tile entries times 32 values, both read as 16-byte vectors (the values as broadcasts)
 __device__ __forceinline__ float row32(const float* a, const float* v) {
@@ -2406,6 +2742,77 @@ int lu_batch_factor(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t st, bo
 }
 
 template <class T>
+int lu_batch_factor_fast(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t st, bool lookahead) {
+    using F = Fast<T>;
+    constexpr int E = sizeof(T) == 4 ? 0 : 1;
+    GB_REQUIRE(B.fail && plan.d_minv, "factorisation without interchanges: no workspace");
+    T* work = reinterpret_cast<T*>(plan.d_minv);
+    lookahead = lookahead && plan.la_stream != nullptr && plan.tc_events == nullptr;
+    bool pending = false;  // a lookahead update in flight on plan.la_stream
+    for (size_t s = 0; s < plan.steps.size(); s++) {
+        const LuStep& S = plan.steps[s];
+        if (S.n_panel == 0 || S.k % F::W != 0) continue;
+        const int32_t* act = plan.d_act + S.act_off;
+        k_lu_diag<T><<<(unsigned)S.n_panel, F::DT, F::diag_smem, st>>>(B, S.k, act, work, plan.base);
+        GB_LAUNCH_CHECK();
+        if (S.fr_blocks[E] == 0) continue;
+        if (pending) {  // the columns that k_lu_rows solves are those the lookahead update is still working on
+            GB_CUDA(cudaStreamWaitEvent(st, plan.la_join, 0));
+            pending = false;
+        }
+        k_lu_rows<T><<<(unsigned)S.fr_blocks[E], F::RT, F::rows_smem, st>>>(B, S.k, act, plan.d_pfx + S.fr_pfx[E],
+                                                                           S.fr_cnt[E], work, plan.base);
+        GB_LAUNCH_CHECK();
+        if constexpr (sizeof(T) == 8) {
+            k_update<T, GT_F64><<<(unsigned)S.fu_blocks, GT_F64 * GT_F64 / 16, 0, st>>>(
+                B, S.k, act, plan.d_pfx + S.fu_pfx, S.fr_cnt[E], 0, 0);
+            GB_LAUNCH_CHECK();
+        } else {
+            const LuStep& U = plan.steps[s + F::W / GK - 1];  // the block's last step holds its update's tables
+            const int32_t* uact = plan.d_act + U.act_off;
+            auto tc_launch = [&](int64_t blocks, int64_t pfx_off, int part, cudaStream_t s_) {
+                const int64_t* pfx = plan.d_pfx + pfx_off;
+                // the next outer panel (part 1) in 128-column tiles, the rest in the plan's width
+                if (part != 1 && plan.tc_wide)
+                    k_update_tc<3, tc::BN_WIDE><<<(unsigned)blocks, tc::THREADS, tc::smem_bytes<tc::BN_WIDE>(), s_>>>(
+                        B, S.k, plan.W, uact, pfx, U.n_tc, plan.d_err, part);
+                else
+                    k_update_tc<3, tc::BN><<<(unsigned)blocks, tc::THREADS, tc::SMEM_BYTES, s_>>>(
+                        B, S.k, plan.W, uact, pfx, U.n_tc, plan.d_err, part);
+            };
+            if (plan.tc_events) {
+                cudaEvent_t e0, e1;
+                GB_CUDA(cudaEventCreate(&e0));
+                GB_CUDA(cudaEventCreate(&e1));
+                plan.tc_events->push_back(e0);
+                plan.tc_events->push_back(e1);
+                GB_CUDA(cudaEventRecord(e0, st));
+            }
+            if (!lookahead) {
+                tc_launch(U.tc_blocks, U.tc_pfx, 0, st);
+                GB_LAUNCH_CHECK();
+            } else {
+                // the next outer panel's columns first; the rest of the trailing
+                // matrix on the side stream while the next diagonal block is factored here
+                tc_launch(U.tcn_blocks, U.tcn_pfx, 1, st);
+                GB_LAUNCH_CHECK();
+                if (U.tcr_blocks > 0) {
+                    GB_CUDA(cudaEventRecord(plan.la_fork, st));
+                    GB_CUDA(cudaStreamWaitEvent(plan.la_stream, plan.la_fork, 0));
+                    tc_launch(U.tcr_blocks, U.tcr_pfx, 2, plan.la_stream);
+                    GB_LAUNCH_CHECK();
+                    GB_CUDA(cudaEventRecord(plan.la_join, plan.la_stream));
+                    pending = true;
+                }
+            }
+            if (plan.tc_events) GB_CUDA(cudaEventRecord(plan.tc_events->back(), st));
+        }
+    }
+    if (pending) GB_CUDA(cudaStreamWaitEvent(st, plan.la_join, 0));
+    return GBVLM_OK;
+}
+
+template <class T>
 int lu_batch_solve(const LuBatch<T>& B, int32_t nsys, int32_t max_nrhs, int64_t maxn, cudaStream_t st, int* err) {
     // X of the largest system in shared memory when it fits, else staged per column
     const size_t full = sizeof(T) * (size_t)maxn * TS_MAXRHS;
@@ -2424,6 +2831,8 @@ int lu_batch_solve(const LuBatch<T>& B, int32_t nsys, int32_t max_nrhs, int64_t 
 
 template int lu_batch_factor<float>(const LuBatch<float>&, const LuPlan&, cudaStream_t, bool);
 template int lu_batch_factor<double>(const LuBatch<double>&, const LuPlan&, cudaStream_t, bool);
+template int lu_batch_factor_fast<float>(const LuBatch<float>&, const LuPlan&, cudaStream_t, bool);
+template int lu_batch_factor_fast<double>(const LuBatch<double>&, const LuPlan&, cudaStream_t, bool);
 template int lu_batch_solve<float>(const LuBatch<float>&, int32_t, int32_t, int64_t, cudaStream_t, int*);
 template int lu_batch_solve<double>(const LuBatch<double>&, int32_t, int32_t, int64_t, cudaStream_t, int*);
 
@@ -2498,6 +2907,16 @@ int lu_plan_build(LuPlan& plan, const std::vector<int64_t>& n_sorted, cudaStream
             GB_CUDA(cudaFuncSetAttribute(k_update_tcp<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::P_SMEM_BYTES));
             GB_CUDA(cudaFuncSetAttribute(k_trs_tcp<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::P_SMEM_BYTES));
             GB_CUDA(cudaFuncSetAttribute(k_trs_tcp<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc::P_SMEM_BYTES));
+        }
+        {
+            // without interchanges: float on the tensor cores' three passes, double always
+            const char* f = getenv("GBVLM_LU_FAST");
+            plan.fast_any = !(f && f[0] == '0');
+            plan.fast = plan.fast_any && plan.tc_passes == 3 && !tc_persistent();
+            GB_CUDA(cudaFuncSetAttribute(k_lu_diag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)Fast<float>::diag_smem));
+            GB_CUDA(cudaFuncSetAttribute(k_lu_rows<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)Fast<float>::rows_smem));
         }
         GB_CUDA(dev_alloc((void**)&plan.d_err, sizeof(int), plan.mem));
         GB_CUDA(cudaMemsetAsync(plan.d_err, 0, sizeof(int), st));
@@ -2737,10 +3156,35 @@ int lu_plan_build(LuPlan& plan, const std::vector<int64_t>& n_sorted, cudaStream
         }
         pfx.push_back(acc);
         S.tcs_blocks = acc;
+        // without interchanges: rows and columns past the block of W columns, and the double update's tiles
+        for (int e = 0; e < 2; e++) {
+            const int64_t w = e == 0 ? Fast<float>::W : Fast<double>::W, rt = e == 0 ? Fast<float>::RT : Fast<double>::RT;
+            S.fr_pfx[e] = (int64_t)pfx.size();
+            acc = 0;
+            ci = 0;
+            if (k % w == 0)
+                while (ci < cnt && n_sorted[ci] > k + w) {
+                    pfx.push_back(acc);
+                    acc += 2 * cdiv(n_sorted[ci] - k - w, rt);
+                    ci++;
+                }
+            pfx.push_back(acc);
+            S.fr_blocks[e] = acc;
+            S.fr_cnt[e] = ci;
+        }
+        S.fu_pfx = (int64_t)pfx.size();
+        acc = 0;
+        for (int i = 0; i < S.fr_cnt[1]; i++) {
+            pfx.push_back(acc);
+            const int64_t t = cdiv(n_sorted[i] - k - GK, (int64_t)GT_F64);
+            acc += t * t;
+        }
+        pfx.push_back(acc);
+        S.fu_blocks = acc;
         plan.steps.push_back(S);
     }
-    if (plan.tc_trsm && plan.nsys > 0)
-        GB_CUDA(dev_alloc((void**)&plan.d_minv, sizeof(float) * LU_OUTER * LU_OUTER * (size_t)plan.nsys, plan.mem));
+    if ((plan.tc_trsm || plan.fast_any) && plan.nsys > 0)
+        GB_CUDA(dev_alloc((void**)&plan.d_minv, sizeof(float) * Fast<float>::WORK * (size_t)plan.nsys, plan.mem));
     if (!act.empty()) {
         GB_CUDA(dev_alloc((void**)&plan.d_act, act.size() * sizeof(int32_t), plan.mem));
         GB_CUDA(cudaMemcpyAsync(plan.d_act, act.data(), act.size() * sizeof(int32_t), cudaMemcpyHostToDevice, st));
@@ -2785,6 +3229,19 @@ int64_t lu_plan_launches(const LuPlan& plan, int es) {
         }
     }
     return n + (plan.nsys > 0);  // + the permutation kernel
+}
+
+int64_t lu_plan_launches_fast(const LuPlan& plan, int es) {
+    const int e = es == 4 ? 0 : 1;
+    const int64_t w = e == 0 ? Fast<float>::W : Fast<double>::W;
+    int64_t n = 0;
+    for (size_t s = 0; s < plan.steps.size(); s++) {
+        const LuStep& S = plan.steps[s];
+        if (S.n_panel == 0 || S.k % w != 0) continue;
+        n += 1 + 2 * (S.fr_blocks[e] > 0);
+        if (e == 0 && S.fr_blocks[0] > 0) n += plan.la_stream && plan.steps[s + w / GK - 1].tcr_blocks > 0;
+    }
+    return n;
 }
 
 int trs_flow_build(TrsFlow& f, const std::vector<int64_t>& n_sorted, cudaStream_t st, int32_t groups) {
@@ -3003,6 +3460,9 @@ struct gbvlm_lu_s {
     // made by the factorisation, so a solve allocates nothing
     void* one = nullptr;
     int64_t one_bytes = 0;
+    // the matrix before its factorisation without interchanges, should it need them
+    void* backup = nullptr;
+    size_t backup_bytes = 0;
 };
 constexpr size_t ONE_Y = 256;
 
@@ -3086,13 +3546,33 @@ static int lu_ensure(gbvlm_lu h, int64_t n, cudaStream_t st) {
     h->d_perm = nullptr;
     GB_CUDA(cudaMalloc(&h->d_ipiv, sizeof(int32_t) * (n > 0 ? n : 1)));
     GB_CUDA(cudaMalloc(&h->d_perm, sizeof(int32_t) * (n > 0 ? n : 1)));
-    GB_CUDA(cudaMalloc(&h->d_info, sizeof(int32_t)));
+    GB_CUDA(cudaMalloc(&h->d_info, 2 * sizeof(int32_t)));  // info, and that interchanges are needed
     std::vector<int64_t> ns(1, n);
     int rc = lu_plan_build(h->plan, ns, st);
     if (rc) return rc;
     h->plan_n = n;
     h->n = n;
     return GBVLM_OK;
+}
+
+// a copy of the matrix; false if there is no memory for one
+template <class T>
+static bool lu_backup(gbvlm_lu h, const T* A, int64_t n, int64_t ld, cudaStream_t st) {
+    const size_t need = sizeof(T) * (size_t)n * (size_t)n;
+    if (h->backup_bytes < need) {
+        if (h->backup) cudaFree(h->backup);
+        h->backup = nullptr;
+        h->backup_bytes = 0;
+        if (cudaMalloc(&h->backup, need) != cudaSuccess) {
+            cudaGetLastError();
+            return false;
+        }
+        h->backup_bytes = need;
+    }
+    const cudaError_t e =
+        cudaMemcpy2DAsync(h->backup, sizeof(T) * n, A, sizeof(T) * ld, sizeof(T) * n, n, cudaMemcpyDeviceToDevice, st);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess;
 }
 
 template <class T>
@@ -3105,11 +3585,29 @@ static int lu_factor_one(gbvlm_lu h, T* A, int64_t n, int64_t ld, cudaStream_t s
     LuBatch<T> B;
     rc = make_single_batch<T>(B, n, ld, A, h->d_ipiv, h->d_perm, h->d_info, nullptr, 0, 0, &h->work, &h->work_bytes, st);
     if (rc) return rc;
-    rc = lu_batch_factor<T>(B, h->plan, st, true);
-    if (rc) return rc;
-    int32_t* hi = (int32_t*)host_scratch(sizeof(int32_t));
-    GB_CUDA(cudaMemcpyAsync(hi, h->d_info, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaStreamSynchronize(st));
+    int32_t* hi = (int32_t*)host_scratch(2 * sizeof(int32_t));
+    bool done = false;
+    // without interchanges first; single-block systems' panel tries that itself
+    const bool fast = (sizeof(T) == 4 ? h->plan.fast : h->plan.fast_any) && n > GK && lu_backup<T>(h, A, n, ld, st);
+    if (fast) {
+        GB_CUDA(cudaMemsetAsync(h->d_info + 1, 0, sizeof(int32_t), st));
+        B.fail = h->d_info + 1;
+        rc = lu_batch_factor_fast<T>(B, h->plan, st, true);
+        B.fail = nullptr;
+        if (rc) return rc;
+        GB_CUDA(cudaMemcpyAsync(hi, h->d_info, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaStreamSynchronize(st));
+        done = hi[1] == 0;
+        if (!done)
+            GB_CUDA(cudaMemcpy2DAsync(A, sizeof(T) * ld, h->backup, sizeof(T) * n, sizeof(T) * n, n,
+                                      cudaMemcpyDeviceToDevice, st));
+    }
+    if (!done) {
+        rc = lu_batch_factor<T>(B, h->plan, st, true);
+        if (rc) return rc;
+        GB_CUDA(cudaMemcpyAsync(hi, h->d_info, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaStreamSynchronize(st));
+    }
     if (*hi != 0) {
         set_error("LU: exactly zero pivot at column %d", *hi);
         return GBVLM_ERR_SINGULAR;
@@ -3286,6 +3784,7 @@ int gbvlm_lu_destroy(gbvlm_lu h) {
     if (h->d_perm) cudaFree(h->d_perm);
     if (h->work) cudaFree(h->work);
     if (h->one) cudaFree(h->one);
+    if (h->backup) cudaFree(h->backup);
     h->plan.release();
     delete h;
     return GBVLM_OK;

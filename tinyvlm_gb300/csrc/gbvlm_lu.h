@@ -27,6 +27,10 @@ struct LuBatch {
     // ends at position k + t, [32 + r] = final offset of the row that started
     // at k + r (null: not recorded)
     int32_t* mv = nullptr;
+    // factorisation without interchanges: set to 1 for a system that needs
+    // them, which the later launches then pass over (zeroed by the caller; null
+    // for the pivoting launches)
+    int32_t* fail = nullptr;
 };
 
 // One panel launch: active systems [first, first + count) of a step, each
@@ -67,6 +71,11 @@ struct LuStep {
     int64_t tcr_pfx = 0, tcr_blocks = 0;      // its other columns of tiles (lookahead)
     int64_t tcs_pfx = 0, tcs_blocks = 0;      // U12 on the tensor cores: tiles of 128 rows x the update's tile width
     int64_t inc_pfx = 0, inc_blocks = 0;      // the inner update on the tensor cores: 128-row tiles
+    // factorisation without interchanges (float at the first step of an outer
+    // block, double at every step): rows and columns past the block
+    int64_t fr_pfx[2] = {0, 0}, fr_blocks[2] = {0, 0};  // k_lu_rows, float and double
+    int32_t fr_cnt[2] = {0, 0};                         // systems past the block (a prefix)
+    int64_t fu_pfx = 0, fu_blocks = 0;                  // double: the trailing update in 32 x 32 tiles
 };
 
 struct LuPlan {
@@ -84,7 +93,11 @@ struct LuPlan {
     bool tc_inner = false;  // inner updates in 128-row tensor-core tiles, K = 32 (GBVLM_TC_INNER=0: CUDA cores)
     bool tc_trsm = false;
     int32_t tc_trsm_min = 1;  // ... for steps with at least this many systems
-    float* d_minv = nullptr;  // nsys x 128 x 128: I - L11^-1 of each system's current outer block
+    // per system 128 x 128 + 128 floats: I - L11^-1 of the current outer block, or the
+    // factored diagonal block and its reciprocal pivots (without interchanges)
+    float* d_minv = nullptr;
+    // systems may be factored without interchanges (GBVLM_LU_FAST=0: not): in double, and in float
+    bool fast_any = false, fast = false;
     int W = LU_NB;      // outer block width of the float factorisation
     int32_t* d_act = nullptr;
     int32_t* d_pack = nullptr;  // PanelGroup pack entries
@@ -119,6 +132,11 @@ int64_t lu_plan_launches(const LuPlan& plan, int es);
 // inner steps (float, tensor-core plans; ignored while timing launches)
 template <class T>
 int lu_batch_factor(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t st, bool lookahead);
+// the same without interchanges; B.fail marks the systems that need them
+template <class T>
+int lu_batch_factor_fast(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t st, bool lookahead);
+// number of kernel launches that makes for element size es (4 or 8)
+int64_t lu_plan_launches_fast(const LuPlan& plan, int es);
 // err: the tensor-core error word of a plan with tensor cores (a single large
 // float system then solves in 128-row blocks on the tensor cores), or null
 template <class T>
