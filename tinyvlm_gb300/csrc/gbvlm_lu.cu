@@ -337,52 +337,115 @@ __device__ __forceinline__ void panel_barrier(int nwa, int bar) {
     }
 }
 
+// Reciprocal of a pivot that pivot_fits: the hardware's approximation and
+// Newton's step (float) or Householder's third-order one (double), to within
+// an ulp; unlike the correctly rounded one it has no branch for subnormals, so
+// the steps around it overlap with it.
+__device__ __forceinline__ float pivot_rcp(float d) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(d));
+    return fmaf(y, fmaf(-d, y, 1.f), y);
+}
+__device__ __forceinline__ double pivot_rcp(double d) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    const double e = fma(-d, y, 1.0);
+    return fma(y, fma(e, e, e), y);
+}
+// normal, and so is its reciprocal (not for NaN)
+__device__ __forceinline__ bool pivot_fits(float d) { return fabsf(d) >= FLT_MIN && fabsf(d) <= 1e37f; }
+__device__ __forceinline__ bool pivot_fits(double d) {
+    const uint32_t e = (uint32_t)__double2hiint(d) & 0x7fffffffu;
+    return e >= 0x00100000u && e < 0x7fd00000u;
+}
+// |x| <= |d| (false for a NaN x or d); in double by the bits, off the fp64 pipe
+__device__ __forceinline__ bool not_above(float x, float d) { return fabsf(x) <= fabsf(d); }
+__device__ __forceinline__ bool not_above(double x, double d) {
+    const unsigned long long m = 0x7fffffffffffffffull, inf = 0x7ff0000000000000ull;
+    const unsigned long long a = (unsigned long long)__double_as_longlong(x) & m;
+    const unsigned long long b = (unsigned long long)__double_as_longlong(d) & m;
+    return a <= b && b <= inf;
+}
+
 // The diagonal block without interchanges, one warp, lane r holding row r:
-// the rows of U and the pivots' reciprocals go to shared memory.  Returns
+// the factored rows and the pivots' reciprocals go to shared memory.  Returns
 // false (in every lane) where partial pivoting would have left the diagonal,
-// or where a pivot is zero, subnormal or not a number.  Each row sees the
-// operations of the pivoting loop in their order.
+// or where a pivot does not fit.  Each row sees the operations of the pivoting
+// loop in their order.
+// A column is one dependent step: pivot, reciprocal, multiplier, the next
+// column's entry.  The pivot row goes round by shuffles, and rows at or above
+// the pivot take a zero multiplier: no branch, so a step's other columns run
+// beside the next one's chain.
 template <class T, int LDU>
 __device__ __forceinline__ bool panel_diag(T (&x)[GK], int nb, T* u, T* rds, int lane) {
     using V2 = typename Vec4<T>::type;
     bool good = true;
+    T myrd = (T)0;
     static_for<0, GK>([&](auto JJ) {
         constexpr int jj = decltype(JJ)::value;
         if (jj < nb) {
             const T d = __shfl_sync(0xffffffffu, x[jj], jj);
-            if (lane == jj) {  // row jj of U is final
+            const T rd = pivot_rcp(d);
+            const bool under = lane > jj;  // rows past nb hold zeros
+            good = good && pivot_fits(d) && (!under || not_above(x[jj], d));
+            const T lm = under ? x[jj] * rd : (T)0;
+            x[jj] = under ? lm : x[jj];
+            myrd = lane == jj ? rd : myrd;
 #pragma unroll
-                for (int t = jj & ~3; t < GK; t += 4) {
-                    V2 v;
-                    v.x = x[t];
-                    v.y = x[t + 1];
-                    v.z = x[t + 2];
-                    v.w = x[t + 3];
-                    *reinterpret_cast<V2*>(u + jj * LDU + t) = v;
-                }
-            }
-            const T rd = rcp_rn(d);
-            if (lane == jj) rds[jj] = rd;
-            __syncwarp();
-            const bool below = lane > jj && lane < nb;
-            good = good && tabs(d) >= (sizeof(T) == 4 ? (T)FLT_MIN : (T)DBL_MIN) &&
-                   (!below || tabs(x[jj]) <= tabs(d));
-            if (below) {
-                const T lm = x[jj] * rd;
+            for (int t = jj + 1; t < GK; t++) x[t] -= lm * __shfl_sync(0xffffffffu, x[t], jj);
+        }
+    });
+    if (lane < nb) rds[lane] = myrd;
+#pragma unroll
+    for (int t = 0; t < GK; t += 4) {  // row `lane`: its entries left of the diagonal are L's
+        V2 v;
+        v.x = x[t];
+        v.y = x[t + 1];
+        v.z = x[t + 2];
+        v.w = x[t + 3];
+        *reinterpret_cast<V2*>(u + lane * LDU + t) = v;
+    }
+    return __all_sync(0xffffffffu, good);
+}
+
+// four consecutive shared-memory values
+__device__ __forceinline__ void load4(const float* p, float (&v)[4]) {
+    const float4 q = *reinterpret_cast<const float4*>(p);
+    v[0] = q.x, v[1] = q.y, v[2] = q.z, v[3] = q.w;
+}
+__device__ __forceinline__ void load4(const double* p, double (&v)[4]) {
+    const double2 a = reinterpret_cast<const double2*>(p)[0], b = reinterpret_cast<const double2*>(p)[1];
+    v[0] = a.x, v[1] = a.y, v[2] = b.x, v[3] = b.y;
+}
+
+// x against 32 rows of a triangle, u its first row and `stride` values per row:
+// ROWS (x a row below, u the rows of U): l_j = x_j / u_jj, x_t -= l_j u_jt, and
+// whether |x_j| <= |u_jj| throughout; else (x a column to the right, u the
+// columns of the unit lower triangle): x_t -= x_j l_tj
+template <class T, bool ROWS>
+__device__ __forceinline__ bool eliminate32(T (&x)[GK], const T* u, int stride, const T* rd, int nb = GK) {
+    bool good = true;
+    static_for<0, GK>([&](auto JJ) {
+        constexpr int jj = decltype(JJ)::value;
+        if (jj < nb) {
+            const T* ua = u + jj * stride;
+            T lm = x[jj];
+            if constexpr (ROWS) {
+                good = good && not_above(lm, ua[jj]);
+                lm = lm * rd[jj];
                 x[jj] = lm;
-                const uint32_t ua = (uint32_t)__cvta_generic_to_shared(u + jj * LDU);
+            }
 #pragma unroll
-                for (int tg = (jj + 1) & ~3; tg < GK; tg += 4) {
-                    T v[4];
-                    lds4(ua + tg * (uint32_t)sizeof(T), v);
+            for (int tg = (jj + 1) & ~3; tg < GK; tg += 4) {
+                T v[4];
+                load4(ua + tg, v);
 #pragma unroll
-                    for (int e = 0; e < 4; e++)
-                        if (tg + e > jj) x[tg + e] -= lm * v[e];
-                }
+                for (int e = 0; e < 4; e++)
+                    if (tg + e > jj) x[tg + e] -= lm * v[e];
             }
         }
     });
-    return __all_sync(0xffffffffu, good);
+    return good;
 }
 
 template <class T, int NT, bool CLUSTER, int RPT>
@@ -475,24 +538,7 @@ __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const
             }
             panel_barrier<NT, CLUSTER>(nwa, bar);
             if (good && sm.f_bad[slice] == 0 && !(first && rank == 0)) {
-                static_for<0, GK>([&](auto JJ) {
-                    constexpr int jj = decltype(JJ)::value;
-                    if (jj < nb) {
-                        const uint32_t ua = (uint32_t)__cvta_generic_to_shared(&fu[jj][0]);
-                        const T d = lds1(ua + jj * (uint32_t)sizeof(T), T(0));
-                        good = good && tabs(x[0][jj]) <= tabs(d);
-                        const T lm = x[0][jj] * frd[jj];
-                        x[0][jj] = lm;
-#pragma unroll
-                        for (int tg = (jj + 1) & ~3; tg < GK; tg += 4) {
-                            T v[4];
-                            lds4(ua + tg * (uint32_t)sizeof(T), v);
-#pragma unroll
-                            for (int e = 0; e < 4; e++)
-                                if (tg + e > jj) x[0][tg + e] -= lm * v[e];
-                        }
-                    }
-                });
+                good = eliminate32<T, true>(x[0], &fu[0][0], GK, frd, nb);
                 if (lid[0] < 0) good = true;  // no row
             }
             // the verdict of the slice, or of every CTA of the cluster
@@ -664,93 +710,57 @@ __device__ __forceinline__ void cp_async_zfill(uint32_t dst, const T* src, bool 
 template <class T> struct Fast {
     static constexpr int W = sizeof(T) == 4 ? LU_OUTER : GK;
     static constexpr int NB = W / GK;
-    static constexpr int LD = W + 16 / (int)sizeof(T);            // diagonal block's row stride: 16-byte aligned rows
-    static constexpr int DT = sizeof(T) == 4 ? 256 : 32;          // threads of k_lu_diag
-    static constexpr int RT = sizeof(T) == 4 ? 128 : 32;          // rows or columns per CTA of k_lu_rows: in double
-                                                                  // few, to reach the fp64 units of many SMs
+    static constexpr int LD = W + 16 / (int)sizeof(T);         // diagonal block's row stride: 16-byte aligned rows
+    static constexpr int DT = sizeof(T) == 4 ? 256 : 128;      // threads of the diagonal block's kernel
+    static constexpr int RT = sizeof(T) == 4 ? 128 : GK;       // rows or columns per CTA
     static constexpr int LDX = RT + 1;
-    static constexpr int MSIZE = NB * (NB + 1) / 2 * GK * GK;     // the blocks on and above the diagonal
-    static constexpr int WORK = W * W + W;                        // per system: the factored block by rows, reciprocal pivots
+    static constexpr int MSIZE = NB * (NB + 1) / 2 * GK * GK;  // the blocks on and above the diagonal
+    static constexpr int WORK = 2 * W * W + W;                 // per system: the factored block by rows, by columns,
+                                                               // and the reciprocal pivots
     static constexpr size_t diag_smem = sizeof(T) * (size_t)(W * LD + GK * GK + W);
     static constexpr size_t rows_smem = sizeof(T) * (size_t)(MSIZE + W + W * LDX);
 };
 
-// x against 32 rows of a triangle, u its address and `stride` bytes per row:
-// ROWS (x a row of A21, u the rows of U): l_j = x_j / u_jj, x_t -= l_j u_jt, and
-// whether |x_j| <= |u_jj| throughout; else (x a column of A12, u the columns of
-// the unit lower triangle): x_t -= x_j l_tj
-template <class T, bool ROWS>
-__device__ __forceinline__ bool eliminate32(T (&x)[GK], uint32_t u, uint32_t stride, const T* rd) {
-    bool good = true;
-    static_for<0, GK>([&](auto JJ) {
-        constexpr int jj = decltype(JJ)::value;
-        const uint32_t ua = u + jj * stride;
-        T lm = x[jj];
-        if constexpr (ROWS) {
-            good = good && tabs(lm) <= tabs(lds1(ua + jj * (uint32_t)sizeof(T), T(0)));
-            lm = lm * rd[jj];
-            x[jj] = lm;
-        }
+// 32-column step c of the diagonal block: RH rows from r0, 32 columns from c0
+// (a lane each) less their product with the step's rows and columns
+template <int RH, int LD>
+__device__ __forceinline__ void diag_update(float* S, int c, int r0, int c0, int lane) {
+    float acc[RH];
 #pragma unroll
-        for (int tg = (jj + 1) & ~3; tg < GK; tg += 4) {
-            T v[4];
-            lds4(ua + tg * (uint32_t)sizeof(T), v);
-#pragma unroll
-            for (int e = 0; e < 4; e++)
-                if (tg + e > jj) x[tg + e] -= lm * v[e];
-        }
-    });
-    return good;
-}
-
-// the block's trailing part after its 32-column step c: rows and columns past
-// it, NC x 32 of each; warp w holds 4 NC rows, a lane NC columns
-template <int NC, int LD>
-__device__ __forceinline__ void diag_update(float* S, int c, int wid, int lane) {
-    const int lo = GK * (c + 1), r0 = lo + 4 * NC * wid;
-    float acc[4 * NC][NC];
-#pragma unroll
-    for (int i = 0; i < 4 * NC; i++)
-#pragma unroll
-        for (int j = 0; j < NC; j++) acc[i][j] = 0.f;
-#pragma unroll 1
+    for (int i = 0; i < RH; i++) acc[i] = 0.f;
+#pragma unroll 2
     for (int k = 0; k < GK; k += 4) {
-        float b[4][NC];
+        float b[4];
 #pragma unroll
-        for (int e = 0; e < 4; e++)
+        for (int e = 0; e < 4; e++) b[e] = S[(GK * c + k + e) * LD + c0 + lane];
 #pragma unroll
-            for (int j = 0; j < NC; j++) b[e][j] = S[(GK * c + k + e) * LD + lo + 32 * j + lane];
+        for (int i = 0; i < RH; i++) {
+            float a[4];
+            load4(S + (r0 + i) * LD + GK * c + k, a);
 #pragma unroll
-        for (int i = 0; i < 4 * NC; i++) {
-            const float4 a = *reinterpret_cast<const float4*>(S + (r0 + i) * LD + GK * c + k);
-#pragma unroll
-            for (int j = 0; j < NC; j++) {
-                acc[i][j] += a.x * b[0][j];
-                acc[i][j] += a.y * b[1][j];
-                acc[i][j] += a.z * b[2][j];
-                acc[i][j] += a.w * b[3][j];
-            }
+            for (int e = 0; e < 4; e++) acc[i] += a[e] * b[e];
         }
     }
 #pragma unroll
-    for (int i = 0; i < 4 * NC; i++)
-#pragma unroll
-        for (int j = 0; j < NC; j++) S[(r0 + i) * LD + lo + 32 * j + lane] -= acc[i][j];
+    for (int i = 0; i < RH; i++) S[(r0 + i) * LD + c0 + lane] -= acc[i];
 }
 
-template <class T>
-__global__ void __launch_bounds__(Fast<T>::DT) k_lu_diag(LuBatch<T> B, int64_t k0, const int32_t* act, T* work,
-                                                         int32_t base) {
-    using F = Fast<T>;
-    constexpr int W = F::W, LD = F::LD, DT = F::DT;
+// Float: the 128 x 128 block, eight warps.  Per 32-column step: the triangle
+// (warp 0), the rows below and the columns to the right (a thread each), the
+// next triangle's update (all warps), then the rest of the update beside
+// warp 0's factorisation of that triangle.
+__global__ void __launch_bounds__(Fast<float>::DT) k_lu_diag(LuBatch<float> B, int64_t k0, const int32_t* act,
+                                                             float* work, int32_t base) {
+    using F = Fast<float>;
+    constexpr int W = F::W, LD = F::LD, DT = F::DT, NB = F::NB;
     extern __shared__ __align__(16) unsigned char fast_smem[];
-    T* S = reinterpret_cast<T*>(fast_smem);  // the block by rows
-    T* LT = S + W * LD;                      // the current 32 x 32 triangle's L by columns
-    T* rds = LT + GK * GK;                   // reciprocal pivots
+    float* S = reinterpret_cast<float*>(fast_smem);  // the block by rows
+    float* LT = S + W * LD;                          // the current 32 x 32 triangle's L by columns
+    float* rds = LT + GK * GK;                       // reciprocal pivots
     __shared__ int s_bad;
     const int32_t sid = act[blockIdx.x];
     const int64_t n = B.n[sid], ld = B.ld[sid];
-    T* A = B.A[sid] + k0 + k0 * ld;
+    float* A = B.A[sid] + k0 + k0 * ld;
     const int w = (int)min((int64_t)W, n - k0);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     // the identity permutation, for a system that fails too: a batch's solves
@@ -761,159 +771,197 @@ __global__ void __launch_bounds__(Fast<T>::DT) k_lu_diag(LuBatch<T> B, int64_t k
     }
     if (B.fail[sid]) return;
     if (tid == 0) s_bad = 0;
-    for (int e = tid; e < W * W; e += DT) {
-        const int r = e & (W - 1), c = e / W;
-        const bool in = r < w && c < w;
-        cp_async_zfill<T>((uint32_t)__cvta_generic_to_shared(S + r * LD + c), in ? A + r + c * ld : A, in);
+    // a thread takes a row's entries in four columns (coalesced down the
+    // columns) and stores them as one vector; past the system's end an
+    // identity, which changes nothing
+    const int r = tid & (W - 1), g0 = tid / W;
+#pragma unroll 1
+    for (int h = 0; h < 2; h++) {
+        float v[8][4];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+#pragma unroll
+            for (int e = 0; e < 4; e++) {
+                const int c = 4 * (g0 + 2 * (8 * h + i)) + e;
+                v[i][e] = r < w && c < w ? A[r + c * ld] : (r == c ? 1.f : 0.f);
+            }
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+            *reinterpret_cast<float4*>(S + r * LD + 4 * (g0 + 2 * (8 * h + i))) =
+                make_float4(v[i][0], v[i][1], v[i][2], v[i][3]);
     }
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
-    if (w < W) {  // past the system's end: an identity, which changes nothing
-        for (int r = w + tid; r < W; r += DT) S[r * LD + r] = (T)1;
+    auto triangle = [&](int c) {  // warp 0
+        float* D = S + GK * c * LD + GK * c;
+        float x[GK];
+#pragma unroll
+        for (int t = 0; t < GK; t += 4) {
+            float v[4];
+            load4(D + lane * LD + t, v);
+#pragma unroll
+            for (int e = 0; e < 4; e++) x[t + e] = v[e];
+        }
+        __syncwarp();
+        const bool good = panel_diag<float, LD>(x, GK, D, rds + GK * c, lane);
+        if (!good && lane == 0) s_bad = 1;
+#pragma unroll
+        for (int t = 0; t < GK; t++) LT[t * GK + lane] = x[t];
+    };
+    if (wid == 0) triangle(0);
+    __syncthreads();
+#pragma unroll 1
+    for (int c = 0; c + 1 < NB; c++) {
+        const float* D = S + GK * c * LD + GK * c;
+        const int i = GK * (c + 1) + (tid & (DT / 2 - 1));
+        if (i < W) {
+            float x[GK];
+            if (tid < DT / 2) {  // a row below
+                float* row = S + i * LD + GK * c;
+#pragma unroll
+                for (int t = 0; t < GK; t += 4) {
+                    float v[4];
+                    load4(row + t, v);
+#pragma unroll
+                    for (int e = 0; e < 4; e++) x[t + e] = v[e];
+                }
+                if (!eliminate32<float, true>(x, D, LD, rds + GK * c)) s_bad = 1;
+#pragma unroll
+                for (int t = 0; t < GK; t += 4)
+                    *reinterpret_cast<float4*>(row + t) = make_float4(x[t], x[t + 1], x[t + 2], x[t + 3]);
+            } else {  // a column to the right
+#pragma unroll
+                for (int t = 0; t < GK; t++) x[t] = S[(GK * c + t) * LD + i];
+                eliminate32<float, false>(x, LT, GK, nullptr);
+#pragma unroll
+                for (int t = 0; t < GK; t++) S[(GK * c + t) * LD + i] = x[t];
+            }
+        }
+        __syncthreads();
+        const int lo = GK * (c + 1);
+        diag_update<4, LD>(S, c, lo + 4 * wid, lo, lane);
+        __syncthreads();
+        if (wid == 0) {
+            triangle(c + 1);
+        } else {
+            // half blocks of 16 rows x 32 columns, but for the triangle's two
+            const int nbk = NB - 1 - c;
+            for (int q = 2 + wid - 1; q < 2 * nbk * nbk; q += DT / 32 - 1) {
+                const int blk = q >> 1;
+                diag_update<16, LD>(S, c, lo + GK * (blk / nbk) + 16 * (q & 1), lo + GK * (blk % nbk), lane);
+            }
+        }
         __syncthreads();
     }
-#pragma unroll 1
-    for (int c = 0; c < F::NB; c++) {
-        T* D = S + GK * c * LD + GK * c;
-        if (wid == 0) {
-            T x[GK];
-#pragma unroll
-            for (int t = 0; t < GK; t++) x[t] = D[lane * LD + t];
-            __syncwarp();
-            const bool good = panel_diag<T, LD>(x, GK, D, rds + GK * c, lane);
-            if (!good && lane == 0) s_bad = 1;
-#pragma unroll
-            for (int t = 0; t < GK; t++) {
-                if (t < lane) D[lane * LD + t] = x[t];
-                LT[t * GK + lane] = x[t];
-            }
-        }
-        if constexpr (F::NB > 1) {
-            __syncthreads();
-            const int lo = GK * (c + 1);
-            const int i = lo + (tid & (DT / 2 - 1));
-            T x[GK];
-            if (i < W) {
-                if (tid < DT / 2) {  // a row below
-                    T* row = S + i * LD + GK * c;
-#pragma unroll
-                    for (int t = 0; t < GK; t += 4) {
-                        T v[4];
-                        lds4((uint32_t)__cvta_generic_to_shared(row + t), v);
-#pragma unroll
-                        for (int e = 0; e < 4; e++) x[t + e] = v[e];
-                    }
-                    const bool good = eliminate32<T, true>(x, (uint32_t)__cvta_generic_to_shared(D),
-                                                           LD * (uint32_t)sizeof(T), rds + GK * c);
-                    if (!good) s_bad = 1;
-                    using V2 = typename Vec4<T>::type;
-#pragma unroll
-                    for (int t = 0; t < GK; t += 4) {
-                        V2 v;
-                        v.x = x[t];
-                        v.y = x[t + 1];
-                        v.z = x[t + 2];
-                        v.w = x[t + 3];
-                        *reinterpret_cast<V2*>(row + t) = v;
-                    }
-                } else {  // a column to the right
-#pragma unroll
-                    for (int t = 0; t < GK; t++) x[t] = S[(GK * c + t) * LD + i];
-                    eliminate32<T, false>(x, (uint32_t)__cvta_generic_to_shared(LT), GK * (uint32_t)sizeof(T), nullptr);
-#pragma unroll
-                    for (int t = 0; t < GK; t++) S[(GK * c + t) * LD + i] = x[t];
-                }
-            }
-            __syncthreads();
-            if (c == 0) diag_update<3, LD>(S, 0, wid, lane);
-            if (c == 1) diag_update<2, LD>(S, 1, wid, lane);
-            if (c == 2) diag_update<1, LD>(S, 2, wid, lane);
-            __syncthreads();
-        }
-    }
-    __syncthreads();
     if (s_bad) {
         if (tid == 0) B.fail[sid] = 1;
         return;
     }
-    for (int e = tid; e < W * W; e += DT) {
-        const int r = e & (W - 1), c = e / W;
-        if (r < w && c < w) A[r + c * ld] = S[r * LD + c];
+    float* wk = work + (int64_t)(sid - base) * F::WORK;
+    float* wc = wk + W * W;
+#pragma unroll 4
+    for (int q = 0; q < 16; q++) {
+        const int c = 4 * (g0 + 2 * q);
+        float v[4];
+        load4(S + r * LD + c, v);
+#pragma unroll
+        for (int e = 0; e < 4; e++) {
+            if (r < w && c + e < w) A[r + (c + e) * ld] = v[e];
+            wc[(c + e) * W + r] = v[e];
+        }
     }
-    T* wk = work + (int64_t)(sid - base) * F::WORK;
-    for (int e = tid; e < W * W; e += DT) wk[e] = S[(e / W) * LD + (e & (W - 1))];
-    for (int e = tid; e < W; e += DT) wk[W * W + e] = rds[e];
+    for (int e = tid; e < W * W / 4; e += DT)
+        reinterpret_cast<float4*>(wk)[e] = *reinterpret_cast<const float4*>(S + (e / (W / 4)) * LD + 4 * (e % (W / 4)));
+    for (int e = tid; e < W; e += DT) wc[W * W + e] = rds[e];
 }
 
-template <class T>
-__global__ void __launch_bounds__(Fast<T>::RT) k_lu_rows(LuBatch<T> B, int64_t k0, const int32_t* act,
-                                                         const int64_t* pfx, int cnt, const T* work, int32_t base) {
-    using F = Fast<T>;
-    constexpr int W = F::W, NB = F::NB, RT = F::RT, LDX = F::LDX;
-    extern __shared__ __align__(16) unsigned char fast_smem[];
-    T* M = reinterpret_cast<T*>(fast_smem);  // block row p: 32 rows of (NB - p) x 32
-    T* rds = M + F::MSIZE;
-    T* Xs = rds + W;                         // solved values, [W][LDX]: a thread's own column
+// What the two row kernels share: the CTA's system and rows (or columns), and
+// the blocks on and above the diagonal of U by rows, or of L by columns, in
+// shared memory (the p-th block row has (NB - p) x 32 values per row).
+struct RowsJob {
+    int32_t sid;
+    int64_t n, ld, i0;
+    float* A;
+    bool rows;
+};
+
+__device__ __forceinline__ int fast_moff(int p) { return GK * GK * (p * Fast<float>::NB - p * (p - 1) / 2); }
+
+template <int RT>
+__device__ __forceinline__ bool rows_job(RowsJob& J, const LuBatch<float>& B, int64_t k0, const int32_t* act,
+                                         const int64_t* pfx, int cnt, const float* work, int32_t base, float* M) {
+    using F = Fast<float>;
     const int a = find_block(pfx, cnt, blockIdx.x);
-    const int32_t sid = act[a];
+    J.sid = act[a];
     // another CTA of the system may set it meanwhile: one thread's reading for all
-    if (__syncthreads_or(threadIdx.x == 0 && *(volatile int32_t*)&B.fail[sid])) return;
-    const int64_t n = B.n[sid], ld = B.ld[sid];
-    T* A = B.A[sid];
-    const int64_t kend = k0 + W;  // systems here have n > kend
-    const int64_t nr = (n - kend + RT - 1) / RT, idx = blockIdx.x - pfx[a];
-    const bool rows = idx < nr;
-    const int64_t i0 = kend + (rows ? idx : idx - nr) * RT;
-    const int tid = threadIdx.x, lane = tid & 31, w0 = tid & ~31;
-    const bool have = i0 + tid < n;
-    const T* wk = work + (int64_t)(sid - base) * F::WORK;
-    auto moff = [](int p) { return GK * GK * (p * NB - p * (p - 1) / 2); };
+    if (__syncthreads_or(threadIdx.x == 0 && *(volatile int32_t*)&B.fail[J.sid])) return false;
+    J.n = B.n[J.sid];
+    J.ld = B.ld[J.sid];
+    J.A = B.A[J.sid];
+    const int64_t kend = k0 + F::W;  // systems here have n > kend
+    const int64_t nr = (J.n - kend + RT - 1) / RT, idx = blockIdx.x - pfx[a];
+    J.rows = idx < nr;
+    J.i0 = kend + (J.rows ? idx : idx - nr) * RT;
+    const float* wk = work + (int64_t)(J.sid - base) * F::WORK;
+    const float* src = J.rows ? wk : wk + F::W * F::W;
 #pragma unroll
-    for (int p = 0; p < NB; p++)
-#pragma unroll
-        for (int c = p; c < NB; c++) {  // one 32 x 32 block, a warp per row
-            const T* src = rows ? wk + (GK * p) * W + GK * c : A + (k0 + GK * c) + (k0 + GK * p) * ld;
-            const int64_t sld = rows ? (int64_t)W : ld;
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(M + moff(p) + GK * (c - p) + lane);
-#pragma unroll
-            for (int j = tid >> 5; j < GK; j += RT / 32)
-                cp_async_zfill<T>(dst + (uint32_t)(j * (NB - p) * GK) * (uint32_t)sizeof(T), src + j * sld + lane, true);
+    for (int p = 0; p < F::NB; p++) {
+        const int q = (F::NB - p) * (GK / 4);  // 16-byte pieces per row
+        const uint32_t dst = (uint32_t)__cvta_generic_to_shared(M + fast_moff(p));
+        for (int e = threadIdx.x; e < GK * q; e += F::RT) {
+            const int j = e / q, t = e - j * q;
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(dst + 16u * (uint32_t)e),
+                         "l"(src + (GK * p + j) * F::W + GK * p + 4 * t)
+                         : "memory");
         }
-    if (rows) {
-        for (int e = tid; e < W; e += RT)
-            cp_async_zfill<T>((uint32_t)__cvta_generic_to_shared(rds + e), wk + W * W + e, true);
-    } else {
-        // columns are read by warps, 32 rows at a time, and turned in shared memory
+    }
+    const uint32_t rd = (uint32_t)__cvta_generic_to_shared(M + F::MSIZE);
+    for (int e = threadIdx.x; e < F::W; e += F::RT)
+        cp_async_zfill<float>(rd + 4u * (uint32_t)e, wk + 2 * F::W * F::W + e, true);
+    return true;
+}
+
+// L21 = A21 U11^-1 and U12 = L11^-1 A12: 128 rows, or columns, per CTA
+__global__ void __launch_bounds__(Fast<float>::RT) k_lu_rows(LuBatch<float> B, int64_t k0, const int32_t* act,
+                                                             const int64_t* pfx, int cnt, const float* work,
+                                                             int32_t base) {
+    using F = Fast<float>;
+    constexpr int NB = F::NB, RT = F::RT, LDX = F::LDX;
+    extern __shared__ __align__(16) unsigned char fast_smem[];
+    float* M = reinterpret_cast<float*>(fast_smem);
+    const float* rds = M + F::MSIZE;
+    float* Xs = M + F::MSIZE + F::W;  // solved values, [W][LDX]: a thread's own column
+    RowsJob J;
+    if (!rows_job<RT>(J, B, k0, act, pfx, cnt, work, base, M)) return;
+    const int tid = threadIdx.x, lane = tid & 31, w0 = tid & ~31;
+    const bool have = J.i0 + tid < J.n, rows = J.rows;
+    if (!rows)  // columns are read by warps, 32 rows at a time, and turned in shared memory
         for (int q = 0; q < 32; q++) {
-            const bool ok = i0 + w0 + q < n;
-            const T* col = ok ? A + k0 + lane + (i0 + w0 + q) * ld : A;
+            const bool ok = J.i0 + w0 + q < J.n;
+            const float* col = ok ? J.A + k0 + lane + (J.i0 + w0 + q) * J.ld : J.A;
             const uint32_t dst = (uint32_t)__cvta_generic_to_shared(Xs + lane * LDX + w0 + q);
 #pragma unroll
             for (int c = 0; c < NB; c++)
-                cp_async_zfill<T>(dst + (uint32_t)(GK * c * LDX) * (uint32_t)sizeof(T), col + (ok ? GK * c : 0), ok);
+                cp_async_zfill<float>(dst + (uint32_t)(GK * c * LDX * 4), col + (ok ? GK * c : 0), ok);
         }
-    }
     asm volatile("cp.async.commit_group;" ::: "memory");
     // a row's entries are read a 32-column step ahead of their use
-    T nx[GK];
-    const T* rsrc = A + i0 + tid + k0 * ld;
+    float nx[GK];
+    const float* rsrc = J.A + J.i0 + tid + k0 * J.ld;
 #pragma unroll
-    for (int t = 0; t < GK; t++) nx[t] = rows && have ? rsrc[t * ld] : (T)0;
+    for (int t = 0; t < GK; t++) nx[t] = rows && have ? rsrc[t * J.ld] : 0.f;
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();
     bool good = true;
-    const uint32_t Ma = (uint32_t)__cvta_generic_to_shared(M);
 #pragma unroll 1
     for (int c = 0; c < NB; c++) {
-        T x[GK];
+        float x[GK];
         if (rows) {
 #pragma unroll
             for (int t = 0; t < GK; t++) x[t] = nx[t];
             if (c + 1 < NB) {
-                rsrc += GK * ld;
+                rsrc += GK * J.ld;
 #pragma unroll
-                for (int t = 0; t < GK; t++) nx[t] = have ? rsrc[t * ld] : (T)0;
+                for (int t = 0; t < GK; t++) nx[t] = have ? rsrc[t * J.ld] : 0.f;
             }
         } else {
 #pragma unroll
@@ -921,47 +969,269 @@ __global__ void __launch_bounds__(Fast<T>::RT) k_lu_rows(LuBatch<T> B, int64_t k
         }
 #pragma unroll 1
         for (int p = 0; p < c; p++) {
-            const uint32_t wb = (uint32_t)((NB - p) * GK) * (uint32_t)sizeof(T);
-            uint32_t ua = Ma + (uint32_t)(moff(p) + GK * (c - p)) * (uint32_t)sizeof(T);
+            const int wp = (NB - p) * GK;
+            const float* u = M + fast_moff(p) + GK * (c - p);
 #pragma unroll 4
-            for (int jj = 0; jj < GK; jj++, ua += wb) {
-                const T l = Xs[(GK * p + jj) * LDX + tid];
+            for (int jj = 0; jj < GK; jj++) {
+                const float l = Xs[(GK * p + jj) * LDX + tid];
 #pragma unroll
                 for (int tg = 0; tg < GK; tg += 4) {
-                    T v[4];
-                    lds4(ua + tg * (uint32_t)sizeof(T), v);
+                    float v[4];
+                    load4(u + jj * wp + tg, v);
 #pragma unroll
                     for (int e = 0; e < 4; e++) x[tg + e] -= l * v[e];
                 }
             }
         }
-        const uint32_t ud = Ma + (uint32_t)moff(c) * (uint32_t)sizeof(T);
-        const uint32_t ub = (uint32_t)((NB - c) * GK) * (uint32_t)sizeof(T);
+        const float* ud = M + fast_moff(c);
         if (rows) {
-            good = eliminate32<T, true>(x, ud, ub, rds + GK * c) && good;
-            T* dst = A + i0 + tid + (k0 + GK * c) * ld;
+            good = eliminate32<float, true>(x, ud, (NB - c) * GK, rds + GK * c) && good;
+            float* dst = J.A + J.i0 + tid + (k0 + GK * c) * J.ld;
             if (have)
 #pragma unroll
-                for (int t = 0; t < GK; t++) dst[t * ld] = x[t];
+                for (int t = 0; t < GK; t++) dst[t * J.ld] = x[t];
         } else {
-            eliminate32<T, false>(x, ud, ub, nullptr);
+            eliminate32<float, false>(x, ud, (NB - c) * GK, nullptr);
         }
         if (!rows || c + 1 < NB)
 #pragma unroll
             for (int t = 0; t < GK; t++) Xs[(GK * c + t) * LDX + tid] = x[t];
     }
     if (rows) {
-        if (have && !good) B.fail[sid] = 1;
+        if (have && !good) B.fail[J.sid] = 1;
         return;
     }
     __syncwarp();  // a warp's 32 columns are its own
 #pragma unroll 4
     for (int q = 0; q < 32; q++) {
-        if (i0 + w0 + q >= n) break;
-        T* col = A + k0 + (i0 + w0 + q) * ld;
+        if (J.i0 + w0 + q >= J.n) break;
+        float* col = J.A + k0 + (J.i0 + w0 + q) * J.ld;
 #pragma unroll
         for (int c = 0; c < NB; c++) col[GK * c + lane] = Xs[(GK * c + lane) * LDX + w0 + q];
     }
+}
+
+// The same for 32 rows, or columns, per CTA (a lane each): warp s takes columns
+// 8 s .. of each 32-column step's products with the steps before it, and warp 0
+// the step's triangle.  Each value sees the operations of k_lu_rows in their
+// order; a third of its latency, for launches that leave SMs idle.
+__global__ void __launch_bounds__(Fast<float>::RT) k_lu_rows_split(LuBatch<float> B, int64_t k0, const int32_t* act,
+                                                                   const int64_t* pfx, int cnt, const float* work,
+                                                                   int32_t base) {
+    using F = Fast<float>;
+    constexpr int NB = F::NB, LDX = GK + 1, S = F::RT / 32, CS = GK / S;
+    extern __shared__ __align__(16) unsigned char fast_smem[];
+    float* M = reinterpret_cast<float*>(fast_smem);
+    const float* rds = M + F::MSIZE;
+    float* Xs = M + F::MSIZE + F::W;  // [W][LDX]
+    RowsJob J;
+    if (!rows_job<GK>(J, B, k0, act, pfx, cnt, work, base, M)) return;
+    const int tid = threadIdx.x, lane = tid & 31, s = tid >> 5;
+    const bool rows = J.rows;
+    if (rows) {
+        const bool ok = J.i0 + lane < J.n;
+        const float* src = ok ? J.A + J.i0 + lane + k0 * J.ld : J.A;
+        for (int t = s; t < F::W; t += S)
+            cp_async_zfill<float>((uint32_t)__cvta_generic_to_shared(Xs + t * LDX + lane), src + (ok ? t * J.ld : 0), ok);
+    } else {
+        for (int q = s; q < 32; q += S) {
+            const bool ok = J.i0 + q < J.n;
+            const float* col = ok ? J.A + k0 + lane + (J.i0 + q) * J.ld : J.A;
+#pragma unroll
+            for (int c = 0; c < NB; c++)
+                cp_async_zfill<float>((uint32_t)__cvta_generic_to_shared(Xs + (GK * c + lane) * LDX + q),
+                                      col + (ok ? GK * c : 0), ok);
+        }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    bool good = true;
+#pragma unroll 1
+    for (int c = 0; c < NB; c++) {
+        if (c > 0) {
+            float x[CS];
+#pragma unroll
+            for (int t = 0; t < CS; t++) x[t] = Xs[(GK * c + CS * s + t) * LDX + lane];
+#pragma unroll 1
+            for (int p = 0; p < c; p++) {
+                const int wp = (NB - p) * GK;
+                const float* u = M + fast_moff(p) + GK * (c - p) + CS * s;
+#pragma unroll 8
+                for (int jj = 0; jj < GK; jj++) {
+                    const float l = Xs[(GK * p + jj) * LDX + lane];
+#pragma unroll
+                    for (int tg = 0; tg < CS; tg += 4) {
+                        float v[4];
+                        load4(u + jj * wp + tg, v);
+#pragma unroll
+                        for (int e = 0; e < 4; e++) x[tg + e] -= l * v[e];
+                    }
+                }
+            }
+#pragma unroll
+            for (int t = 0; t < CS; t++) Xs[(GK * c + CS * s + t) * LDX + lane] = x[t];
+            __syncthreads();
+        }
+        if (s == 0) {
+            float x[GK];
+#pragma unroll
+            for (int t = 0; t < GK; t++) x[t] = Xs[(GK * c + t) * LDX + lane];
+            const float* ud = M + fast_moff(c);
+            if (rows) good = eliminate32<float, true>(x, ud, (NB - c) * GK, rds + GK * c) && good;
+            else eliminate32<float, false>(x, ud, (NB - c) * GK, nullptr);
+#pragma unroll
+            for (int t = 0; t < GK; t++) Xs[(GK * c + t) * LDX + lane] = x[t];
+        }
+        __syncthreads();
+    }
+    if (rows) {
+        if (J.i0 + lane < J.n) {
+            float* dst = J.A + J.i0 + lane + k0 * J.ld;
+            for (int t = s; t < F::W; t += S) dst[t * J.ld] = Xs[t * LDX + lane];
+            if (!good) B.fail[J.sid] = 1;
+        }
+        return;
+    }
+    for (int q = s; q < 32; q += S) {
+        if (J.i0 + q >= J.n) break;
+        float* col = J.A + k0 + (J.i0 + q) * J.ld;
+#pragma unroll
+        for (int c = 0; c < NB; c++) col[GK * c + lane] = Xs[(GK * c + lane) * LDX + q];
+    }
+}
+
+// Double: 32-column blocks.  A sub-partition issues half an fp64 lane per
+// cycle, so a warp's fp64 instruction takes 64 cycles: the columns are dealt out to
+// four warps (column t to warp t mod 4, a lane per row), one per sub-partition,
+// and a column's multipliers go round through shared memory.  (One warp per 32
+// rows: the block 39 us, 32 rows against it 26 us; four: see below.)
+__device__ __forceinline__ const double* fast64_work(const double* work, int32_t i) {
+    return work + (int64_t)i * Fast<double>::WORK;
+}
+
+__global__ void __launch_bounds__(Fast<double>::DT) k_lu_diag64(LuBatch<double> B, int64_t k0, const int32_t* act,
+                                                                double* work, int32_t base) {
+    __shared__ double ls[2][GK], rds[GK];
+    const int32_t sid = act[blockIdx.x];
+    const int64_t n = B.n[sid], ld = B.ld[sid];
+    double* A = B.A[sid] + k0 + k0 * ld;
+    const int w = (int)min((int64_t)GK, n - k0);
+    const int tid = threadIdx.x, lane = tid & 31, s = tid >> 5;
+    if (tid < w) {
+        B.ipiv[sid][k0 + tid] = (int32_t)(k0 + tid);
+        B.perm[sid][k0 + tid] = (int32_t)(k0 + tid);
+    }
+    if (B.fail[sid]) return;
+    double x[8];  // row `lane`, columns s, s + 4, ..; past the system's end an identity
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const int t = 4 * q + s;
+        x[q] = lane < w && t < w ? A[lane + t * ld] : (lane == t ? 1.0 : 0.0);
+    }
+    bool good = true;
+    static_for<0, GK>([&](auto JJ) {
+        constexpr int jj = decltype(JJ)::value, q = jj >> 2;
+        if (s == (jj & 3)) {
+            const double d = __shfl_sync(0xffffffffu, x[q], jj);
+            const double rd = pivot_rcp(d);
+            const bool under = lane > jj;
+            good = good && pivot_fits(d) && (!under || not_above(x[q], d));
+            const double lm = under ? x[q] * rd : 0.0;
+            x[q] = under ? lm : x[q];
+            ls[jj & 1][lane] = lm;
+            if (lane == 0) rds[jj] = rd;
+        }
+        __syncthreads();
+        const double lm = ls[jj & 1][lane];
+#pragma unroll
+        for (int e = q; e < 8; e++)
+            if (e > q || s > (jj & 3)) x[e] -= lm * __shfl_sync(0xffffffffu, x[e], jj);
+    });
+    const bool bad = __syncthreads_or(!good);
+    if (bad) {
+        if (tid == 0) B.fail[sid] = 1;
+        return;
+    }
+    double* wk = work + (int64_t)(sid - base) * Fast<double>::WORK;
+#pragma unroll
+    for (int q = 0; q < 8; q++) {
+        const int t = 4 * q + s;
+        if (lane < w && t < w) A[lane + t * ld] = x[q];
+        wk[lane * GK + t] = x[q];            // by rows
+        wk[GK * GK + t * GK + lane] = x[q];  // by columns
+    }
+    if (tid < GK) wk[2 * GK * GK + tid] = rds[tid];
+}
+
+__global__ void __launch_bounds__(Fast<double>::DT) k_lu_rows64(LuBatch<double> B, int64_t k0, const int32_t* act,
+                                                                const int64_t* pfx, int cnt, const double* work,
+                                                                int32_t base) {
+    constexpr int LDX = GK + 1;
+    __shared__ __align__(16) double M[GK * GK];
+    __shared__ double ls[2][GK], rds[GK], Xs[GK * LDX];
+    const int a = find_block(pfx, cnt, blockIdx.x);
+    const int32_t sid = act[a];
+    if (__syncthreads_or(threadIdx.x == 0 && *(volatile int32_t*)&B.fail[sid])) return;
+    const int64_t n = B.n[sid], ld = B.ld[sid];
+    double* A = B.A[sid];
+    const int64_t kend = k0 + GK;
+    const int64_t nr = (n - kend + GK - 1) / GK, idx = blockIdx.x - pfx[a];
+    const bool rows = idx < nr;
+    const int64_t i0 = kend + (rows ? idx : idx - nr) * GK;
+    const int tid = threadIdx.x, lane = tid & 31, s = tid >> 5;
+    const bool have = i0 + lane < n;
+    const double* wk = fast64_work(work, sid - base);
+    double v[8], x[8];
+#pragma unroll
+    for (int q = 0; q < 8; q++) v[q] = wk[(rows ? 0 : GK * GK) + tid + 128 * q];
+    if (rows) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) x[q] = have ? A[i0 + lane + (k0 + 4 * q + s) * ld] : 0.0;
+    } else {  // columns 8 s ..: read down the column, turned in shared memory
+#pragma unroll
+        for (int q = 0; q < 8; q++) x[q] = i0 + 8 * s + q < n ? A[k0 + lane + (i0 + 8 * s + q) * ld] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; q++) Xs[lane * LDX + 8 * s + q] = x[q];
+    }
+    if (tid < GK) rds[tid] = wk[2 * GK * GK + tid];
+#pragma unroll
+    for (int q = 0; q < 8; q++) M[tid + 128 * q] = v[q];
+    __syncthreads();
+    if (!rows) {
+#pragma unroll
+        for (int q = 0; q < 8; q++) x[q] = Xs[(4 * q + s) * LDX + lane];
+    }
+    bool good = true;
+    static_for<0, GK>([&](auto JJ) {
+        constexpr int jj = decltype(JJ)::value, q = jj >> 2;
+        if (s == (jj & 3)) {
+            if (rows) {
+                good = good && not_above(x[q], M[jj * GK + jj]);
+                x[q] *= rds[jj];
+            }
+            ls[jj & 1][lane] = x[q];
+        }
+        __syncthreads();
+        const double lm = ls[jj & 1][lane];
+#pragma unroll
+        for (int e = q; e < 8; e++)
+            if (e > q || s > (jj & 3)) x[e] -= lm * M[jj * GK + 4 * e + s];
+    });
+    if (rows) {
+        if (have) {
+#pragma unroll
+            for (int q = 0; q < 8; q++) A[i0 + lane + (k0 + 4 * q + s) * ld] = x[q];
+            if (!good) B.fail[sid] = 1;
+        }
+        return;
+    }
+#pragma unroll
+    for (int q = 0; q < 8; q++) Xs[(4 * q + s) * LDX + lane] = x[q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 8; q++)
+        if (i0 + 8 * s + q < n) A[k0 + lane + (i0 + 8 * s + q) * ld] = Xs[lane * LDX + 8 * s + q];
 }
 
 template <class T>
@@ -2753,15 +3023,29 @@ int lu_batch_factor_fast(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t s
         const LuStep& S = plan.steps[s];
         if (S.n_panel == 0 || S.k % F::W != 0) continue;
         const int32_t* act = plan.d_act + S.act_off;
-        k_lu_diag<T><<<(unsigned)S.n_panel, F::DT, F::diag_smem, st>>>(B, S.k, act, work, plan.base);
+        if constexpr (sizeof(T) == 4)
+            k_lu_diag<<<(unsigned)S.n_panel, F::DT, F::diag_smem, st>>>(B, S.k, act, work, plan.base);
+        else
+            k_lu_diag64<<<(unsigned)S.n_panel, F::DT, 0, st>>>(B, S.k, act, work, plan.base);
         GB_LAUNCH_CHECK();
         if (S.fr_blocks[E] == 0) continue;
         if (pending) {  // the columns that k_lu_rows solves are those the lookahead update is still working on
             GB_CUDA(cudaStreamWaitEvent(st, plan.la_join, 0));
             pending = false;
         }
-        k_lu_rows<T><<<(unsigned)S.fr_blocks[E], F::RT, F::rows_smem, st>>>(B, S.k, act, plan.d_pfx + S.fr_pfx[E],
-                                                                           S.fr_cnt[E], work, plan.base);
+        const int64_t* fpfx = plan.d_pfx + S.fr_pfx[E];
+        if constexpr (sizeof(T) == 8) {
+            k_lu_rows64<<<(unsigned)S.fr_blocks[E], F::DT, 0, st>>>(B, S.k, act, fpfx, S.fr_cnt[E], work, plan.base);
+        } else {
+            // in 32-row CTAs of four warps while they fit the SMs at once
+            // (shortest chain), else in 128-row CTAs; the same arithmetic
+            if (S.fs_blocks <= 2 * tc_num_sms())
+                k_lu_rows_split<<<(unsigned)S.fs_blocks, F::RT, F::rows_smem, st>>>(B, S.k, act, plan.d_pfx + S.fs_pfx,
+                                                                                   S.fr_cnt[E], work, plan.base);
+            else
+                k_lu_rows<<<(unsigned)S.fr_blocks[E], F::RT, F::rows_smem, st>>>(B, S.k, act, fpfx, S.fr_cnt[E], work,
+                                                                                plan.base);
+        }
         GB_LAUNCH_CHECK();
         if constexpr (sizeof(T) == 8) {
             k_update<T, GT_F64><<<(unsigned)S.fu_blocks, GT_F64 * GT_F64 / 16, 0, st>>>(
@@ -2913,9 +3197,11 @@ int lu_plan_build(LuPlan& plan, const std::vector<int64_t>& n_sorted, cudaStream
             const char* f = getenv("GBVLM_LU_FAST");
             plan.fast_any = !(f && f[0] == '0');
             plan.fast = plan.fast_any && plan.tc_passes == 3 && !tc_persistent();
-            GB_CUDA(cudaFuncSetAttribute(k_lu_diag<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            GB_CUDA(cudaFuncSetAttribute(k_lu_diag, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)Fast<float>::diag_smem));
-            GB_CUDA(cudaFuncSetAttribute(k_lu_rows<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+            GB_CUDA(cudaFuncSetAttribute(k_lu_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)Fast<float>::rows_smem));
+            GB_CUDA(cudaFuncSetAttribute(k_lu_rows_split, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)Fast<float>::rows_smem));
         }
         GB_CUDA(dev_alloc((void**)&plan.d_err, sizeof(int), plan.mem));
@@ -3172,6 +3458,14 @@ int lu_plan_build(LuPlan& plan, const std::vector<int64_t>& n_sorted, cudaStream
             S.fr_blocks[e] = acc;
             S.fr_cnt[e] = ci;
         }
+        S.fs_pfx = (int64_t)pfx.size();
+        acc = 0;
+        for (int i = 0; i < S.fr_cnt[0]; i++) {
+            pfx.push_back(acc);
+            acc += 2 * cdiv(n_sorted[i] - k - Fast<float>::W, (int64_t)GK);
+        }
+        pfx.push_back(acc);
+        S.fs_blocks = acc;
         S.fu_pfx = (int64_t)pfx.size();
         acc = 0;
         for (int i = 0; i < S.fr_cnt[1]; i++) {

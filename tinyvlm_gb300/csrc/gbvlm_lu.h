@@ -75,6 +75,7 @@ struct LuStep {
     // block, double at every step): rows and columns past the block
     int64_t fr_pfx[2] = {0, 0}, fr_blocks[2] = {0, 0};  // k_lu_rows, float and double
     int32_t fr_cnt[2] = {0, 0};                         // systems past the block (a prefix)
+    int64_t fs_pfx = 0, fs_blocks = 0;                  // float: k_lu_rows_split, 32 rows or columns per CTA
     int64_t fu_pfx = 0, fu_blocks = 0;                  // double: the trailing update in 32 x 32 tiles
 };
 
@@ -93,8 +94,8 @@ struct LuPlan {
     bool tc_inner = false;  // inner updates in 128-row tensor-core tiles, K = 32 (GBVLM_TC_INNER=0: CUDA cores)
     bool tc_trsm = false;
     int32_t tc_trsm_min = 1;  // ... for steps with at least this many systems
-    // per system 128 x 128 + 128 floats: I - L11^-1 of the current outer block, or the
-    // factored diagonal block and its reciprocal pivots (without interchanges)
+    // per system 2 x 128 x 128 + 128 floats: I - L11^-1 of the current outer block, or the factored
+    // diagonal block by rows and by columns and its reciprocal pivots (without interchanges)
     float* d_minv = nullptr;
     // systems may be factored without interchanges (GBVLM_LU_FAST=0: not): in double, and in float
     bool fast_any = false, fast = false;
