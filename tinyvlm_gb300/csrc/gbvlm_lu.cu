@@ -1130,23 +1130,33 @@ __global__ void __launch_bounds__(Fast<double>::DT) k_lu_diag64(LuBatch<double> 
         x[q] = lane < w && t < w ? A[lane + t * ld] : (lane == t ? 1.0 : 0.0);
     }
     bool good = true;
+    // column j, by its warp: the multipliers to shared memory
+    auto column = [&](auto J) {
+        constexpr int j = decltype(J)::value, q = j >> 2;
+        const double d = __shfl_sync(0xffffffffu, x[q], j);
+        const double rd = pivot_rcp(d);
+        const bool under = lane > j;
+        good = good && pivot_fits(d) && (!under || not_above(x[q], d));
+        const double lm = under ? x[q] * rd : 0.0;
+        x[q] = under ? lm : x[q];
+        ls[j & 1][lane] = lm;
+        if (lane == 0) rds[j] = rd;
+    };
+    if (s == 0) column(std::integral_constant<int, 0>{});
     static_for<0, GK>([&](auto JJ) {
-        constexpr int jj = decltype(JJ)::value, q = jj >> 2;
-        if (s == (jj & 3)) {
-            const double d = __shfl_sync(0xffffffffu, x[q], jj);
-            const double rd = pivot_rcp(d);
-            const bool under = lane > jj;
-            good = good && pivot_fits(d) && (!under || not_above(x[q], d));
-            const double lm = under ? x[q] * rd : 0.0;
-            x[q] = under ? lm : x[q];
-            ls[jj & 1][lane] = lm;
-            if (lane == 0) rds[jj] = rd;
-        }
+        constexpr int jj = decltype(JJ)::value, q = jj >> 2, j1 = jj + 1, q1 = j1 >> 2;
         __syncthreads();
         const double lm = ls[jj & 1][lane];
+        // the next column first: the others wait for its multipliers
+        if constexpr (j1 < GK)
+            if (s == (j1 & 3)) {
+                x[q1] -= lm * __shfl_sync(0xffffffffu, x[q1], jj);
+                column(std::integral_constant<int, j1>{});
+            }
 #pragma unroll
         for (int e = q; e < 8; e++)
-            if (e > q || s > (jj & 3)) x[e] -= lm * __shfl_sync(0xffffffffu, x[e], jj);
+            if ((e > q || s > (jj & 3)) && !(e == q1 && s == (j1 & 3)))
+                x[e] -= lm * __shfl_sync(0xffffffffu, x[e], jj);
     });
     const bool bad = __syncthreads_or(!good);
     if (bad) {
@@ -1203,20 +1213,27 @@ __global__ void __launch_bounds__(Fast<double>::DT) k_lu_rows64(LuBatch<double> 
         for (int q = 0; q < 8; q++) x[q] = Xs[(4 * q + s) * LDX + lane];
     }
     bool good = true;
-    static_for<0, GK>([&](auto JJ) {
-        constexpr int jj = decltype(JJ)::value, q = jj >> 2;
-        if (s == (jj & 3)) {
-            if (rows) {
-                good = good && not_above(x[q], M[jj * GK + jj]);
-                x[q] *= rds[jj];
-            }
-            ls[jj & 1][lane] = x[q];
+    auto column = [&](auto J) {
+        constexpr int j = decltype(J)::value, q = j >> 2;
+        if (rows) {
+            good = good && not_above(x[q], M[j * GK + j]);
+            x[q] *= rds[j];
         }
+        ls[j & 1][lane] = x[q];
+    };
+    if (s == 0) column(std::integral_constant<int, 0>{});
+    static_for<0, GK>([&](auto JJ) {
+        constexpr int jj = decltype(JJ)::value, q = jj >> 2, j1 = jj + 1, q1 = j1 >> 2;
         __syncthreads();
         const double lm = ls[jj & 1][lane];
+        if constexpr (j1 < GK)
+            if (s == (j1 & 3)) {
+                x[q1] -= lm * M[jj * GK + j1];
+                column(std::integral_constant<int, j1>{});
+            }
 #pragma unroll
         for (int e = q; e < 8; e++)
-            if (e > q || s > (jj & 3)) x[e] -= lm * M[jj * GK + 4 * e + s];
+            if ((e > q || s > (jj & 3)) && !(e == q1 && s == (j1 & 3))) x[e] -= lm * M[jj * GK + 4 * e + s];
     });
     if (rows) {
         if (have) {

@@ -182,16 +182,19 @@ static int mesh_metrics(T alpha, int32_t nsurf, const gbvlm_dims* dims, const T*
 
 // ---------------------------------------------------------------------------
 // a1: AIC assembly, one launch per (influenced, influencing) surface pair
-// (vlm_backend_cpu.cpp:84-148).  Block = 128 collocation points (one per
-// thread, each with its y-mirror) x one chordwise ring row (chunked along
-// the span) of the influencing surface; that row's two vertex lines are
-// staged in shared memory and read as broadcasts.  Along the span a thread
-// keeps the left vertex terms and left chordwise segment of the previous
-// ring, so each ring costs two vertex terms and three segment terms per
-// evaluation point.
+// (vlm_backend_cpu.cpp:84-148).  Block = LHS_THREADS collocation points (one per
+// thread, each with its y-mirror) x a piece of the influencing surface, ROWS
+// ring rows x `span` rings, staged in shared memory with its segment vectors;
+// lattice_rings evaluates each segment once for the two rings it bounds, 2.25
+// to 2.5 segments and 1.25 to 1.5 vertices per ring and point where the
+// ring-by-ring walk took three and two.  The block of the last ring row adds
+// the wake rows to the trailing-edge columns.
+// Bound: the fp32 (fp64) pipe; small surfaces, the number of blocks, so the
+// pieces shrink until the launch covers the SMs twice (a ring's value does not
+// depend on the cut).
 // ---------------------------------------------------------------------------
-constexpr int LHS_THREADS = 128;
-constexpr int LHS_SCHUNK = 256;
+constexpr int LHS_THREADS = 64;
+constexpr int LHS_SPAN = 32;  // rings of a piece at most
 
 template <class T>
 struct LhsPair {
@@ -209,47 +212,49 @@ struct LhsPair {
     int64_t row_off, col_off;
 };
 
-template <class T, bool SIGMA>
-__global__ void __launch_bounds__(LHS_THREADS) k_lhs_pair(LhsPair<T> a) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    T* sv = reinterpret_cast<T*>(smem_raw);
-    constexpr int W = LHS_SCHUNK + 1;
-    const int64_t c = blockIdx.y;
-    const int64_t s0 = (int64_t)blockIdx.z * LHS_SCHUNK;
-    const int64_t s1 = min(s0 + (int64_t)LHS_SCHUNK, a.ns);
-    const int nv = (int)(s1 - s0 + 1);
-    const int64_t vld = (a.ns + 1) * (a.nc + 1);
-    for (int t = threadIdx.x; t < 2 * nv; t += blockDim.x) {
-        int r = t / nv, sl = t - r * nv;
-        int64_t vi = (s0 + sl) + (c + r) * (a.ns + 1);
-        sv[(r * 3 + 0) * W + sl] = a.vw[vi];
-        sv[(r * 3 + 1) * W + sl] = a.vw[vld + vi];
-        sv[(r * 3 + 2) * W + sl] = a.vw[2 * vld + vi];
+// lines [r0, r0 + nl) and vertices [k0, k0 + nk] of the lattice v (n vertices per line) into shared memory
+template <class T>
+__device__ __forceinline__ void stage_piece(const T* v, int64_t n, int64_t vld, int64_t r0, int64_t k0, int nl, int nk,
+                                            int W, Quad<T>* sv, Quad<T>* ss, Quad<T>* sc) {
+    for (int e = threadIdx.x; e < nl * (nk + 1); e += blockDim.x) {
+        const int li = e / (nk + 1), k = e - li * (nk + 1);
+        const int64_t vi = k0 + k + (r0 + li) * n;
+        const T x = v[vi], y = v[vld + vi], z = v[2 * vld + vi];
+        sv[li * W + k] = Quad<T>{x, y, z, 0};
+        if (k > 0) ss[li * W + k] = Quad<T>{x - v[vi - 1], y - v[vld + vi - 1], z - v[2 * vld + vi - 1], 0};
+        if (li + 1 < nl) sc[li * W + k] = Quad<T>{v[vi + n] - x, v[vld + vi + n] - y, v[2 * vld + vi + n] - z, 0};
     }
-    __syncthreads();
+}
+
+template <class T, bool SIGMA, int ROWS>
+__global__ void __launch_bounds__(LHS_THREADS) k_lhs_pair(LhsPair<T> a) {
+    constexpr int LR = ROWS + 1, W = LHS_SPAN + 1;
+    __shared__ Quad<T> sv[LR * W], ss[LR * W], sc[LR * W];
+    const int64_t c0 = (int64_t)blockIdx.y * ROWS;
+    const int64_t s0 = (int64_t)blockIdx.z * a.ns / gridDim.z, s1 = (int64_t)(blockIdx.z + 1) * a.ns / gridDim.z;
+    const int nr = (int)min((int64_t)ROWS, a.nc - c0), nk = (int)(s1 - s0);
+    const int64_t n = a.ns + 1;
+    stage_piece<T>(a.vw, n, n * (a.nc + 1), c0, s0, nr + 1, nk, W, sv, ss, sc);
     const int64_t i = (int64_t)blockIdx.x * LHS_THREADS + threadIdx.x;
-    if (i >= a.np_i) return;
-    const T px = a.colloc[i], py = a.colloc[a.np_i + i], pz = a.colloc[2 * a.np_i + i];
-    const T nx = a.normals[i], ny = a.normals[a.np_i + i], nz = a.normals[2 * a.np_i + i];
-    const T sg = a.sigma2;
-    const bool te = (c == a.nc - 1) && a.iteration > 0;
-    const int64_t wk_ld = (a.ns + 1) * a.nwv;
-    T* out = a.lhs + (a.row_off + i) + (a.col_off + c * a.ns) * a.ld;
-    strip_normal<T, SIGMA>(sv, sv + 3 * W, W, nv, px, py, pz, nx, ny, nz, sg, [&](int kk, T val) {
-        const int64_t s = s0 + kk;
-        if (te) {
-            for (int32_t it = 0; it < a.iteration; it++) {
-                const int64_t r0 = a.nwv - 2 - it;
-                const int64_t i0 = s + r0 * (a.ns + 1), i1 = i0 + 1, i2 = i1 + (a.ns + 1), i3 = i0 + (a.ns + 1);
-                V3<T> q[4] = {{a.vk[i0], a.vk[wk_ld + i0], a.vk[2 * wk_ld + i0]},
-                              {a.vk[i1], a.vk[wk_ld + i1], a.vk[2 * wk_ld + i1]},
-                              {a.vk[i2], a.vk[wk_ld + i2], a.vk[2 * wk_ld + i2]},
-                              {a.vk[i3], a.vk[wk_ld + i3], a.vk[2 * wk_ld + i3]}};
-                val += ring_normal_full<T, SIGMA>(px, py, pz, nx, ny, nz, q, sg);
-            }
-        }
-        out[s * a.ld] += val * inv_four_pi<T>();
+    const bool active = i < a.np_i;
+    const int64_t ip = active ? i : 0;
+    const T px = a.colloc[ip], py = a.colloc[a.np_i + ip], pz = a.colloc[2 * a.np_i + ip];
+    const T nx = a.normals[ip], ny = a.normals[a.np_i + ip], nz = a.normals[2 * a.np_i + ip];
+    T* out = a.lhs + (a.row_off + ip) + (a.col_off + c0 * a.ns + s0) * a.ld;
+    __syncthreads();
+    lattice_rings<T, SIGMA, LR>(sv, ss, sc, W, nr + 1, nk, px, py, pz, nx, ny, nz, a.sigma2, [&](int r, int k, T val) {
+        if (active) out[(r * a.ns + k) * a.ld] += val * inv_four_pi<T>();
     });
+    if (c0 + nr < a.nc) return;
+    out += (int64_t)(nr - 1) * a.ns * a.ld;
+    for (int32_t it = 0; it < a.iteration; it++) {
+        __syncthreads();
+        stage_piece<T>(a.vk, n, n * a.nwv, a.nwv - 2 - it, s0, 2, nk, W, sv, ss, sc);
+        __syncthreads();
+        lattice_rings<T, SIGMA, 2>(sv, ss, sc, W, 2, nk, px, py, pz, nx, ny, nz, a.sigma2, [&](int, int k, T val) {
+            if (active) out[k * a.ld] += val * inv_four_pi<T>();
+        });
+    }
 }
 
 template <class T>
@@ -270,7 +275,6 @@ static int lhs_assemble(T* lhs, int64_t ld, int32_t nsurf, const gbvlm_dims* dim
             GB_REQUIRE(dims[m].nwv >= iteration + 1, "surface %d: nwv=%lld < iteration+1", m, (long long)dims[m].nwv);
         }
     }
-    const size_t smem = 2 * 3 * (LHS_SCHUNK + 1) * sizeof(T);
     for (int mj = 0; mj < nsurf; mj++) {
         for (int mi = 0; mi < nsurf; mi++) {
             LhsPair<T> a;
@@ -288,11 +292,21 @@ static int lhs_assemble(T* lhs, int64_t ld, int32_t nsurf, const gbvlm_dims* dim
             a.sigma2 = sigma * sigma;
             a.row_off = s.poff[mi];
             a.col_off = s.poff[mj];
-            dim3 grid((unsigned)cdiv(a.np_i, LHS_THREADS), (unsigned)a.nc, (unsigned)cdiv(a.ns, LHS_SCHUNK));
-            if (sigma != (T)0)
-                k_lhs_pair<T, true><<<grid, LHS_THREADS, smem, st>>>(a);
-            else
-                k_lhs_pair<T, false><<<grid, LHS_THREADS, smem, st>>>(a);
+            // four ring rows x 32 rings per piece, fewer until the blocks cover the SMs twice
+            int rows = 4;
+            int64_t span = LHS_SPAN;
+            auto blocks = [&]() { return cdiv(a.np_i, (int64_t)LHS_THREADS) * cdiv(a.nc, (int64_t)rows) * cdiv(a.ns, span); };
+            if (blocks() < 2 * sm_count()) rows = 2;
+            while (span > 8 && blocks() < 2 * sm_count()) span /= 2;
+            dim3 grid((unsigned)cdiv(a.np_i, (int64_t)LHS_THREADS), (unsigned)cdiv(a.nc, (int64_t)rows),
+                      (unsigned)cdiv(a.ns, span));
+            auto launch = [&](auto SIGMA) {
+                constexpr bool sg = decltype(SIGMA)::value;
+                if (rows == 4) k_lhs_pair<T, sg, 4><<<grid, LHS_THREADS, 0, st>>>(a);
+                else k_lhs_pair<T, sg, 2><<<grid, LHS_THREADS, 0, st>>>(a);
+            };
+            if (sigma != (T)0) launch(std::true_type{});
+            else launch(std::false_type{});
             GB_LAUNCH_CHECK();
         }
     }

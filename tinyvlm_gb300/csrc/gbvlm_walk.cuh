@@ -239,4 +239,48 @@ __device__ __forceinline__ void lattice_walk(const Quad<T>* v, const Quad<T>* s,
     }
 }
 
+// Every ring of a lattice piece (laid out as for lattice_walk, at most LR - 1
+// ring rows) at unit strength: calls emit(row, ring, 4 pi (v . n + v_image .
+// n_image)).  A segment is evaluated once, forward, for the two rings it bounds,
+// so a ring's value does not depend on how the lattice was cut into pieces.
+template <class T, bool SIGMA, int LR, class F>
+__device__ __forceinline__ void lattice_rings(const Quad<T>* v, const Quad<T>* s, const Quad<T>* c, int W, int nl, int nk,
+                                              T px, T py, T pz, T nx, T ny, T nz, T sg, F&& emit) {
+    RelPair<T> prev[LR];
+    T left[LR - 1];  // the chordwise segments of the vertex before
+    auto seg = [&](const RelPair<T>& a, const RelPair<T>& b, const Quad<T>& e) {
+        T k0, k1, cy, cx0, cx1, cz0, cz1;
+        seg_pair<T, SIGMA>(a, b, e.x, e.y, e.z, sg, k0, k1, cy, cx0, cx1, cz0, cz1);
+        const T tn = cy * ny;
+        return k0 * (cx0 * nx + tn + cz0 * nz) + k1 * (cx1 * nx - tn + cz1 * nz);
+    };
+#pragma unroll
+    for (int l = 0; l < LR; l++)
+        if (l < nl) {
+            const Quad<T> q = v[l * W];
+            prev[l] = make_rel_pair<T>(px, py, pz, q.x, q.y, q.z);
+            if (l > 0) left[l - 1] = seg(prev[l > 0 ? l - 1 : 0], prev[l], c[(l - 1) * W]);
+        }
+#pragma unroll 1
+    for (int k = 1; k <= nk; k++) {
+        RelPair<T> up = prev[0];
+        T above = 0;
+#pragma unroll
+        for (int l = 0; l < LR; l++)
+            if (l < nl) {
+                const Quad<T> q = v[l * W + k];
+                const RelPair<T> cur = make_rel_pair<T>(px, py, pz, q.x, q.y, q.z);
+                const T span = seg(prev[l], cur, s[l * W + k]);
+                if (l > 0) {
+                    const T right = seg(up, cur, c[(l - 1) * W + k]);
+                    emit(l - 1, k - 1, (above - span) + (right - left[l - 1]));
+                    left[l - 1] = right;
+                }
+                up = cur;
+                above = span;
+                prev[l] = cur;
+            }
+    }
+}
+
 }  // namespace gbvlm
