@@ -65,9 +65,16 @@ __device__ __forceinline__ void hb_rot_y(double px, double a, double& r00, doubl
     t2 = 0.0 - (-sn) * px;
 }
 
-__global__ void k_hb_chain(const double* prm, int H, int64_t rows, int32_t nsurf, int32_t m, double* Tall) {
+// grid y: the parameter set (its steps and the offsets of its transforms and wake in `sets`)
+struct HbSet {
+    int64_t rows, tw, wake;
+};
+__global__ void k_hb_chain(const double* prm, int64_t stride, const HbSet* sets, int H, int32_t nsurf, int32_t m,
+                           double* Tall) {
     const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (i >= rows) return;
+    if (i >= sets[blockIdx.y].rows) return;
+    prm += blockIdx.y * stride;
+    Tall += sets[blockIdx.y].tw;
     const int U = 2 * H + 1;
     const double sigma = prm[0], omega = prm[1], dt = prm[2], px = prm[3], qx = prm[4];
     const bool flap = prm[5] != 0.0;
@@ -110,10 +117,12 @@ __global__ void k_hb_chain(const double* prm, int H, int64_t rows, int32_t nsurf
 
 // wake pre-generation in one launch (libhbvlm3.cpp:307-319): wake row
 // nwv-1-i = T(i dt) applied to the trailing-edge vertices, every step i
-__global__ void k_pregen_wake(const double* Tall, int32_t nsurf, int32_t m, const double* vinit, int64_t ns, int64_t nc,
-                              int64_t max_t, double* wake) {
+__global__ void k_pregen_wake(const double* Tall, const HbSet* sets, int32_t nsurf, int32_t m, const double* vinit,
+                              int64_t ns, int64_t nc, double* wake) {
     const int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    const int64_t n1 = ns + 1;
+    const int64_t n1 = ns + 1, max_t = sets[blockIdx.y].rows;
+    Tall += sets[blockIdx.y].tw;
+    wake += sets[blockIdx.y].wake;
     if (g >= n1 * max_t) return;
     const int64_t j = g % n1, i = g / n1;
     const double* T = Tall + 16 * ((size_t)i * nsurf + m);
@@ -171,6 +180,7 @@ struct WopArgs {
     float* basis_f2;           // the basis rows as float pairs, 2 floats per entry of the double rows
     const double* basis0;      // start of the double basis rows
     int32_t c0;                // the first Fourier coefficient this launch accumulates
+    int64_t slices;
 };
 
 // ---------------------------------------------------------------------------
@@ -263,37 +273,56 @@ __global__ void k_hb_basis(WopArgs a) {
     }
 }
 
+// a wake vertex seen from the point (y0, n0) and from its image (y1, n1); what
+// has no y in it is formed once
 struct RelF2 {
-    F2 x, y, z, n;
+    F2 x, z, y0, y1, n0, n1;
 };
-__device__ __forceinline__ RelF2 rel_f2(F2 px, F2 py, F2 pz, F2 vx, F2 vy, F2 vz) {
+__device__ __forceinline__ RelF2 rel_f2(F2 px, F2 py, F2 qy, F2 pz, F2 vx, F2 vy, F2 vz) {
     RelF2 r;
     r.x = f2_sub(px, vx);
-    r.y = f2_sub(py, vy);
     r.z = f2_sub(pz, vz);
-    r.n = f2_sqrt(f2_add(f2_add(f2_mul(r.x, r.x), f2_mul(r.y, r.y)), f2_mul(r.z, r.z)));
+    r.y0 = f2_sub(py, vy);
+    r.y1 = f2_sub(qy, vy);
+    const F2 xx = f2_mul(r.x, r.x), zz = f2_mul(r.z, r.z);
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+        const F2 y = k ? r.y1 : r.y0;
+        const F2 n = f2_sqrt(f2_add(f2_add(xx, f2_mul(y, y)), zz));
+        if (k) r.n1 = n;
+        else r.n0 = n;
+    }
     return r;
 }
-// seg_normal of the operator library (4 pi (v(A->B) . n), no core) in float pairs
-__device__ __forceinline__ F2 seg_normal_f2(const RelF2& a, const RelF2& b, F2 nx, F2 ny, F2 nz) {
-    const F2 r0x = f2_sub(a.x, b.x), r0y = f2_sub(a.y, b.y), r0z = f2_sub(a.z, b.z);  // B - A
-    const F2 cx = f2_sub(f2_mul(r0y, a.z), f2_mul(r0z, a.y));
-    const F2 cy = f2_sub(f2_mul(r0z, a.x), f2_mul(r0x, a.z));
-    const F2 cz = f2_sub(f2_mul(r0x, a.y), f2_mul(r0y, a.x));
-    const F2 sq = f2_add(f2_add(f2_mul(cx, cx), f2_mul(cy, cy)), f2_mul(cz, cz));
-    if (sq.h < RCUT_SQ || a.n.h < (float)RCUT_NORM_D || b.n.h < (float)RCUT_NORM_D) return F2{0.f, 0.f};
-    const F2 ab = f2_add(f2_add(f2_mul(a.x, b.x), f2_mul(a.y, b.y)), f2_mul(a.z, b.z));
-    const F2 nab = f2_mul(a.n, b.n), sum = f2_add(a.n, b.n);
-    F2 num, den;
-    if (ab.h >= 0.f) {
-        num = sum;
-        den = f2_mul(nab, f2_add(nab, ab));
-    } else {
-        num = f2_mul(sum, f2_sub(nab, ab));
-        den = f2_mul(nab, sq);
+// seg_normal of the operator library (4 pi (v(A->B) . n), no core) in float
+// pairs, at the point (va) and at its image (vb)
+__device__ __forceinline__ void seg_normal_f2(const RelF2& a, const RelF2& b, F2 nx, F2 ny, F2 nz, F2& va, F2& vb) {
+    const F2 rx = f2_sub(a.x, b.x), rz = f2_sub(a.z, b.z);  // B - A
+    const F2 cy = f2_sub(f2_mul(rz, a.x), f2_mul(rx, a.z)), cyy = f2_mul(cy, cy), cyn = f2_mul(cy, ny);
+    const F2 abx = f2_mul(a.x, b.x), abz = f2_mul(a.z, b.z);
+    va = vb = F2{0.f, 0.f};
+#pragma unroll 1
+    for (int k = 0; k < 2; k++) {
+        const F2 ay = k ? a.y1 : a.y0, by = k ? b.y1 : b.y0, an = k ? a.n1 : a.n0, bn = k ? b.n1 : b.n0;
+        const F2 ry = f2_sub(ay, by);
+        const F2 cx = f2_sub(f2_mul(ry, a.z), f2_mul(rz, ay)), cz = f2_sub(f2_mul(rx, ay), f2_mul(ry, a.x));
+        const F2 sq = f2_add(f2_add(f2_mul(cx, cx), cyy), f2_mul(cz, cz));
+        if (sq.h < RCUT_SQ || an.h < (float)RCUT_NORM_D || bn.h < (float)RCUT_NORM_D) continue;
+        const F2 ab = f2_add(f2_add(abx, f2_mul(ay, by)), abz);
+        const F2 nab = f2_mul(an, bn), sum = f2_add(an, bn);
+        F2 num, den;
+        if (ab.h >= 0.f) {
+            num = sum;
+            den = f2_mul(nab, f2_add(nab, ab));
+        } else {
+            num = f2_mul(sum, f2_sub(nab, ab));
+            den = f2_mul(nab, sq);
+        }
+        const F2 cn = f2_add(f2_add(f2_mul(cx, nx), k ? f2_neg(cyn) : cyn), f2_mul(cz, nz));
+        const F2 v = f2_mul(f2_div(num, den), cn);
+        if (k) vb = v;
+        else va = v;
     }
-    const F2 cn = f2_add(f2_add(f2_mul(cx, nx), f2_mul(cy, ny)), f2_mul(cz, nz));
-    return f2_mul(f2_div(num, den), cn);
 }
 
 // the wake of each instance's set relative to the instance's origin (its
@@ -314,14 +343,25 @@ __global__ void k_wake_shift(const WopInst* inst, int64_t wns, float* out, const
     }
 }
 
-// one thread per (target p, wake span i) of instance blockIdx.y over the
-// rows of slice blockIdx.z: the ring values along the rows in float pairs,
-// each line's spanwise segment shared by the two rings it bounds
+// one thread per (slice of rows, target p, wake span i) of instance blockIdx.y:
+// the ring values along the slice's rows in float pairs, each line's spanwise
+// segment shared by the two rings it bounds.  Bound: issue of fp32
+// instructions.  Slices and points side by side leave no lane of a warp idle
+// (45 points on 64 threads did), a point and its image share what has no y in
+// it and the code of the rest (two copies of it overflowed the instruction
+// cache), and NC, the coefficients a launch accumulates, is known to the
+// compiler.  Every value is formed by the operations that it was formed by
+// before, in their order: the fixed-point iteration ends on a residual of
+// 1e-9, and another rounding here moves its result by more than that.
+// 44 sets of 11 instances, 45 points, about 2500 rows: 10.4 -> 6.4 ms; one set
+// 335 -> 221 us.
+template <int NC>
 __global__ void __launch_bounds__(WOP_THREADS) k_wake_operator(WopArgs a) {
     const WopInst& I = a.inst[blockIdx.y];
     const int64_t n = a.poff[a.nsurf], npairs = n * a.wns;
-    const int64_t g = blockIdx.x * (int64_t)WOP_THREADS + threadIdx.x;
-    if (g >= npairs) return;
+    const int64_t t = blockIdx.x * (int64_t)WOP_THREADS + threadIdx.x;
+    const int64_t slice = t / npairs, g = t - slice * npairs;
+    if (slice >= a.slices) return;
     const int64_t p = g / a.wns, i = g - p * a.wns;
     int m = 0;
     while (p >= a.poff[m + 1]) m++;
@@ -331,14 +371,13 @@ __global__ void __launch_bounds__(WOP_THREADS) k_wake_operator(WopArgs a) {
     const F2 Px = f2_of(px - O[0]), Py = f2_of(py - O[1]), Pz = f2_of(pz - O[2]);
     const F2 Qy = f2_of(-py - O[1]);  // the mirror point's y
     const F2 nx = f2_of(I.normals[m][pl]), ny = f2_of(I.normals[m][np + pl]), nz = f2_of(I.normals[m][2 * np + pl]);
-    const F2 mny = f2_neg(ny);
     const int64_t start = I.nwv - 1 - I.it;
-    const int64_t j0 = start + (int64_t)blockIdx.z * I.rps;
+    const int64_t j0 = start + slice * I.rps;
     const int64_t j1 = min(j0 + I.rps, I.nwv - 1);
-    const int nco = a.N - a.c0;  // coefficients of this launch (at most WOP_NMAX used)
-    F2 acc[WOP_NMAX];
+    const int nco = min(a.N - a.c0, NC);
+    F2 acc[NC];
 #pragma unroll
-    for (int c = 0; c < WOP_NMAX; c++) acc[c] = F2{0.f, 0.f};
+    for (int c = 0; c < NC; c++) acc[c] = F2{0.f, 0.f};
     if (j0 < j1) {
         const int64_t n1 = a.wns + 1, nv = n1 * I.nwv;
         const float* W = a.wshift + a.wshift_off[blockIdx.y];
@@ -351,30 +390,32 @@ __global__ void __launch_bounds__(WOP_THREADS) k_wake_operator(WopArgs a) {
         F2 x0, y0, z0, x1, y1, z1;
         V(j0, i, x0, y0, z0);
         V(j0, i + 1, x1, y1, z1);
-        RelF2 A0 = rel_f2(Px, Py, Pz, x0, y0, z0), A1 = rel_f2(Px, Py, Pz, x1, y1, z1);
-        RelF2 B0 = rel_f2(Px, Qy, Pz, x0, y0, z0), B1 = rel_f2(Px, Qy, Pz, x1, y1, z1);
-        F2 Ta = seg_normal_f2(A0, A1, nx, ny, nz), Tb = seg_normal_f2(B0, B1, nx, mny, nz);
+        RelF2 A0 = rel_f2(Px, Py, Qy, Pz, x0, y0, z0), A1 = rel_f2(Px, Py, Qy, Pz, x1, y1, z1);
+        F2 Ta, Tb;
+        seg_normal_f2(A0, A1, nx, ny, nz, Ta, Tb);
+#pragma unroll 1
         for (int64_t j = j0; j < j1; j++) {
             F2 x3, y3, z3, x2, y2, z2;  // line j + 1: v3 = (j + 1, i), v2 = (j + 1, i + 1)
             V(j + 1, i, x3, y3, z3);
             V(j + 1, i + 1, x2, y2, z2);
-            const RelF2 A3 = rel_f2(Px, Py, Pz, x3, y3, z3), A2 = rel_f2(Px, Py, Pz, x2, y2, z2);
-            const RelF2 B3 = rel_f2(Px, Qy, Pz, x3, y3, z3), B2 = rel_f2(Px, Qy, Pz, x2, y2, z2);
-            const F2 Na = seg_normal_f2(A3, A2, nx, ny, nz), Nb = seg_normal_f2(B3, B2, nx, mny, nz);
-            F2 val = f2_add(f2_sub(f2_add(Ta, seg_normal_f2(A1, A2, nx, ny, nz)), Na), seg_normal_f2(A3, A0, nx, ny, nz));
-            val = f2_add(val, f2_add(f2_sub(f2_add(Tb, seg_normal_f2(B1, B2, nx, mny, nz)), Nb),
-                                     seg_normal_f2(B3, B0, nx, mny, nz)));
+            const RelF2 A3 = rel_f2(Px, Py, Qy, Pz, x3, y3, z3), A2 = rel_f2(Px, Py, Qy, Pz, x2, y2, z2);
+            F2 Na, Nb, Ra, Rb, La, Lb;
+            seg_normal_f2(A3, A2, nx, ny, nz, Na, Nb);
+            seg_normal_f2(A1, A2, nx, ny, nz, Ra, Rb);
+            seg_normal_f2(A3, A0, nx, ny, nz, La, Lb);
+            F2 val = f2_add(f2_sub(f2_add(Ta, Ra), Na), La);
+            val = f2_add(val, f2_add(f2_sub(f2_add(Tb, Rb), Nb), Lb));
             const float* br = a.basis_f2 + (I.basis - a.basis0 + (j - start) * a.N + a.c0) * 2;
 #pragma unroll
-            for (int c = 0; c < WOP_NMAX; c++)
+            for (int c = 0; c < NC; c++)
                 if (c < nco) acc[c] = f2_add(acc[c], f2_mul(val, F2{br[2 * c], br[2 * c + 1]}));
-            A0 = A3, A1 = A2, B0 = B3, B1 = B2;
+            A0 = A3, A1 = A2;
             Ta = Na, Tb = Nb;
         }
     }
-    double* out = a.partial + (((int64_t)blockIdx.z * gridDim.y + blockIdx.y) * npairs + g) * a.N + a.c0;
+    double* out = a.partial + ((slice * gridDim.y + blockIdx.y) * npairs + g) * a.N + a.c0;
 #pragma unroll
-    for (int c = 0; c < WOP_NMAX; c++)
+    for (int c = 0; c < NC; c++)
         if (c < nco) out[c] = f2_dbl(acc[c]);
 }
 
@@ -702,6 +743,7 @@ struct HbState {
     DBuf wop_basis, wop_part, wop_M;
     Buf<float> wop_basis_f2, wop_shift;
     Buf<int64_t> wop_shift_off;
+    Buf<HbSet> set_buf;
     bool wop_valid = false;
     // inputs and outputs of k_hb_loads
     DBuf ld_C, ld_D, ld_DD, ld_T, ld_Td, ld_fs, ld_ra, ld_rb, ld_out;
@@ -783,10 +825,10 @@ struct HbState {
                                          areas.data(), s)))
             return rc;
         GB_CUDA(cudaMemsetAsync(lhs, 0, sizeof(double) * n * n, st));
-        if ((rc = gbvlm_lhs_assemble_f64(lhs, n, nsurf, dims.data(), C(colloc_h).data(), C(normals).data(),
-                                         C(verts).data(), nullptr, 0, 0.0, s)))
+        if ((rc = lhs_assemble_rings_f64(lhs, n, nsurf, dims.data(), C(colloc_h).data(), C(normals).data(),
+                                         C(verts).data(), st)))
             return rc;
-        if ((rc = gbvlm_lu_factor_f64(lu, lhs, n, n, s))) return rc;
+        if ((rc = lu_factor_pivoting_f64(lu, lhs, n, st))) return rc;
         if (n <= HB_INV_MAX) {  // A^-1 from the factors: the identity solved for
             if ((rc = ainv.grow(n * n))) return rc;
             std::vector<double> I((size_t)(n * n), 0.0);
@@ -836,7 +878,8 @@ struct HbState {
             if ((rc = chain_buf.grow(K * cstride))) return rc;
             GB_CUDA(cudaMemcpyAsync(chain_buf.p, chain, sizeof(double) * K * cstride, cudaMemcpyHostToDevice, st));
         }
-        int64_t wo = 0, two = 0;
+        int64_t wo = 0, two = 0, most = 1;
+        std::vector<HbSet> sets(K);
         for (int c = 0; c < K; c++) {
             HbCol& col = cols[c];
             col.max_t = max_t[c];
@@ -845,21 +888,24 @@ struct HbState {
             col.wake.assign(nsurf, nullptr);
             col.wake[wake_surf] = wake_buf.p + wo;
             double* Tall = tw_buf.p + two;
-            if (chain) {
-                k_hb_chain<<<(unsigned)cdiv(col.max_t, 128), 128, 0, st>>>(chain_buf.p + c * cstride, harmonics,
-                                                                          col.max_t, nsurf, wake_surf, Tall);
-                GB_LAUNCH_CHECK();
-            } else {
+            if (!chain)
                 GB_CUDA(cudaMemcpyAsync(Tall, wake_T[c], sizeof(double) * 16 * nsurf * col.max_t,
                                         cudaMemcpyHostToDevice, st));
-            }
-            const int64_t cnt = wn1 * col.max_t;
-            k_pregen_wake<<<(unsigned)cdiv(cnt, 128), 128, 0, st>>>(Tall, nsurf, wake_surf, vinit[wake_surf], W.ns,
-                                                                     W.nc, col.max_t, col.wake[wake_surf]);
-            GB_LAUNCH_CHECK();
+            sets[c] = HbSet{col.max_t, two, wo};
+            most = std::max(most, col.max_t);
             wo += 4 * wn1 * col.max_t;
             two += 16 * nsurf * col.max_t;
         }
+        if ((rc = set_buf.grow(K))) return rc;
+        GB_CUDA(cudaMemcpyAsync(set_buf.p, sets.data(), sizeof(HbSet) * K, cudaMemcpyHostToDevice, st));
+        if (chain) {
+            k_hb_chain<<<dim3((unsigned)cdiv(most, 128), (unsigned)K), 128, 0, st>>>(
+                chain_buf.p, cstride, set_buf.p, harmonics, nsurf, wake_surf, tw_buf.p);
+            GB_LAUNCH_CHECK();
+        }
+        k_pregen_wake<<<dim3((unsigned)cdiv(wn1 * most, 128), (unsigned)K), 128, 0, st>>>(
+            tw_buf.p, set_buf.p, nsurf, wake_surf, vinit[wake_surf], W.ns, W.nc, wake_buf.p);
+        GB_LAUNCH_CHECK();
         // instances
         GB_CUDA(cudaMemcpyAsync(tdev.p, Th, sizeof(double) * ninst * nsurf * 16, cudaMemcpyHostToDevice, st));
         GB_CUDA(cudaMemcpyAsync(tddev.p, Tdh, sizeof(double) * ninst * nsurf * 16, cudaMemcpyHostToDevice, st));
@@ -1003,8 +1049,16 @@ struct HbState {
         a.wshift_off = wop_shift_off.p;
         k_hb_basis<<<dim3((unsigned)cdiv(max_it, 128), (unsigned)ninst), 128, 0, st>>>(a);
         GB_LAUNCH_CHECK();
+        a.slices = zs;
+        const dim3 og((unsigned)cdiv(zs * npairs, WOP_THREADS), (unsigned)ninst);
         for (a.c0 = 0; a.c0 < N; a.c0 += WOP_NMAX) {  // the ring values again for each block of coefficients
-            k_wake_operator<<<dim3((unsigned)xb, (unsigned)ninst, (unsigned)zs), WOP_THREADS, 0, st>>>(a);
+            const int nc = std::min(N - a.c0, WOP_NMAX);
+            if (nc <= 3) k_wake_operator<3><<<og, WOP_THREADS, 0, st>>>(a);
+            else if (nc <= 5) k_wake_operator<5><<<og, WOP_THREADS, 0, st>>>(a);
+            else if (nc <= 7) k_wake_operator<7><<<og, WOP_THREADS, 0, st>>>(a);
+            else if (nc <= 11) k_wake_operator<11><<<og, WOP_THREADS, 0, st>>>(a);
+            else if (nc <= 17) k_wake_operator<17><<<og, WOP_THREADS, 0, st>>>(a);
+            else k_wake_operator<WOP_NMAX><<<og, WOP_THREADS, 0, st>>>(a);
             GB_LAUNCH_CHECK();
         }
         k_wake_operator_sum<<<(unsigned)cdiv(len, 256), 256, 0, st>>>(wop_part.p, zs, len, wop_M.p);

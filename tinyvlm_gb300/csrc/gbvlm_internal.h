@@ -66,6 +66,16 @@ void* host_scratch(size_t bytes);
 // Per-device small device buffer for reductions (grown on demand).
 int device_scratch(size_t bytes, void** out, cudaStream_t s);
 
+// The harmonic-balance solver's AIC and factors.  Its fixed-point iteration ends
+// on a residual, and a rounding in the AIC moves the result by more than what
+// callers compare at, so these keep the order of operations that its
+// results were established with: ring by ring (no wake rows, no core), and the
+// pivoting launches.
+int lhs_assemble_rings_f64(double* lhs, int64_t ld, int32_t nsurf, const gbvlm_dims* dims,
+                           const double* const* colloc, const double* const* normals,
+                           const double* const* verts_wing, cudaStream_t st);
+int lu_factor_pivoting_f64(gbvlm_lu h, double* A, int64_t n, cudaStream_t st);
+
 // ---------------------------------------------------------------------------
 // Launch-only forms of a few operators for code captured into a CUDA graph
 // and replayed at every time step: the step-dependent argument (wake rows,

@@ -376,7 +376,8 @@ __device__ __forceinline__ bool not_above(double x, double d) {
 // column's entry.  The pivot row goes round by shuffles, and rows at or above
 // the pivot take a zero multiplier: no branch, so a step's other columns run
 // beside the next one's chain.
-template <class T, int LDU>
+// EXACT: the reciprocals correctly rounded, as the pivoting loop takes them.
+template <class T, int LDU, bool EXACT>
 __device__ __forceinline__ bool panel_diag(T (&x)[GK], int nb, T* u, T* rds, int lane) {
     using V2 = typename Vec4<T>::type;
     bool good = true;
@@ -385,7 +386,7 @@ __device__ __forceinline__ bool panel_diag(T (&x)[GK], int nb, T* u, T* rds, int
         constexpr int jj = decltype(JJ)::value;
         if (jj < nb) {
             const T d = __shfl_sync(0xffffffffu, x[jj], jj);
-            const T rd = pivot_rcp(d);
+            const T rd = EXACT ? rcp_rn(d) : pivot_rcp(d);
             const bool under = lane > jj;  // rows past nb hold zeros
             good = good && pivot_fits(d) && (!under || not_above(x[jj], d));
             const T lm = under ? x[jj] * rd : (T)0;
@@ -532,7 +533,7 @@ __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const
             const bool first = tid < 32;  // the slice's first warp factors the diagonal block
             if (first) {
                 if (rank != 0) load_row(lane, lane < nb);  // rank 0's first warp holds those rows
-                good = panel_diag<T, GK>(x[0], nb, &fu[0][0], frd, lane);
+                good = panel_diag<T, GK, true>(x[0], nb, &fu[0][0], frd, lane);
                 if (rank != 0) load_row(lid[0], lid[0] >= 0);
                 if (lane == 0) sm.f_bad[slice] = good ? 0 : 1;
             }
@@ -802,7 +803,7 @@ __global__ void __launch_bounds__(Fast<float>::DT) k_lu_diag(LuBatch<float> B, i
             for (int e = 0; e < 4; e++) x[t + e] = v[e];
         }
         __syncwarp();
-        const bool good = panel_diag<float, LD>(x, GK, D, rds + GK * c, lane);
+        const bool good = panel_diag<float, LD, false>(x, GK, D, rds + GK * c, lane);
         if (!good && lane == 0) s_bad = 1;
 #pragma unroll
         for (int t = 0; t < GK; t++) LT[t * GK + lane] = x[t];
@@ -1101,11 +1102,12 @@ __global__ void __launch_bounds__(Fast<float>::RT) k_lu_rows_split(LuBatch<float
     }
 }
 
-// Double: 32-column blocks.  A sub-partition issues half an fp64 lane per
-// cycle, so a warp's fp64 instruction takes 64 cycles: the columns are dealt out to
+// Double: 32-column blocks.  A warp's fp64 instruction takes a sub-partition
+// about 100 cycles: the columns are dealt out to
 // four warps (column t to warp t mod 4, a lane per row), one per sub-partition,
-// and a column's multipliers go round through shared memory.  (One warp per 32
-// rows: the block 39 us, 32 rows against it 26 us; four: see below.)
+// and a column's multipliers go round through shared memory: the block 14.7 us,
+// 32 rows against it 10.2 us (one warp: 39 and 26; one warp with eight rows and
+// every fourth column to a lane: 14.9 and 10.2, and the whole solve slower).
 __device__ __forceinline__ const double* fast64_work(const double* work, int32_t i) {
     return work + (int64_t)i * Fast<double>::WORK;
 }
@@ -3887,7 +3889,7 @@ static bool lu_backup(gbvlm_lu h, const T* A, int64_t n, int64_t ld, cudaStream_
 }
 
 template <class T>
-static int lu_factor_one(gbvlm_lu h, T* A, int64_t n, int64_t ld, cudaStream_t st) {
+static int lu_factor_one(gbvlm_lu h, T* A, int64_t n, int64_t ld, cudaStream_t st, bool pivot = false) {
     GB_REQUIRE(h && A && n >= 1 && ld >= n, "bad LU arguments");
     int rc = lu_ensure(h, n, st);
     if (rc) return rc;
@@ -3899,7 +3901,8 @@ static int lu_factor_one(gbvlm_lu h, T* A, int64_t n, int64_t ld, cudaStream_t s
     int32_t* hi = (int32_t*)host_scratch(2 * sizeof(int32_t));
     bool done = false;
     // without interchanges first; single-block systems' panel tries that itself
-    const bool fast = (sizeof(T) == 4 ? h->plan.fast : h->plan.fast_any) && n > GK && lu_backup<T>(h, A, n, ld, st);
+    const bool fast =
+        !pivot && (sizeof(T) == 4 ? h->plan.fast : h->plan.fast_any) && n > GK && lu_backup<T>(h, A, n, ld, st);
     if (fast) {
         GB_CUDA(cudaMemsetAsync(h->d_info + 1, 0, sizeof(int32_t), st));
         B.fail = h->d_info + 1;
@@ -3947,6 +3950,10 @@ static int lu_solve_one(gbvlm_lu h, const T* A, int64_t n, int64_t ld, T* X, int
 }
 
 namespace gbvlm {
+
+int lu_factor_pivoting_f64(gbvlm_lu h, double* A, int64_t n, cudaStream_t st) {
+    return lu_factor_one<double>(h, A, n, n, st, true);
+}
 
 struct LuSolveTables {
     LuBatch<float> B;

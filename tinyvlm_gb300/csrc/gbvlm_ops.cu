@@ -313,6 +313,62 @@ static int lhs_assemble(T* lhs, int64_t ld, int32_t nsurf, const gbvlm_dims* dim
     return GBVLM_OK;
 }
 
+// The same AIC ring by ring, for the harmonic-balance solver
+// (gbvlm_internal.h): block = 128 collocation points x one ring row in chunks of
+// 256 rings; along the span a thread keeps the left vertex terms and the left
+// chordwise segment of the previous ring.
+constexpr int LHR_THREADS = 128, LHR_SPAN = 256;
+
+__global__ void __launch_bounds__(LHR_THREADS) k_lhs_rings(LhsPair<double> a) {
+    constexpr int W = LHR_SPAN + 1;
+    __shared__ double sv[6 * W];
+    const int64_t c = blockIdx.y, s0 = (int64_t)blockIdx.z * LHR_SPAN;
+    const int nv = (int)(min(s0 + (int64_t)LHR_SPAN, a.ns) - s0 + 1);
+    const int64_t vld = (a.ns + 1) * (a.nc + 1);
+    for (int t = threadIdx.x; t < 2 * nv; t += LHR_THREADS) {
+        const int r = t / nv, sl = t - r * nv;
+        const int64_t vi = (s0 + sl) + (c + r) * (a.ns + 1);
+        for (int k = 0; k < 3; k++) sv[(r * 3 + k) * W + sl] = a.vw[k * vld + vi];
+    }
+    __syncthreads();
+    const int64_t i = (int64_t)blockIdx.x * LHR_THREADS + threadIdx.x;
+    if (i >= a.np_i) return;
+    const double px = a.colloc[i], py = a.colloc[a.np_i + i], pz = a.colloc[2 * a.np_i + i];
+    const double nx = a.normals[i], ny = a.normals[a.np_i + i], nz = a.normals[2 * a.np_i + i];
+    double* out = a.lhs + (a.row_off + i) + (a.col_off + c * a.ns) * a.ld;
+    strip_normal<double, false>(sv, sv + 3 * W, W, nv, px, py, pz, nx, ny, nz, 0.0, [&](int k, double val) {
+        out[(s0 + k) * a.ld] += val * inv_four_pi<double>();
+    });
+}
+
+int lhs_assemble_rings_f64(double* lhs, int64_t ld, int32_t nsurf, const gbvlm_dims* dims,
+                           const double* const* colloc, const double* const* normals,
+                           const double* const* verts_wing, cudaStream_t st) {
+    Surfs<double> s;
+    int rc = make_surfs(s, nsurf, dims);
+    if (rc) return rc;
+    GB_REQUIRE(lhs && ld >= s.poff[nsurf], "bad lhs");
+    for (int mj = 0; mj < nsurf; mj++)
+        for (int mi = 0; mi < nsurf; mi++) {
+            LhsPair<double> a = {};
+            a.lhs = lhs;
+            a.ld = ld;
+            a.colloc = colloc[mi];
+            a.normals = normals[mi];
+            a.np_i = s.ns[mi] * s.nc[mi];
+            a.vw = verts_wing[mj];
+            a.ns = s.ns[mj];
+            a.nc = s.nc[mj];
+            a.row_off = s.poff[mi];
+            a.col_off = s.poff[mj];
+            k_lhs_rings<<<dim3((unsigned)cdiv(a.np_i, (int64_t)LHR_THREADS), (unsigned)a.nc,
+                               (unsigned)cdiv(a.ns, (int64_t)LHR_SPAN)),
+                          LHR_THREADS, 0, st>>>(a);
+            GB_LAUNCH_CHECK();
+        }
+    return GBVLM_OK;
+}
+
 // ---------------------------------------------------------------------------
 // a2: rhs += -(V . n) (vlm_backend_cpu.cpp:156-179)
 // ---------------------------------------------------------------------------
