@@ -97,13 +97,6 @@ int wake_influence_dev_f32(float* rhs, int32_t nsurf, const gbvlm_dims* dims, co
                            const float* const* colloc, const float* const* normals, const float* const* verts_wake,
                            const int32_t* lifting, const int64_t* it_dev, int32_t it_max, float* scratch,
                            cudaStream_t st);
-// wake row nwv - 1 - *it_dev <- the wing's trailing-edge row
-int wake_shed_dev_f32(int32_t nsurf, const gbvlm_dims* dims, const float* const* verts_wing, float* const* verts_wake,
-                      const int64_t* it_dev, cudaStream_t st);
-// gbvlm_gamma_update_f32 with the wake column col_base - *it_dev
-int gamma_update_dev_f32(int64_t ns, int64_t nc, const float* x, float* gamma, float* gamma_delta, float* gamma_wake,
-                         int64_t col_base, const int64_t* it_dev, const float* gamma_prev, float* dgamma_dt, float dt,
-                         cudaStream_t st);
 // gbvlm_newmark_step with v_i = v + ndof * (*i_dev), a_i = a + ndof * (*i_dev)
 int newmark_step_dev(gbvlm_newmark h, const double* M, const double* C, const double* v, const double* a,
                      const int64_t* i_dev, double* du, double* dv, double* da, const double* delta_F, double dt,

@@ -963,41 +963,6 @@ __global__ void k_gamma_update(int64_t ns, int64_t nc, const T* x, T* g, T* gd, 
     if (dgdt) dgdt[p] = (v - gp[p]) * inv_dt;
 }
 
-// the same two with the iteration read on the device (graph replay)
-template <class T>
-__global__ void k_wake_shed_dev(Surfs<T> s, const int64_t* it_dev) {
-    int64_t g = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    int m = 0;
-    int64_t base = 0;
-    while (m < s.n) {
-        int64_t cnt = 4 * (s.ns[m] + 1);
-        if (g < base + cnt) break;
-        base += cnt;
-        m++;
-    }
-    if (m >= s.n) return;
-    const int64_t it = *it_dev;
-    if (it < 0 || it >= s.nwv[m]) return;
-    int64_t r = g - base, n = s.ns[m] + 1;
-    int64_t k = r / n, i = r % n;
-    int64_t vld = n * (s.nc[m] + 1), kld = n * s.nwv[m];
-    s.o0[m][k * kld + i + (s.nwv[m] - 1 - it) * n] = s.a[m][k * vld + i + s.nc[m] * n];
-}
-
-template <class T>
-__global__ void k_gamma_update_dev(int64_t ns, int64_t nc, const T* x, T* g, T* gd, T* gw, int64_t col_base,
-                                   const int64_t* it_dev, const T* gp, T* dgdt, T inv_dt, int64_t ncols) {
-    int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= ns * nc) return;
-    int64_t i = p % ns, j = p / ns;
-    T v = x[p];
-    g[p] = v;
-    gd[p] = (j > 0) ? v - x[p - ns] : v;
-    const int64_t wcol = col_base - *it_dev;
-    if (gw && j == nc - 1 && wcol >= 0 && wcol < ncols) gw[i + wcol * ns] = v;
-    if (dgdt) dgdt[p] = (v - gp[p]) * inv_dt;
-}
-
 // ---------------------------------------------------------------------------
 // Trefftz-plane drag (ispc:273-323): one block per spanwise ring
 // ---------------------------------------------------------------------------
@@ -1114,35 +1079,6 @@ int wake_influence_dev_f32(float* rhs, int32_t nsurf, const gbvlm_dims* dims, co
     for (int m = 0; m < nsurf; m++) ntg += dims[m].ns * dims[m].nc;
     return wake_influence<float>(rhs, nsurf, dims, gamma_wake, colloc, normals, verts_wake, lifting, it_max, 0.f, 5000,
                                  scratch, (size_t)(WAKE_DEV_MAX_SLICES * ntg), st, it_dev);
-}
-
-int wake_shed_dev_f32(int32_t nsurf, const gbvlm_dims* dims, const float* const* verts_wing, float* const* verts_wake,
-                      const int64_t* it_dev, cudaStream_t st) {
-    Surfs<float> s;
-    int rc = make_surfs(s, nsurf, dims);
-    if (rc) return rc;
-    int64_t total = 0;
-    for (int m = 0; m < nsurf; m++) {
-        GB_REQUIRE(verts_wing[m] && verts_wake[m], "null pointer surface %d", m);
-        s.a[m] = verts_wing[m];
-        s.o0[m] = verts_wake[m];
-        total += 4 * (dims[m].ns + 1);
-    }
-    k_wake_shed_dev<float><<<(unsigned)cdiv(total, 256), 256, 0, st>>>(s, it_dev);
-    GB_LAUNCH_CHECK();
-    return GBVLM_OK;
-}
-
-int gamma_update_dev_f32(int64_t ns, int64_t nc, const float* x, float* gamma, float* gamma_delta, float* gamma_wake,
-                         int64_t col_base, const int64_t* it_dev, const float* gamma_prev, float* dgamma_dt, float dt,
-                         cudaStream_t st) {
-    GB_REQUIRE(ns >= 1 && nc >= 1 && x && gamma && gamma_delta && it_dev, "bad arguments");
-    GB_REQUIRE(!dgamma_dt || (gamma_prev && dt != 0.f), "dgamma_dt needs gamma_prev and dt != 0");
-    k_gamma_update_dev<float><<<(unsigned)cdiv(ns * nc, 256), 256, 0, st>>>(
-        ns, nc, x, gamma, gamma_delta, gamma_wake, col_base, it_dev, gamma_prev, dgamma_dt, dgamma_dt ? 1.f / dt : 0.f,
-        col_base + 1);
-    GB_LAUNCH_CHECK();
-    return GBVLM_OK;
 }
 
 }  // namespace gbvlm

@@ -28,94 +28,311 @@
 
 namespace gbvlm {
 
+// ---------------------------------------------------------------------------
+// The elementwise parts of a time step, three launches per step whatever the
+// number of surfaces (they were about ten, each of one or two microseconds of
+// work and as much again of launch):
+//   k_step_start  wake shed, panel velocities, the kinematic right-hand side;
+//   k_step_loads  circulation, forces, CL and CM of the solution;
+//   k_step_move   wing to its next pose, panel metrics.
+// The step index is `step`, or idx[0] when idx is set (graphs replayed for any
+// step).  by_step: the transforms, free streams, moment points and records are
+// indexed by the step; otherwise they are the caller's current ones.
+// ---------------------------------------------------------------------------
 template <class T>
-__global__ void k_dual_velocity(const T* Td, const T* c0, T* vel, int64_t np) {
-    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= np) return;
-    const T x = c0[p], y = c0[np + p], z = c0[2 * np + p];
-    // -(dT/dt) [x y z 1], column-major 4x4
-    for (int r = 0; r < 3; r++) vel[r * np + p] = -(Td[r] * x + Td[r + 4] * y + Td[r + 8] * z + Td[r + 12]);
-}
-
-// Multibody CL and CM of one step (vlm/src/vlm_backend.cpp:72-139) in
-// double, written to out[0] (cl) and out[1..3] (cm).  One block.
-template <class T>
-struct CoefArgs {
-    int32_t n;
+struct StepArgs {
+    int32_t n = 0;
     int64_t ns[GBVLM_MAX_SURFACES], nc[GBVLM_MAX_SURFACES];
-    const T* forces[GBVLM_MAX_SURFACES];
-    const T* verts[GBVLM_MAX_SURFACES];
-    const T* areas[GBVLM_MAX_SURFACES];
+    int64_t poff[GBVLM_MAX_SURFACES + 1];  // first panel of each surface
+    const T* vpos[GBVLM_MAX_SURFACES];     // vertices that the transforms move
+    const T* colloc0[GBVLM_MAX_SURFACES];  // collocation points that the velocities belong to
+    T *verts[GBVLM_MAX_SURFACES], *wake[GBVLM_MAX_SURFACES], *vel[GBVLM_MAX_SURFACES], *colloc[GBVLM_MAX_SURFACES],
+        *normals[GBVLM_MAX_SURFACES], *areas[GBVLM_MAX_SURFACES], *gamma[GBVLM_MAX_SURFACES],
+        *gprev[GBVLM_MAX_SURFACES], *gwake[GBVLM_MAX_SURFACES];
+    int64_t nwv = 0;                        // wake vertex rows
+    T* rhs = nullptr;                       // right-hand side, then the solution
+    const T *Tm = nullptr, *Tdm = nullptr;  // [step][surface][16] column-major
+    const T *fs = nullptr, *ref = nullptr;  // [step][3]
+    double* out = nullptr;                  // [step][4]: CL, CM
+    T inv_dt = 0;
+    double rho = 1;
+    double* part = nullptr;    // [step_load_blocks][6]
+    unsigned* done = nullptr;  // blocks finished, zero between launches
+    const int64_t* idx = nullptr;
+    bool by_step = true;
+    bool keep = true;   // gprev = gamma after use
+    bool flap = false;  // the second surface's leading row carries the first's trailing-edge circulation off
+
+    __device__ __forceinline__ int64_t at(int64_t step) const { return idx ? idx[0] : step; }
+    __device__ __forceinline__ int surf(int64_t g) const {
+        int m = 0;
+        while (m + 1 < n && g >= poff[m + 1]) m++;
+        return m;
+    }
 };
 
-__device__ double blk_sum(double v, double* sh) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[wid] = v;
-    __syncthreads();
-    double r = 0;
-    for (int k = 0; k < (int)(blockDim.x >> 5); k++) r += sh[k];
-    return r;
+constexpr int STEP_THREADS = 128;
+constexpr int STEP_CHORDS = STEP_THREADS - 1;  // strips of a chord block (a strip needs two chords)
+
+template <class T>
+static void step_dims(StepArgs<T>& a, const std::vector<gbvlm_dims>& dims) {
+    a.n = (int32_t)dims.size();
+    a.poff[0] = 0;
+    for (int m = 0; m < a.n; m++) {
+        a.ns[m] = dims[m].ns;
+        a.nc[m] = dims[m].nc;
+        a.poff[m + 1] = a.poff[m] + dims[m].ns * dims[m].nc;
+    }
+}
+
+static int64_t step_load_blocks(const std::vector<gbvlm_dims>& dims) {
+    int64_t b = 0;
+    for (auto& d : dims) b += cdiv(d.ns * d.nc, STEP_THREADS) + cdiv(d.ns, STEP_CHORDS);
+    return b;
 }
 
 template <class T>
-__global__ void __launch_bounds__(512) k_step_coeffs(CoefArgs<T> a, const T* fs_all, const T* ref_all, int64_t step,
-                                                    double rho, double* out) {
-    __shared__ double sh[32];
-    const T* fsp = fs_all + 3 * step;
-    const T* rp = ref_all + 3 * step;
-    const double fx = fsp[0], fy = fsp[1], fz = fsp[2];
-    double lx = -fz, lz = fx;
-    const double ll = sqrt(lx * lx + lz * lz);
-    lx /= ll;
-    lz /= ll;
-    const double v2 = fx * fx + fy * fy + fz * fz;
-    double cl = 0, ta = 0, tm = 0, cm[3] = {0, 0, 0};
-    for (int m = 0; m < a.n; m++) {
-        const int64_t ns = a.ns[m], nc = a.nc[m], np = ns * nc, vld = (ns + 1) * (nc + 1);
-        const T* F = a.forces[m];
-        const T* v = a.verts[m];
-        CSum sl, sa, sx, sy, sz, smac;
-        for (int64_t p = threadIdx.x; p < np; p += blockDim.x) {
-            const int64_t i = p % ns, j = p / ns, ia = i + j * (ns + 1), ib = ia + 1;
-            const double Fx = F[p], Fy = F[np + p], Fz = F[2 * np + p];
-            sl.add(Fx * lx + Fz * lz);
-            sa.add((double)a.areas[m][p]);
-            const double ex = 0.5 * ((double)v[ia] + v[ib]) - rp[0];
-            const double ey = 0.5 * ((double)v[vld + ia] + v[vld + ib]) - rp[1];
-            const double ez = 0.5 * ((double)v[2 * vld + ia] + v[2 * vld + ib]) - rp[2];
-            sx.add(ey * Fz - ez * Fy);
-            sy.add(ez * Fx - ex * Fz);
-            sz.add(ex * Fy - ey * Fx);
+__global__ void __launch_bounds__(STEP_THREADS) k_step_start(StepArgs<T> a, int64_t step) {
+    const int64_t i = a.at(step), g = blockIdx.x * (int64_t)STEP_THREADS + threadIdx.x;
+    const T* Tdm = a.Tdm + (a.by_step ? 16 * a.n * i : 0);
+    if (g < a.poff[a.n]) {
+        const int m = a.surf(g);
+        const int64_t p = g - a.poff[m], np = a.ns[m] * a.nc[m];
+        const T *c0 = a.colloc0[m], *n = a.normals[m], *Td = Tdm + 16 * m;
+        T* vel = a.vel[m];
+        const T x = c0[p], y = c0[np + p], z = c0[2 * np + p];
+        T v[3];
+        // -(dT/dt) [x y z 1]
+#pragma unroll
+        for (int r = 0; r < 3; r++) {
+            v[r] = -(Td[r] * x + Td[r + 4] * y + Td[r + 8] * z + Td[r + 12]);
+            vel[r * np + p] = v[r];
         }
-        const int64_t last = nc * (ns + 1);
-        for (int64_t i = threadIdx.x; i < ns; i += blockDim.x) {
-            auto chord = [&](int64_t q) {
-                const double dx = (double)v[q] - v[last + q], dy = (double)v[vld + q] - v[vld + last + q];
-                const double dz = (double)v[2 * vld + q] - v[2 * vld + last + q];
-                return sqrt(dx * dx + dy * dy + dz * dz);
-            };
-            const double c0 = chord(i), c1 = chord(i + 1);
+        a.rhs[g] = (T)0 + -(v[0] * n[p] + v[1] * n[np + p] + v[2] * n[2 * np + p]);
+        return;
+    }
+    // trailing edge to wake row i
+    int64_t r = g - a.poff[a.n];
+    for (int m = 0; m < a.n; m++) {
+        const int64_t nv = a.ns[m] + 1;
+        if (r < 4 * nv) {
+            const int64_t k = r / nv, q = r - k * nv;
+            if (i >= 0 && i < a.nwv)
+                a.wake[m][k * nv * a.nwv + q + (a.nwv - 1 - i) * nv] =
+                    a.verts[m][k * nv * (a.nc[m] + 1) + q + a.nc[m] * nv];
+            return;
+        }
+        r -= 4 * nv;
+    }
+}
+
+// verts = T vpos and the metrics of the moved panels (k_displace, then
+// k_mesh_metrics with the collocation point at 3/4 chord): a panel's thread
+// moves its four corners and writes the one at its origin, the last strip and
+// row those beyond.
+template <class T>
+__global__ void __launch_bounds__(STEP_THREADS) k_step_move(StepArgs<T> a, int64_t step) {
+    const int64_t g = blockIdx.x * (int64_t)STEP_THREADS + threadIdx.x;
+    if (g >= a.poff[a.n]) return;
+    const int m = a.surf(g);
+    const T* tr = a.Tm + (a.by_step ? 16 * a.n * (a.at(step) + 1) : 0) + 16 * m;
+    const int64_t p = g - a.poff[m], ns = a.ns[m], nc = a.nc[m], np = ns * nc, vld = (ns + 1) * (nc + 1);
+    const int64_t j = p / ns, i = p - j * ns, v = i + j * (ns + 1);
+    const T* in = a.vpos[m];
+    T* out = a.verts[m];
+    auto move = [&](int64_t q, bool write) {
+        T x[4] = {in[q], in[vld + q], in[2 * vld + q], in[3 * vld + q]}, y[4];
+#pragma unroll
+        for (int c = 0; c < 4; c++) {
+            T acc = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) acc += x[k] * tr[c + 4 * k];
+            y[c] = acc;
+            if (write) out[c * vld + q] = acc;
+        }
+        return V3<T>{y[0], y[1], y[2]};
+    };
+    const bool lc = i == ns - 1, lr = j == nc - 1;
+    const V3<T> v0 = move(v, true), v1 = move(v + 1, lc), v2 = move(v + ns + 2, lc && lr), v3_ = move(v + ns + 1, lr);
+    const V3<T> nn = cross(v3_ - v1, v2 - v0);
+    const T l = dsqrt(len2(nn));
+    T *col = a.colloc[m], *nor = a.normals[m];
+    nor[p] = nn.x / l;
+    nor[np + p] = nn.y / l;
+    nor[2 * np + p] = nn.z / l;
+    const V3<T> f = v3_ - v0, bb = v2 - v0, e = v1 - v0;
+    a.areas[m][p] = (T)0.5 * (dsqrt(len2(cross(f, bb))) + dsqrt(len2(cross(bb, e))));
+    const V3<T> ch = (T)0.5 * (((v2 + v3_) - v0) - v1);
+    const V3<T> cp = (T)0.5 * (v0 + v1) + (T)0.5 * ch;
+    col[p] = cp.x;
+    col[np + p] = cp.y;
+    col[2 * np + p] = cp.z;
+}
+
+// Circulation of the solution (gamma, the trailing edge's into the wake), with
+// `loads` the unsteady forces (vlm_backend_cpu.cpp:276-321) and the multibody
+// CL and CM about ref (vlm/src/vlm_backend.cpp:72-139): the sums in double,
+// out[0] cl and out[1..3] cm.
+//
+// Bound: latency.  A warp's double instruction takes about 100 cycles on this
+// device, so what a block does in double is kept short: one panel per thread,
+// six sums of a block's panels through shared memory (8 additions and 4
+// exchanges on three warps where six warp-wide trees spend 30), blocks of their
+// own for the chords (three square roots a strip), and the block that finishes
+// last adds the blocks' sums in a fixed order and forms the coefficients.  The
+// sums over all panels in a single block took 70 us a step for 1600 panels.
+template <class T>
+__global__ void __launch_bounds__(STEP_THREADS) k_step_loads(StepArgs<T> a, int64_t step, bool loads) {
+    __shared__ double sh[6][STEP_THREADS];
+    __shared__ double tot[6];
+    __shared__ bool last;
+    const int64_t it = a.at(step), o = a.by_step ? it : 0;
+    const int t = threadIdx.x;
+    const T *fsp = a.fs + 3 * o, *rp = a.ref + 3 * o;
+    int64_t blk = blockIdx.x;
+    int m = 0;
+    bool chords = false;
+    for (; m < a.n; m++) {
+        const int64_t pb = (a.ns[m] * a.nc[m] + STEP_THREADS - 1) / STEP_THREADS;
+        const int64_t cb = loads ? (a.ns[m] + STEP_CHORDS - 1) / STEP_CHORDS : 0;
+        if (blk < pb) break;
+        blk -= pb;
+        if (blk < cb) {
+            chords = true;
+            break;
+        }
+        blk -= cb;
+    }
+    const int64_t ns = a.ns[m], nc = a.nc[m], np = ns * nc, vld = (ns + 1) * (nc + 1);
+    const T* v = a.verts[m];
+    if (!chords) {
+        const int64_t p = blk * STEP_THREADS + t;
+        double s[5] = {0, 0, 0, 0, 0};
+        if (p < np) {
+            const int64_t j = p / ns, i = p - j * ns;
+            const T* x = a.rhs + a.poff[m];
+            const T g = x[p];
+            a.gamma[m][p] = g;
+            const int64_t wcol = a.nwv - 2 - it;
+            if (j == nc - 1 && wcol >= 0 && wcol < a.nwv - 1) a.gwake[m][i + wcol * ns] = g;
+            if (loads) {
+                T gd = (j > 0) ? g - x[p - ns] : g;
+                // the reference's wing-flap coupling (uvlm_2dof.cpp:578-584)
+                if (a.flap && m == 1 && j == 0) gd -= a.rhs[a.poff[0] + i + (a.nc[0] - 1) * a.ns[0]];
+                const T dg = (g - a.gprev[m][p]) * a.inv_dt;
+                const T *vel = a.vel[m], *nor = a.normals[m];
+                const T area = a.areas[m][p], rho = 1;
+                const int64_t ia = i + j * (ns + 1), ib = ia + 1;
+                const V3<T> V{vel[p], vel[np + p], vel[2 * np + p]}, n{nor[p], nor[np + p], nor[2 * np + p]};
+                const V3<T> v0{v[ia], v[vld + ia], v[2 * vld + ia]}, v1{v[ib], v[vld + ib], v[2 * vld + ib]};
+                V3<T> F = (rho * gd) * cross(V, v1 - v0);
+                F = F + (rho * dg * area) * n;
+                const double Fx = F.x, Fy = F.y, Fz = F.z;
+                const double ex = 0.5 * ((double)v0.x + v1.x) - rp[0];
+                const double ey = 0.5 * ((double)v0.y + v1.y) - rp[1];
+                const double ez = 0.5 * ((double)v0.z + v1.z) - rp[2];
+                s[0] = Fz * fsp[0] - Fx * fsp[2];  // lift times the length of (-fz, fx)
+                s[1] = area;
+                s[2] = ey * Fz - ez * Fy;
+                s[3] = ez * Fx - ex * Fz;
+                s[4] = ex * Fy - ey * Fx;
+            }
+            if (a.keep) a.gprev[m][p] = g;
+        }
+#pragma unroll
+        for (int q = 0; q < 5; q++) sh[q][t] = s[q];
+    } else {
+        const int64_t i = blk * STEP_CHORDS + t, end = nc * (ns + 1);
+        double c = 0;
+        if (i <= ns) {
+            const double dx = (double)v[i] - v[end + i], dy = (double)v[vld + i] - v[vld + end + i];
+            const double dz = (double)v[2 * vld + i] - v[2 * vld + end + i];
+            c = dx * dx + dy * dy + dz * dz;
+        }
+        sh[1][t] = sqrt(c);
+        __syncthreads();
+        double s = 0;
+        if (t < STEP_CHORDS && i < ns) {
+            const double c0 = sh[1][t], c1 = sh[1][t + 1];
             const double dx = (double)v[i + 1] - v[i], dy = (double)v[vld + i + 1] - v[vld + i];
             const double dz = (double)v[2 * vld + i + 1] - v[2 * vld + i];
-            smac.add(0.5 * (c0 * c0 + c1 * c1) * sqrt(dx * dx + dy * dy + dz * dz));
+            s = 0.5 * (c0 * c0 + c1 * c1) * sqrt(dx * dx + dy * dy + dz * dz);
         }
-        const double L = blk_sum(sl.value(), sh), S = blk_sum(sa.value(), sh);
-        const double Mx = blk_sum(sx.value(), sh), My = blk_sum(sy.value(), sh), Mz = blk_sum(sz.value(), sh);
-        const double mac = blk_sum(smac.value(), sh) / S;
-        const double q = 0.5 * rho * v2;
-        cl += L / (q * S) * S;
-        cm[0] += Mx / (q * S * mac) * S * mac;
-        cm[1] += My / (q * S * mac) * S * mac;
-        cm[2] += Mz / (q * S * mac) * S * mac;
-        ta += S;
-        tm += mac;
+        sh[0][t] = s;
     }
-    if (threadIdx.x == 0) {
-        out[0] = cl / ta;
-        for (int k = 0; k < 3; k++) out[1 + k] = cm[k] / (ta * tm);
+    if (!loads) return;
+    __syncthreads();
+    const int q = t >> 4, l = t & 15;  // 16 lanes per sum
+    auto lanes = [&](double x) {
+#pragma unroll
+        for (int d = 8; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
+        return x;
+    };
+    if (t < 96) {
+        double x = 0;
+        if (q < (chords ? 1 : 5)) {
+#pragma unroll
+            for (int k = 0; k < STEP_THREADS / 16; k++) x += sh[q][l + 16 * k];
+        }
+        x = lanes(x);
+        if (l == 0) a.part[6 * (int64_t)blockIdx.x + q] = x;
     }
+    __threadfence();
+    __syncthreads();
+    if (t == 0) last = atomicInc(a.done, gridDim.x - 1) == gridDim.x - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double cl = 0, ta = 0, tm = 0;  // of thread t < 4: CL, CM x, y, z
+    const double fx = fsp[0], fy = fsp[1], fz = fsp[2];
+    const double qd = 0.5 * a.rho * (fx * fx + fy * fy + fz * fz), ll = sqrt(fz * fz + fx * fx);
+    int64_t b0 = 0;
+    for (int k = 0; k < a.n; k++) {
+        const int64_t pb = (a.ns[k] * a.nc[k] + STEP_THREADS - 1) / STEP_THREADS;
+        const int64_t cb = (a.ns[k] + STEP_CHORDS - 1) / STEP_CHORDS;
+        if (t < 96) {
+            CSum s;
+            // sum q of the panel blocks; the sixth: the chord blocks' strips
+            const int64_t first = b0 + (q < 5 ? 0 : pb), cnt = q < 5 ? pb : cb;
+            for (int64_t e = l; e < cnt; e += 16) s.add(__ldcg(a.part + 6 * (first + e) + (q < 5 ? q : 0)));
+            const double x = lanes(s.value());
+            if (l == 0) tot[q] = x;
+        }
+        __syncthreads();
+        if (t < 4) {
+            const double S = tot[1], mac = tot[5] / S;
+            cl += t == 0 ? tot[0] / ll / (qd * S) * S : tot[1 + t] / (qd * S * mac) * S * mac;
+            ta += S;
+            tm += mac;
+        }
+        __syncthreads();
+        b0 += pb + cb;
+    }
+    if (t < 4) a.out[4 * o + t] = t == 0 ? cl / ta : cl / (ta * tm);
+}
+
+template <class T>
+static int step_start(const StepArgs<T>& a, int64_t step, cudaStream_t st) {
+    int64_t n = a.poff[a.n];
+    for (int m = 0; m < a.n; m++) n += 4 * (a.ns[m] + 1);
+    k_step_start<T><<<(unsigned)cdiv(n, STEP_THREADS), STEP_THREADS, 0, st>>>(a, step);
+    GB_LAUNCH_CHECK();
+    return GBVLM_OK;
+}
+template <class T>
+static int step_move(const StepArgs<T>& a, int64_t step, cudaStream_t st) {
+    k_step_move<T><<<(unsigned)cdiv(a.poff[a.n], STEP_THREADS), STEP_THREADS, 0, st>>>(a, step);
+    GB_LAUNCH_CHECK();
+    return GBVLM_OK;
+}
+template <class T>
+static int step_loads(const StepArgs<T>& a, int64_t step, bool loads, cudaStream_t st) {
+    int64_t blocks = 0;
+    for (int m = 0; m < a.n; m++)
+        blocks += cdiv(a.ns[m] * a.nc[m], STEP_THREADS) + (loads ? cdiv(a.ns[m], STEP_CHORDS) : 0);
+    k_step_loads<T><<<(unsigned)blocks, STEP_THREADS, 0, st>>>(a, step, loads);
+    GB_LAUNCH_CHECK();
+    return GBVLM_OK;
 }
 
 template <class T>
@@ -135,14 +352,6 @@ struct Ops2;
                             gbvlm_stream s) {                                                                       \
             return gbvlm_displace_wing_##sfx(ns, d, t, v, vi, s);                                                  \
         }                                                                                                           \
-        static int shed(int32_t ns, const gbvlm_dims* d, const T* const* v, T* const* k, int32_t it,                \
-                        gbvlm_stream s) {                                                                           \
-            return gbvlm_wake_shed_##sfx(ns, d, v, k, it, s);                                                      \
-        }                                                                                                           \
-        static int rhsv(T* r, int32_t ns, const gbvlm_dims* d, const T* const* n, const T* const* v,                \
-                        gbvlm_stream s) {                                                                           \
-            return gbvlm_rhs_assemble_velocities_##sfx(r, ns, d, n, v, s);                                         \
-        }                                                                                                           \
         static int wake(T* r, int32_t ns, const gbvlm_dims* d, const T* const* g, const T* const* c,                \
                         const T* const* n, const T* const* k, const int32_t* lf, int32_t it, T sg, gbvlm_stream s) { \
             return gbvlm_rhs_assemble_wake_influence_##sfx(r, ns, d, g, c, n, k, lf, it, sg, s);                   \
@@ -155,43 +364,14 @@ struct Ops2;
         static int solve(gbvlm_lu h, const T* a, int64_t n, T* x, gbvlm_stream s) {                                 \
             return gbvlm_lu_solve_##sfx(h, a, n, n, x, n, 1, s);                                                    \
         }                                                                                                           \
-        static int gupd(int64_t ns, int64_t nc, const T* x, T* g, T* gd, T* gw, int64_t col, const T* gp, T* dg,    \
-                        T dt, gbvlm_stream s) {                                                                     \
-            return gbvlm_gamma_update_##sfx(ns, nc, x, g, gd, gw, col, gp, dg, dt, s);                              \
-        }                                                                                                           \
-        static int forces(int64_t ns, int64_t nc, const T* v, const T* gd, const T* dg, const T* vel, const T* ar,  \
-                          const T* nr, T* f, gbvlm_stream s) {                                                      \
-            return gbvlm_forces_unsteady_##sfx(ns, nc, v, gd, dg, vel, ar, nr, f, s);                              \
-        }                                                                                                           \
     };
 OPS2(float, f32)
 OPS2(double, f64)
 
 // Device-indexed UVLM step (float, no roll-up): the step index i lives in
-// idx[0] on the device.  The pose kernel stages T(i+1) and Td(i) of every
-// surface and the step's free stream and moment point into fixed buffers,
-// so one captured graph advances the case any number of times.
-template <class T>
-__global__ void k_uvlm_dev_pose(const int64_t* idx, const T* Tm, const T* Tdm, const T* fs, const T* ref, int nsurf,
-                                T* pose) {
-    const int64_t i = idx[0];
-    for (int q = threadIdx.x; q < 16 * nsurf; q += blockDim.x) {
-        pose[q] = Tm[16 * (i + 1) * nsurf + q];
-        pose[16 * nsurf + q] = Tdm[16 * i * nsurf + q];
-    }
-    if (threadIdx.x < 3) {
-        pose[32 * nsurf + threadIdx.x] = fs[3 * i + threadIdx.x];
-        pose[32 * nsurf + 3 + threadIdx.x] = ref[3 * i + threadIdx.x];
-    }
-}
-
-// the step's coefficients into the run's record, then i -> i + 1
-__global__ void k_uvlm_dev_end(int64_t* idx, const double* coef, double* res) {
-    const int64_t i = idx[0];
-    if (threadIdx.x < 4) res[4 * i + threadIdx.x] = coef[threadIdx.x];
-    __syncthreads();
-    if (threadIdx.x == 0) idx[0] = i + 1;
-}
+// idx[0] on the device, so one captured graph advances the case any number of
+// times.  Its last launch: i -> i + 1.
+__global__ void k_uvlm_dev_end(int64_t* idx) { idx[0] += 1; }
 
 struct UvlmBase {
     virtual ~UvlmBase() = default;
@@ -213,18 +393,15 @@ struct UvlmState : UvlmBase {
     std::vector<gbvlm_dims> dims;
     std::vector<int32_t> lifting;
     void* mem = nullptr;
-    std::vector<T*> vinit, vpos, verts, wake, colloc, colloc0, normals, areas, gamma, gprev, gdelta, gdt, gwake, vel,
-        forces;
+    std::vector<T*> vinit, vpos, verts, wake, colloc, colloc0, normals, areas, gamma, gprev, gwake, vel;
     T *lhs = nullptr, *rhs = nullptr, *Tm = nullptr, *Tdm = nullptr, *fs = nullptr, *ref = nullptr;
     double* res = nullptr;  // [t_steps][4]
     gbvlm_lu lu = nullptr;
 
-    // device-indexed step (step_graph): counter, staged pose, wake scratch,
-    // coefficients, the staged LU solve and the captured graph
+    // device-indexed step (step_graph): counter, wake scratch, the staged LU
+    // solve and the captured graph
     int64_t* d_idx = nullptr;
-    T* d_pose = nullptr;
     float* wsc = nullptr;
-    double* d_coef = nullptr;
     void* dmem = nullptr;
     void* lut = nullptr;
     int64_t dev_idx = -1;  // the value idx[0] holds on the device (-1: unknown)
@@ -254,11 +431,12 @@ struct UvlmState : UvlmBase {
             x.nwv = t_steps;  // wake (ns+1, t_steps, 4) (vlm.cpp:388-399)
             const int64_t np = x.ns * x.nc, nv = (x.ns + 1) * (x.nc + 1);
             n += np;
-            bytes += al(sizeof(T) * 4 * nv) * 3 + al(sizeof(T) * 4 * (x.ns + 1) * t_steps) + al(sizeof(T) * 3 * np) * 5 +
-                     al(sizeof(T) * np) * 5 + al(sizeof(T) * x.ns * (t_steps - 1));
+            bytes += al(sizeof(T) * 4 * nv) * 3 + al(sizeof(T) * 4 * (x.ns + 1) * t_steps) + al(sizeof(T) * 3 * np) * 4 +
+                     al(sizeof(T) * np) * 3 + al(sizeof(T) * x.ns * (t_steps - 1));
         }
         bytes += al(sizeof(T) * n * n) + al(sizeof(T) * n) + 2 * al(sizeof(T) * 16 * nsurf * (t_steps + 1)) +
-                 2 * al(sizeof(T) * 3 * (t_steps + 1)) + al(sizeof(double) * 4 * t_steps);
+                 2 * al(sizeof(T) * 3 * (t_steps + 1)) + al(sizeof(double) * 4 * t_steps) +
+                 al(sizeof(double) * 6 * step_load_blocks(dims)) + al(sizeof(unsigned));
         GB_CUDA(cudaMalloc(&mem, bytes));
         GB_CUDA(cudaMemset(mem, 0, bytes));
         char* p = (char*)mem;
@@ -275,6 +453,10 @@ struct UvlmState : UvlmBase {
         ref = take(3 * (t_steps + 1));
         res = (double*)p;
         p += al(sizeof(double) * 4 * t_steps);
+        sa.part = (double*)p;
+        p += al(sizeof(double) * 6 * step_load_blocks(dims));
+        sa.done = (unsigned*)p;
+        p += al(sizeof(unsigned));
         for (auto& x : dims) {
             const int64_t np = x.ns * x.nc, nv = (x.ns + 1) * (x.nc + 1);
             vinit.push_back(take(4 * nv));
@@ -285,12 +467,9 @@ struct UvlmState : UvlmBase {
             colloc0.push_back(take(3 * np));
             normals.push_back(take(3 * np));
             vel.push_back(take(3 * np));
-            forces.push_back(take(3 * np));
             areas.push_back(take(np));
             gamma.push_back(take(np));
             gprev.push_back(take(np));
-            gdelta.push_back(take(np));
-            gdt.push_back(take(np));
             gwake.push_back(take(x.ns * (t_steps - 1)));
         }
         for (int m = 0; m < nsurf; m++) {
@@ -302,6 +481,27 @@ struct UvlmState : UvlmBase {
             GB_CUDA(cudaMemcpy(wake[m] + 3 * (dims[m].ns + 1) * t_steps, ones.data(), sizeof(T) * ones.size(),
                                cudaMemcpyHostToDevice));
         }
+        step_dims(sa, dims);
+        for (int m = 0; m < nsurf; m++) {
+            sa.vpos[m] = vpos[m];
+            sa.colloc0[m] = colloc0[m];
+            sa.verts[m] = verts[m];
+            sa.wake[m] = wake[m];
+            sa.vel[m] = vel[m];
+            sa.colloc[m] = colloc[m];
+            sa.normals[m] = normals[m];
+            sa.areas[m] = areas[m];
+            sa.gamma[m] = gamma[m];
+            sa.gprev[m] = gprev[m];
+            sa.gwake[m] = gwake[m];
+        }
+        sa.nwv = t_steps;
+        sa.rhs = rhs;
+        sa.Tm = Tm;
+        sa.Tdm = Tdm;
+        sa.fs = fs;
+        sa.ref = ref;
+        sa.out = res;
         int rc = gbvlm_lu_create(&lu);
         if (rc) return rc;
         return gbvlm_lu_init(lu, n);
@@ -331,7 +531,7 @@ struct UvlmState : UvlmBase {
         return out;
     }
 
-    CoefArgs<T> ca;
+    StepArgs<T> sa;
     T dt_ = 0, sigma_ = 0;
     int32_t roll_ = 0;
     int64_t next_step = 0;
@@ -381,15 +581,7 @@ struct UvlmState : UvlmBase {
         if ((rc = Ops2<T>::lhs(lhs, n, nsurf, dims.data(), C(colloc).data(), C(normals).data(), C(verts).data(), sigma, s)))
             return rc;
         if ((rc = Ops2<T>::factor(lu, lhs, n, s))) return rc;
-        memset(&ca, 0, sizeof(ca));
-        ca.n = nsurf;
-        for (int m = 0; m < nsurf; m++) {
-            ca.ns[m] = dims[m].ns;
-            ca.nc[m] = dims[m].nc;
-            ca.forces[m] = forces[m];
-            ca.verts[m] = verts[m];
-            ca.areas[m] = areas[m];
-        }
+        sa.inv_dt = (T)1 / dt;
         GB_CUDA(cudaMemsetAsync(res, 0, sizeof(double) * 4 * t_steps, st));
         return GBVLM_OK;
     }
@@ -404,50 +596,18 @@ struct UvlmState : UvlmBase {
         const int32_t roll = roll_;
         int rc;
         {
-            if ((rc = Ops2<T>::shed(nsurf, dims.data(), C(verts).data(), wake.data(), (int32_t)i, s))) return rc;
-            for (int m = 0; m < nsurf; m++) {
-                const int64_t np = dims[m].ns * dims[m].nc;
-                k_dual_velocity<T><<<(unsigned)cdiv(np, 256), 256, 0, st>>>(Tdm + 16 * ((size_t)i * nsurf + m),
-                                                                           colloc0[m], vel[m], np);
-                GB_LAUNCH_CHECK();
-            }
-            GB_CUDA(cudaMemsetAsync(rhs, 0, sizeof(T) * n, st));
-            if ((rc = Ops2<T>::rhsv(rhs, nsurf, dims.data(), C(normals).data(), C(vel).data(), s))) return rc;
+            if ((rc = step_start(sa, i, st))) return rc;
             if ((rc = Ops2<T>::wake(rhs, nsurf, dims.data(), C(gwake).data(), C(colloc).data(), C(normals).data(),
                                     C(wake).data(), lifting.data(), (int32_t)i, sigma, s)))
                 return rc;
             if ((rc = Ops2<T>::solve(lu, lhs, n, rhs, s))) return rc;
-            int64_t off = 0;
-            for (int m = 0; m < nsurf; m++) {
-                const int64_t ns = dims[m].ns, nc = dims[m].nc;
-                if ((rc = Ops2<T>::gupd(ns, nc, rhs + off, gamma[m], gdelta[m], gwake[m], t_steps - 2 - i, gprev[m],
-                                        gdt[m], dt, s)))
-                    return rc;
-                off += ns * nc;
-            }
-            if (i > 0) {
-                for (int m = 0; m < nsurf; m++) {
-                    if ((rc = Ops2<T>::forces(dims[m].ns, dims[m].nc, verts[m], gdelta[m], gdt[m], vel[m], areas[m],
-                                              normals[m], forces[m], s)))
-                        return rc;
-                }
-                k_step_coeffs<T><<<1, 512, 0, st>>>(ca, fs, ref, i, 1.0, res + 4 * i);
-                GB_LAUNCH_CHECK();
-            }
+            if ((rc = step_loads(sa, i, i > 0, st))) return rc;
             if (roll && i > 0) {
                 if ((rc = Ops2<T>::rollup(nsurf, dims.data(), wake.data(), C(verts).data(), C(gamma).data(),
                                           C(gwake).data(), lifting.data(), sigma, dt, (int32_t)i, s)))
                     return rc;
             }
-            for (int m = 0; m < nsurf; m++) {
-                const int64_t np = dims[m].ns * dims[m].nc;
-                GB_CUDA(cudaMemcpyAsync(gprev[m], gamma[m], sizeof(T) * np, cudaMemcpyDeviceToDevice, st));
-            }
-            auto tn = tr_at(Tm, i + 1);
-            if ((rc = Ops2<T>::displace(nsurf, dims.data(), tn.data(), verts.data(), C(vpos).data(), s))) return rc;
-            if ((rc = Ops2<T>::metrics(nsurf, dims.data(), C(verts).data(), colloc.data(), normals.data(), areas.data(),
-                                       s)))
-                return rc;
+            if ((rc = step_move(sa, i, st))) return rc;
         }
         return GBVLM_OK;
     }
@@ -482,49 +642,18 @@ struct UvlmState : UvlmBase {
     // the device-indexed step on stream c (captured by step_graph and by the
     // request loop of gbvlm_uvlm_loop_*)
     int enqueue_dev_step(cudaStream_t c) {
-        gbvlm_stream cs = (gbvlm_stream)c;
+        StepArgs<T> a = sa;
+        a.idx = d_idx;
         int r;
-        k_uvlm_dev_pose<T><<<1, 128, 0, c>>>(d_idx, Tm, Tdm, fs, ref, nsurf, d_pose);
-        GB_LAUNCH_CHECK();
-        if ((r = wake_shed_dev_f32(nsurf, dims.data(), C(verts).data(), wake.data(), d_idx, c))) return r;
-        for (int m = 0; m < nsurf; m++) {
-            const int64_t np = dims[m].ns * dims[m].nc;
-            k_dual_velocity<T><<<(unsigned)cdiv(np, 256), 256, 0, c>>>(d_pose + 16 * nsurf + 16 * m,
-                                                                      colloc0[m], vel[m], np);
-            GB_LAUNCH_CHECK();
-        }
-        GB_CUDA(cudaMemsetAsync(rhs, 0, sizeof(T) * n, c));
-        if ((r = Ops2<T>::rhsv(rhs, nsurf, dims.data(), C(normals).data(), C(vel).data(), cs))) return r;
+        if ((r = step_start(a, 0, c))) return r;
         if ((r = wake_influence_dev_f32(rhs, nsurf, dims.data(), C(gwake).data(), C(colloc).data(),
                                         C(normals).data(), C(wake).data(), lifting.data(), d_idx,
                                         (int32_t)(t_steps - 2), wsc, c)))
             return r;
         if ((r = lu_solve_prepared_f32(lu, lut, n, c))) return r;
-        int64_t off = 0;
-        for (int m = 0; m < nsurf; m++) {
-            const int64_t ns = dims[m].ns, nc = dims[m].nc;
-            if ((r = gamma_update_dev_f32(ns, nc, rhs + off, gamma[m], gdelta[m], gwake[m], t_steps - 2, d_idx,
-                                          gprev[m], gdt[m], dt_, c)))
-                return r;
-            off += ns * nc;
-        }
-        for (int m = 0; m < nsurf; m++)
-            if ((r = Ops2<T>::forces(dims[m].ns, dims[m].nc, verts[m], gdelta[m], gdt[m], vel[m], areas[m],
-                                     normals[m], forces[m], cs)))
-                return r;
-        k_step_coeffs<T><<<1, 512, 0, c>>>(ca, d_pose + 32 * nsurf, d_pose + 32 * nsurf + 3, 0, 1.0, d_coef);
-        GB_LAUNCH_CHECK();
-        for (int m = 0; m < nsurf; m++) {
-            const int64_t np = dims[m].ns * dims[m].nc;
-            GB_CUDA(cudaMemcpyAsync(gprev[m], gamma[m], sizeof(T) * np, cudaMemcpyDeviceToDevice, c));
-        }
-        std::vector<const T*> tn(nsurf);
-        for (int m = 0; m < nsurf; m++) tn[m] = d_pose + 16 * m;
-        if ((r = Ops2<T>::displace(nsurf, dims.data(), tn.data(), verts.data(), C(vpos).data(), cs))) return r;
-        if ((r = Ops2<T>::metrics(nsurf, dims.data(), C(verts).data(), colloc.data(), normals.data(),
-                                  areas.data(), cs)))
-            return r;
-        k_uvlm_dev_end<<<1, 32, 0, c>>>(d_idx, d_coef, res);
+        if ((r = step_loads(a, 0, true, c))) return r;
+        if ((r = step_move(a, 0, c))) return r;
+        k_uvlm_dev_end<<<1, 1, 0, c>>>(d_idx);
         GB_LAUNCH_CHECK();
         return GBVLM_OK;
     }
@@ -532,12 +661,9 @@ struct UvlmState : UvlmBase {
     // device buffers of the device-indexed step and the staged LU solve
     int prepare_dev(cudaStream_t st) {
         if (!dmem) {
-            const size_t pose = sizeof(T) * (32 * nsurf + 6), wb = sizeof(float) * WAKE_DEV_MAX_SLICES * n;
-            GB_CUDA(cudaMalloc(&dmem, 256 + 256 + (pose + 255) / 256 * 256 + wb));
+            GB_CUDA(cudaMalloc(&dmem, 256 + sizeof(float) * WAKE_DEV_MAX_SLICES * n));
             d_idx = (int64_t*)dmem;
-            d_coef = (double*)((char*)dmem + 256);
-            d_pose = (T*)((char*)dmem + 512);
-            wsc = (float*)((char*)dmem + 512 + (pose + 255) / 256 * 256);
+            wsc = (float*)((char*)dmem + 256);
         }
         if constexpr (std::is_same<T, float>::value) {
             if (!lut) {
@@ -688,13 +814,6 @@ __global__ void k_a2_pose(A2Dev* d, double* u, double* v, double* a, float dtf, 
         }
 }
 
-// the reference's wing-flap coupling: the flap's first chordwise row of
-// gamma_delta also subtracts the wing's trailing-edge gamma (uvlm_2dof.cpp:578-584)
-__global__ void k_a2_flap(float* gdelta1, const float* gamma0, int64_t ns, int64_t nc0) {
-    const int64_t s_ = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (s_ < ns) gdelta1[s_] -= gamma0[s_ + (nc0 - 1) * ns];
-}
-
 __host__ __device__ inline double torsional_cubic(double al) { return 0.1 * al + 40.0 * al * al * al; }
 
 // loads of the iterate (uvlm_2dof.cpp:728-744) and the Newton test; the
@@ -755,15 +874,14 @@ struct Aero2Dof {
     double dt = 0;
     int64_t t_steps = 0, n = 0, done = 0;  // steps advanced
     void* mem = nullptr;
-    std::vector<float*> vinit, verts, wake, colloc, colloch, normals, areas, gamma, gprev, gdelta, gdt, gwake, vel,
-        forces;
+    std::vector<float*> vinit, verts, wake, colloc, colloch, normals, areas, gamma, gprev, gwake, vel;
     float *lhs = nullptr, *rhs = nullptr, *T_all = nullptr, *dT_all = nullptr;
     double *u = nullptr, *v = nullptr, *a = nullptr, *F = nullptr;
     A2Dev* dev = nullptr;
     gbvlm_lu lu = nullptr;
     gbvlm_newmark nm = nullptr;
     std::vector<int32_t> iters;
-    CoefArgs<float> ca;
+    StepArgs<float> sa;
     // one time step as a CUDA graph: the Newton iterations in a conditional
     // while node, replayed step after step without host round trips
     void* aux = nullptr;             // iteration counts per step, wake-influence scratch
@@ -820,10 +938,11 @@ struct Aero2Dof {
             x.nwv = t_steps;
             const int64_t np = x.ns * x.nc, nv = (x.ns + 1) * (x.nc + 1);
             n += np;
-            bytes += al(4 * 4 * nv) * 2 + al(4 * 4 * (x.ns + 1) * t_steps) + al(4 * 3 * np) * 5 + al(4 * np) * 5 +
+            bytes += al(4 * 4 * nv) * 2 + al(4 * 4 * (x.ns + 1) * t_steps) + al(4 * 3 * np) * 4 + al(4 * np) * 3 +
                      al(4 * x.ns * (t_steps - 1));
         }
-        bytes += al(4 * n * n) + al(4 * n) + 2 * al(4 * 16 * nsurf) + 4 * al(8 * 2 * t_steps) + al(sizeof(A2Dev));
+        bytes += al(4 * n * n) + al(4 * n) + 2 * al(4 * 16 * nsurf) + 4 * al(8 * 2 * t_steps) + al(sizeof(A2Dev)) +
+                 al(sizeof(double) * 6 * step_load_blocks(dims)) + al(sizeof(unsigned));
         GB_CUDA(cudaMalloc(&mem, bytes));
         GB_CUDA(cudaMemset(mem, 0, bytes));
         char* p = (char*)mem;
@@ -841,6 +960,8 @@ struct Aero2Dof {
         a = (double*)take(8 * 2 * t_steps);
         F = (double*)take(8 * 2 * t_steps);
         dev = (A2Dev*)take(sizeof(A2Dev));
+        sa.part = (double*)take(sizeof(double) * 6 * step_load_blocks(dims));
+        sa.done = (unsigned*)take(sizeof(unsigned));
         {
             const size_t ib = (sizeof(int32_t) * t_steps + 255) / 256 * 256;
             GB_CUDA(cudaMalloc(&aux, ib + sizeof(float) * WAKE_DEV_MAX_SLICES * n));
@@ -856,12 +977,9 @@ struct Aero2Dof {
             colloch.push_back((float*)take(4 * 3 * np));
             normals.push_back((float*)take(4 * 3 * np));
             vel.push_back((float*)take(4 * 3 * np));
-            forces.push_back((float*)take(4 * 3 * np));
             areas.push_back((float*)take(4 * np));
             gamma.push_back((float*)take(4 * np));
             gprev.push_back((float*)take(4 * np));
-            gdelta.push_back((float*)take(4 * np));
-            gdt.push_back((float*)take(4 * np));
             gwake.push_back((float*)take(4 * x.ns * (t_steps - 1)));
         }
         for (int m = 0; m < nsurf; m++) {
@@ -896,15 +1014,31 @@ struct Aero2Dof {
         if ((rc = gbvlm_newmark_init(nm, 2, dev->M, dev->C, dev->K, dt, (gbvlm_stream)st))) return rc;
         if ((rc = gbvlm_lu_create(&lu))) return rc;
         if ((rc = gbvlm_lu_init(lu, n))) return rc;
-        memset(&ca, 0, sizeof(ca));
-        ca.n = nsurf;
+        step_dims(sa, dims);
         for (int m = 0; m < nsurf; m++) {
-            ca.ns[m] = dims[m].ns;
-            ca.nc[m] = dims[m].nc;
-            ca.forces[m] = forces[m];
-            ca.verts[m] = verts[m];
-            ca.areas[m] = areas[m];
+            sa.vpos[m] = vinit[m];
+            sa.colloc0[m] = colloch[m];
+            sa.verts[m] = verts[m];
+            sa.wake[m] = wake[m];
+            sa.vel[m] = vel[m];
+            sa.colloc[m] = colloc[m];
+            sa.normals[m] = normals[m];
+            sa.areas[m] = areas[m];
+            sa.gamma[m] = gamma[m];
+            sa.gprev[m] = gprev[m];
+            sa.gwake[m] = gwake[m];
         }
+        sa.nwv = t_steps;
+        sa.rhs = rhs;
+        sa.Tm = T_all;
+        sa.Tdm = dT_all;
+        sa.fs = dev->fs;
+        sa.ref = dev->ref;
+        sa.out = dev->coef;
+        sa.inv_dt = 1.f / (float)dt;
+        sa.rho = vars.rho;
+        sa.by_step = sa.keep = false;  // the pose and loads of the iterate; gprev stays the step's
+        sa.flap = nsurf > 1 && dims[1].ns == dims[0].ns;
         return start(st);
     }
 
@@ -940,92 +1074,45 @@ struct Aero2Dof {
             return rc;
         if ((rc = Ops2<float>::factor(lu, lhs, n, s))) return rc;
         if (!lut && (rc = lu_solve_prepare_f32(lu, lhs, n, rhs, &lut, st))) return rc;
-        if ((rc = Ops2<float>::shed(nsurf, dims.data(), C(verts).data(), wake.data(), 0, s))) return rc;
         if ((rc = aero_solve(0, st))) return rc;
         done = 0;
         iters.clear();
         return GBVLM_OK;
     }
 
-    // velocities, RHS, solve and circulation of the current pose (wake rows 0..it)
+    // wake shed, velocities, RHS, solve and circulation of the current pose (wake rows 0..it)
     int aero_solve(int64_t it, cudaStream_t st) {
         gbvlm_stream s = (gbvlm_stream)st;
         int rc;
-        for (int m = 0; m < nsurf; m++) {
-            const int64_t np = dims[m].ns * dims[m].nc;
-            k_dual_velocity<float><<<(unsigned)cdiv(np, 256), 256, 0, st>>>(dT_all + 16 * m, colloch[m], vel[m], np);
-            GB_LAUNCH_CHECK();
-        }
-        GB_CUDA(cudaMemsetAsync(rhs, 0, 4 * n, st));
-        if ((rc = Ops2<float>::rhsv(rhs, nsurf, dims.data(), C(normals).data(), C(vel).data(), s))) return rc;
+        if ((rc = step_start(sa, it, st))) return rc;
         if ((rc = Ops2<float>::wake(rhs, nsurf, dims.data(), C(gwake).data(), C(colloc).data(), C(normals).data(),
                                     C(wake).data(), lifting.data(), (int32_t)it, 0.f, s)))
             return rc;
         if ((rc = Ops2<float>::solve(lu, lhs, n, rhs, s))) return rc;
-        int64_t off = 0;
-        for (int m = 0; m < nsurf; m++) {
-            const int64_t ns = dims[m].ns, nc = dims[m].nc;
-            if ((rc = Ops2<float>::gupd(ns, nc, rhs + off, gamma[m], gdelta[m], gwake[m], t_steps - 2 - it, gprev[m],
-                                        gdt[m], (float)dt, s)))
-                return rc;
-            off += ns * nc;
-        }
-        if (nsurf > 1 && dims[1].ns == dims[0].ns) {
-            k_a2_flap<<<(unsigned)cdiv(dims[1].ns, 128), 128, 0, st>>>(gdelta[1], gamma[0], dims[0].ns, dims[0].nc);
-            GB_LAUNCH_CHECK();
-        }
-        return GBVLM_OK;
+        return step_loads(sa, it, false, st);
     }
 
     // one Newton iteration of the step dev->step (uvlm_2dof.cpp:639-751), with
     // every step-dependent index read on the device: captured into the body
     // of the step graph's while node
     int iterate_dev(cudaStream_t st, cudaGraphConditionalHandle loop) {
-        gbvlm_stream s = (gbvlm_stream)st;
         int rc;
         GB_CUDA(cudaMemcpyAsync(dev->du_prev, dev->du, sizeof(double) * 2, cudaMemcpyDeviceToDevice, st));
         if ((rc = newmark_step_dev(nm, dev->M, dev->C, v, a, &dev->step, dev->du, dev->dv, dev->da, dev->dF, dt, st)))
             return rc;
         k_a2_pose<<<1, 32, 0, st>>>(dev, u, v, a, (float)dt, vars.a_h, nsurf, T_all, dT_all);
         GB_LAUNCH_CHECK();
-        std::vector<const float*> tr(nsurf);
-        for (int m = 0; m < nsurf; m++) tr[m] = T_all + 16 * m;
-        if ((rc = Ops2<float>::displace(nsurf, dims.data(), tr.data(), verts.data(), C(vinit).data(), s))) return rc;
-        if ((rc = Ops2<float>::metrics(nsurf, dims.data(), C(verts).data(), colloc.data(), normals.data(),
-                                       areas.data(), s)))
-            return rc;
-        if ((rc = wake_shed_dev_f32(nsurf, dims.data(), C(verts).data(), wake.data(), &dev->wit, st))) return rc;
-        // velocities, RHS, solve and circulation of the pose (wake rows 0..step+1)
-        for (int m = 0; m < nsurf; m++) {
-            const int64_t np = dims[m].ns * dims[m].nc;
-            k_dual_velocity<float><<<(unsigned)cdiv(np, 256), 256, 0, st>>>(dT_all + 16 * m, colloch[m], vel[m], np);
-            GB_LAUNCH_CHECK();
-        }
-        GB_CUDA(cudaMemsetAsync(rhs, 0, 4 * n, st));
-        if ((rc = Ops2<float>::rhsv(rhs, nsurf, dims.data(), C(normals).data(), C(vel).data(), s))) return rc;
+        StepArgs<float> d = sa;
+        d.idx = &dev->wit;
+        if ((rc = step_move(d, 0, st))) return rc;
+        // wake shed, velocities, RHS, solve and loads of the pose (wake rows 0..step+1)
+        if ((rc = step_start(d, 0, st))) return rc;
         if ((rc = wake_influence_dev_f32(rhs, nsurf, dims.data(), C(gwake).data(), C(colloc).data(),
                                          C(normals).data(), C(wake).data(), lifting.data(), &dev->wit,
                                          (int32_t)(t_steps - 2), wscratch, st)))
             return rc;
         if ((rc = lu_solve_prepared_f32(lu, lut, n, st))) return rc;
-        int64_t off = 0;
-        for (int m = 0; m < nsurf; m++) {
-            const int64_t ns = dims[m].ns, nc = dims[m].nc;
-            if ((rc = gamma_update_dev_f32(ns, nc, rhs + off, gamma[m], gdelta[m], gwake[m], t_steps - 2, &dev->wit,
-                                           gprev[m], gdt[m], (float)dt, st)))
-                return rc;
-            off += ns * nc;
-        }
-        if (nsurf > 1 && dims[1].ns == dims[0].ns) {
-            k_a2_flap<<<(unsigned)cdiv(dims[1].ns, 128), 128, 0, st>>>(gdelta[1], gamma[0], dims[0].ns, dims[0].nc);
-            GB_LAUNCH_CHECK();
-        }
-        for (int m = 0; m < nsurf; m++)
-            if ((rc = Ops2<float>::forces(dims[m].ns, dims[m].nc, verts[m], gdelta[m], gdt[m], vel[m], areas[m],
-                                          normals[m], forces[m], s)))
-                return rc;
-        k_step_coeffs<float><<<1, 512, 0, st>>>(ca, dev->fs, dev->ref, 0, vars.rho, dev->coef);
-        GB_LAUNCH_CHECK();
+        if ((rc = step_loads(d, 0, true, st))) return rc;
         k_a2_loads<<<1, 32, 0, st>>>(dev, u, F, vars.mu, vars.r_a, vars.omega, vars.U_a,
                                      (double)1.1920928955078125e-07, loop);
         GB_LAUNCH_CHECK();
