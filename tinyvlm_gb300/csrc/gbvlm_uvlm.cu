@@ -50,7 +50,8 @@ struct StepArgs {
         *normals[GBVLM_MAX_SURFACES], *areas[GBVLM_MAX_SURFACES], *gamma[GBVLM_MAX_SURFACES],
         *gprev[GBVLM_MAX_SURFACES], *gwake[GBVLM_MAX_SURFACES];
     int64_t nwv = 0;                        // wake vertex rows
-    T* rhs = nullptr;                       // right-hand side, then the solution
+    T* rhs = nullptr;                       // right-hand side
+    const T* sol = nullptr;                 // solution (rhs itself after a solve in place)
     const T *Tm = nullptr, *Tdm = nullptr;  // [step][surface][16] column-major
     const T *fs = nullptr, *ref = nullptr;  // [step][3]
     double* out = nullptr;                  // [step][4]: CL, CM
@@ -210,7 +211,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_step_loads(StepArgs<T> a, int6
         double s[5] = {0, 0, 0, 0, 0};
         if (p < np) {
             const int64_t j = p / ns, i = p - j * ns;
-            const T* x = a.rhs + a.poff[m];
+            const T* x = a.sol + a.poff[m];
             const T g = x[p];
             a.gamma[m][p] = g;
             const int64_t wcol = a.nwv - 2 - it;
@@ -218,7 +219,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_step_loads(StepArgs<T> a, int6
             if (loads) {
                 T gd = (j > 0) ? g - x[p - ns] : g;
                 // the reference's wing-flap coupling (uvlm_2dof.cpp:578-584)
-                if (a.flap && m == 1 && j == 0) gd -= a.rhs[a.poff[0] + i + (a.nc[0] - 1) * a.ns[0]];
+                if (a.flap && m == 1 && j == 0) gd -= a.sol[a.poff[0] + i + (a.nc[0] - 1) * a.ns[0]];
                 const T dg = (g - a.gprev[m][p]) * a.inv_dt;
                 const T *vel = a.vel[m], *nor = a.normals[m];
                 const T area = a.areas[m][p], rho = 1;
@@ -335,6 +336,83 @@ static int step_loads(const StepArgs<T>& a, int64_t step, bool loads, cudaStream
     return GBVLM_OK;
 }
 
+// ---------------------------------------------------------------------------
+// The AIC is factored once and solved for at every step, a chain of n / 128
+// (n / 64 in double) dependent blocks twice over.  A run of many steps forms
+// the inverse instead, as the solution for the identity, and a step's solve is
+// a product with it: every row by a warp of its own, no chain, the matrix read
+// from L2.  1600 panels in float: a solve 71 us, the product 6, the inverse
+// once 0.52 ms (500 steps 126 -> 97 ms); 576 in double: 147, 5 and 1.15 ms (160
+// steps 140 -> 120 ms).
+// inv_steps: the number of steps from which the inverse is formed.  It costs
+// as much as 3 to 13 solves up to 2304 unknowns and 36 at 4096 (double: 1 to 12
+// up to 1024, 50 at 2304, beyond that the solve for many columns is out of
+// shared memory and slow), with about as many again kept in hand.
+// ---------------------------------------------------------------------------
+template <class T>
+static int64_t inv_steps(int64_t n) {
+    if (n > (sizeof(T) == 4 ? 4096 : 2304)) return INT64_MAX;
+    return 16 + n / (sizeof(T) == 4 ? 64 : 32);
+}
+constexpr int INV_WARPS = 4;       // rows of a block
+
+template <class T>
+static int64_t inv_ld(int64_t n) {
+    constexpr int64_t V = 16 / sizeof(T);
+    return (n + V - 1) / V * V;
+}
+
+template <class T>
+__global__ void k_set_diagonal(T* m, int64_t n, int64_t ld) {
+    const int64_t r = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (r < n) m[r * (ld + 1)] = (T)1;
+}
+
+// m = m^T in place, a pair of 32 x 32 tiles per block (grid: tiles x tiles, the lower ones at work)
+template <class T>
+__global__ void __launch_bounds__(256) k_transpose(T* m, int64_t n, int64_t ld) {
+    __shared__ T s0[32][33], s1[32][33];
+    const int64_t i0 = 32 * (int64_t)blockIdx.x, j0 = 32 * (int64_t)blockIdx.y;
+    if (j0 > i0) return;
+    const int x = threadIdx.x & 31;
+    for (int y = threadIdx.x >> 5; y < 32; y += 8) {
+        if (j0 + y < n && i0 + x < n) s0[y][x] = m[(j0 + y) * ld + i0 + x];
+        if (i0 + y < n && j0 + x < n) s1[y][x] = m[(i0 + y) * ld + j0 + x];
+    }
+    __syncthreads();
+    for (int y = threadIdx.x >> 5; y < 32; y += 8) {
+        if (j0 + y < n && i0 + x < n) m[(j0 + y) * ld + i0 + x] = s1[x][y];
+        if (i0 + y < n && j0 + x < n) m[(i0 + y) * ld + j0 + x] = s0[x][y];
+    }
+}
+
+// x = M b, M by rows with a leading dimension of whole 16-byte vectors (M and b
+// zero from n to there)
+template <class T>
+__global__ void __launch_bounds__(32 * INV_WARPS) k_inverse_apply(const T* M, int64_t n, int64_t ld, const T* b, T* x) {
+    constexpr int V = 16 / sizeof(T);
+    struct alignas(16) Vec {
+        T v[V];
+    };
+    const int64_t r = blockIdx.x * (int64_t)INV_WARPS + (threadIdx.x >> 5);
+    if (r >= n) return;
+    const Vec *mv = reinterpret_cast<const Vec*>(M + r * ld), *bv = reinterpret_cast<const Vec*>(b);
+    T acc[V];
+#pragma unroll
+    for (int e = 0; e < V; e++) acc[e] = 0;
+#pragma unroll 4
+    for (int64_t k = threadIdx.x & 31; k < ld / V; k += 32) {
+        const Vec p = mv[k], q = bv[k];
+#pragma unroll
+        for (int e = 0; e < V; e++) acc[e] += p.v[e] * q.v[e];
+    }
+    T s = acc[0] + acc[1];
+    if constexpr (V == 4) s += acc[2] + acc[3];
+#pragma unroll
+    for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+    if ((threadIdx.x & 31) == 0) x[r] = s;
+}
+
 template <class T>
 struct Ops2;
 #define OPS2(T, sfx)                                                                                                \
@@ -363,6 +441,9 @@ struct Ops2;
         static int factor(gbvlm_lu h, T* a, int64_t n, gbvlm_stream s) { return gbvlm_lu_factor_##sfx(h, a, n, n, s); } \
         static int solve(gbvlm_lu h, const T* a, int64_t n, T* x, gbvlm_stream s) {                                 \
             return gbvlm_lu_solve_##sfx(h, a, n, n, x, n, 1, s);                                                    \
+        }                                                                                                           \
+        static int solve_many(gbvlm_lu h, const T* a, int64_t n, T* x, int64_t ldx, int64_t nrhs, gbvlm_stream s) {  \
+            return gbvlm_lu_solve_##sfx(h, a, n, n, x, ldx, nrhs, s);                                               \
         }                                                                                                           \
     };
 OPS2(float, f32)
@@ -396,6 +477,8 @@ struct UvlmState : UvlmBase {
     std::vector<T*> vinit, vpos, verts, wake, colloc, colloc0, normals, areas, gamma, gprev, gwake, vel;
     T *lhs = nullptr, *rhs = nullptr, *Tm = nullptr, *Tdm = nullptr, *fs = nullptr, *ref = nullptr;
     double* res = nullptr;  // [t_steps][4]
+    T *inv = nullptr, *sol = nullptr;  // the AIC's inverse by rows and its product, where the run pays for it
+    int64_t ldi = 0;
     gbvlm_lu lu = nullptr;
 
     // device-indexed step (step_graph): counter, wake scratch, the staged LU
@@ -437,6 +520,8 @@ struct UvlmState : UvlmBase {
         bytes += al(sizeof(T) * n * n) + al(sizeof(T) * n) + 2 * al(sizeof(T) * 16 * nsurf * (t_steps + 1)) +
                  2 * al(sizeof(T) * 3 * (t_steps + 1)) + al(sizeof(double) * 4 * t_steps) +
                  al(sizeof(double) * 6 * step_load_blocks(dims)) + al(sizeof(unsigned));
+        ldi = t_steps - 1 >= inv_steps<T>(n) ? inv_ld<T>(n) : 0;
+        bytes += al(sizeof(T) * n * ldi) + al(sizeof(T) * ldi);
         GB_CUDA(cudaMalloc(&mem, bytes));
         GB_CUDA(cudaMemset(mem, 0, bytes));
         char* p = (char*)mem;
@@ -446,7 +531,11 @@ struct UvlmState : UvlmBase {
             return r;
         };
         lhs = take(n * n);
-        rhs = take(n);
+        rhs = take(n);  // (to a multiple of 256 bytes, zero past n)
+        if (ldi) {
+            inv = take(n * ldi);
+            sol = take(ldi);
+        }
         Tm = take(16 * nsurf * (t_steps + 1));
         Tdm = take(16 * nsurf * (t_steps + 1));
         fs = take(3 * (t_steps + 1));
@@ -497,6 +586,7 @@ struct UvlmState : UvlmBase {
         }
         sa.nwv = t_steps;
         sa.rhs = rhs;
+        sa.sol = inv ? sol : rhs;
         sa.Tm = Tm;
         sa.Tdm = Tdm;
         sa.fs = fs;
@@ -581,8 +671,23 @@ struct UvlmState : UvlmBase {
         if ((rc = Ops2<T>::lhs(lhs, n, nsurf, dims.data(), C(colloc).data(), C(normals).data(), C(verts).data(), sigma, s)))
             return rc;
         if ((rc = Ops2<T>::factor(lu, lhs, n, s))) return rc;
+        if (inv) {
+            GB_CUDA(cudaMemsetAsync(inv, 0, sizeof(T) * n * ldi, st));
+            k_set_diagonal<T><<<(unsigned)cdiv(n, 256), 256, 0, st>>>(inv, n, ldi);
+            GB_LAUNCH_CHECK();
+            if ((rc = Ops2<T>::solve_many(lu, lhs, n, inv, ldi, n, s))) return rc;
+            const dim3 g((unsigned)cdiv(n, 32), (unsigned)cdiv(n, 32));
+            k_transpose<T><<<g, 256, 0, st>>>(inv, n, ldi);
+            GB_LAUNCH_CHECK();
+        }
         sa.inv_dt = (T)1 / dt;
         GB_CUDA(cudaMemsetAsync(res, 0, sizeof(double) * 4 * t_steps, st));
+        return GBVLM_OK;
+    }
+
+    int apply_inverse(cudaStream_t st) {
+        k_inverse_apply<T><<<(unsigned)cdiv(n, INV_WARPS), 32 * INV_WARPS, 0, st>>>(inv, n, ldi, rhs, sol);
+        GB_LAUNCH_CHECK();
         return GBVLM_OK;
     }
 
@@ -600,7 +705,7 @@ struct UvlmState : UvlmBase {
             if ((rc = Ops2<T>::wake(rhs, nsurf, dims.data(), C(gwake).data(), C(colloc).data(), C(normals).data(),
                                     C(wake).data(), lifting.data(), (int32_t)i, sigma, s)))
                 return rc;
-            if ((rc = Ops2<T>::solve(lu, lhs, n, rhs, s))) return rc;
+            if ((rc = inv ? apply_inverse(st) : Ops2<T>::solve(lu, lhs, n, rhs, s))) return rc;
             if ((rc = step_loads(sa, i, i > 0, st))) return rc;
             if (roll && i > 0) {
                 if ((rc = Ops2<T>::rollup(nsurf, dims.data(), wake.data(), C(verts).data(), C(gamma).data(),
@@ -650,7 +755,7 @@ struct UvlmState : UvlmBase {
                                         C(normals).data(), C(wake).data(), lifting.data(), d_idx,
                                         (int32_t)(t_steps - 2), wsc, c)))
             return r;
-        if ((r = lu_solve_prepared_f32(lu, lut, n, c))) return r;
+        if ((r = inv ? apply_inverse(c) : lu_solve_prepared_f32(lu, lut, n, c))) return r;
         if ((r = step_loads(a, 0, true, c))) return r;
         if ((r = step_move(a, 0, c))) return r;
         k_uvlm_dev_end<<<1, 1, 0, c>>>(d_idx);
@@ -666,7 +771,7 @@ struct UvlmState : UvlmBase {
             wsc = (float*)((char*)dmem + 256);
         }
         if constexpr (std::is_same<T, float>::value) {
-            if (!lut) {
+            if (!lut && !inv) {
                 int rc = lu_solve_prepare_f32(lu, lhs, n, rhs, &lut, st);
                 if (rc) return rc;
             }
@@ -1030,6 +1135,7 @@ struct Aero2Dof {
         }
         sa.nwv = t_steps;
         sa.rhs = rhs;
+        sa.sol = rhs;
         sa.Tm = T_all;
         sa.Tdm = dT_all;
         sa.fs = dev->fs;
