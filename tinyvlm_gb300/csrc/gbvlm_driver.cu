@@ -1,9 +1,11 @@
 // Host drivers above the operator C ABI: the steady VLM simulation
 // (vlm/src/vlm.cpp:17-151), the nonlinear VLM (vlm.cpp:153-295) and the
 // plot3d reader (vlm/src/vlm_mesh.cpp).
-// These are the "plain per-solve" paths: one operator call per reference
-// backend call, scalars read back synchronously, in float (the reference's
-// semantics) or double.
+// These are the per-solve paths, in float (the reference's semantics) or double:
+// AIC assembly, factorisation and solve are the operators of the C ABI, and what
+// lies around them is one launch before the assembly (wake, pose, metrics), one
+// before the solve (right-hand side) and one after it (circulation, forces and
+// every sum), read back together.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>
@@ -14,16 +16,157 @@
 #include <vector>
 
 #include "gbvlm_internal.h"
+#include "gbvlm_loads.cuh"
 
 namespace gbvlm {
 
 template <class T>
-__global__ void k_fill3(T* v, int64_t np, T x, T y, T z) {
-    int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= np) return;
-    v[p] = x;
-    v[np + p] = y;
-    v[2 * np + p] = z;
+struct SteadyArgs {
+    int32_t n = 0;
+    int64_t ns[GBVLM_MAX_SURFACES], nc[GBVLM_MAX_SURFACES];
+    int64_t poff[GBVLM_MAX_SURFACES + 1], soff[GBVLM_MAX_SURFACES + 1];  // first panel, first strip
+    const T* vinit[GBVLM_MAX_SURFACES];
+    T *verts[GBVLM_MAX_SURFACES], *wake[GBVLM_MAX_SURFACES], *colloc[GBVLM_MAX_SURFACES],
+        *normals[GBVLM_MAX_SURFACES], *areas[GBVLM_MAX_SURFACES];
+    T* rhs = nullptr;          // right-hand side, then the solution
+    T* strip = nullptr;        // angles of the strips (nonlinear)
+    double* part = nullptr;    // [blocks][LOAD_PART]
+    double* out = nullptr;     // [n][7]: lift, area, moment x, y, z, chord numerator, drag sum
+    unsigned* done = nullptr;  // blocks finished, zero between launches
+    T tr[16];                  // pose of every surface
+    T factor = 0;              // collocation point's share of the chord
+    T V[3], la[3], ref[3];     // panel velocity, lift axis, moment point
+    T sigma = 0;
+
+    __device__ __forceinline__ int surf(int64_t g) const {
+        int m = 0;
+        while (m + 1 < n && g >= poff[m + 1]) m++;
+        return m;
+    }
+};
+
+// the wake row from the trailing edge at rest to that of the moved wing, the
+// moved wing and its metrics (wake_shed, displace, wake_shed, mesh_metrics)
+template <class T>
+__global__ void __launch_bounds__(LOAD_THREADS) k_vlm_place(SteadyArgs<T> a) {
+    const int64_t g = blockIdx.x * (int64_t)LOAD_THREADS + threadIdx.x;
+    if (g < a.poff[a.n]) {
+        const int m = a.surf(g);
+        move_panel(a.vinit[m], a.verts[m], a.tr, a.ns[m], a.nc[m], g - a.poff[m], a.factor, a.colloc[m], a.normals[m],
+                   a.areas[m]);
+        return;
+    }
+    int64_t r = g - a.poff[a.n];
+    for (int m = 0; m < a.n; m++) {
+        const int64_t nv = a.ns[m] + 1;
+        if (r < nv) {
+            const int64_t vld = nv * (a.nc[m] + 1), q = r + a.nc[m] * nv;
+            T y[4];
+            move_vertex(a.vinit[m], vld, q, a.tr, y);
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+                a.wake[m][2 * k * nv + r] = y[k];
+                a.wake[m][2 * k * nv + nv + r] = a.vinit[m][k * vld + q];
+            }
+            return;
+        }
+        r -= nv;
+    }
+}
+
+// right-hand side -V . n: V the free stream, or with strip angles theirs
+// (vlm.cpp:186-196: freestream(u_inf, alpha_strip, 0))
+template <class T>
+__global__ void __launch_bounds__(LOAD_THREADS) k_vlm_rhs(SteadyArgs<T> a, bool strips, T u) {
+    const int64_t g = blockIdx.x * (int64_t)LOAD_THREADS + threadIdx.x;
+    if (g >= a.poff[a.n]) return;
+    const int m = a.surf(g);
+    const int64_t p = g - a.poff[m], np = a.ns[m] * a.nc[m];
+    const T* n = a.normals[m];
+    T V[3] = {a.V[0], a.V[1], a.V[2]};
+    if (strips) {
+        const T al = a.strip[a.soff[m] + p % a.ns[m]];
+        V[0] = u * cos(al);
+        V[1] = 0;
+        V[2] = u * sin(al);
+    }
+    a.rhs[g] = (T)0 + -(V[0] * n[p] + V[1] * n[np + p] + V[2] * n[2 * np + p]);
+}
+
+// the steady force on the bound segment of panel (i, j) (vlm_backend_cpu.cpp:276-297), rho = 1
+template <class T>
+__device__ __forceinline__ V3<T> steady_force(const T* x, const T* v, int64_t ns, int64_t nc, int64_t i, int64_t j,
+                                              V3<T> V, V3<T>& v0, V3<T>& v1) {
+    const int64_t p = i + j * ns, ia = i + j * (ns + 1), ib = ia + 1, vld = (ns + 1) * (nc + 1);
+    const T g = x[p], gd = (j > 0) ? g - x[p - ns] : g, rho = 1;
+    v0 = V3<T>{v[ia], v[vld + ia], v[2 * vld + ia]};
+    v1 = V3<T>{v[ib], v[vld + ib], v[2 * vld + ib]};
+    return (rho * gd) * cross(V, v1 - v0);
+}
+
+// The sums that the coefficients are made of (vlm_backend.cpp:72-139,
+// ispc:273-323) from the solution, one launch: panel blocks, chord blocks, a
+// block per wake ring.  all: with the chords and the drag.  alpha: the panel
+// velocity u (cos, 0, sin) of it instead of V.  Four sums and the drag by a
+// launch and a read-back each took 90 us of a 256-panel case.
+template <class T>
+__global__ void __launch_bounds__(LOAD_THREADS) k_vlm_loads(SteadyArgs<T> a, bool all, bool from_alpha, T u, T alpha) {
+    __shared__ LoadShared sh;
+    __shared__ double red[32];
+    const int t = threadIdx.x;
+    int64_t blk = blockIdx.x;
+    int m = 0, kind = 0;
+    for (; m < a.n; m++) {
+        const int64_t cnt[3] = {(a.ns[m] * a.nc[m] + LOAD_THREADS - 1) / LOAD_THREADS,
+                                all ? (a.ns[m] + LOAD_CHORDS - 1) / LOAD_CHORDS : 0, all ? a.ns[m] : 0};
+        for (kind = 0; kind < 3; kind++) {
+            if (blk < cnt[kind]) break;
+            blk -= cnt[kind];
+        }
+        if (kind < 3) break;
+    }
+    const int64_t ns = a.ns[m], nc = a.nc[m], np = ns * nc;
+    const T *x = a.rhs + a.poff[m], *v = a.verts[m];
+    double* part = a.part + LOAD_PART * (int64_t)blockIdx.x;
+    if (kind == 0) {
+        const int64_t p = blk * LOAD_THREADS + t;
+        double s[LOAD_SUMS] = {0, 0, 0, 0, 0};
+        if (p < np) {
+            V3<T> V{a.V[0], a.V[1], a.V[2]}, v0, v1;
+            if (from_alpha) V = V3<T>{u * cos(alpha), (T)0, u * sin(alpha)};
+            const int64_t j = p / ns, i = p - j * ns;
+            const V3<T> F = steady_force(x, v, ns, nc, i, j, V, v0, v1);
+            const double Fx = F.x, Fy = F.y, Fz = F.z;
+            s[0] = Fx * a.la[0] + Fy * a.la[1] + Fz * a.la[2];
+            s[1] = a.areas[m][p];
+            if (all) {
+                const double ex = 0.5 * ((double)v0.x + v1.x) - a.ref[0];
+                const double ey = 0.5 * ((double)v0.y + v1.y) - a.ref[1];
+                const double ez = 0.5 * ((double)v0.z + v1.z) - a.ref[2];
+                s[2] = ey * Fz - ez * Fy;
+                s[3] = ez * Fx - ex * Fz;
+                s[4] = ex * Fy - ey * Fx;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < LOAD_SUMS; q++) sh.s[q][t] = s[q];
+        block_sums(sh, LOAD_SUMS, part);
+    } else if (kind == 1) {
+        chord_terms(sh, v, ns, nc, blk);
+        block_sums(sh, 1, part);
+    } else {
+        const double d = trefftz_ring(ns + 1, (int64_t)2, (const T*)a.wake[m], x + (nc - 1) * ns, a.sigma, blk, red);
+        if (t == 0) part[0] = d;
+    }
+    if (!last_block(sh, a.done)) return;
+    int64_t b0 = 0;
+    for (int k = 0; k < a.n; k++) {
+        const int64_t pb = (a.ns[k] * a.nc[k] + LOAD_THREADS - 1) / LOAD_THREADS;
+        const int64_t cb = all ? (a.ns[k] + LOAD_CHORDS - 1) / LOAD_CHORDS : 0, rb = all ? a.ns[k] : 0;
+        add_parts(sh, a.part, b0, pb, cb, rb);
+        if (t < 7) a.out[7 * k + t] = sh.tot[t];
+        b0 += pb + cb + rb;
+    }
 }
 
 template <class T>
@@ -41,45 +184,9 @@ struct Ops;
                        const T* const* vw, const T* const* vk, int32_t it, T sg, gbvlm_stream s) {                    \
             return gbvlm_lhs_assemble_##sfx(a, ld, ns, d, c, n, vw, vk, it, sg, s);                                  \
         }                                                                                                            \
-        static int rhsv(T* r, int32_t ns, const gbvlm_dims* d, const T* const* n, const T* const* v, gbvlm_stream s) { \
-            return gbvlm_rhs_assemble_velocities_##sfx(r, ns, d, n, v, s);                                          \
-        }                                                                                                            \
-        static int metrics(T a, int32_t ns, const gbvlm_dims* d, const T* const* v, T* const* c, T* const* n,        \
-                           T* const* ar, gbvlm_stream s) {                                                           \
-            return gbvlm_mesh_metrics_##sfx(a, ns, d, v, c, n, ar, s);                                              \
-        }                                                                                                            \
-        static int displace(int32_t ns, const gbvlm_dims* d, const T* const* t, T* const* v, const T* const* vi,     \
-                            gbvlm_stream s) {                                                                        \
-            return gbvlm_displace_wing_##sfx(ns, d, t, v, vi, s);                                                   \
-        }                                                                                                            \
-        static int shed(int32_t ns, const gbvlm_dims* d, const T* const* v, T* const* k, int32_t it, gbvlm_stream s) { \
-            return gbvlm_wake_shed_##sfx(ns, d, v, k, it, s);                                                       \
-        }                                                                                                            \
         static int factor(gbvlm_lu h, T* a, int64_t n, gbvlm_stream s) { return gbvlm_lu_factor_##sfx(h, a, n, n, s); } \
         static int solve(gbvlm_lu h, const T* a, int64_t n, T* x, gbvlm_stream s) {                                  \
             return gbvlm_lu_solve_##sfx(h, a, n, n, x, n, 1, s);                                                     \
-        }                                                                                                            \
-        static int gupd(int64_t ns, int64_t nc, const T* x, T* g, T* gd, T* gw, gbvlm_stream s) {                    \
-            return gbvlm_gamma_update_##sfx(ns, nc, x, g, gd, gw, 0, nullptr, nullptr, (T)0, s);                     \
-        }                                                                                                            \
-        static int forces(int64_t ns, int64_t nc, const T* v, const T* gd, const T* vel, T* f, gbvlm_stream s) {     \
-            return gbvlm_forces_steady_##sfx(ns, nc, v, gd, vel, f, s);                                             \
-        }                                                                                                            \
-        static int sum(const T* x, int64_t n, T* o, gbvlm_stream s) { return gbvlm_sum_##sfx(x, n, o, s); }          \
-        static int cl(int64_t ns, int64_t nc, const T* f, const T* la, const T* fs, T rho, T area, T* o,             \
-                      gbvlm_stream s) {                                                                              \
-            return gbvlm_coeff_cl_##sfx(ns, nc, f, la, fs, rho, area, o, s);                                        \
-        }                                                                                                            \
-        static int cm(int64_t ns, int64_t nc, const T* f, const T* v, const T* r, const T* fs, T rho, T area, T mac, \
-                      T* o, gbvlm_stream s) {                                                                        \
-            return gbvlm_coeff_cm_##sfx(ns, nc, f, v, r, fs, rho, area, mac, o, s);                                 \
-        }                                                                                                            \
-        static int mac(int64_t ns, int64_t nc, const T* v, const T* a, T* o, gbvlm_stream s) {                       \
-            return gbvlm_mesh_mac_##sfx(ns, nc, v, a, o, s);                                                        \
-        }                                                                                                            \
-        static int cd(int64_t ns, int64_t nwv, const T* vk, const T* gw, const T* fs, T area, T sg, T* o,            \
-                      gbvlm_stream s) {                                                                              \
-            return gbvlm_trefftz_cd_##sfx(ns, nwv, vk, gw, fs, area, sg, o, s);                                     \
         }                                                                                                            \
     };
 OPS(float, f32)
@@ -100,7 +207,9 @@ struct VlmState : VlmBase {
     std::vector<gbvlm_dims> dims;
     int64_t n = 0;
     void* mem = nullptr;
-    std::vector<T*> verts_init, verts, wake, colloc, normals, areas, gamma, gdelta, gwake, vel, forces, transform;
+    std::vector<T*> verts_init, verts, wake, colloc, normals, areas;
+    SteadyArgs<T> sa;
+    int64_t loads_blocks = 0, lift_blocks = 0;  // of k_vlm_loads with and without the chords and the drag
     T* lhs = nullptr;
     T* rhs = nullptr;
     gbvlm_lu lu = nullptr;
@@ -120,9 +229,11 @@ struct VlmState : VlmBase {
             x.nwv = 2;  // single row of wake panels (vlm.cpp:73)
             int64_t np = x.ns * x.nc, nv = (x.ns + 1) * (x.nc + 1);
             n += np;
-            bytes += sizeof(T) * (2 * 4 * nv + 4 * (x.ns + 1) * 2 + 3 * 3 * np + 3 * np + 3 * np + x.ns + 16 + 3 * np);
+            bytes += sizeof(T) * (2 * 4 * nv + 4 * (x.ns + 1) * 2 + 7 * np);
+            lift_blocks += cdiv(np, LOAD_THREADS);
+            loads_blocks += cdiv(np, LOAD_THREADS) + cdiv(x.ns, LOAD_CHORDS) + x.ns;
         }
-        bytes += sizeof(T) * (n * n + n) + 4096 * 8;
+        bytes += sizeof(T) * (n * n + n) + 256 * (6 * ns_ + 5) + sizeof(double) * (LOAD_PART * loads_blocks + 7 * ns_);
         GB_CUDA(cudaMalloc(&mem, bytes));
         GB_CUDA(cudaMemset(mem, 0, bytes));
         char* p = (char*)mem;
@@ -141,12 +252,6 @@ struct VlmState : VlmBase {
             colloc.push_back(take(3 * np));
             normals.push_back(take(3 * np));
             areas.push_back(take(np));
-            gamma.push_back(take(np));
-            gdelta.push_back(take(np));
-            gwake.push_back(take(x.ns));
-            vel.push_back(take(3 * np));
-            forces.push_back(take(3 * np));
-            transform.push_back(take(16));
         }
         // upload initial vertices (float host) and set wake w = 1
         for (int m = 0; m < nsurf; m++) {
@@ -162,6 +267,29 @@ struct VlmState : VlmBase {
             GB_CUDA(cudaMemcpy(wake[m] + 3 * 2 * (dims[m].ns + 1), ones.data(), sizeof(T) * ones.size(),
                                cudaMemcpyHostToDevice));
         }
+        sa.n = nsurf;
+        sa.poff[0] = sa.soff[0] = 0;
+        for (int m = 0; m < nsurf; m++) {
+            sa.ns[m] = dims[m].ns;
+            sa.nc[m] = dims[m].nc;
+            sa.poff[m + 1] = sa.poff[m] + dims[m].ns * dims[m].nc;
+            sa.soff[m + 1] = sa.soff[m] + dims[m].ns;
+            sa.vinit[m] = verts_init[m];
+            sa.verts[m] = verts[m];
+            sa.wake[m] = wake[m];
+            sa.colloc[m] = colloc[m];
+            sa.normals[m] = normals[m];
+            sa.areas[m] = areas[m];
+        }
+        sa.rhs = rhs;
+        auto take_bytes = [&](size_t b) {
+            void* r = p;
+            p += (b + 255) / 256 * 256;
+            return r;
+        };
+        sa.part = (double*)take_bytes(sizeof(double) * LOAD_PART * loads_blocks);
+        sa.out = (double*)take_bytes(sizeof(double) * 7 * nsurf);
+        sa.done = (unsigned*)take_bytes(sizeof(unsigned));
         int rc = gbvlm_lu_create(&lu);
         if (rc) return rc;
         return gbvlm_lu_init(lu, n);
@@ -184,25 +312,19 @@ struct VlmState : VlmBase {
     // high-AoA factor of alpha; `tr` receives the wake translation.
     int assemble(T alpha, T u, T* tr, gbvlm_stream s, cudaStream_t st) {
         GB_CUDA(cudaMemsetAsync(lhs, 0, sizeof(T) * n * n, st));
-        for (int m = 0; m < nsurf; m++) {
-            int64_t nv = (dims[m].ns + 1) * (dims[m].nc + 1);
-            GB_CUDA(cudaMemcpyAsync(verts[m], verts_init[m], sizeof(T) * 4 * nv, cudaMemcpyDeviceToDevice, st));
-        }
         // 100-chord wake (vlm.cpp:104-114)
         const T t16[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, (T)-100 * u * (T)cos(alpha), 0,
                            (T)-100 * u * (T)sin(alpha), 1};
         for (int k = 0; k < 16; k++) tr[k] = t16[k];
-        for (int m = 0; m < nsurf; m++)
-            GB_CUDA(cudaMemcpyAsync(transform[m], t16, sizeof(t16), cudaMemcpyHostToDevice, st));
-        std::vector<const T*> cverts(verts.begin(), verts.end()), cinit(verts_init.begin(), verts_init.end()),
-            ctr(transform.begin(), transform.end()), ccol(colloc.begin(), colloc.end()),
+        for (int k = 0; k < 16; k++) sa.tr[k] = t16[k];
+        sa.factor = aoa_factor(alpha);
+        std::vector<const T*> cverts(verts.begin(), verts.end()), ccol(colloc.begin(), colloc.end()),
             cnor(normals.begin(), normals.end()), cwake(wake.begin(), wake.end());
+        int64_t cnt = n;
+        for (auto& x : dims) cnt += x.ns + 1;
+        k_vlm_place<T><<<(unsigned)cdiv(cnt, LOAD_THREADS), LOAD_THREADS, 0, st>>>(sa);
+        GB_LAUNCH_CHECK();
         int rc;
-        if ((rc = Ops<T>::shed(nsurf, dims.data(), cverts.data(), wake.data(), 0, s))) return rc;
-        if ((rc = Ops<T>::displace(nsurf, dims.data(), ctr.data(), verts.data(), cinit.data(), s))) return rc;
-        if ((rc = Ops<T>::shed(nsurf, dims.data(), cverts.data(), wake.data(), 1, s))) return rc;
-        if ((rc = Ops<T>::metrics(alpha, nsurf, dims.data(), cverts.data(), colloc.data(), normals.data(), areas.data(), s)))
-            return rc;
         if ((rc = Ops<T>::lhs(lhs, n, nsurf, dims.data(), ccol.data(), cnor.data(), cverts.data(), cwake.data(), 1, sigma, s)))
             return rc;
         return Ops<T>::factor(lu, lhs, n, s);
@@ -212,53 +334,54 @@ struct VlmState : VlmBase {
     // update and the loads (vlm.cpp:115-151) on the factored AIC.
     int solve_loads(const T* fs, const T* la, T rho, const T* tr, const double* ref_pt, gbvlm_coeffs* out,
                     double* gamma_out, gbvlm_stream s, cudaStream_t st) {
-        GB_CUDA(cudaMemsetAsync(rhs, 0, sizeof(T) * n, st));
-        std::vector<const T*> cnor(normals.begin(), normals.end()), cvel(vel.begin(), vel.end());
+        for (int k = 0; k < 3; k++) {
+            sa.V[k] = fs[k];
+            sa.la[k] = la[k];
+        }
+        sa.sigma = (T)sqrt((double)(sigma * sigma));
+        k_vlm_rhs<T><<<(unsigned)cdiv(n, LOAD_THREADS), LOAD_THREADS, 0, st>>>(sa, false, (T)0);
+        GB_LAUNCH_CHECK();
         int rc;
-        for (int m = 0; m < nsurf; m++) {
-            int64_t np = dims[m].ns * dims[m].nc;
-            k_fill3<T><<<(unsigned)cdiv(np, 256), 256, 0, st>>>(vel[m], np, fs[0], fs[1], fs[2]);
-            GB_LAUNCH_CHECK();
-        }
-        if ((rc = Ops<T>::rhsv(rhs, nsurf, dims.data(), cnor.data(), cvel.data(), s))) return rc;
         if ((rc = Ops<T>::solve(lu, lhs, n, rhs, s))) return rc;
-        int64_t off = 0;
-        for (int m = 0; m < nsurf; m++) {
-            if ((rc = Ops<T>::gupd(dims[m].ns, dims[m].nc, rhs + off, gamma[m], gdelta[m], gwake[m], s))) return rc;
-            if ((rc = Ops<T>::forces(dims[m].ns, dims[m].nc, verts[m], gdelta[m], vel[m], forces[m], s))) return rc;
-            off += dims[m].ns * dims[m].nc;
-        }
         // coefficient reductions (vlm_backend.cpp:72-139) + Trefftz drag
         // the wing sits displaced by the wake translation; move the moment
         // reference with it so CM is the body-frame moment about ref_pt
         T ref[3] = {(T)(ref_pt ? ref_pt[0] : 0) + tr[12], (T)(ref_pt ? ref_pt[1] : 0) + tr[13],
                     (T)(ref_pt ? ref_pt[2] : 0) + tr[14]};
+        for (int k = 0; k < 3; k++) sa.ref[k] = ref[k];
+        k_vlm_loads<T><<<(unsigned)loads_blocks, LOAD_THREADS, 0, st>>>(sa, true, false, (T)0, (T)0);
+        GB_LAUNCH_CHECK();
+        // the sums, the circulations and the solve's error words in one wait
+        const size_t sums = sizeof(double) * 7 * nsurf;
+        char* h = (char*)host_scratch(16 + sums + sizeof(T) * n);
+        GB_REQUIRE(h != nullptr, "pinned host allocation failed");
+        const double* r = (const double*)(h + 16);
+        const T* g = (const T*)(h + 16 + sums);
+        if ((rc = lu_solve_words(lu, (int*)h, st))) return rc;
+        GB_CUDA(cudaMemcpyAsync(h + 16, sa.out, sums, cudaMemcpyDeviceToHost, st));
+        if (gamma_out) GB_CUDA(cudaMemcpyAsync(h + 16 + sums, rhs, sizeof(T) * n, cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaStreamSynchronize(st));
+        const T v2 = fs[0] * fs[0] + fs[1] * fs[1] + fs[2] * fs[2];
+        const double v2d = (double)fs[0] * fs[0] + (double)fs[1] * fs[1] + (double)fs[2] * fs[2];
         T cl = 0, ta = 0, tm = 0, cdn = 0;
         T cm[3] = {0, 0, 0};
-        for (int m = 0; m < nsurf; m++) {
-            int64_t ns = dims[m].ns, nc = dims[m].nc;
-            T area, clm, mac, cmm[3], cdm;
-            if ((rc = Ops<T>::sum(areas[m], ns * nc, &area, s))) return rc;
-            if ((rc = Ops<T>::cl(ns, nc, forces[m], la, fs, rho, area, &clm, s))) return rc;
-            if ((rc = Ops<T>::mac(ns, nc, verts[m], areas[m], &mac, s))) return rc;
-            if ((rc = Ops<T>::cm(ns, nc, forces[m], verts[m], ref, fs, rho, area, mac, cmm, s))) return rc;
-            if ((rc = Ops<T>::cd(ns, 2, wake[m], gwake[m], fs, area, sigma, &cdm, s))) return rc;
+        for (int m = 0; m < nsurf; m++, r += 7) {
+            const T area = (T)r[1], mac = (T)(r[5] / r[1]);
+            const T clm = (T)(r[0] / ((double)((T)0.5 * rho * v2 * area)));
+            const double d = (double)((T)0.5 * rho * v2 * area * mac);
+            const T cdm = (T)(r[6] / (v2d * (double)area));
             cl += clm * area;
             cdn += cdm * area;
-            for (int k = 0; k < 3; k++) cm[k] += cmm[k] * area * mac;
+            for (int k = 0; k < 3; k++) cm[k] += (T)(r[2 + k] / d) * area * mac;
             ta += area;
             tm += mac;
         }
         out->cl = (double)(cl / ta);
         out->cdi = (double)(cdn / ta);
         for (int k = 0; k < 3; k++) out->cm[k] = (double)(cm[k] / (ta * tm));
-        if (gamma_out) {
-            std::vector<T> h(n);
-            GB_CUDA(cudaMemcpyAsync(h.data(), rhs, sizeof(T) * n, cudaMemcpyDeviceToHost, st));
-            GB_CUDA(cudaStreamSynchronize(st));
-            for (int64_t i = 0; i < n; i++) gamma_out[i] = (double)h[i];
-        }
-        return lu_solve_check(lu, st);  // the solve finished its bounded waits
+        if (gamma_out)
+            for (int64_t i = 0; i < n; i++) gamma_out[i] = (double)g[i];
+        return lu_solve_verdict(lu, (const int*)h, st);  // the solve finished its bounded waits
     }
 
     int run(double alpha_d, double beta_d, double u_inf_d, double rho_d, const double* ref_pt, gbvlm_coeffs* out,
@@ -317,56 +440,69 @@ __device__ T akima_at(const T* x, const T* y, const T* m, const T* s, int n, T x
     return y[i] + s[i] * dxx + c * dxx * dxx + d * dxx * dxx * dxx;
 }
 
-// panel velocities of a surface from its strip angles (vlm.cpp:186-196:
-// freestream(u_inf, alpha_strip, 0), one value per spanwise strip)
-template <class T>
-__global__ void k_strip_vel(T* vel, const T* strip, int64_t ns, int64_t nc, T u) {
-    const int64_t np = ns * nc, p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (p >= np) return;
-    const T a = strip[p % ns];
-    vel[p] = u * cos(a);
-    vel[np + p] = (T)0;
-    vel[2 * np + p] = u * sin(a);
-}
+// a strip per thread: its circulation differences and forces, its CL about its
+// own lift axis, the effective angle and the correction toward the polar
+// (vlm.cpp:257-276); *err = the sum of |correction| over all surfaces
+constexpr int STRIP_THREADS = 32;
 
-// one CTA per surface: for every spanwise strip its CL about the strip's own
-// lift axis, the effective angle and the correction toward the polar
-// (vlm.cpp:257-276); err_out = the surface's sum of |correction|
 template <class T>
-__global__ void __launch_bounds__(256) k_strip_correct(T* strip, const T* forces, const T* areas, int64_t ns, int64_t nc,
-                                                       T alpha, T beta, T u, T rho, const T* tx, const T* ty,
-                                                       const T* tm, const T* ts, int ntab, double* err_out) {
-    __shared__ double red[256];
-    const int64_t np = ns * nc;
+__global__ void __launch_bounds__(STRIP_THREADS) k_strip_correct(SteadyArgs<T> a, T alpha, T beta, T u, T rho,
+                                                                 const T* tx, const T* ty, const T* tm, const T* ts,
+                                                                 int ntab, double* err) {
+    __shared__ bool last;
     const T two_pi = (T)(2.0f * 3.141593f);  // 2 PI_f with the reference's float pi (vlm_types.hpp:22)
+    const int64_t q = blockIdx.x * (int64_t)STRIP_THREADS + threadIdx.x;
     double e = 0;
-    for (int64_t i = threadIdx.x; i < ns; i += blockDim.x) {
-        const T a = strip[i];
+    if (q < a.soff[a.n]) {
+        int m = 0;
+        while (m + 1 < a.n && q >= a.soff[m + 1]) m++;
+        const int64_t i = q - a.soff[m], ns = a.ns[m], nc = a.nc[m];
+        const T* x = a.rhs + a.poff[m];
+        const T al = a.strip[q];
         // FlowData of the strip (vlm_utils.cpp:5-19): freestream and lift axis
-        const T fx = u * cos(a) * cos(beta), fy = -(u * cos(a) * sin(beta)), fz = u * sin(a);
+        const T fx = u * cos(al) * cos(beta), fy = -(u * cos(al) * sin(beta)), fz = u * sin(al);
         T lx = -fz, lz = fx;
         const T ll = sqrt(lx * lx + lz * lz);
         lx /= ll;
         lz /= ll;
+        const V3<T> V{u * cos(al), (T)0, u * sin(al)};
         T fl = 0, area = 0;
         for (int64_t j = 0; j < nc; j++) {
-            const int64_t p = i + j * ns;
-            fl += forces[p] * lx + forces[2 * np + p] * lz;  // the lift axis has no y component
-            area += areas[p];
+            V3<T> v0, v1;
+            const V3<T> F = steady_force(x, (const T*)a.verts[m], ns, nc, i, j, V, v0, v1);
+            fl += F.x * lx + F.z * lz;  // the lift axis has no y component
+            area += a.areas[m][i + j * ns];
         }
         const T cl = fl / ((T)0.5 * rho * (fx * fx + fy * fy + fz * fz) * area);
-        const T eff = cl / two_pi - a + alpha;
+        const T eff = cl / two_pi - al + alpha;
         const T corr = (akima_at<T>(tx, ty, tm, ts, ntab, eff) - cl) / two_pi;
-        strip[i] = a + corr;
-        e += fabs((double)corr);
+        a.strip[q] = al + corr;
+        e = fabs((double)corr);
     }
-    red[threadIdx.x] = e;
+    auto lanes = [&](double y) {
+#pragma unroll
+        for (int d = 16; d > 0; d >>= 1) y += __shfl_xor_sync(0xffffffffu, y, d);
+        return y;
+    };
+    e = lanes(e);
+    if (threadIdx.x == 0) {
+        a.part[blockIdx.x] = e;
+        __threadfence();
+        last = atomicInc(a.done, gridDim.x - 1) == gridDim.x - 1;
+    }
     __syncthreads();
-    for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-        if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *err_out = red[0];
+    if (!last) return;
+    __threadfence();
+    CSum s;
+    for (int64_t b = threadIdx.x; b < gridDim.x; b += STRIP_THREADS) s.add(__ldcg(a.part + b));
+    e = lanes(s.value());
+    if (threadIdx.x == 0) *err = e;
+}
+
+template <class T>
+__global__ void k_fill(T* v, int64_t n, T x) {
+    const int64_t p = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (p < n) v[p] = x;
 }
 
 struct NlvlmBase {
@@ -380,7 +516,8 @@ template <class T>
 struct NlvlmState : NlvlmBase {
     VlmState<T> w;  // wing, wake, AIC and per-panel buffers of the steady simulation
     void* mem = nullptr;
-    std::vector<T*> strip;
+    T* strip = nullptr;  // angles, all surfaces' strips
+    int64_t strips = 0;
     double* d_err = nullptr;
     T* tab = nullptr;  // x, y, m, s of the polar
     int32_t tab_cap = 0;
@@ -393,15 +530,11 @@ struct NlvlmState : NlvlmBase {
     int init(int32_t ns_, const gbvlm_dims* d, const float* const* vinit) {
         int rc = w.init(ns_, d, vinit);
         if (rc) return rc;
-        int64_t strips = 0;
         for (auto& x : w.dims) strips += x.ns;
-        GB_CUDA(cudaMalloc(&mem, sizeof(T) * strips + sizeof(double) * w.nsurf + 256));
+        GB_CUDA(cudaMalloc(&mem, 256 + sizeof(T) * strips));
         d_err = (double*)mem;
-        T* p = (T*)((char*)mem + ((sizeof(double) * w.nsurf + 255) / 256) * 256);
-        for (auto& x : w.dims) {
-            strip.push_back(p);
-            p += x.ns;
-        }
+        strip = (T*)((char*)mem + 256);
+        w.sa.strip = strip;
         return GBVLM_OK;
     }
 
@@ -412,7 +545,8 @@ struct NlvlmState : NlvlmBase {
         const int32_t nsurf = w.nsurf;
         const T alpha = (T)alpha_d, beta = (T)beta_d, u = (T)u_inf_d, rho = (T)rho_d;
         // the polar's Akima coefficients (tinyinterpolate.hpp:29-54), as the reference builds them on the host
-        std::vector<T> tx(ndb), ty(ndb), tm(ndb - 1), ts(ndb);
+        std::vector<T> table(4 * ndb);  // x, y, m, s as in `tab`
+        T *tx = table.data(), *ty = tx + ndb, *tm = ty + ndb, *ts = tm + ndb;
         for (int i = 0; i < ndb; i++) {
             tx[i] = (T)db_alpha[i];
             ty[i] = (T)db_cl[i];
@@ -437,101 +571,50 @@ struct NlvlmState : NlvlmBase {
         T* dy = tab + ndb;
         T* dm = tab + 2 * ndb;
         T* dsp = tab + 3 * ndb;
-        GB_CUDA(cudaMemcpyAsync(dx, tx.data(), sizeof(T) * ndb, cudaMemcpyHostToDevice, st));
-        GB_CUDA(cudaMemcpyAsync(dy, ty.data(), sizeof(T) * ndb, cudaMemcpyHostToDevice, st));
-        GB_CUDA(cudaMemcpyAsync(dm, tm.data(), sizeof(T) * (ndb - 1), cudaMemcpyHostToDevice, st));
-        GB_CUDA(cudaMemcpyAsync(dsp, ts.data(), sizeof(T) * ndb, cudaMemcpyHostToDevice, st));
+        GB_CUDA(cudaMemcpyAsync(tab, tx, sizeof(T) * 4 * ndb, cudaMemcpyHostToDevice, st));  // (pageable: staged at return)
         // the wing with its 100-chord wake row and the factored AIC (vlm.cpp:201-217)
-        GB_CUDA(cudaMemsetAsync(w.lhs, 0, sizeof(T) * w.n * w.n, st));
-        for (int m = 0; m < nsurf; m++) {
-            const int64_t nv = (w.dims[m].ns + 1) * (w.dims[m].nc + 1);
-            GB_CUDA(cudaMemcpyAsync(w.verts[m], w.verts_init[m], sizeof(T) * 4 * nv, cudaMemcpyDeviceToDevice, st));
-        }
-        T tr[16] = {1, 0, 0, 0, 0, 1, 0, 0, 0, 0, 1, 0, (T)-100 * u * (T)cos(alpha), 0, (T)-100 * u * (T)sin(alpha), 1};
-        for (int m = 0; m < nsurf; m++)
-            GB_CUDA(cudaMemcpyAsync(w.transform[m], tr, sizeof(tr), cudaMemcpyHostToDevice, st));
-        std::vector<const T*> cverts(w.verts.begin(), w.verts.end()), cinit(w.verts_init.begin(), w.verts_init.end()),
-            ctr(w.transform.begin(), w.transform.end()), ccol(w.colloc.begin(), w.colloc.end()),
-            cnor(w.normals.begin(), w.normals.end()), cwake(w.wake.begin(), w.wake.end()),
-            cvel(w.vel.begin(), w.vel.end());
+        T tr[16];
         int rc;
-        if ((rc = Ops<T>::shed(nsurf, w.dims.data(), cverts.data(), w.wake.data(), 0, s))) return rc;
-        if ((rc = Ops<T>::displace(nsurf, w.dims.data(), ctr.data(), w.verts.data(), cinit.data(), s))) return rc;
-        if ((rc = Ops<T>::shed(nsurf, w.dims.data(), cverts.data(), w.wake.data(), 1, s))) return rc;
-        if ((rc = Ops<T>::metrics(alpha, nsurf, w.dims.data(), cverts.data(), w.colloc.data(), w.normals.data(),
-                                  w.areas.data(), s)))
-            return rc;
-        if ((rc = Ops<T>::lhs(w.lhs, w.n, nsurf, w.dims.data(), ccol.data(), cnor.data(), cverts.data(),
-                              cwake.data(), 1, (T)0, s)))
-            return rc;
-        if ((rc = Ops<T>::factor(w.lu, w.lhs, w.n, s))) return rc;
-        for (int m = 0; m < nsurf; m++) {
-            std::vector<T> a0(w.dims[m].ns, alpha);
-            GB_CUDA(cudaMemcpyAsync(strip[m], a0.data(), sizeof(T) * a0.size(), cudaMemcpyHostToDevice, st));
-            GB_CUDA(cudaStreamSynchronize(st));  // a0 goes out of scope
-        }
-        auto velocities = [&]() -> int {
-            for (int m = 0; m < nsurf; m++) {
-                const int64_t np = w.dims[m].ns * w.dims[m].nc;
-                k_strip_vel<T><<<(unsigned)cdiv(np, 256), 256, 0, st>>>(w.vel[m], strip[m], w.dims[m].ns,
-                                                                        w.dims[m].nc, u);
-                GB_LAUNCH_CHECK();
-            }
-            return GBVLM_OK;
-        };
-        std::vector<double> herr(nsurf);
+        if ((rc = w.assemble(alpha, u, tr, s, st))) return rc;
+        k_fill<T><<<(unsigned)cdiv(strips, 128), 128, 0, st>>>(strip, strips, alpha);
+        GB_LAUNCH_CHECK();
+        double* herr = (double*)host_scratch(sizeof(double) * (1 + 7 * nsurf) + sizeof(T) * strips);
+        GB_REQUIRE(herr != nullptr, "pinned host allocation failed");
         double err = 1.0;
         int32_t it = 0;
         for (; it < max_iter && err > tol; it++) {
-            if ((rc = velocities())) return rc;
-            GB_CUDA(cudaMemsetAsync(w.rhs, 0, sizeof(T) * w.n, st));
-            if ((rc = Ops<T>::rhsv(w.rhs, nsurf, w.dims.data(), cnor.data(), cvel.data(), s))) return rc;
+            k_vlm_rhs<T><<<(unsigned)cdiv(w.n, LOAD_THREADS), LOAD_THREADS, 0, st>>>(w.sa, true, u);
+            GB_LAUNCH_CHECK();
             if ((rc = Ops<T>::solve(w.lu, w.lhs, w.n, w.rhs, s))) return rc;
-            int64_t off = 0;
-            for (int m = 0; m < nsurf; m++) {
-                const int64_t ns = w.dims[m].ns, nc = w.dims[m].nc;
-                if ((rc = Ops<T>::gupd(ns, nc, w.rhs + off, w.gamma[m], w.gdelta[m], w.gwake[m], s))) return rc;
-                if ((rc = Ops<T>::forces(ns, nc, w.verts[m], w.gdelta[m], w.vel[m], w.forces[m], s))) return rc;
-                k_strip_correct<T><<<1, 256, 0, st>>>(strip[m], w.forces[m], w.areas[m], ns, nc, alpha, beta, u, rho,
-                                                      dx, dy, dm, dsp, ndb, d_err + m);
-                GB_LAUNCH_CHECK();
-                off += ns * nc;
-            }
-            GB_CUDA(cudaMemcpyAsync(herr.data(), d_err, sizeof(double) * nsurf, cudaMemcpyDeviceToHost, st));
+            k_strip_correct<T><<<(unsigned)cdiv(strips, STRIP_THREADS), STRIP_THREADS, 0, st>>>(
+                w.sa, alpha, beta, u, rho, dx, dy, dm, dsp, ndb, d_err);
+            GB_LAUNCH_CHECK();
+            GB_CUDA(cudaMemcpyAsync(herr, d_err, sizeof(double), cudaMemcpyDeviceToHost, st));
             GB_CUDA(cudaStreamSynchronize(st));
-            err = 0;
-            for (int m = 0; m < nsurf; m++) err += herr[m];
+            err = *herr;
             err /= (double)w.n;  // per panel, as the reference normalises
         }
-        if (strip_out) {
-            int64_t o = 0;
-            for (int m = 0; m < nsurf; m++) {
-                std::vector<T> h(w.dims[m].ns);
-                GB_CUDA(cudaMemcpyAsync(h.data(), strip[m], sizeof(T) * h.size(), cudaMemcpyDeviceToHost, st));
-                GB_CUDA(cudaStreamSynchronize(st));
-                for (auto v : h) strip_out[o++] = (float)v;
-            }
-        }
+        T* hs = (T*)(herr + 1 + 7 * nsurf);
+        if (strip_out) GB_CUDA(cudaMemcpyAsync(hs, strip, sizeof(T) * strips, cudaMemcpyDeviceToHost, st));
         // final loads with the strips back at alpha (vlm.cpp:281-291)
-        for (int m = 0; m < nsurf; m++) {
-            std::vector<T> a0(w.dims[m].ns, alpha);
-            GB_CUDA(cudaMemcpyAsync(strip[m], a0.data(), sizeof(T) * a0.size(), cudaMemcpyHostToDevice, st));
-            GB_CUDA(cudaStreamSynchronize(st));
-        }
-        if ((rc = velocities())) return rc;
         T fs[3] = {u * (T)cos(alpha) * (T)cos(beta), -(u * (T)cos(alpha) * (T)sin(beta)), u * (T)sin(alpha)};
         T la[3] = {-fs[2], (T)0, fs[0]};
         const T ll = (T)sqrt(la[0] * la[0] + la[2] * la[2]);
         la[0] /= ll;
         la[2] /= ll;
+        for (int k = 0; k < 3; k++) w.sa.la[k] = la[k];
+        k_vlm_loads<T><<<(unsigned)w.lift_blocks, LOAD_THREADS, 0, st>>>(w.sa, false, true, u, alpha);
+        GB_LAUNCH_CHECK();
+        GB_CUDA(cudaMemcpyAsync(herr + 1, w.sa.out, sizeof(double) * 7 * nsurf, cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaStreamSynchronize(st));
+        if (strip_out)
+            for (int64_t i = 0; i < strips; i++) strip_out[i] = (float)hs[i];
+        const T v2 = fs[0] * fs[0] + fs[1] * fs[1] + fs[2] * fs[2];
         T cl = 0, ta = 0;
         for (int m = 0; m < nsurf; m++) {
-            const int64_t ns = w.dims[m].ns, nc = w.dims[m].nc;
-            if ((rc = Ops<T>::forces(ns, nc, w.verts[m], w.gdelta[m], w.vel[m], w.forces[m], s))) return rc;
-            T area, clm;
-            if ((rc = Ops<T>::sum(w.areas[m], ns * nc, &area, s))) return rc;
-            if ((rc = Ops<T>::cl(ns, nc, w.forces[m], la, fs, rho, area, &clm, s))) return rc;
-            cl += clm * area;
+            const double* r = herr + 1 + 7 * m;
+            const T area = (T)r[1];
+            cl += (T)(r[0] / ((double)((T)0.5 * rho * v2 * area))) * area;
             ta += area;
         }
         *cl_out = (double)(cl / ta);

@@ -87,9 +87,16 @@ int lu_factor_pivoting_f64(gbvlm_lu h, double* A, int64_t n, cudaStream_t st);
 int lu_solve_prepare_f32(gbvlm_lu h, const float* A, int64_t n, float* X, void** tables, cudaStream_t st);
 int lu_solve_prepared_f32(gbvlm_lu h, void* tables, int64_t n, cudaStream_t st);
 void lu_solve_tables_free(void* tables);
+// share of the chord vector from mid-span quarter chord to the collocation point
+float aoa_factor(float alpha);
+double aoa_factor(double alpha);
 // GBVLM_OK, or an error if a bounded wait of a float solve since the last
 // factorisation ran out (synchronises st)
 int lu_solve_check(gbvlm_lu h, cudaStream_t st);
+// the same in two parts around the caller's own wait: the error words on their
+// way to `words` (2, pinned), and once they are there the verdict on them
+int lu_solve_words(gbvlm_lu h, int* words, cudaStream_t st);
+int lu_solve_verdict(gbvlm_lu h, const int* words, cudaStream_t st);
 // rhs -= wake influence with *it_dev active ring rows per lifting wake
 // (it_dev <= it_max); scratch of WAKE_DEV_MAX_SLICES x (total panels) floats
 constexpr int64_t WAKE_DEV_MAX_SLICES = 608;

@@ -3514,16 +3514,10 @@ int lu_plan_build(LuPlan& plan, const std::vector<int64_t>& n_sorted, cudaStream
     return GBVLM_OK;
 }
 
-int lu_plan_check(const LuPlan& plan, cudaStream_t st) {
-    if (!plan.d_err) return GBVLM_OK;
-    int* h = (int*)host_scratch(sizeof(int));
-    GB_CUDA(cudaMemcpyAsync(h, plan.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaStreamSynchronize(st));
-    if (*h != 0) {
-        set_error("LU: a tensor-core update tile timed out waiting for its MMAs");
-        return GBVLM_ERR_CUDA;
-    }
-    return GBVLM_OK;
+int lu_plan_verdict(int word) {
+    if (word == 0) return GBVLM_OK;
+    set_error("LU: a tensor-core update tile timed out waiting for its MMAs");
+    return GBVLM_ERR_CUDA;
 }
 
 int64_t lu_plan_launches(const LuPlan& plan, int es) {
@@ -3811,17 +3805,34 @@ static int lu_one_ready(gbvlm_lu h, int64_t bytes, cudaStream_t st) {
     return GBVLM_OK;
 }
 
-// GBVLM_OK, or an error if a wait of a single-column solve ran out (synchronises st)
-static int lu_one_check(gbvlm_lu h, cudaStream_t st) {
-    if (!h->one) return GBVLM_OK;
-    int* e = (int*)host_scratch(sizeof(int));
-    GB_CUDA(cudaMemcpyAsync(e, h->one, sizeof(int), cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaStreamSynchronize(st));
-    if (*e == 0) return GBVLM_OK;
-    GB_CUDA(cudaMemsetAsync(h->one, 0, ONE_Y, st));  // the counters of the solve that gave up
+namespace gbvlm {
+
+int lu_solve_words(gbvlm_lu h, int* words, cudaStream_t st) {
+    GB_REQUIRE(h && words, "null argument");
+    words[0] = words[1] = 0;
+    if (h->one) GB_CUDA(cudaMemcpyAsync(words, h->one, sizeof(int), cudaMemcpyDeviceToHost, st));
+    if (h->flow_n >= 0 && h->flow.d_ctl)
+        GB_CUDA(cudaMemcpyAsync(words + 1, h->flow.d_ctl + 1, sizeof(int), cudaMemcpyDeviceToHost, st));
+    return GBVLM_OK;
+}
+
+int lu_solve_verdict(gbvlm_lu h, const int* words, cudaStream_t st) {
+    if (words[0] != 0) GB_CUDA(cudaMemsetAsync(h->one, 0, ONE_Y, st));  // the counters of the solve that gave up
+    if (words[0] == 0 && words[1] == 0) return GBVLM_OK;
     set_error("triangular solve: a block timed out waiting for the blocks it depends on");
     return GBVLM_ERR_CUDA;
 }
+
+int lu_solve_check(gbvlm_lu h, cudaStream_t st) {
+    int* w = (int*)host_scratch(2 * sizeof(int));
+    GB_REQUIRE(w != nullptr, "pinned host allocation failed");
+    const int rc = lu_solve_words(h, w, st);
+    if (rc) return rc;
+    GB_CUDA(cudaStreamSynchronize(st));
+    return lu_solve_verdict(h, w, st);
+}
+
+}  // namespace gbvlm
 
 // one right-hand side by k_trs_one: systems beyond ONE_MIN unknowns, unless
 // GBVLM_TRS_FLOW=0 selects the one-CTA solve
@@ -3898,7 +3909,17 @@ static int lu_factor_one(gbvlm_lu h, T* A, int64_t n, int64_t ld, cudaStream_t s
     LuBatch<T> B;
     rc = make_single_batch<T>(B, n, ld, A, h->d_ipiv, h->d_perm, h->d_info, nullptr, 0, 0, &h->work, &h->work_bytes, st);
     if (rc) return rc;
-    int32_t* hi = (int32_t*)host_scratch(2 * sizeof(int32_t));
+    int32_t* hi = (int32_t*)host_scratch(5 * sizeof(int32_t));  // info, needs interchanges, solve words, tile word
+    GB_REQUIRE(hi != nullptr, "pinned host allocation failed");
+    auto read = [&](int words) -> int {
+        hi[4] = 0;
+        GB_CUDA(cudaMemcpyAsync(hi, h->d_info, words * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+        const int r = lu_solve_words(h, hi + 2, st);
+        if (r) return r;
+        if (h->plan.d_err) GB_CUDA(cudaMemcpyAsync(hi + 4, h->plan.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaStreamSynchronize(st));
+        return GBVLM_OK;
+    };
     bool done = false;
     // without interchanges first; single-block systems' panel tries that itself
     const bool fast =
@@ -3909,8 +3930,7 @@ static int lu_factor_one(gbvlm_lu h, T* A, int64_t n, int64_t ld, cudaStream_t s
         rc = lu_batch_factor_fast<T>(B, h->plan, st, true);
         B.fail = nullptr;
         if (rc) return rc;
-        GB_CUDA(cudaMemcpyAsync(hi, h->d_info, 2 * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        GB_CUDA(cudaStreamSynchronize(st));
+        if ((rc = read(2))) return rc;
         done = hi[1] == 0;
         if (!done)
             GB_CUDA(cudaMemcpy2DAsync(A, sizeof(T) * ld, h->backup, sizeof(T) * n, sizeof(T) * n, n,
@@ -3918,17 +3938,15 @@ static int lu_factor_one(gbvlm_lu h, T* A, int64_t n, int64_t ld, cudaStream_t s
     }
     if (!done) {
         rc = lu_batch_factor<T>(B, h->plan, st, true);
-        if (rc) return rc;
-        GB_CUDA(cudaMemcpyAsync(hi, h->d_info, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        GB_CUDA(cudaStreamSynchronize(st));
+        if (rc || (rc = read(1))) return rc;
     }
     if (*hi != 0) {
         set_error("LU: exactly zero pivot at column %d", *hi);
         return GBVLM_ERR_SINGULAR;
     }
-    if (h->flow_n >= 0 && (rc = trs_flow_check(h->flow, st))) return rc;  // a solve since the last factorisation
-    if ((rc = lu_one_check(h, st))) return rc;
-    return lu_plan_check(h->plan, st);
+    // the words read beside info: a tile of this factorisation, and the solves since the last one
+    if ((rc = lu_solve_verdict(h, hi + 2, st))) return rc;
+    return lu_plan_verdict(hi[4]);
 }
 
 template <class T>
@@ -3991,13 +4009,6 @@ int lu_solve_prepared_f32(gbvlm_lu h, void* tables, int64_t n, cudaStream_t st) 
     if (t->one_A) return lu_solve_column<float>(h, t->one_A, n, n, t->one_X, st);
     if (t->flow && h->flow_n == n) return trs_flow_solve(t->B, h->flow, 1, st);
     return lu_batch_solve<float>(t->B, 1, 1, n, st, h->plan.tc_passes ? h->plan.d_err : nullptr);
-}
-
-int lu_solve_check(gbvlm_lu h, cudaStream_t st) {
-    GB_REQUIRE(h, "null argument");
-    const int rc = lu_one_check(h, st);
-    if (rc) return rc;
-    return h->flow_n >= 0 ? trs_flow_check(h->flow, st) : GBVLM_OK;
 }
 
 void lu_solve_tables_free(void* tables) {

@@ -17,6 +17,7 @@
 #include <vector>
 
 #include "gbvlm_internal.h"
+#include "gbvlm_loads.cuh"
 #include "gbvlm_math.cuh"
 #include "gbvlm_walk.cuh"
 
@@ -150,14 +151,10 @@ __global__ void k_mesh_metrics(Surfs<T> s, T factor) {
     col[2 * np + p] = cp.z;
 }
 
-template <class T>
-static T aoa_factor(T alpha);
-template <>
-float aoa_factor<float>(float alpha) {
+float aoa_factor(float alpha) {
     return (alpha < EPS_F) ? 0.5f : 0.5f * (alpha / (sinf(alpha) + EPS_F));
 }
-template <>
-double aoa_factor<double>(double alpha) {
+double aoa_factor(double alpha) {
     return (alpha < (double)EPS_F) ? 0.5 : 0.5 * (alpha / (sin(alpha) + (double)EPS_F));
 }
 
@@ -175,7 +172,7 @@ static int mesh_metrics(T alpha, int32_t nsurf, const gbvlm_dims* dims, const T*
         s.o2[m] = areas[m];
     }
     int64_t n = s.poff[nsurf];
-    k_mesh_metrics<T><<<(unsigned)cdiv(n, 256), 256, 0, st>>>(s, aoa_factor<T>(alpha));
+    k_mesh_metrics<T><<<(unsigned)cdiv(n, 256), 256, 0, st>>>(s, aoa_factor(alpha));
     GB_LAUNCH_CHECK();
     return GBVLM_OK;
 }
@@ -793,19 +790,6 @@ __global__ void k_forces(int64_t ns, int64_t nc, const T* vw, const T* gd, const
 // ---------------------------------------------------------------------------
 constexpr int RED_THREADS = 512;
 
-__device__ __forceinline__ double block_sum(double v, double* sh) {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    if (lane == 0) sh[wid] = v;
-    __syncthreads();
-    double r = 0;
-    if (threadIdx.x == 0) {
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) r += sh[k];
-    }
-    __syncthreads();
-    return r;
-}
-
 // kind 0: cl = sum F.L ; kind 1: cm = sum (0.5(v0+v1) - ref) x F ; kind 2: sum x ; kind 3: mac numerator
 template <class T>
 __global__ void __launch_bounds__(RED_THREADS) k_reduce(int kind, int64_t ns, int64_t nc, const T* x, const T* vw,
@@ -966,30 +950,11 @@ __global__ void k_gamma_update(int64_t ns, int64_t nc, const T* x, T* g, T* gd, 
 // ---------------------------------------------------------------------------
 // Trefftz-plane drag (ispc:273-323): one block per spanwise ring
 // ---------------------------------------------------------------------------
-template <class T, bool SIGMA>
-__global__ void k_trefftz(int64_t nv, int64_t nwv, const T* v, const T* gam, T sigma2, double* partial) {
+template <class T>
+__global__ void k_trefftz(int64_t nv, int64_t nwv, const T* v, const T* gam, T sigma, double* partial) {
     __shared__ double sh[32];
-    const int64_t i = nwv - 2, ld = nv * nwv;
-    const int64_t j = blockIdx.x;
-    auto P = [&](int64_t idx) { return V3<T>{v[idx], v[ld + idx], v[2 * ld + idx]}; };
-    V3<T> a = P(i * nv + j), b = P(i * nv + j + 1), d = P((i + 1) * nv + j + 1), e = P((i + 1) * nv + j);
-    V3<T> c = (T)0.25 * (((a + b) + d) + e);
-    V3<T> nn = cross(e - b, d - a);
-    T l = dsqrt(len2(nn));
-    V3<T> n{nn.x / l, nn.y / l, nn.z / l};
-    double acc = 0;
-    for (int64_t jj = threadIdx.x; jj < nv - 1; jj += blockDim.x) {
-        V3<T> w0 = P(i * nv + jj), w1 = P(i * nv + jj + 1), w2 = P((i + 1) * nv + jj + 1), w3 = P((i + 1) * nv + jj);
-        V3<T> inf2{0, 0, 0};
-        symmetry_ref(inf2, c, w1, w2, (T)sqrt((double)sigma2));
-        symmetry_ref(inf2, c, w3, w0, (T)sqrt((double)sigma2));
-        acc += (double)gam[i * (nv - 1) + jj] * (double)dot(inf2, n);
-    }
-    double iv = block_sum(acc, sh);
-    if (threadIdx.x == 0) {
-        V3<T> dl = b - a;
-        partial[j] = -(double)gam[i * (nv - 1) + j] * iv * sqrt((double)len2(dl));
-    }
+    const double d = trefftz_ring(nv, nwv, v, gam, sigma, (int64_t)blockIdx.x, sh);
+    if (threadIdx.x == 0) partial[blockIdx.x] = d;
 }
 
 __global__ void k_sum_partials(const double* p, int64_t n, double* out) {
@@ -1009,10 +974,7 @@ static int trefftz(int64_t ns, int64_t nwv, const T* vk, const T* gw, const T* f
     int rc = device_scratch(sizeof(double) * (ns + 2), &d, st);
     if (rc) return rc;
     double* part = (double*)d;
-    if (sigma != (T)0)
-        k_trefftz<T, true><<<(unsigned)ns, 128, 0, st>>>(ns + 1, nwv, vk, gw, sigma * sigma, part);
-    else
-        k_trefftz<T, false><<<(unsigned)ns, 128, 0, st>>>(ns + 1, nwv, vk, gw, (T)0, part);
+    k_trefftz<T><<<(unsigned)ns, 128, 0, st>>>(ns + 1, nwv, vk, gw, (T)sqrt((double)(sigma * sigma)), part);
     GB_LAUNCH_CHECK();
     k_sum_partials<<<1, 256, 0, st>>>(part, ns, part + ns);
     GB_LAUNCH_CHECK();

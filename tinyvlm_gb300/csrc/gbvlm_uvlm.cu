@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "gbvlm_internal.h"
+#include "gbvlm_loads.cuh"
 #include "gbvlm_math.cuh"
 
 namespace gbvlm {
@@ -57,7 +58,7 @@ struct StepArgs {
     double* out = nullptr;                  // [step][4]: CL, CM
     T inv_dt = 0;
     double rho = 1;
-    double* part = nullptr;    // [step_load_blocks][6]
+    double* part = nullptr;    // [step_load_blocks][LOAD_PART]
     unsigned* done = nullptr;  // blocks finished, zero between launches
     const int64_t* idx = nullptr;
     bool by_step = true;
@@ -72,8 +73,7 @@ struct StepArgs {
     }
 };
 
-constexpr int STEP_THREADS = 128;
-constexpr int STEP_CHORDS = STEP_THREADS - 1;  // strips of a chord block (a strip needs two chords)
+constexpr int STEP_THREADS = LOAD_THREADS;
 
 template <class T>
 static void step_dims(StepArgs<T>& a, const std::vector<gbvlm_dims>& dims) {
@@ -88,7 +88,7 @@ static void step_dims(StepArgs<T>& a, const std::vector<gbvlm_dims>& dims) {
 
 static int64_t step_load_blocks(const std::vector<gbvlm_dims>& dims) {
     int64_t b = 0;
-    for (auto& d : dims) b += cdiv(d.ns * d.nc, STEP_THREADS) + cdiv(d.ns, STEP_CHORDS);
+    for (auto& d : dims) b += cdiv(d.ns * d.nc, STEP_THREADS) + cdiv(d.ns, LOAD_CHORDS);
     return b;
 }
 
@@ -127,66 +127,25 @@ __global__ void __launch_bounds__(STEP_THREADS) k_step_start(StepArgs<T> a, int6
     }
 }
 
-// verts = T vpos and the metrics of the moved panels (k_displace, then
-// k_mesh_metrics with the collocation point at 3/4 chord): a panel's thread
-// moves its four corners and writes the one at its origin, the last strip and
-// row those beyond.
+// verts = T vpos and the metrics of the moved panels, the collocation point at 3/4 chord
 template <class T>
 __global__ void __launch_bounds__(STEP_THREADS) k_step_move(StepArgs<T> a, int64_t step) {
     const int64_t g = blockIdx.x * (int64_t)STEP_THREADS + threadIdx.x;
     if (g >= a.poff[a.n]) return;
     const int m = a.surf(g);
     const T* tr = a.Tm + (a.by_step ? 16 * a.n * (a.at(step) + 1) : 0) + 16 * m;
-    const int64_t p = g - a.poff[m], ns = a.ns[m], nc = a.nc[m], np = ns * nc, vld = (ns + 1) * (nc + 1);
-    const int64_t j = p / ns, i = p - j * ns, v = i + j * (ns + 1);
-    const T* in = a.vpos[m];
-    T* out = a.verts[m];
-    auto move = [&](int64_t q, bool write) {
-        T x[4] = {in[q], in[vld + q], in[2 * vld + q], in[3 * vld + q]}, y[4];
-#pragma unroll
-        for (int c = 0; c < 4; c++) {
-            T acc = 0;
-#pragma unroll
-            for (int k = 0; k < 4; k++) acc += x[k] * tr[c + 4 * k];
-            y[c] = acc;
-            if (write) out[c * vld + q] = acc;
-        }
-        return V3<T>{y[0], y[1], y[2]};
-    };
-    const bool lc = i == ns - 1, lr = j == nc - 1;
-    const V3<T> v0 = move(v, true), v1 = move(v + 1, lc), v2 = move(v + ns + 2, lc && lr), v3_ = move(v + ns + 1, lr);
-    const V3<T> nn = cross(v3_ - v1, v2 - v0);
-    const T l = dsqrt(len2(nn));
-    T *col = a.colloc[m], *nor = a.normals[m];
-    nor[p] = nn.x / l;
-    nor[np + p] = nn.y / l;
-    nor[2 * np + p] = nn.z / l;
-    const V3<T> f = v3_ - v0, bb = v2 - v0, e = v1 - v0;
-    a.areas[m][p] = (T)0.5 * (dsqrt(len2(cross(f, bb))) + dsqrt(len2(cross(bb, e))));
-    const V3<T> ch = (T)0.5 * (((v2 + v3_) - v0) - v1);
-    const V3<T> cp = (T)0.5 * (v0 + v1) + (T)0.5 * ch;
-    col[p] = cp.x;
-    col[np + p] = cp.y;
-    col[2 * np + p] = cp.z;
+    move_panel(a.vpos[m], a.verts[m], tr, a.ns[m], a.nc[m], g - a.poff[m], (T)0.5, a.colloc[m], a.normals[m],
+               a.areas[m]);
 }
 
 // Circulation of the solution (gamma, the trailing edge's into the wake), with
 // `loads` the unsteady forces (vlm_backend_cpu.cpp:276-321) and the multibody
 // CL and CM about ref (vlm/src/vlm_backend.cpp:72-139): the sums in double,
-// out[0] cl and out[1..3] cm.
-//
-// Bound: latency.  A warp's double instruction takes about 100 cycles on this
-// device, so what a block does in double is kept short: one panel per thread,
-// six sums of a block's panels through shared memory (8 additions and 4
-// exchanges on three warps where six warp-wide trees spend 30), blocks of their
-// own for the chords (three square roots a strip), and the block that finishes
-// last adds the blocks' sums in a fixed order and forms the coefficients.  The
-// sums over all panels in a single block took 70 us a step for 1600 panels.
+// out[0] cl and out[1..3] cm.  The sums over all panels in a single block took
+// 70 us a step for 1600 panels.
 template <class T>
 __global__ void __launch_bounds__(STEP_THREADS) k_step_loads(StepArgs<T> a, int64_t step, bool loads) {
-    __shared__ double sh[6][STEP_THREADS];
-    __shared__ double tot[6];
-    __shared__ bool last;
+    __shared__ LoadShared sh;
     const int64_t it = a.at(step), o = a.by_step ? it : 0;
     const int t = threadIdx.x;
     const T *fsp = a.fs + 3 * o, *rp = a.ref + 3 * o;
@@ -195,7 +154,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_step_loads(StepArgs<T> a, int6
     bool chords = false;
     for (; m < a.n; m++) {
         const int64_t pb = (a.ns[m] * a.nc[m] + STEP_THREADS - 1) / STEP_THREADS;
-        const int64_t cb = loads ? (a.ns[m] + STEP_CHORDS - 1) / STEP_CHORDS : 0;
+        const int64_t cb = loads ? (a.ns[m] + LOAD_CHORDS - 1) / LOAD_CHORDS : 0;
         if (blk < pb) break;
         blk -= pb;
         if (blk < cb) {
@@ -208,7 +167,7 @@ __global__ void __launch_bounds__(STEP_THREADS) k_step_loads(StepArgs<T> a, int6
     const T* v = a.verts[m];
     if (!chords) {
         const int64_t p = blk * STEP_THREADS + t;
-        double s[5] = {0, 0, 0, 0, 0};
+        double s[LOAD_SUMS] = {0, 0, 0, 0, 0};
         if (p < np) {
             const int64_t j = p / ns, i = p - j * ns;
             const T* x = a.sol + a.poff[m];
@@ -241,72 +200,27 @@ __global__ void __launch_bounds__(STEP_THREADS) k_step_loads(StepArgs<T> a, int6
             if (a.keep) a.gprev[m][p] = g;
         }
 #pragma unroll
-        for (int q = 0; q < 5; q++) sh[q][t] = s[q];
+        for (int q = 0; q < LOAD_SUMS; q++) sh.s[q][t] = s[q];
     } else {
-        const int64_t i = blk * STEP_CHORDS + t, end = nc * (ns + 1);
-        double c = 0;
-        if (i <= ns) {
-            const double dx = (double)v[i] - v[end + i], dy = (double)v[vld + i] - v[vld + end + i];
-            const double dz = (double)v[2 * vld + i] - v[2 * vld + end + i];
-            c = dx * dx + dy * dy + dz * dz;
-        }
-        sh[1][t] = sqrt(c);
-        __syncthreads();
-        double s = 0;
-        if (t < STEP_CHORDS && i < ns) {
-            const double c0 = sh[1][t], c1 = sh[1][t + 1];
-            const double dx = (double)v[i + 1] - v[i], dy = (double)v[vld + i + 1] - v[vld + i];
-            const double dz = (double)v[2 * vld + i + 1] - v[2 * vld + i];
-            s = 0.5 * (c0 * c0 + c1 * c1) * sqrt(dx * dx + dy * dy + dz * dz);
-        }
-        sh[0][t] = s;
+        chord_terms(sh, v, ns, nc, blk);
     }
     if (!loads) return;
-    __syncthreads();
-    const int q = t >> 4, l = t & 15;  // 16 lanes per sum
-    auto lanes = [&](double x) {
-#pragma unroll
-        for (int d = 8; d > 0; d >>= 1) x += __shfl_xor_sync(0xffffffffu, x, d);
-        return x;
-    };
-    if (t < 96) {
-        double x = 0;
-        if (q < (chords ? 1 : 5)) {
-#pragma unroll
-            for (int k = 0; k < STEP_THREADS / 16; k++) x += sh[q][l + 16 * k];
-        }
-        x = lanes(x);
-        if (l == 0) a.part[6 * (int64_t)blockIdx.x + q] = x;
-    }
-    __threadfence();
-    __syncthreads();
-    if (t == 0) last = atomicInc(a.done, gridDim.x - 1) == gridDim.x - 1;
-    __syncthreads();
-    if (!last) return;
-    __threadfence();
+    block_sums(sh, chords ? 1 : LOAD_SUMS, a.part + LOAD_PART * (int64_t)blockIdx.x);
+    if (!last_block(sh, a.done)) return;
     double cl = 0, ta = 0, tm = 0;  // of thread t < 4: CL, CM x, y, z
     const double fx = fsp[0], fy = fsp[1], fz = fsp[2];
     const double qd = 0.5 * a.rho * (fx * fx + fy * fy + fz * fz), ll = sqrt(fz * fz + fx * fx);
     int64_t b0 = 0;
     for (int k = 0; k < a.n; k++) {
         const int64_t pb = (a.ns[k] * a.nc[k] + STEP_THREADS - 1) / STEP_THREADS;
-        const int64_t cb = (a.ns[k] + STEP_CHORDS - 1) / STEP_CHORDS;
-        if (t < 96) {
-            CSum s;
-            // sum q of the panel blocks; the sixth: the chord blocks' strips
-            const int64_t first = b0 + (q < 5 ? 0 : pb), cnt = q < 5 ? pb : cb;
-            for (int64_t e = l; e < cnt; e += 16) s.add(__ldcg(a.part + 6 * (first + e) + (q < 5 ? q : 0)));
-            const double x = lanes(s.value());
-            if (l == 0) tot[q] = x;
-        }
-        __syncthreads();
+        const int64_t cb = (a.ns[k] + LOAD_CHORDS - 1) / LOAD_CHORDS;
+        add_parts(sh, a.part, b0, pb, cb, 0);
         if (t < 4) {
-            const double S = tot[1], mac = tot[5] / S;
-            cl += t == 0 ? tot[0] / ll / (qd * S) * S : tot[1 + t] / (qd * S * mac) * S * mac;
+            const double S = sh.tot[1], mac = sh.tot[5] / S;
+            cl += t == 0 ? sh.tot[0] / ll / (qd * S) * S : sh.tot[1 + t] / (qd * S * mac) * S * mac;
             ta += S;
             tm += mac;
         }
-        __syncthreads();
         b0 += pb + cb;
     }
     if (t < 4) a.out[4 * o + t] = t == 0 ? cl / ta : cl / (ta * tm);
@@ -330,7 +244,7 @@ template <class T>
 static int step_loads(const StepArgs<T>& a, int64_t step, bool loads, cudaStream_t st) {
     int64_t blocks = 0;
     for (int m = 0; m < a.n; m++)
-        blocks += cdiv(a.ns[m] * a.nc[m], STEP_THREADS) + (loads ? cdiv(a.ns[m], STEP_CHORDS) : 0);
+        blocks += cdiv(a.ns[m] * a.nc[m], STEP_THREADS) + (loads ? cdiv(a.ns[m], LOAD_CHORDS) : 0);
     k_step_loads<T><<<(unsigned)blocks, STEP_THREADS, 0, st>>>(a, step, loads);
     GB_LAUNCH_CHECK();
     return GBVLM_OK;
@@ -519,7 +433,7 @@ struct UvlmState : UvlmBase {
         }
         bytes += al(sizeof(T) * n * n) + al(sizeof(T) * n) + 2 * al(sizeof(T) * 16 * nsurf * (t_steps + 1)) +
                  2 * al(sizeof(T) * 3 * (t_steps + 1)) + al(sizeof(double) * 4 * t_steps) +
-                 al(sizeof(double) * 6 * step_load_blocks(dims)) + al(sizeof(unsigned));
+                 al(sizeof(double) * LOAD_PART * step_load_blocks(dims)) + al(sizeof(unsigned));
         ldi = t_steps - 1 >= inv_steps<T>(n) ? inv_ld<T>(n) : 0;
         bytes += al(sizeof(T) * n * ldi) + al(sizeof(T) * ldi);
         GB_CUDA(cudaMalloc(&mem, bytes));
@@ -543,7 +457,7 @@ struct UvlmState : UvlmBase {
         res = (double*)p;
         p += al(sizeof(double) * 4 * t_steps);
         sa.part = (double*)p;
-        p += al(sizeof(double) * 6 * step_load_blocks(dims));
+        p += al(sizeof(double) * LOAD_PART * step_load_blocks(dims));
         sa.done = (unsigned*)p;
         p += al(sizeof(unsigned));
         for (auto& x : dims) {
@@ -1047,7 +961,7 @@ struct Aero2Dof {
                      al(4 * x.ns * (t_steps - 1));
         }
         bytes += al(4 * n * n) + al(4 * n) + 2 * al(4 * 16 * nsurf) + 4 * al(8 * 2 * t_steps) + al(sizeof(A2Dev)) +
-                 al(sizeof(double) * 6 * step_load_blocks(dims)) + al(sizeof(unsigned));
+                 al(sizeof(double) * LOAD_PART * step_load_blocks(dims)) + al(sizeof(unsigned));
         GB_CUDA(cudaMalloc(&mem, bytes));
         GB_CUDA(cudaMemset(mem, 0, bytes));
         char* p = (char*)mem;
@@ -1065,7 +979,7 @@ struct Aero2Dof {
         a = (double*)take(8 * 2 * t_steps);
         F = (double*)take(8 * 2 * t_steps);
         dev = (A2Dev*)take(sizeof(A2Dev));
-        sa.part = (double*)take(sizeof(double) * 6 * step_load_blocks(dims));
+        sa.part = (double*)take(sizeof(double) * LOAD_PART * step_load_blocks(dims));
         sa.done = (unsigned*)take(sizeof(unsigned));
         {
             const size_t ib = (sizeof(int32_t) * t_steps + 255) / 256 * 256;
