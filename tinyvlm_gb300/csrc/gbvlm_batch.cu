@@ -90,18 +90,22 @@ __device__ __forceinline__ void split_hl(double x, float& h, float& l) {
 }
 
 // ---------------------------------------------------------------------------
-// geometry: one block per system
+// geometry: the blocks of a system (grid y) share its vertices, wake and panels;
+// one block where the batch fills the SMs, else as many as that takes: 16384
+// panels in one block took 785 us
 // ---------------------------------------------------------------------------
 __global__ void __launch_bounds__(256) k_batch_geom(BatchArgs a) {
     SysDesc& S = a.sys[blockIdx.x];
     const int64_t ns = S.ns, nc = S.nc, nv = (ns + 1) * (nc + 1), np = ns * nc;
     const double al = S.alpha_geom;
-    if (threadIdx.x == 0 && !a.only_failed) a.fail[blockIdx.x] = 0;
+    if (threadIdx.x == 0 && blockIdx.y == 0 && !a.only_failed) a.fail[blockIdx.x] = 0;
     int bad = 0;
-    for (int64_t v = threadIdx.x; v < nv; v += blockDim.x) {
+    const int64_t t0 = threadIdx.x + blockIdx.y * (int64_t)blockDim.x, stride = gridDim.y * (int64_t)blockDim.x;
+    if (blockIdx.y == 0)
+        for (int64_t e = threadIdx.x; e < 3 * nv; e += blockDim.x) bad |= !isfinite(S.vinit[e]);
+    for (int64_t v = t0; v < nv; v += stride) {
         for (int k = 0; k < 3; k++) {
             double x = (double)S.vinit[k * nv + v];
-            bad |= !isfinite(x);
             S.vd[k * nv + v] = x;
             split_hl(x, S.vh[k * nv + v], S.vl[k * nv + v]);
         }
@@ -109,7 +113,7 @@ __global__ void __launch_bounds__(256) k_batch_geom(BatchArgs a) {
     // a case with a non-finite coordinate is reported by gbvlm_batch_results
     // (its solves come out non-finite; the other cases are unaffected)
     bad = __syncthreads_or(bad);
-    if (threadIdx.x == 0) a.bad[blockIdx.x] = bad;
+    if (threadIdx.x == 0 && blockIdx.y == 0) a.bad[blockIdx.x] = bad;
     // the angle's double trigonometry once per block (long on the fp64 units)
     __shared__ double s_trig[5];
     if (threadIdx.x == 0) {
@@ -125,7 +129,7 @@ __global__ void __launch_bounds__(256) k_batch_geom(BatchArgs a) {
     // edge, row 1 = trailing edge + 100 u (cos a, 0, sin a)
     const double dx = s_trig[0], dz = s_trig[1], ca = s_trig[3], sa = s_trig[4];
     const int64_t wl = 2 * (ns + 1);
-    for (int64_t i = threadIdx.x; i <= ns; i += blockDim.x) {
+    for (int64_t i = t0; i <= ns; i += stride) {
         const int64_t te = i + nc * (ns + 1);
         double x = S.vinit[te], y = S.vinit[nv + te], z = S.vinit[2 * nv + te];
         double w0[3] = {x, y, z}, w1[3] = {x + dx, y, z + dz};
@@ -146,10 +150,9 @@ __global__ void __launch_bounds__(256) k_batch_geom(BatchArgs a) {
             S.wd[2 * wl + o] = fma(ca, q[2], -(sa * q[0]));
         }
     }
-    __syncthreads();
     const double factor = s_trig[2];
-    const double* v = S.vd;
-    for (int64_t p = threadIdx.x; p < np; p += blockDim.x) {
+    const float* v = S.vinit;  // (S.vd is being written by all of the system's blocks)
+    for (int64_t p = t0; p < np; p += stride) {
         const int64_t i = p % ns, j = p / ns;
         const int64_t ia = i + j * (ns + 1), ib = ia + 1, ic = ib + (ns + 1), id = ia + (ns + 1);
         V3<double> v0{v[ia], v[nv + ia], v[2 * nv + ia]}, v1{v[ib], v[nv + ib], v[2 * nv + ib]};
@@ -567,53 +570,77 @@ __global__ void k_batch_accum(BatchArgs a) {
 
 // R = B - A2 Xd (B - (A2 + Alo) Xd in FP64 residual plans); X = (float)R.
 // One thread per row, tiles (system, row
-// block).  The products of the float matrix A2 with the double solution Xd
-// are accumulated in double-float arithmetic on the fp32 units (Xd split as
-// hi + lo floats, each product a*hi exact through an FMA, running sums
-// (sh, sl) kept with a compensated addition): about 2^-44 relative per term,
-// where the fp64 units of this part run at a small fraction of the fp32 rate.
+// block).
+// The products of the float matrix A2 with the double solution Xd
+// (split as hi + lo floats) are accumulated in double-float arithmetic on the
+// fp32 units, about 2^-44 relative per term, where the fp64 units of this part
+// run at a small fraction of the fp32 rate.
+//
+// Bound: the fp32 pipe.  RS_CB columns at a time are added to a bias that is 32
+// times the largest product they can form, so that the running sum stays
+// within a factor two of it and a term costs four operations instead of a
+// product, its error and a branch-free two-sum (nine): with t = s + a x rounded
+// once, t - s is exact (Sterbenz), and a x - (t - s), one FMA, is the rounding
+// error.  The bias is subtracted again (exact), and the chunk's sum joins
+// (sh, sl) by a two-sum.  16384 panels, 64 right-hand sides: 8.5 -> 6.8 ms (with the
+// columns and X fetched ahead; the arithmetic alone 8.7, waiting for them).
 constexpr int RS_THREADS = 64;
 constexpr int RS_MAXRHS = 8;  // (the inner loop reads them as two float4)
-constexpr int RS_CB = 8;  // columns of Xd staged per step
+constexpr int RS_CB = 8;  // columns of Xd staged per step (the bias allows for 8 of them)
+static_assert(RS_CB * RS_MAXRHS == RS_THREADS, "a thread stages one value");
 constexpr int RS_ROWS = 2;  // rows per thread
-
-// (sh, sl) += a * (xh + xl); XL = false: xl is zero
-template <bool XL>
-__device__ __forceinline__ void df_mac(float& sh, float& sl, float a, float xh, float xl) {
-    const float p = __fmul_rn(a, xh);
-    const float pe = __fmaf_rn(a, xh, -p);  // a*xh - p exactly
-    const float s = __fadd_rn(sh, p);
-    const float bb = __fsub_rn(s, sh);
-    const float e = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bb)), __fsub_rn(p, bb));  // sh + p - s exactly
-    sh = s;
-    sl = XL ? __fmaf_rn(a, xl, __fadd_rn(sl, __fadd_rn(e, pe))) : __fadd_rn(sl, __fadd_rn(e, pe));
-}
 
 // LO: the plan keeps the correction Alo of the stored AIC; its products with
 // the hi part of Xd join the low-order sums (Alo is about 2^-24 of A, so
 // the float product is exact to far below the residual's accuracy).
 // XL = false: Xd holds float values (the first sweep: Xd = 0 + the float
 // solve), so its lo part is zero and its products are left out.
+constexpr int RS_STAGES = 3;
+constexpr int RS_MIN_BLOCKS = 6;
+
+// 4 bytes to shared memory, asynchronously; zero where !valid (src is still an address of the matrix)
+__device__ __forceinline__ void copy4_async(float* dst, const float* src, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst), bytes = valid ? 4u : 0u;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
 template <bool LO, bool XL>
-__global__ void __launch_bounds__(RS_THREADS) k_batch_residual(BatchArgs a, const int64_t* rpfx) {
-    __shared__ __align__(16) float xh[RS_CB][RS_MAXRHS];
-    __shared__ __align__(16) float xl[RS_CB][RS_MAXRHS];
+__global__ void __launch_bounds__(RS_THREADS, RS_MIN_BLOCKS) k_batch_residual(BatchArgs a, const int64_t* rpfx) {
+    constexpr int ROWS = RS_THREADS * RS_ROWS;
+    __shared__ __align__(16) float xh[2][RS_CB][RS_MAXRHS];
+    __shared__ __align__(16) float xl[XL ? 2 : 1][RS_CB][RS_MAXRHS];
+    __shared__ __align__(16) float xm[2][2][RS_MAXRHS];  // largest |hi| of a warp's columns
+    __shared__ float sa[RS_STAGES][RS_CB][ROWS];         // a thread reads what it copied itself
+    __shared__ float sl_[LO ? RS_STAGES : 1][LO ? RS_CB : 1][LO ? ROWS : 1];
     const int si = find_sys(rpfx, a.nsys, blockIdx.x);
     const SysDesc& S = a.sys[si];
     // RS_ROWS rows per thread, RS_THREADS apart: each staged value of X is
     // read once from shared memory for all of them
-    const int64_t r0 = (blockIdx.x - rpfx[si]) * (RS_THREADS * RS_ROWS) + threadIdx.x;
+    const int64_t r0 = (blockIdx.x - rpfx[si]) * ROWS + threadIdx.x;
     const int64_t n = S.n;
     bool rv[RS_ROWS];
-    const float* arow[RS_ROWS];
-    const float* lrow[RS_ROWS];
 #pragma unroll
-    for (int k = 0; k < RS_ROWS; k++) {
-        const int64_t r = r0 + k * RS_THREADS;
-        rv[k] = r < n;
-        arow[k] = S.A2 + (rv[k] ? r : 0);
-        lrow[k] = LO ? S.Alo + (rv[k] ? r : 0) : nullptr;
-    }
+    for (int k = 0; k < RS_ROWS; k++) rv[k] = r0 + k * RS_THREADS < n;
+    const int64_t nchunk = (n + RS_CB - 1) / RS_CB;
+    // chunk c's columns of this thread's rows, one group of asynchronous copies (empty past the last chunk)
+    auto fetch = [&](int64_t c) {
+        if (c < nchunk) {
+            const int st = (int)(c % RS_STAGES);
+#pragma unroll
+            for (int cc = 0; cc < RS_CB; cc++) {
+                const int64_t col = c * RS_CB + cc;
+#pragma unroll
+                for (int k = 0; k < RS_ROWS; k++) {
+                    const bool ok = col < n && rv[k];
+                    const int64_t off = ok ? r0 + k * RS_THREADS + col * n : 0;
+                    copy4_async(&sa[st][cc][threadIdx.x + k * RS_THREADS], S.A2 + off, ok);
+                    if constexpr (LO)
+                        copy4_async(&sl_[st][cc][threadIdx.x + k * RS_THREADS], S.Alo + off, ok);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     // grid.y: blocks of RS_MAXRHS right-hand sides
     for (int q0 = blockIdx.y * RS_MAXRHS; q0 < S.nrhs; q0 += RS_MAXRHS * gridDim.y) {
         const int nq = min(RS_MAXRHS, S.nrhs - q0);
@@ -622,49 +649,85 @@ __global__ void __launch_bounds__(RS_THREADS) k_batch_residual(BatchArgs a, cons
         for (int k = 0; k < RS_ROWS; k++)
 #pragma unroll
             for (int q = 0; q < RS_MAXRHS; q++) sh[k][q] = sl[k][q] = 0.f;
-        for (int64_t c0 = 0; c0 < n; c0 += RS_CB) {
-            __syncthreads();
-            for (int e = threadIdx.x; e < RS_CB * RS_MAXRHS; e += RS_THREADS) {
-                const int cc = e / RS_MAXRHS, q = e % RS_MAXRHS;
-                const double v = (c0 + cc < n && q < nq) ? S.Xd[(c0 + cc) + (q0 + q) * n] : 0.0;
-                const float h = (float)v;
-                xh[cc][q] = h;
-                if (XL) xl[cc][q] = (float)(v - (double)h);
+        const int xc = threadIdx.x / RS_MAXRHS, xq = threadIdx.x % RS_MAXRHS;  // the value of X this thread stages
+        auto xval = [&](int64_t c) {
+            const int64_t col = c * RS_CB + xc;
+            return (col < n && xq < nq) ? S.Xd[col + (q0 + xq) * n] : 0.0;
+        };
+        double xnext = xval(0);
+#pragma unroll
+        for (int c = 0; c < RS_STAGES - 1; c++) fetch(c);
+        __syncthreads();  // the last sweep's readers of xh are done
+        for (int64_t c = 0; c < nchunk; c++) {
+            const int b = (int)(c & 1), st = (int)(c % RS_STAGES);
+            {
+                const float h = (float)xnext;
+                xh[b][xc][xq] = h;
+                if (XL) xl[b][xc][xq] = (float)(xnext - (double)h);
+                float big = fabsf(h);  // over the warp's four columns
+                big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 8));
+                big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 16));
+                if ((threadIdx.x & 31) < RS_MAXRHS) xm[b][threadIdx.x >> 5][xq] = big;
             }
+            xnext = xval(c + 1);
+            fetch(c + RS_STAGES - 1);
+            asm volatile("cp.async.wait_group %0;" ::"n"(RS_STAGES - 1) : "memory");  // chunk c is there
             __syncthreads();
-            if (rv[0]) {
-                const int cn = (int)min((int64_t)RS_CB, n - c0);
-                float av[RS_ROWS][RS_CB], lv[RS_ROWS][RS_CB];
+            float s[RS_ROWS][RS_MAXRHS], lo[RS_ROWS][RS_MAXRHS], bias[RS_ROWS][RS_MAXRHS];
 #pragma unroll
-                for (int k = 0; k < RS_ROWS; k++)
+            for (int k = 0; k < RS_ROWS; k++) {
+                float big = 0.f;
 #pragma unroll
-                    for (int cc = 0; cc < RS_CB; cc++) {
-                        av[k][cc] = (cc < cn && rv[k]) ? arow[k][(c0 + cc) * n] : 0.f;
-                        if (LO) lv[k][cc] = (cc < cn && rv[k]) ? lrow[k][(c0 + cc) * n] : 0.f;
-                    }
+                for (int cc = 0; cc < RS_CB; cc++)
+                    big = fmaxf(big, fabsf(sa[st][cc][threadIdx.x + k * RS_THREADS]));
 #pragma unroll
-                for (int cc = 0; cc < RS_CB; cc++) {
-                    // the 8 hi and 8 lo values of column cc as four 16-byte broadcasts
-                    const float4 h0 = *reinterpret_cast<const float4*>(&xh[cc][0]);
-                    const float4 h1 = *reinterpret_cast<const float4*>(&xh[cc][4]);
-                    const float hh[RS_MAXRHS] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-                    float ll[RS_MAXRHS] = {};
-                    if (XL) {
-                        const float4 l0 = *reinterpret_cast<const float4*>(&xl[cc][0]);
-                        const float4 l1 = *reinterpret_cast<const float4*>(&xl[cc][4]);
-                        ll[0] = l0.x, ll[1] = l0.y, ll[2] = l0.z, ll[3] = l0.w;
-                        ll[4] = l1.x, ll[5] = l1.y, ll[6] = l1.z, ll[7] = l1.w;
-                    }
-#pragma unroll
-                    for (int k = 0; k < RS_ROWS; k++)
-#pragma unroll
-                        for (int q = 0; q < RS_MAXRHS; q++) {
-                            df_mac<XL>(sh[k][q], sl[k][q], av[k][cc], hh[q], ll[q]);
-                            if (LO) sl[k][q] = __fmaf_rn(lv[k][cc], hh[q], sl[k][q]);
-                        }
+                for (int q = 0; q < RS_MAXRHS; q++) {
+                    bias[k][q] = s[k][q] = __fmul_rn(32.f * big, fmaxf(xm[b][0][q], xm[b][1][q]));
+                    lo[k][q] = 0.f;
                 }
             }
+#pragma unroll
+            for (int cc = 0; cc < RS_CB; cc++) {
+                // the 8 hi and 8 lo values of column cc as four 16-byte broadcasts
+                const float4 h0 = *reinterpret_cast<const float4*>(&xh[b][cc][0]);
+                const float4 h1 = *reinterpret_cast<const float4*>(&xh[b][cc][4]);
+                const float hh[RS_MAXRHS] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                float ll[RS_MAXRHS] = {};
+                if (XL) {
+                    const float4 l0 = *reinterpret_cast<const float4*>(&xl[XL ? b : 0][cc][0]);
+                    const float4 l1 = *reinterpret_cast<const float4*>(&xl[XL ? b : 0][cc][4]);
+                    ll[0] = l0.x, ll[1] = l0.y, ll[2] = l0.z, ll[3] = l0.w;
+                    ll[4] = l1.x, ll[5] = l1.y, ll[6] = l1.z, ll[7] = l1.w;
+                }
+#pragma unroll
+                for (int k = 0; k < RS_ROWS; k++) {
+                    const float av = sa[st][cc][threadIdx.x + k * RS_THREADS];
+                    float lv = 0.f;
+                    if constexpr (LO) lv = sl_[st][cc][threadIdx.x + k * RS_THREADS];
+#pragma unroll
+                    for (int q = 0; q < RS_MAXRHS; q++) {
+                        const float t = __fmaf_rn(av, hh[q], s[k][q]);
+                        const float d = __fsub_rn(t, s[k][q]);
+                        lo[k][q] = __fadd_rn(lo[k][q], __fmaf_rn(av, hh[q], -d));
+                        s[k][q] = t;
+                        if (XL) lo[k][q] = __fmaf_rn(av, ll[q], lo[k][q]);
+                        if (LO) lo[k][q] = __fmaf_rn(lv, hh[q], lo[k][q]);
+                    }
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < RS_ROWS; k++)
+#pragma unroll
+                for (int q = 0; q < RS_MAXRHS; q++) {
+                    const float p = __fsub_rn(s[k][q], bias[k][q]);
+                    const float h = __fadd_rn(sh[k][q], p);
+                    const float bb = __fsub_rn(h, sh[k][q]);
+                    const float e = __fadd_rn(__fsub_rn(sh[k][q], __fsub_rn(h, bb)), __fsub_rn(p, bb));  // sh + p - h
+                    sh[k][q] = h;
+                    sl[k][q] = __fadd_rn(sl[k][q], __fadd_rn(e, lo[k][q]));
+                }
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
         for (int k = 0; k < RS_ROWS; k++) {
             if (!rv[k]) continue;
@@ -1019,7 +1082,11 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
         return cudaGetLastError();
     };
     mark(0);
-    k_batch_geom<<<h->nsys, 256, 0, st>>>(a);
+    {
+        const int64_t fill = 2 * tc_num_sms() / std::max<int64_t>(1, h->nsys);
+        const dim3 g((unsigned)h->nsys, (unsigned)std::max<int64_t>(1, std::min(cdiv(h->maxn, 256), fill)));
+        k_batch_geom<<<g, 256, 0, st>>>(a);
+    }
     GB_LAUNCH_CHECK();
     if (staged) GB_CUDA(trefftz());
     mark(1);

@@ -2691,7 +2691,7 @@ __global__ void __launch_bounds__(tc::P_THREADS, 1) k_trs_tcp(LuBatch<float> B, 
     tc::update_persistent<3>(ntiles, job, tc_smem, err);
 }
 
-static int tc_num_sms() {
+int tc_num_sms() {
     static int sms[64];
     int dev = 0;
     cudaGetDevice(&dev);

@@ -125,6 +125,7 @@ struct LuPlan {
 
 // n_sorted: sizes of systems [base, base + n_sorted.size()) of the batch, descending
 int lu_plan_build(LuPlan& plan, const std::vector<int64_t>& n_sorted, cudaStream_t st, int32_t base = 0);
+int tc_num_sms();  // SMs of the current device
 int lu_plan_verdict(int word);  // GBVLM_OK, or the error that a tile's wait ran out, of the plan's word d_err
 // number of kernel launches lu_batch_factor makes for element size es (4 or 8)
 int64_t lu_plan_launches(const LuPlan& plan, int es);
