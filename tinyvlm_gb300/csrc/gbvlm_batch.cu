@@ -1167,8 +1167,25 @@ static int batch_factor(gbvlm_batch h, int g, cudaStream_t st, bool lookahead, b
 }
 
 // pivot: repeat the systems that d_fail marks, with interchanges
+static bool batch_fast(gbvlm_batch h) {
+    for (int g = 0; g < h->ngroups; g++)
+        if (h->plans[g].fast) return true;
+    return false;
+}
+
+// phases: FACTOR up to the factorisation, SOLVE from the solves on.
+// pivot: again, with interchanges, for the systems that the run before left; where
+// the unfactored AICs are kept they are copied back, else assembled again.
+enum { BATCH_FACTOR = 1, BATCH_SOLVE = 2 };
+
+__global__ void k_batch_restore(BatchArgs a) {
+    const SysDesc& S = a.sys[blockIdx.y];
+    const int64_t total = S.n * S.n, stride = gridDim.x * (int64_t)blockDim.x;
+    for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += stride) S.A[e] = S.A2[e];
+}
+
 static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullptr, bool serial_lu = false,
-                         bool pivot = false) {
+                         bool pivot = false, int phases = BATCH_FACTOR | BATCH_SOLVE) {
     auto mark = [&](int k) { if (ev) cudaEventRecord(ev[k], st); };
     int64_t nlaunch = 0;
     for (int g = 0; g < h->ngroups; g++)
@@ -1179,7 +1196,7 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
     // geometry, Trefftz, the groups' assemblies, RHS, the factorisations, the
     // solves and accumulations, the refinement sweeps, the loads
     h->launches = 3 + h->ngroups * (h->fp64_residual ? 2 : 1) + nlaunch + solves + 1 +
-                  (int64_t)h->refine * (1 + solves + 1) + 1;
+                  (int64_t)h->refine * (1 + solves + 1) + 1 + (batch_fast(h) ? 1 : 0);
     BatchArgs a;
     a.sys = h->d_sys;
     a.nsys = h->nsys;
@@ -1208,58 +1225,68 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
         k_batch_trefftz_k<<<gk, 128, 0, st>>>(a);
         return cudaGetLastError();
     };
-    mark(0);
-    {
-        const int64_t fill = 2 * tc_num_sms() / std::max<int64_t>(1, h->nsys);
-        const dim3 g((unsigned)h->nsys, (unsigned)std::max<int64_t>(1, std::min(cdiv(h->maxn, 256), fill)));
-        k_batch_geom<<<g, 256, 0, st>>>(a);
-    }
-    GB_LAUNCH_CHECK();
-    if (staged) GB_CUDA(trefftz());
-    mark(1);
-    if (staged) {
-        GB_CUDA(launch_assemble(h, (unsigned)(h->asm_rows > 1 ? h->assembly_tiles_rows : h->assembly_tiles), 0, a, st));
-        if (h->fp64_residual)
-            GB_CUDA(launch_assemble_lo(h, (unsigned)(lo_rows(h) ? h->assembly_tiles_rows : h->assembly_tiles), 0, a, st));
-    }
-    mark(2);
+    const bool restore = pivot && h->refine > 0;
     dim3 gp((unsigned)cdiv(h->maxn, 256), (unsigned)h->nsys);  // one thread per row of every system
-    if (staged) {
-        k_batch_rhs<<<gp, 256, 0, st>>>(a);
-        GB_LAUNCH_CHECK();
-    }
-    mark(3);
-    if (staged) {
-        for (int g = 0; g < h->ngroups; g++) {
-            int rc = batch_factor(h, g, st, !serial_lu, pivot);
-            if (rc) return rc;
+    if (phases & BATCH_FACTOR) {
+        mark(0);
+        if (restore) {
+            const dim3 g((unsigned)std::min<int64_t>(cdiv(h->maxn * h->maxn, 1024), 1024), (unsigned)h->nsys);
+            k_batch_restore<<<g, 256, 0, st>>>(a);
+        } else {
+            const int64_t fill = 2 * tc_num_sms() / std::max<int64_t>(1, h->nsys);
+            const dim3 g((unsigned)h->nsys, (unsigned)std::max<int64_t>(1, std::min(cdiv(h->maxn, 256), fill)));
+            k_batch_geom<<<g, 256, 0, st>>>(a);
         }
-    } else {
-        GB_CUDA(cudaEventRecord(h->fork, st));
-        for (int g = 0; g < h->ngroups; g++) {
-            GB_CUDA(cudaStreamWaitEvent(h->side[g], h->fork, 0));
-            if (h->gtile[g][1] > 0) {
-                const int64_t(&gt)[2] = h->asm_rows > 1 ? h->gtile_rows[g] : h->gtile[g];
-                GB_CUDA(launch_assemble(h, (unsigned)gt[1], gt[0], a, h->side[g]));
-                if (h->fp64_residual) {
-                    GB_CUDA(cudaEventRecord(h->asm_done[g], h->side[g]));
-                    GB_CUDA(cudaStreamWaitEvent(h->lo_side, h->asm_done[g], 0));
-                    const int64_t(&lt)[2] = lo_rows(h) ? h->gtile_rows[g] : h->gtile[g];
-                    GB_CUDA(launch_assemble_lo(h, (unsigned)lt[1], lt[0], a, h->lo_side));
-                }
+        GB_LAUNCH_CHECK();
+        if (staged && !restore) GB_CUDA(trefftz());
+        mark(1);
+        if (staged && !restore) {
+            GB_CUDA(launch_assemble(h, (unsigned)(h->asm_rows > 1 ? h->assembly_tiles_rows : h->assembly_tiles), 0, a, st));
+            if (h->fp64_residual)
+                GB_CUDA(launch_assemble_lo(h, (unsigned)(lo_rows(h) ? h->assembly_tiles_rows : h->assembly_tiles), 0, a, st));
+        }
+        mark(2);
+        if (staged) {
+            k_batch_rhs<<<gp, 256, 0, st>>>(a);
+            GB_LAUNCH_CHECK();
+        }
+        mark(3);
+        if (staged) {
+            for (int g = 0; g < h->ngroups; g++) {
+                int rc = batch_factor(h, g, st, !serial_lu, pivot);
+                if (rc) return rc;
             }
-            int rc = batch_factor(h, g, h->side[g], true, pivot);
-            if (rc) return rc;
-            GB_CUDA(cudaEventRecord(h->join[g], h->side[g]));
+        } else {
+            GB_CUDA(cudaEventRecord(h->fork, st));
+            for (int g = 0; g < h->ngroups; g++) {
+                GB_CUDA(cudaStreamWaitEvent(h->side[g], h->fork, 0));
+                if (h->gtile[g][1] > 0 && !restore) {
+                    const int64_t(&gt)[2] = h->asm_rows > 1 ? h->gtile_rows[g] : h->gtile[g];
+                    GB_CUDA(launch_assemble(h, (unsigned)gt[1], gt[0], a, h->side[g]));
+                    if (h->fp64_residual) {
+                        GB_CUDA(cudaEventRecord(h->asm_done[g], h->side[g]));
+                        GB_CUDA(cudaStreamWaitEvent(h->lo_side, h->asm_done[g], 0));
+                        const int64_t(&lt)[2] = lo_rows(h) ? h->gtile_rows[g] : h->gtile[g];
+                        GB_CUDA(launch_assemble_lo(h, (unsigned)lt[1], lt[0], a, h->lo_side));
+                    }
+                }
+                int rc = batch_factor(h, g, h->side[g], true, pivot);
+                if (rc) return rc;
+                GB_CUDA(cudaEventRecord(h->join[g], h->side[g]));
+            }
+            if (!restore) GB_CUDA(trefftz());
+            k_batch_rhs<<<gp, 256, 0, st>>>(a);
+            GB_LAUNCH_CHECK();
+            for (int gi = 0; gi < h->ngroups; gi++) GB_CUDA(cudaStreamWaitEvent(st, h->join[gi], 0));
+            if (h->fp64_residual && !restore) GB_CUDA(cudaEventRecord(h->lo_join, h->lo_side));
         }
-        GB_CUDA(trefftz());
-        k_batch_rhs<<<gp, 256, 0, st>>>(a);
-        GB_LAUNCH_CHECK();
-        for (int gi = 0; gi < h->ngroups; gi++) GB_CUDA(cudaStreamWaitEvent(st, h->join[gi], 0));
-        if (h->fp64_residual) GB_CUDA(cudaEventRecord(h->lo_join, h->lo_side));
+        mark(4);
+    }
+    if (!(phases & BATCH_SOLVE)) {
+        if (h->fp64_residual && !staged && !restore) GB_CUDA(cudaStreamWaitEvent(st, h->lo_join, 0));
+        return GBVLM_OK;
     }
     int rc = GBVLM_OK;
-    mark(4);
     int32_t maxrhs = 0;
     for (auto& s : h->sys) maxrhs = std::max(maxrhs, s.nrhs);
     auto solve = [&]() {
@@ -1271,7 +1298,8 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
     if (rc) return rc;
     k_batch_accum<<<gp, 256, 0, st>>>(a);
     GB_LAUNCH_CHECK();
-    if (h->fp64_residual && !staged && h->refine > 0) GB_CUDA(cudaStreamWaitEvent(st, h->lo_join, 0));
+    if (h->fp64_residual && !staged && !restore && (phases & BATCH_FACTOR))
+        GB_CUDA(cudaStreamWaitEvent(st, h->lo_join, 0));
     for (int it = 0; it < h->refine; it++) {
         const dim3 rg((unsigned)h->residual_tiles, (unsigned)cdiv(maxrhs, RS_MAXRHS));
         if (h->fp64_residual) {
@@ -1306,9 +1334,95 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
     return GBVLM_OK;
 }
 
-// After a run: repeats, with row interchanges, the solves of the systems whose
+// the graph's conditions: a system is factored, a system needs interchanges
+__global__ void k_batch_conditions(const int32_t* fail, int32_t n, cudaGraphConditionalHandle done,
+                                   cudaGraphConditionalHandle left) {
+    int ok = 0, bad = 0;
+    for (int32_t k = threadIdx.x; k < n; k += blockDim.x) {
+        ok |= fail[k] == 0;
+        bad |= fail[k] != 0;
+    }
+    ok = __syncthreads_or(ok);
+    bad = __syncthreads_or(bad);
+    if (threadIdx.x == 0) {
+        cudaGraphSetConditional(done, ok ? 1u : 0u);
+        cudaGraphSetConditional(left, bad ? 1u : 0u);
+    }
+}
+
+// The run as a graph.  Where the factorisation may leave systems that need
+// interchanges: the launches up to it, the solves under the condition that a
+// system is factored, and the run again with interchanges under the condition
+// that one is not (16384 panels that need them: 80 ms, with the solves before
+// and the assembly after them as well 105).
+static int batch_capture(gbvlm_batch h) {
+    cudaGraph_t g = nullptr;
+    GB_CUDA(cudaGraphCreate(&g, 0));
+    auto fail = [&](int rc) {
+        cudaGraphDestroy(g);
+        return rc;
+    };
+    cudaGraphConditionalHandle cond[2] = {};
+    // launches on h->cap into graph `into`
+    auto capture = [&](cudaGraph_t into, int phases, bool pivot, bool conditions) -> int {
+        GB_CUDA(cudaStreamBeginCaptureToGraph(h->cap, into, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
+        int rc = batch_enqueue(h, h->cap, nullptr, false, pivot, phases);
+        if (rc == GBVLM_OK && conditions) {
+            k_batch_conditions<<<1, 256, 0, h->cap>>>(h->d_fail, h->nsys, cond[0], cond[1]);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) rc = cuda_fail(e, "k_batch_conditions", __FILE__, __LINE__);
+        }
+        cudaGraph_t got = nullptr;
+        const cudaError_t e = cudaStreamEndCapture(h->cap, &got);
+        if (rc) return rc;
+        GB_CUDA(e);
+        return GBVLM_OK;
+    };
+    auto build = [&]() -> int {
+        if (!batch_fast(h)) return capture(g, BATCH_FACTOR | BATCH_SOLVE, false, false);
+        for (auto& c : cond) GB_CUDA(cudaGraphConditionalHandleCreate(&c, g, 0, cudaGraphCondAssignDefault));
+        int rc = capture(g, BATCH_FACTOR, false, true);
+        if (rc) return rc;
+        // the captured launches' last one, which every branch has joined
+        size_t nn = 0, ne = 0;
+        GB_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
+        std::vector<cudaGraphNode_t> nodes(nn);
+        GB_CUDA(cudaGraphGetNodes(g, nodes.data(), &nn));
+        GB_CUDA(cudaGraphGetEdges(g, nullptr, nullptr, nullptr, &ne));
+        std::vector<cudaGraphNode_t> from(ne), to(ne), last;
+        std::vector<cudaGraphEdgeData> data(ne);
+        GB_CUDA(cudaGraphGetEdges(g, from.data(), to.data(), data.data(), &ne));
+        std::sort(from.begin(), from.end());
+        for (auto x : nodes)
+            if (!std::binary_search(from.begin(), from.end(), x)) last.push_back(x);
+        for (int k = 0; k < 2; k++) {
+            cudaGraphNode_t nif;
+            cudaGraphNodeParams np = {};
+            np.type = cudaGraphNodeTypeConditional;
+            np.conditional.handle = cond[k];
+            np.conditional.type = cudaGraphCondTypeIf;
+            np.conditional.size = 1;
+            GB_CUDA(cudaGraphAddNode(&nif, g, last.data(), nullptr, last.size(), &np));
+            last.assign(1, nif);
+            rc = capture(np.conditional.phGraph_out[0], k ? BATCH_FACTOR | BATCH_SOLVE : BATCH_SOLVE, k == 1, false);
+            if (rc) return rc;
+        }
+        return GBVLM_OK;
+    };
+    const int rc = build();
+    if (rc) return fail(rc);
+    const cudaError_t e = cudaGraphInstantiate(&h->exec, g, cudaGraphInstantiateFlagUseNodePriority);
+    if (e != cudaSuccess) {
+        h->exec = nullptr;
+        return fail(cuda_fail(e, "cudaGraphInstantiate", __FILE__, __LINE__));
+    }
+    h->graph = g;
+    return GBVLM_OK;
+}
+
+// After a run without the graph: repeats, with row interchanges, the solves of the systems whose
 // factorisation needed them (synchronises st).  The others' outputs stay.
-static int batch_settle(gbvlm_batch h, cudaStream_t st) {
+static int batch_settle(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullptr, bool* repeated = nullptr) {
     if (!h->unchecked) return GBVLM_OK;
     GB_CUDA(cudaStreamWaitEvent(st, h->done, 0));
     std::vector<int32_t> f(h->nsys);
@@ -1316,8 +1430,9 @@ static int batch_settle(gbvlm_batch h, cudaStream_t st) {
     GB_CUDA(cudaStreamSynchronize(st));
     h->unchecked = false;
     if (std::none_of(f.begin(), f.end(), [](int32_t x) { return x != 0; })) return GBVLM_OK;
-    const int rc = batch_enqueue(h, st, nullptr, false, true);
+    const int rc = batch_enqueue(h, st, ev, false, true);
     if (rc) return rc;
+    if (repeated) *repeated = true;
     GB_CUDA(cudaEventRecord(h->done, st));
     return GBVLM_OK;
 }
@@ -1754,19 +1869,10 @@ int gbvlm_batch_run(gbvlm_batch h, int32_t want_gamma, gbvlm_stream stream) {
             cudaGraphDestroy(h->graph);
             h->graph = nullptr;
         }
-        GB_CUDA(cudaStreamBeginCapture(h->cap, cudaStreamCaptureModeThreadLocal));
-        int rc = batch_enqueue(h, h->cap);
-        cudaGraph_t g = nullptr;
-        cudaError_t e = cudaStreamEndCapture(h->cap, &g);
-        if (rc) {
-            if (g) cudaGraphDestroy(g);
-            return rc;
-        }
-        GB_CUDA(e);
-        h->graph = g;
-        GB_CUDA(cudaGraphInstantiate(&h->exec, h->graph, cudaGraphInstantiateFlagUseNodePriority));
+        const int rc = batch_capture(h);
+        if (rc) return rc;
     }
-    h->unchecked = true;
+    h->unchecked = false;  // the graph repeats what needs it
     GB_CUDA(cudaGraphLaunch(h->exec, st));
     GB_CUDA(cudaEventRecord(h->done, st));
     return GBVLM_OK;
@@ -1783,9 +1889,19 @@ int gbvlm_batch_profile(gbvlm_batch h, float* stage_ms, gbvlm_stream stream) {
         cudaEventRecord(h->done, st);
         cudaError_t e = cudaEventSynchronize(ev[6]);
         if (e != cudaSuccess) rc = cuda_fail(e, "cudaEventSynchronize", __FILE__, __LINE__);
-        for (int k = 0; k < 6 && rc == GBVLM_OK; k++) {
-            e = cudaEventElapsedTime(&stage_ms[k], ev[k], ev[k + 1]);
-            if (e != cudaSuccess) rc = cuda_fail(e, "cudaEventElapsedTime", __FILE__, __LINE__);
+        bool again = false;  // the systems that need interchanges: their stages' times are added
+        for (int pass = 0; pass < 2 && rc == GBVLM_OK; pass++) {
+            for (int k = 0; k < 6 && rc == GBVLM_OK; k++) {
+                float ms = 0;
+                e = cudaEventElapsedTime(&ms, ev[k], ev[k + 1]);
+                if (e != cudaSuccess) rc = cuda_fail(e, "cudaEventElapsedTime", __FILE__, __LINE__);
+                stage_ms[k] = (pass ? stage_ms[k] : 0.f) + ms;
+            }
+            if (pass || rc) break;
+            rc = batch_settle(h, st, ev, &again);
+            if (rc || !again) break;
+            e = cudaEventSynchronize(ev[6]);
+            if (e != cudaSuccess) rc = cuda_fail(e, "cudaEventSynchronize", __FILE__, __LINE__);
         }
     }
     for (int k = 0; k < 7; k++) cudaEventDestroy(ev[k]);
