@@ -412,7 +412,7 @@ static int rhs_velocities(T* rhs, int32_t nsurf, const gbvlm_dims* dims, const T
 // scheduling.
 //
 // Bound: issue slots and the fp32 pipe (float), the fp64 pipe (double, 89 % busy).
-// Per point and ring two segments and 1.25 vertices, each with its image: 190
+// Per point and ring two segments and 1.25 vertices, each with its image: 150
 // instructions, where the ring-by-ring walk spent 370.
 // LatticeRows: a piece's last vertex line is formed again by the next piece, so
 // (rows + 1) / rows vertices per ring; a line's relative vectors are 6
