@@ -426,7 +426,7 @@ static int rhs_velocities(T* rhs, int32_t nsurf, const gbvlm_dims* dims, const T
 // 8000 rings in double 7.0 -> 2.90 ms; roll-up of 12,150 vertices (95 blocks
 // before, one per 128 points, which left SMs idle) 3417 -> 763 us.
 // Not kept: the point and its image as the two halves of packed fp32
-// instructions (issue slots per ring 190 -> 150, but 128 registers: 320 us),
+// instructions (a fifth fewer issue slots per ring, but 128 registers: 320 us),
 // and the cut-offs left out of a first walk that a second one repeats where a
 // lane met one (298 us, but the roll-up 763 -> 819).
 // ---------------------------------------------------------------------------
