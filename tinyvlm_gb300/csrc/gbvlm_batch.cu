@@ -81,6 +81,7 @@ struct BatchArgs {
     const int32_t* uidx;    // batch solve -> the caller's solve index
     int32_t* bad;           // per system: 1 if its case's vertices hold a non-finite coordinate
     int32_t* fail;          // per system: 1 if its factorisation needs row interchanges (LuBatch::fail)
+    int32_t* info;          // per system: first zero pivot's column + 1 (LuBatch::info)
     int32_t only_failed;    // the run repeats those systems with interchanges: the others' outputs stay
 };
 
@@ -98,7 +99,10 @@ __global__ void __launch_bounds__(256) k_batch_geom(BatchArgs a) {
     SysDesc& S = a.sys[blockIdx.x];
     const int64_t ns = S.ns, nc = S.nc, nv = (ns + 1) * (nc + 1), np = ns * nc;
     const double al = S.alpha_geom;
-    if (threadIdx.x == 0 && blockIdx.y == 0 && !a.only_failed) a.fail[blockIdx.x] = 0;
+    if (threadIdx.x == 0 && blockIdx.y == 0 && !a.only_failed) {  // the verdicts of this run
+        a.fail[blockIdx.x] = 0;
+        a.info[blockIdx.x] = 0;
+    }
     int bad = 0;
     const int64_t t0 = threadIdx.x + blockIdx.y * (int64_t)blockDim.x, stride = gridDim.y * (int64_t)blockDim.x;
     if (blockIdx.y == 0)
@@ -1211,6 +1215,7 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
     a.uidx = h->d_uidx;
     a.bad = h->d_bad;
     a.fail = h->d_fail;
+    a.info = h->lub.info;
     a.only_failed = pivot ? 1 : 0;
     // staged: every phase after the previous one on `st` (stage timing, or
     // kernel timing without the groups' launches overlapping); otherwise each
