@@ -1,0 +1,66 @@
+"""What a batch pays for one system that needs row interchanges: that system's
+own factorisation, not a second one of every system.  A repeat of the whole
+batch took 1.96 times the batch without it (512 wings x 8 angles), one of the
+single system about 1.2 times; the bar lies between.  And the mates of systems
+that are factored again, with none, some and all of the batch among them,
+keep their results to the bit in graph and launch-by-launch runs alike."""
+import time
+
+import numpy as np
+import pytest
+
+from tinyvlm_gb300 import mesh as M
+from tinyvlm_gb300.batch import BatchSolver, pack_alphas, pack_verts
+
+pytestmark = pytest.mark.gpu
+
+
+def _spoil(case, seed=1):
+    v = case.verts
+    rng = np.random.default_rng(seed)
+    v[:3, 1:-1, 1:-1] += rng.normal(0.0, 0.4, v[:3, 1:-1, 1:-1].shape).astype(np.float32)
+
+
+def _run(cases, mode="shared", refine=1, graph=True, **kw):
+    bs = BatchSolver(cases, mode=mode, refine=refine, **kw)
+    bs.set_inputs(pack_verts(cases), pack_alphas(cases))
+    bs.run(want_gamma=True, graph=graph)
+    return bs.results(gamma=True)
+
+
+def _best(bs, n=7):
+    t = []
+    for _ in range(n):
+        t0 = time.perf_counter()
+        bs.run()
+        bs.results()
+        t.append(time.perf_counter() - t0)
+    return min(t)
+
+
+def test_one_system_is_repeated_alone(cuda):
+    clean = M.batch_cases(512, n_alpha=8)
+    mixed = M.batch_cases(512, n_alpha=8)
+    _spoil(mixed[sorted(range(512), key=lambda k: mixed[k].verts[0].size)[256]])
+    t = []
+    for cases in (clean, mixed):
+        bs = BatchSolver(cases)
+        bs.set_inputs(pack_verts(cases), pack_alphas(cases))
+        t.append(_best(bs))
+    assert t[1] <= 1.5 * t[0], t
+
+
+@pytest.mark.parametrize("mode,refine,kw", [("shared", 1, {}), ("exact", 1, {}), ("shared", 0, {}),
+                                            ("shared", 2, {"fp64_residual": True})])
+@pytest.mark.parametrize("spoilt", [(), (0, 3), (0, 1, 2, 3, 4, 5)])
+def test_graph_and_launches_agree(cuda, mode, refine, kw, spoilt):
+    cases = M.batch_cases(6, seed=11, n_alpha=2, nc_range=(5, 20), ns_range=(8, 40))
+    alone = {k: _run(cases[k:k + 1], mode, refine, **kw) for k in range(6) if k not in spoilt}
+    for k in spoilt:
+        _spoil(cases[k], k)
+    co, g = _run(cases, mode, refine, True, **kw)
+    ce, ge = _run(cases, mode, refine, False, **kw)
+    assert np.isfinite(co).all()
+    assert (co == ce).all() and all((a == b).all() for a, b in zip(g, ge))
+    for k, (ca, ga) in alone.items():
+        assert (co[2 * k:2 * k + 2] == ca).all() and all((a == b).all() for a, b in zip(g[2 * k:2 * k + 2], ga))

@@ -82,7 +82,9 @@ struct BatchArgs {
     int32_t* bad;           // per system: 1 if its case's vertices hold a non-finite coordinate
     int32_t* fail;          // per system: 1 if its factorisation needs row interchanges (LuBatch::fail)
     int32_t* info;          // per system: first zero pivot's column + 1 (LuBatch::info)
-    int32_t only_failed;    // the run repeats those systems with interchanges: the others' outputs stay
+    int32_t only_failed;    // the launches factor those systems again, with interchanges, and pass over the others
+
+    __device__ __forceinline__ bool skips(int si) const { return only_failed && !fail[si]; }
 };
 
 __device__ __forceinline__ void split_hl(double x, float& h, float& l) {
@@ -99,7 +101,7 @@ __global__ void __launch_bounds__(256) k_batch_geom(BatchArgs a) {
     SysDesc& S = a.sys[blockIdx.x];
     const int64_t ns = S.ns, nc = S.nc, nv = (ns + 1) * (nc + 1), np = ns * nc;
     const double al = S.alpha_geom;
-    if (threadIdx.x == 0 && blockIdx.y == 0 && !a.only_failed) {  // the verdicts of this run
+    if (threadIdx.x == 0 && blockIdx.y == 0) {  // the verdicts of this run
         a.fail[blockIdx.x] = 0;
         a.info[blockIdx.x] = 0;
     }
@@ -286,6 +288,7 @@ __global__ void __launch_bounds__(BA_THREADS, 8) k_batch_assemble(BatchArgs a, c
     __shared__ float4 sseg[3][BA_W];      // the strip's segment vectors (strip_hl)
     const int64_t tile = tile0 + blockIdx.x;
     const int si = find_sys(tpfx, a.nsys, tile);
+    if (a.skips(si)) return;
     const SysDesc& S = a.sys[si];
     const int64_t ns = S.ns, nc = S.nc, n = S.n;
     const int64_t nchunk = (ns + BA_SPAN - 1) / BA_SPAN, nrb = (n + BA_THREADS - 1) / BA_THREADS;
@@ -361,6 +364,7 @@ __global__ void __launch_bounds__(BA_THREADS, R <= 3 ? 8 : 6) k_batch_assemble_r
     __shared__ float4 schord[R][BA_W];        // ring row r: line r -> line r+1 at vertex k
     const int64_t tile = tile0 + blockIdx.x;
     const int si = find_sys(tpfx, a.nsys, tile);
+    if (a.skips(si)) return;
     const SysDesc& S = a.sys[si];
     const int64_t ns = S.ns, nc = S.nc, n = S.n;
     const int64_t nchunk = (ns + BA_SPAN - 1) / BA_SPAN, nrb = (n + BA_THREADS - 1) / BA_THREADS;
@@ -917,7 +921,6 @@ template <int LD_THREADS>
 __global__ void __launch_bounds__(LD_THREADS) k_batch_loads(BatchArgs a, const int32_t* solve_sys, int32_t want_gamma) {
     const int32_t sol = blockIdx.x;
     const int32_t si = solve_sys[sol];
-    if (a.only_failed && !a.fail[si]) return;
     const SysDesc& S = a.sys[si];
     const int q = sol - S.rhs_off;
     const int64_t ns = S.ns, nc = S.nc, n = S.n, nv = (ns + 1) * (nc + 1);
@@ -1032,10 +1035,6 @@ struct gbvlm_batch_s {
     int32_t* d_uidx = nullptr;   // batch solve -> the caller's solve
     int32_t* d_bad = nullptr;    // per system: non-finite input vertices
     int32_t* d_fail = nullptr;   // per system: its factorisation needs row interchanges
-    // a run factors without interchanges; whether a system needed them is
-    // looked up, and its solves repeated, before the run's results are handed
-    // out or its inputs replaced
-    bool unchecked = false;
     void* status = nullptr;      // pinned: error words and pivot flags read back with the results
     SysDesc* d_sys = nullptr;
     int32_t* d_solve_sys = nullptr;
@@ -1162,34 +1161,42 @@ static cudaError_t launch_assemble_lo(gbvlm_batch h, unsigned tiles, int64_t til
     return cudaGetLastError();
 }
 
-// one size group's factorisation: without interchanges, or (pivot) with them
-static int batch_factor(gbvlm_batch h, int g, cudaStream_t st, bool lookahead, bool pivot) {
-    if (pivot || !h->plans[g].fast) return lu_batch_factor<float>(h->lub, h->plans[g], st, lookahead);
-    LuBatch<float> B = h->lub;
-    B.fail = h->d_fail;
-    return lu_batch_factor_fast<float>(B, h->plans[g], st, lookahead);
-}
-
-// pivot: repeat the systems that d_fail marks, with interchanges
+// whether a run factors systems without interchanges first, and so may have to
+// factor some again
 static bool batch_fast(gbvlm_batch h) {
     for (int g = 0; g < h->ngroups; g++)
         if (h->plans[g].fast) return true;
     return false;
 }
 
-// phases: FACTOR up to the factorisation, SOLVE from the solves on.
-// pivot: again, with interchanges, for the systems that the run before left; where
-// the unfactored AICs are kept they are copied back, else assembled again.
-enum { BATCH_FACTOR = 1, BATCH_SOLVE = 2 };
+// one size group's factorisation: without interchanges, d_fail marking the
+// systems that need them, or (pivot) with them, those systems only
+static int batch_factor(gbvlm_batch h, int g, cudaStream_t st, bool lookahead, bool pivot) {
+    LuBatch<float> B = h->lub;
+    if (!h->plans[g].fast) return pivot ? GBVLM_OK : lu_batch_factor<float>(B, h->plans[g], st, lookahead);
+    if (pivot) {
+        B.only = h->d_fail;
+        return lu_batch_factor<float>(B, h->plans[g], st, lookahead);
+    }
+    B.fail = h->d_fail;
+    return lu_batch_factor_fast<float>(B, h->plans[g], st, lookahead);
+}
 
 __global__ void k_batch_restore(BatchArgs a) {
+    if (a.skips(blockIdx.y)) return;
     const SysDesc& S = a.sys[blockIdx.y];
     const int64_t total = S.n * S.n, stride = gridDim.x * (int64_t)blockDim.x;
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += stride) S.A[e] = S.A2[e];
 }
 
-static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullptr, bool serial_lu = false,
-                         bool pivot = false, int phases = BATCH_FACTOR | BATCH_SOLVE) {
+// A run's phases: FACTOR, up to the factorisation without interchanges; REPEAT,
+// the systems that need them once more (their unfactored AICs copied back where
+// they are kept, else assembled again; every other system's blocks leave at
+// entry); SOLVE, from the solves on, all systems.
+enum { BATCH_FACTOR = 1, BATCH_REPEAT = 2, BATCH_SOLVE = 4 };
+
+static int batch_enqueue(gbvlm_batch h, cudaStream_t st, int phases, cudaEvent_t* ev = nullptr,
+                         bool serial_lu = false) {
     auto mark = [&](int k) { if (ev) cudaEventRecord(ev[k], st); };
     int64_t nlaunch = 0;
     for (int g = 0; g < h->ngroups; g++)
@@ -1204,11 +1211,11 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
     BatchArgs a;
     a.sys = h->d_sys;
     a.nsys = h->nsys;
-    a.alphas = h->d_alpha;
     a.u_inf = h->u_inf;
-    a.rho = h->rho;
     a.beta = h->beta;
+    a.rho = h->rho;
     for (int k = 0; k < 3; k++) a.ref[k] = h->ref[k];
+    a.alphas = h->d_alpha;
     a.out = h->d_out;
     a.gamma_out = h->d_gamma;
     a.goff = h->d_goff;
@@ -1216,37 +1223,58 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
     a.bad = h->d_bad;
     a.fail = h->d_fail;
     a.info = h->lub.info;
-    a.only_failed = pivot ? 1 : 0;
+    a.only_failed = 0;
     // staged: every phase after the previous one on `st` (stage timing, or
     // kernel timing without the groups' launches overlapping); otherwise each
     // size group's assembly and factorisation run on its own branch, group 0
-    // (the largest systems, the critical path) at high priority, with the
-    // Trefftz kernel and the right-hand sides on the main stream beside them
+    // (the longest chain) on a high-priority stream
     const bool staged = ev != nullptr || serial_lu;
+    // the Trefftz influence matrices need only the geometry: launched where
+    // they run beside the assembly and the factorisation
     auto trefftz = [&]() {
         int64_t maxns = 1;
-        for (auto& S : h->sys) maxns = std::max(maxns, S.ns);
-        dim3 gk((unsigned)cdiv(maxns * maxns, 128), (unsigned)h->nsys);
+        for (auto& s : h->sys) maxns = std::max(maxns, s.ns);
+        const dim3 gk((unsigned)cdiv(maxns * maxns, 128), (unsigned)h->nsys);
         k_batch_trefftz_k<<<gk, 128, 0, st>>>(a);
         return cudaGetLastError();
     };
-    const bool restore = pivot && h->refine > 0;
-    dim3 gp((unsigned)cdiv(h->maxn, 256), (unsigned)h->nsys);  // one thread per row of every system
+    auto assemble_all = [&]() {
+        return launch_assemble(h, (unsigned)(h->asm_rows > 1 ? h->assembly_tiles_rows : h->assembly_tiles), 0, a, st);
+    };
+    const dim3 gp((unsigned)cdiv(h->maxn, 256), (unsigned)h->nsys);  // one thread per row of every system
+    // the size groups' factorisations: one after another on `st`, or each on its branch, joined on `st`
+    auto factor = [&](bool pivot, auto&& before, auto&& beside) -> int {
+        if (staged) {
+            for (int g = 0; g < h->ngroups; g++) {
+                const int rc = batch_factor(h, g, st, !serial_lu, pivot);
+                if (rc) return rc;
+            }
+            return GBVLM_OK;
+        }
+        GB_CUDA(cudaEventRecord(h->fork, st));
+        for (int g = 0; g < h->ngroups; g++) {
+            GB_CUDA(cudaStreamWaitEvent(h->side[g], h->fork, 0));
+            int rc = before(g);
+            if (rc == GBVLM_OK) rc = batch_factor(h, g, h->side[g], true, pivot);
+            if (rc) return rc;
+            GB_CUDA(cudaEventRecord(h->join[g], h->side[g]));
+        }
+        const int rc = beside();
+        if (rc) return rc;
+        for (int g = 0; g < h->ngroups; g++) GB_CUDA(cudaStreamWaitEvent(st, h->join[g], 0));
+        return GBVLM_OK;
+    };
+    int rc = GBVLM_OK;
     if (phases & BATCH_FACTOR) {
         mark(0);
-        if (restore) {
-            const dim3 g((unsigned)std::min<int64_t>(cdiv(h->maxn * h->maxn, 1024), 1024), (unsigned)h->nsys);
-            k_batch_restore<<<g, 256, 0, st>>>(a);
-        } else {
-            const int64_t fill = 2 * tc_num_sms() / std::max<int64_t>(1, h->nsys);
-            const dim3 g((unsigned)h->nsys, (unsigned)std::max<int64_t>(1, std::min(cdiv(h->maxn, 256), fill)));
-            k_batch_geom<<<g, 256, 0, st>>>(a);
-        }
+        const int64_t fill = 2 * tc_num_sms() / std::max<int64_t>(1, h->nsys);
+        const dim3 gg((unsigned)h->nsys, (unsigned)std::max<int64_t>(1, std::min(cdiv(h->maxn, 256), fill)));
+        k_batch_geom<<<gg, 256, 0, st>>>(a);
         GB_LAUNCH_CHECK();
-        if (staged && !restore) GB_CUDA(trefftz());
+        if (staged) GB_CUDA(trefftz());
         mark(1);
-        if (staged && !restore) {
-            GB_CUDA(launch_assemble(h, (unsigned)(h->asm_rows > 1 ? h->assembly_tiles_rows : h->assembly_tiles), 0, a, st));
+        if (staged) {
+            GB_CUDA(assemble_all());
             if (h->fp64_residual)
                 GB_CUDA(launch_assemble_lo(h, (unsigned)(lo_rows(h) ? h->assembly_tiles_rows : h->assembly_tiles), 0, a, st));
         }
@@ -1256,42 +1284,47 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
             GB_LAUNCH_CHECK();
         }
         mark(3);
-        if (staged) {
-            for (int g = 0; g < h->ngroups; g++) {
-                int rc = batch_factor(h, g, st, !serial_lu, pivot);
-                if (rc) return rc;
-            }
-        } else {
-            GB_CUDA(cudaEventRecord(h->fork, st));
-            for (int g = 0; g < h->ngroups; g++) {
-                GB_CUDA(cudaStreamWaitEvent(h->side[g], h->fork, 0));
-                if (h->gtile[g][1] > 0 && !restore) {
-                    const int64_t(&gt)[2] = h->asm_rows > 1 ? h->gtile_rows[g] : h->gtile[g];
-                    GB_CUDA(launch_assemble(h, (unsigned)gt[1], gt[0], a, h->side[g]));
-                    if (h->fp64_residual) {
-                        GB_CUDA(cudaEventRecord(h->asm_done[g], h->side[g]));
-                        GB_CUDA(cudaStreamWaitEvent(h->lo_side, h->asm_done[g], 0));
-                        const int64_t(&lt)[2] = lo_rows(h) ? h->gtile_rows[g] : h->gtile[g];
-                        GB_CUDA(launch_assemble_lo(h, (unsigned)lt[1], lt[0], a, h->lo_side));
-                    }
+        rc = factor(
+            false,
+            [&](int g) -> int {
+                if (h->gtile[g][1] == 0) return GBVLM_OK;
+                const int64_t(&gt)[2] = h->asm_rows > 1 ? h->gtile_rows[g] : h->gtile[g];
+                GB_CUDA(launch_assemble(h, (unsigned)gt[1], gt[0], a, h->side[g]));
+                if (h->fp64_residual) {
+                    GB_CUDA(cudaEventRecord(h->asm_done[g], h->side[g]));
+                    GB_CUDA(cudaStreamWaitEvent(h->lo_side, h->asm_done[g], 0));
+                    const int64_t(&lt)[2] = lo_rows(h) ? h->gtile_rows[g] : h->gtile[g];
+                    GB_CUDA(launch_assemble_lo(h, (unsigned)lt[1], lt[0], a, h->lo_side));
                 }
-                int rc = batch_factor(h, g, h->side[g], true, pivot);
-                if (rc) return rc;
-                GB_CUDA(cudaEventRecord(h->join[g], h->side[g]));
-            }
-            if (!restore) GB_CUDA(trefftz());
-            k_batch_rhs<<<gp, 256, 0, st>>>(a);
-            GB_LAUNCH_CHECK();
-            for (int gi = 0; gi < h->ngroups; gi++) GB_CUDA(cudaStreamWaitEvent(st, h->join[gi], 0));
-            if (h->fp64_residual && !restore) GB_CUDA(cudaEventRecord(h->lo_join, h->lo_side));
+                return GBVLM_OK;
+            },
+            [&]() -> int {
+                GB_CUDA(trefftz());
+                k_batch_rhs<<<gp, 256, 0, st>>>(a);
+                GB_LAUNCH_CHECK();
+                return GBVLM_OK;
+            });
+        if (rc) return rc;
+        if (h->fp64_residual && !staged) {
+            GB_CUDA(cudaEventRecord(h->lo_join, h->lo_side));
+            if (!(phases & BATCH_SOLVE)) GB_CUDA(cudaStreamWaitEvent(st, h->lo_join, 0));
         }
-        mark(4);
     }
-    if (!(phases & BATCH_SOLVE)) {
-        if (h->fp64_residual && !staged && !restore) GB_CUDA(cudaStreamWaitEvent(st, h->lo_join, 0));
-        return GBVLM_OK;
+    if (phases & BATCH_REPEAT) {
+        a.only_failed = 1;
+        if (h->refine > 0) {
+            const dim3 g((unsigned)std::min<int64_t>(cdiv(h->maxn * h->maxn, 1024), 1024), (unsigned)h->nsys);
+            k_batch_restore<<<g, 256, 0, st>>>(a);
+            GB_LAUNCH_CHECK();
+        } else {
+            GB_CUDA(assemble_all());
+        }
+        rc = factor(true, [](int) { return GBVLM_OK; }, []() { return GBVLM_OK; });
+        if (rc) return rc;
+        a.only_failed = 0;
     }
-    int rc = GBVLM_OK;
+    if (!(phases & BATCH_SOLVE)) return GBVLM_OK;
+    mark(4);
     int32_t maxrhs = 0;
     for (auto& s : h->sys) maxrhs = std::max(maxrhs, s.nrhs);
     auto solve = [&]() {
@@ -1303,7 +1336,7 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
     if (rc) return rc;
     k_batch_accum<<<gp, 256, 0, st>>>(a);
     GB_LAUNCH_CHECK();
-    if (h->fp64_residual && !staged && !restore && (phases & BATCH_FACTOR))
+    if (h->fp64_residual && !staged && (phases & BATCH_FACTOR))
         GB_CUDA(cudaStreamWaitEvent(st, h->lo_join, 0));
     for (int it = 0; it < h->refine; it++) {
         const dim3 rg((unsigned)h->residual_tiles, (unsigned)cdiv(maxrhs, RS_MAXRHS));
@@ -1339,27 +1372,18 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullp
     return GBVLM_OK;
 }
 
-// the graph's conditions: a system is factored, a system needs interchanges
-__global__ void k_batch_conditions(const int32_t* fail, int32_t n, cudaGraphConditionalHandle done,
-                                   cudaGraphConditionalHandle left) {
-    int ok = 0, bad = 0;
-    for (int32_t k = threadIdx.x; k < n; k += blockDim.x) {
-        ok |= fail[k] == 0;
-        bad |= fail[k] != 0;
-    }
-    ok = __syncthreads_or(ok);
+// the graph's condition: a system needs interchanges
+__global__ void k_batch_condition(const int32_t* fail, int32_t n, cudaGraphConditionalHandle left) {
+    int bad = 0;
+    for (int32_t k = threadIdx.x; k < n; k += blockDim.x) bad |= fail[k] != 0;
     bad = __syncthreads_or(bad);
-    if (threadIdx.x == 0) {
-        cudaGraphSetConditional(done, ok ? 1u : 0u);
-        cudaGraphSetConditional(left, bad ? 1u : 0u);
-    }
+    if (threadIdx.x == 0) cudaGraphSetConditional(left, bad ? 1u : 0u);
 }
 
 // The run as a graph.  Where the factorisation may leave systems that need
-// interchanges: the launches up to it, the solves under the condition that a
-// system is factored, and the run again with interchanges under the condition
-// that one is not (16384 panels that need them: 80 ms, with the solves before
-// and the assembly after them as well 105).
+// interchanges, their factorisation lies between it and the solves, under the
+// condition that there is one.  Measured, 512 wings x 8 angles: none 10.0 ms,
+// one of middle size 12.1 (13.5 with interchanges for all from the start).
 static int batch_capture(gbvlm_batch h) {
     cudaGraph_t g = nullptr;
     GB_CUDA(cudaGraphCreate(&g, 0));
@@ -1367,15 +1391,16 @@ static int batch_capture(gbvlm_batch h) {
         cudaGraphDestroy(g);
         return rc;
     };
-    cudaGraphConditionalHandle cond[2] = {};
-    // launches on h->cap into graph `into`
-    auto capture = [&](cudaGraph_t into, int phases, bool pivot, bool conditions) -> int {
-        GB_CUDA(cudaStreamBeginCaptureToGraph(h->cap, into, nullptr, nullptr, 0, cudaStreamCaptureModeThreadLocal));
-        int rc = batch_enqueue(h, h->cap, nullptr, false, pivot, phases);
-        if (rc == GBVLM_OK && conditions) {
-            k_batch_conditions<<<1, 256, 0, h->cap>>>(h->d_fail, h->nsys, cond[0], cond[1]);
+    cudaGraphConditionalHandle left = 0;
+    // launches on h->cap into graph `into`, after its node `dep`
+    auto capture = [&](cudaGraph_t into, const cudaGraphNode_t* dep, int phases, bool condition) -> int {
+        GB_CUDA(cudaStreamBeginCaptureToGraph(h->cap, into, dep, nullptr, dep ? 1 : 0,
+                                              cudaStreamCaptureModeThreadLocal));
+        int rc = batch_enqueue(h, h->cap, phases);
+        if (rc == GBVLM_OK && condition) {
+            k_batch_condition<<<1, 256, 0, h->cap>>>(h->d_fail, h->nsys, left);
             const cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess) rc = cuda_fail(e, "k_batch_conditions", __FILE__, __LINE__);
+            if (e != cudaSuccess) rc = cuda_fail(e, "k_batch_condition", __FILE__, __LINE__);
         }
         cudaGraph_t got = nullptr;
         const cudaError_t e = cudaStreamEndCapture(h->cap, &got);
@@ -1384,9 +1409,9 @@ static int batch_capture(gbvlm_batch h) {
         return GBVLM_OK;
     };
     auto build = [&]() -> int {
-        if (!batch_fast(h)) return capture(g, BATCH_FACTOR | BATCH_SOLVE, false, false);
-        for (auto& c : cond) GB_CUDA(cudaGraphConditionalHandleCreate(&c, g, 0, cudaGraphCondAssignDefault));
-        int rc = capture(g, BATCH_FACTOR, false, true);
+        if (!batch_fast(h)) return capture(g, nullptr, BATCH_FACTOR | BATCH_SOLVE, false);
+        GB_CUDA(cudaGraphConditionalHandleCreate(&left, g, 0, cudaGraphCondAssignDefault));
+        int rc = capture(g, nullptr, BATCH_FACTOR, true);
         if (rc) return rc;
         // the captured launches' last one, which every branch has joined
         size_t nn = 0, ne = 0;
@@ -1400,19 +1425,15 @@ static int batch_capture(gbvlm_batch h) {
         std::sort(from.begin(), from.end());
         for (auto x : nodes)
             if (!std::binary_search(from.begin(), from.end(), x)) last.push_back(x);
-        for (int k = 0; k < 2; k++) {
-            cudaGraphNode_t nif;
-            cudaGraphNodeParams np = {};
-            np.type = cudaGraphNodeTypeConditional;
-            np.conditional.handle = cond[k];
-            np.conditional.type = cudaGraphCondTypeIf;
-            np.conditional.size = 1;
-            GB_CUDA(cudaGraphAddNode(&nif, g, last.data(), nullptr, last.size(), &np));
-            last.assign(1, nif);
-            rc = capture(np.conditional.phGraph_out[0], k ? BATCH_FACTOR | BATCH_SOLVE : BATCH_SOLVE, k == 1, false);
-            if (rc) return rc;
-        }
-        return GBVLM_OK;
+        cudaGraphNode_t nif;
+        cudaGraphNodeParams np = {};
+        np.type = cudaGraphNodeTypeConditional;
+        np.conditional.handle = left;
+        np.conditional.type = cudaGraphCondTypeIf;
+        np.conditional.size = 1;
+        GB_CUDA(cudaGraphAddNode(&nif, g, last.data(), nullptr, last.size(), &np));
+        if ((rc = capture(np.conditional.phGraph_out[0], nullptr, BATCH_REPEAT, false))) return rc;
+        return capture(g, &nif, BATCH_SOLVE, false);
     };
     const int rc = build();
     if (rc) return fail(rc);
@@ -1425,21 +1446,19 @@ static int batch_capture(gbvlm_batch h) {
     return GBVLM_OK;
 }
 
-// After a run without the graph: repeats, with row interchanges, the solves of the systems whose
-// factorisation needed them (synchronises st).  The others' outputs stay.
-static int batch_settle(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev = nullptr, bool* repeated = nullptr) {
-    if (!h->unchecked) return GBVLM_OK;
-    GB_CUDA(cudaStreamWaitEvent(st, h->done, 0));
-    std::vector<int32_t> f(h->nsys);
-    GB_CUDA(cudaMemcpyAsync(f.data(), h->d_fail, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
-    GB_CUDA(cudaStreamSynchronize(st));
-    h->unchecked = false;
-    if (std::none_of(f.begin(), f.end(), [](int32_t x) { return x != 0; })) return GBVLM_OK;
-    const int rc = batch_enqueue(h, st, ev, false, true);
+// A run launch by launch for the profiles, which wait anyway: the host looks
+// whether a system needs interchanges.
+static int batch_enqueue_checked(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev, bool serial_lu) {
+    int rc = batch_enqueue(h, st, BATCH_FACTOR, ev, serial_lu);
     if (rc) return rc;
-    if (repeated) *repeated = true;
-    GB_CUDA(cudaEventRecord(h->done, st));
-    return GBVLM_OK;
+    std::vector<int32_t> f(h->nsys, 0);
+    if (batch_fast(h)) {
+        GB_CUDA(cudaMemcpyAsync(f.data(), h->d_fail, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaStreamSynchronize(st));
+    }
+    const bool left = std::any_of(f.begin(), f.end(), [](int32_t x) { return x != 0; });
+    if (left && (rc = batch_enqueue(h, st, BATCH_REPEAT, ev, serial_lu))) return rc;
+    return batch_enqueue(h, st, BATCH_SOLVE, ev, serial_lu);
 }
 
 extern "C" {
@@ -1811,10 +1830,6 @@ int gbvlm_batch_set_inputs(gbvlm_batch h, const float* verts, const double* alph
     for (int32_t u = 0; u < h->nsolve; u++)
         GB_REQUIRE(isfinite(alphas[u]), "alpha %d is not finite", u);
     cudaStream_t st = to_cuda(stream);
-    {
-        const int rc = batch_settle(h, st);  // the last run still needs its inputs
-        if (rc) return rc;
-    }
     // conditions baked into the graph: rebuild it if they change
     const double r[3] = {ref_pt ? ref_pt[0] : 0, ref_pt ? ref_pt[1] : 0, ref_pt ? ref_pt[2] : 0};
     if (u_inf != h->u_inf || rho != h->rho || r[0] != h->ref[0] || r[1] != h->ref[1] || r[2] != h->ref[2]) {
@@ -1854,8 +1869,8 @@ int gbvlm_batch_run_eager(gbvlm_batch h, int32_t want_gamma, gbvlm_stream stream
         cudaGraphExecDestroy(h->exec);
         h->exec = nullptr;
     }
-    h->unchecked = true;
-    int rc = batch_enqueue(h, to_cuda(stream));
+    // (no host wait: the launches for systems that need interchanges are always there, and leave where there is none)
+    int rc = batch_enqueue(h, to_cuda(stream), BATCH_FACTOR | BATCH_SOLVE | (batch_fast(h) ? BATCH_REPEAT : 0));
     if (rc == GBVLM_OK) GB_CUDA(cudaEventRecord(h->done, to_cuda(stream)));
     return rc;
 }
@@ -1877,7 +1892,6 @@ int gbvlm_batch_run(gbvlm_batch h, int32_t want_gamma, gbvlm_stream stream) {
         const int rc = batch_capture(h);
         if (rc) return rc;
     }
-    h->unchecked = false;  // the graph repeats what needs it
     GB_CUDA(cudaGraphLaunch(h->exec, st));
     GB_CUDA(cudaEventRecord(h->done, st));
     return GBVLM_OK;
@@ -1888,25 +1902,14 @@ int gbvlm_batch_profile(gbvlm_batch h, float* stage_ms, gbvlm_stream stream) {
     cudaStream_t st = to_cuda(stream);
     cudaEvent_t ev[7];
     for (int k = 0; k < 7; k++) GB_CUDA(cudaEventCreate(&ev[k]));
-    h->unchecked = true;
-    int rc = batch_enqueue(h, st, ev);
+    int rc = batch_enqueue_checked(h, st, ev, false);
     if (rc == GBVLM_OK) {
         cudaEventRecord(h->done, st);
         cudaError_t e = cudaEventSynchronize(ev[6]);
         if (e != cudaSuccess) rc = cuda_fail(e, "cudaEventSynchronize", __FILE__, __LINE__);
-        bool again = false;  // the systems that need interchanges: their stages' times are added
-        for (int pass = 0; pass < 2 && rc == GBVLM_OK; pass++) {
-            for (int k = 0; k < 6 && rc == GBVLM_OK; k++) {
-                float ms = 0;
-                e = cudaEventElapsedTime(&ms, ev[k], ev[k + 1]);
-                if (e != cudaSuccess) rc = cuda_fail(e, "cudaEventElapsedTime", __FILE__, __LINE__);
-                stage_ms[k] = (pass ? stage_ms[k] : 0.f) + ms;
-            }
-            if (pass || rc) break;
-            rc = batch_settle(h, st, ev, &again);
-            if (rc || !again) break;
-            e = cudaEventSynchronize(ev[6]);
-            if (e != cudaSuccess) rc = cuda_fail(e, "cudaEventSynchronize", __FILE__, __LINE__);
+        for (int k = 0; k < 6 && rc == GBVLM_OK; k++) {
+            e = cudaEventElapsedTime(&stage_ms[k], ev[k], ev[k + 1]);
+            if (e != cudaSuccess) rc = cuda_fail(e, "cudaEventElapsedTime", __FILE__, __LINE__);
         }
     }
     for (int k = 0; k < 7; k++) cudaEventDestroy(ev[k]);
@@ -1918,8 +1921,7 @@ int gbvlm_batch_update_profile(gbvlm_batch h, double* out, gbvlm_stream stream) 
     cudaStream_t st = to_cuda(stream);
     std::vector<cudaEvent_t> ev;
     for (int g = 0; g < h->ngroups; g++) h->plans[g].tc_events = &ev;
-    h->unchecked = true;
-    int rc = batch_enqueue(h, st, nullptr, true);
+    int rc = batch_enqueue_checked(h, st, nullptr, true);
     for (int g = 0; g < h->ngroups; g++) h->plans[g].tc_events = nullptr;
     double ms = 0;
     if (rc == GBVLM_OK) {
@@ -1951,8 +1953,8 @@ int gbvlm_batch_results(gbvlm_batch h, double* coeffs, float* gamma, gbvlm_strea
     cudaStream_t st = to_cuda(stream);
     constexpr int G = gbvlm_batch_s::MAX_GROUPS;
     // status words (bounded-wait errors of the LU plans and the triangular
-    // solve, pivot flags, systems that need interchanges) with the same synchronisation
-    const size_t sbytes = sizeof(int32_t) * (G + 1 + 3 * (size_t)h->nsys);
+    // solve, pivot flags) with the same synchronisation
+    const size_t sbytes = sizeof(int32_t) * (G + 1 + 2 * (size_t)h->nsys);
     if (!h->status) {
         h->status = pinned_take(sbytes);
         if (!h->status) {
@@ -1962,29 +1964,19 @@ int gbvlm_batch_results(gbvlm_batch h, double* coeffs, float* gamma, gbvlm_strea
         h->status_bytes = sbytes;
     }
     int32_t* hs = (int32_t*)h->status;
-    const int32_t* fail = hs + G + 1 + 2 * h->nsys;
-    while (true) {
-        // outputs are already in the caller's order: straight into the caller's buffers
-        GB_CUDA(cudaMemcpyAsync(coeffs, h->d_out, sizeof(double) * 5 * h->nsolve, cudaMemcpyDeviceToHost, st));
-        if (gamma)
-            GB_CUDA(cudaMemcpyAsync(gamma, h->d_gamma, sizeof(float) * h->gamma_floats, cudaMemcpyDeviceToHost, st));
-        memset(hs, 0, sizeof(int32_t) * (G + 1));
-        for (int g = 0; g < h->ngroups; g++)
-            if (h->plans[g].d_err)
-                GB_CUDA(cudaMemcpyAsync(hs + g, h->plans[g].d_err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        if (h->use_flow && h->flow.d_ctl)
-            GB_CUDA(cudaMemcpyAsync(hs + G, h->flow.d_ctl + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
-        GB_CUDA(cudaMemcpyAsync(hs + G + 1, h->lub.info, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
-        GB_CUDA(cudaMemcpyAsync(hs + G + 1 + h->nsys, h->d_bad, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
-        GB_CUDA(cudaMemcpyAsync(hs + G + 1 + 2 * h->nsys, h->d_fail, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost,
-                                st));
-        GB_CUDA(cudaStreamSynchronize(st));
-        const bool again = h->unchecked && std::any_of(fail, fail + h->nsys, [](int32_t x) { return x != 0; });
-        h->unchecked = h->unchecked && again;
-        if (!again) break;
-        const int rc = batch_settle(h, st);  // repeats them, with interchanges
-        if (rc) return rc;
-    }
+    // outputs are already in the caller's order: straight into the caller's buffers
+    GB_CUDA(cudaMemcpyAsync(coeffs, h->d_out, sizeof(double) * 5 * h->nsolve, cudaMemcpyDeviceToHost, st));
+    if (gamma)
+        GB_CUDA(cudaMemcpyAsync(gamma, h->d_gamma, sizeof(float) * h->gamma_floats, cudaMemcpyDeviceToHost, st));
+    memset(hs, 0, sizeof(int32_t) * (G + 1));
+    for (int g = 0; g < h->ngroups; g++)
+        if (h->plans[g].d_err)
+            GB_CUDA(cudaMemcpyAsync(hs + g, h->plans[g].d_err, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    if (h->use_flow && h->flow.d_ctl)
+        GB_CUDA(cudaMemcpyAsync(hs + G, h->flow.d_ctl + 1, sizeof(int32_t), cudaMemcpyDeviceToHost, st));
+    GB_CUDA(cudaMemcpyAsync(hs + G + 1, h->lub.info, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
+    GB_CUDA(cudaMemcpyAsync(hs + G + 1 + h->nsys, h->d_bad, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
+    GB_CUDA(cudaStreamSynchronize(st));
     for (int g = 0; g < h->ngroups; g++)
         if (hs[g]) {
             set_error("LU: a tensor-core update tile timed out waiting for its MMAs");

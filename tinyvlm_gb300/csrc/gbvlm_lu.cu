@@ -77,6 +77,7 @@ __device__ __forceinline__ void staged_copy(int64_t total, int tid, int nthreads
 template <class T>
 __global__ void __launch_bounds__(PANEL_THREADS) k_panel(LuBatch<T> B, int64_t k, const int32_t* act) {
     const int32_t sid = act[blockIdx.x];
+    if (B.skips(sid)) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     T* A = B.A[sid];
     int32_t* ipiv = B.ipiv[sid];
@@ -477,6 +478,7 @@ __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const
         }
     }
     const int32_t sid = act[sidx];
+    if (B.skips(sid)) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     T* A = B.A[sid];
     int32_t* ipiv = B.ipiv[sid];
@@ -1260,6 +1262,7 @@ __global__ void k_swap(LuBatch<T> B, int64_t k, const int32_t* act, const int64_
     if (g >= tot) return;
     const int a = find_block(pfx, cnt, g);
     const int32_t sid = act[a];
+    if (B.skips(sid)) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     const int nb = (int)min((int64_t)GK, n - k);
     int64_t j = g - pfx[a];  // 0 .. n-nb-1
@@ -1290,6 +1293,7 @@ __global__ void __launch_bounds__(SW2_THREADS) k_swap2(LuBatch<T> B, const int32
     __shared__ int32_t s_ip[LU_OUTER];
     const int a = find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
+    if (B.skips(sid)) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     const int32_t* ip = B.ipiv[sid];
     const int nr = (int)(min(n, r_hi) - r_lo);
@@ -1325,6 +1329,7 @@ __global__ void __launch_bounds__(TRSM_COLS) k_trsm(LuBatch<T> B, int64_t k, con
     __shared__ T L[GK][GK + 1];
     const int a = find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
+    if (B.skips(sid)) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     T* A = B.A[sid];
     const int nb = (int)min((int64_t)GK, n - k);
@@ -1394,6 +1399,7 @@ __global__ void __launch_bounds__(256, 2) k_trsm_wide(LuBatch<float> B, int64_t 
     float* X = L + WW * TW_LS;     // X[r * TW_XS + j]
     const int a = INV ? (int)(blockIdx.x / CTAS) : find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
+    if (B.skips(sid)) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     float* A = B.A[sid];
     // columns of A12 (systems here have n > k0 + WW), or of the identity
@@ -1499,6 +1505,7 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_inner_tc(LuBatch<float> B, i
     __shared__ uint32_t tslot;
     const int a = find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
+    if (B.skips(sid)) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     float* A = B.A[sid];
     const int64_t lo = k + GK, ke = min(n, kend);
@@ -1521,6 +1528,7 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_trsm_tc12(LuBatch<float> B, 
     __shared__ uint32_t tslot;
     const int a = find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
+    if (B.skips(sid)) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     float* A = B.A[sid];
     const int64_t c0 = k0 + LU_OUTER + (int64_t)(blockIdx.x - pfx[a]) * TBN;
@@ -1552,6 +1560,7 @@ __global__ void __launch_bounds__(IN_THREADS) k_inner(LuBatch<float> B, int64_t 
     __shared__ int32_t msrc[GK], mdst[GK];
     const int a = find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
+    if (B.skips(sid)) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     float* A = B.A[sid];
     const int nb = (int)min((int64_t)GK, n - k);  // rows k .. k + nb - 1 and their pivots move
@@ -1614,6 +1623,7 @@ __global__ void __launch_bounds__(GT * GT / 16) k_update(LuBatch<T> B, int64_t k
     __shared__ __align__(16) T sB[GK][SW];  // U12 tile: [kk][col]
     const int a = find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
+    if (B.skips(sid)) return;
     if (B.fail && B.fail[sid]) return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     T* A = B.A[sid];
@@ -1705,6 +1715,7 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_update_tc(LuBatch<float> B, 
     __shared__ uint32_t tslot;
     const int a = find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
+    if (B.skips(sid)) return;
     // without interchanges: nothing to do for a system that needs them (the next
     // diagonal block may set it meanwhile: one thread's reading for all)
     if (part != 1 && B.fail && __syncthreads_or(threadIdx.x == 0 && *(volatile int32_t*)&B.fail[sid])) return;
@@ -1759,6 +1770,7 @@ template <class T>
 __global__ void k_perm(LuBatch<T> B, int32_t base) {
     extern __shared__ int32_t sp[];
     const int32_t sid = base + blockIdx.x;
+    if (B.skips(sid)) return;
     const int64_t n = B.n[sid];
     const int32_t* ip = B.ipiv[sid];
     int32_t* pm = B.perm[sid];

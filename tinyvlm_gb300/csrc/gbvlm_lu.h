@@ -31,6 +31,11 @@ struct LuBatch {
     // them, which the later launches then pass over (zeroed by the caller; null
     // for the pivoting launches)
     int32_t* fail = nullptr;
+    // pivoting launches: the systems to work on, the marked ones (null: all).
+    // Every block of another system leaves at entry.
+    const int32_t* only = nullptr;
+
+    __device__ __forceinline__ bool skips(int32_t sid) const { return only && !only[sid]; }
 };
 
 // One panel launch: active systems [first, first + count) of a step, each
