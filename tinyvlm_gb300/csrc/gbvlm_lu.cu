@@ -23,6 +23,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <chrono>
 #include <mutex>
 #include <type_traits>
 #include <vector>
@@ -450,6 +451,84 @@ __device__ __forceinline__ bool eliminate32(T (&x)[GK], const T* u, int stride, 
     return good;
 }
 
+// A panel's attempt without interchanges.  The pivot search is the panel's serial
+// chain (a barrier, two reductions and a broadcast per column); if every
+// pivot is the diagonal, as it is throughout an AIC, none of it is needed.
+// So one warp factors the 32 x 32 diagonal block, the other rows are
+// eliminated against it, each on its own, and every row checks on the way
+// that |a| <= |pivot| held in each column: exactly then partial pivoting
+// would have kept the diagonal (it comes first on ties).  The operations
+// of a row and their order are those of the pivoting loop, so the factors
+// are the same bits; nothing is written before the verdict.  False, and
+// nothing written: the panel takes the pivoting loop.
+// It is tried unless the panel before moved rows, or, for a system that has
+// been looked over (LuBatch::hint), where the look found no column that needs
+// an interchange: an attempt in vain costs 20 us, in double 65, one that
+// succeeds saves about as much.
+// Out of line, so that the pivoting loop keeps the registers it had without it
+// (in line it spilled with 1024 threads: 3.7 us a panel).
+template <class T, int NT, bool CLUSTER>
+__device__ __noinline__ bool panel_attempt(T* A, int64_t ld, int64_t k, int rows, int slab, int snt, int slice, int nwa,
+                                           int32_t* ipiv, int32_t* mv) {
+    namespace cg = cooperative_groups;
+    using SM = PanelSmem<T, NT, CLUSTER>;
+    extern __shared__ __align__(16) unsigned char pr_smem[];
+    SM& sm = *reinterpret_cast<SM*>(pr_smem);
+    int csize = 1, rank = 0;
+    if constexpr (CLUSTER) {
+        csize = (int)cg::this_cluster().num_blocks();
+        rank = (int)cg::this_cluster().block_rank();
+    }
+    const int tid = (int)threadIdx.x - slice * snt, lane = tid & 31, bar = 1 + slice, nb = min(GK, rows);
+    const int own = rank * slab + tid;
+    const bool have = (CLUSTER ? tid < slab : tid < snt) && own < rows;
+    T(*fu)[GK] = sm.f_u[slice];
+    T* frd = sm.f_rd[slice];
+    T x[GK];
+    auto load_row = [&](int r, bool ok) {
+        const T* src = A + (k + r) + k * ld;
+#pragma unroll
+        for (int t = 0; t < GK; t++) x[t] = (ok && t < nb) ? src[t * ld] : (T)0;
+    };
+    bool good = true;
+    const bool first = tid < 32;  // the slice's first warp factors the diagonal block
+    if (first) {
+        load_row(lane, lane < nb);
+        good = panel_diag<T, GK, true>(x, nb, &fu[0][0], frd, lane);
+        if (rank != 0) load_row(own, have);  // (rank 0's first warp holds those rows)
+        if (lane == 0) sm.f_bad[slice] = good ? 0 : 1;
+    } else {
+        load_row(own, have);
+    }
+    panel_barrier<NT, CLUSTER>(nwa, bar);
+    if (good && sm.f_bad[slice] == 0 && !(first && rank == 0)) {
+        good = eliminate32<T, true>(x, &fu[0][0], GK, frd, nb);
+        if (!have) good = true;  // no row
+    }
+    // the verdict of the slice, or of every CTA of the cluster
+    if (!__all_sync(0xffffffffu, good) && lane == 0) sm.f_bad[slice] = 1;
+    panel_barrier<NT, CLUSTER>(nwa, bar);
+    bool fast = *(volatile int*)&sm.f_bad[slice] == 0;
+    if constexpr (CLUSTER) {
+        cg::cluster_group cl = cg::this_cluster();
+        if (tid < csize) *cl.map_shared_rank(&sm.f_cta[rank], tid) = fast ? 0 : 1;
+        cl.sync();
+        fast = __all_sync(0xffffffffu, lane >= csize || *(volatile int*)&sm.f_cta[lane < csize ? lane : 0] == 0);
+    }
+    if (!fast) return false;
+    if (rank == 0 && tid < nb) {
+        ipiv[k + tid] = (int32_t)(k + tid);
+        if (mv) mv[tid] = mv[GK + tid] = tid;
+    }
+    if (have) {
+        T* dst = A + (k + own) + k * ld;
+#pragma unroll
+        for (int t = 0; t < GK; t++)
+            if (t < nb) dst[t * ld] = x[t];
+    }
+    return true;
+}
+
 template <class T, int NT, bool CLUSTER, int RPT>
 __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const int32_t* act, int slab, int trim,
                                                    const int32_t* pack, int count) {
@@ -495,6 +574,21 @@ __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const
             if (wid - wbase >= nwa) return;
         }
     }
+    if constexpr (RPT == 1) {
+        const auto moved = [&]() {
+            return !__all_sync(0xffffffffu, ipiv[k - GK + lane] == (int32_t)(k - GK + lane));
+        };
+        bool tried;
+        if (B.hint) {
+            const int32_t* hint = B.hint + (int64_t)sid * B.hint_ld + k / GK;
+            tried = hint[0] == 0 && (k < GK || hint[-1] != 0 || !moved());
+        } else {
+            tried = k < GK || !moved();
+        }
+        if (tried && panel_attempt<T, NT, CLUSTER>(A, ld, k, rows, slab, snt, slice, nwa, ipiv,
+                                                   B.mv ? B.mv + (int64_t)sid * 64 : nullptr))
+            return;
+    }
 
     // own rows: slab-relative tid, tid + NT, ...; lid = logical position, -1: no row
     int lid[RPT];
@@ -507,66 +601,12 @@ __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const
 #pragma unroll
         for (int t = 0; t < GK; t++) x[i][t] = (lid[i] >= 0 && t < nb) ? src[t * ld] : (T)0;
     }
-
-    // Attempt without interchanges.  The pivot search is the panel's serial
-    // chain (a barrier, two reductions and a broadcast per column); if every
-    // pivot is the diagonal, as it is throughout an AIC, none of it is needed.
-    // So one warp factors the 32 x 32 diagonal block, the other rows are
-    // eliminated against it, each on its own, and every row checks on the way
-    // that |a| <= |pivot| held in each column: exactly then partial pivoting
-    // would have kept the diagonal (it comes first on ties).  The operations
-    // of a row and their order are those of the pivoting loop, so the factors
-    // are the same bits; nothing is written before the verdict.  A panel that
-    // fails is read again and takes the pivoting loop, and so, without an
-    // attempt, does one whose predecessor moved rows.
-    bool fast = false;
-    if constexpr (RPT == 1) {
-        const bool tried =
-            k < GK || __all_sync(0xffffffffu, ipiv[k - GK + lane] == (int32_t)(k - GK + lane));
-        if (tried) {
-            T(*fu)[GK] = sm.f_u[slice];
-            T* frd = sm.f_rd[slice];
-            auto load_row = [&](int r, bool have) {
-                const T* src = A + (k + r) + k * ld;
-#pragma unroll
-                for (int t = 0; t < GK; t++) x[0][t] = (have && t < nb) ? src[t * ld] : (T)0;
-            };
-            bool good = true;
-            const bool first = tid < 32;  // the slice's first warp factors the diagonal block
-            if (first) {
-                if (rank != 0) load_row(lane, lane < nb);  // rank 0's first warp holds those rows
-                good = panel_diag<T, GK, true>(x[0], nb, &fu[0][0], frd, lane);
-                if (rank != 0) load_row(lid[0], lid[0] >= 0);
-                if (lane == 0) sm.f_bad[slice] = good ? 0 : 1;
-            }
-            panel_barrier<NT, CLUSTER>(nwa, bar);
-            if (good && sm.f_bad[slice] == 0 && !(first && rank == 0)) {
-                good = eliminate32<T, true>(x[0], &fu[0][0], GK, frd, nb);
-                if (lid[0] < 0) good = true;  // no row
-            }
-            // the verdict of the slice, or of every CTA of the cluster
-            if (!__all_sync(0xffffffffu, good) && lane == 0) sm.f_bad[slice] = 1;
-            panel_barrier<NT, CLUSTER>(nwa, bar);
-            fast = *(volatile int*)&sm.f_bad[slice] == 0;
-            if constexpr (CLUSTER) {
-                cg::cluster_group cl = cg::this_cluster();
-                if (tid < csize) *cl.map_shared_rank(&sm.f_cta[rank], tid) = fast ? 0 : 1;
-                cl.sync();
-                fast = __all_sync(0xffffffffu, lane >= csize || *(volatile int*)&sm.f_cta[lane < csize ? lane : 0] == 0);
-            }
-            if (fast) {
-                if (rank == 0 && tid < nb) ipiv[k + tid] = (int32_t)(k + tid);
-            } else {
-                load_row(lid[0], lid[0] >= 0);
-            }
-        }
-    }
     Key cand = Key::none();  // best candidate of the own rows for the current column
 #pragma unroll
     for (int i = 0; i < RPT; i++)
         if (lid[i] >= 0) cand = Key::kmax(cand, Key::make(x[i][0], lid[i]));
 
-    if (!fast) static_for<0, GK>([&](auto JJ) {
+    static_for<0, GK>([&](auto JJ) {
         constexpr int jj = decltype(JJ)::value;
         if (jj < nb) {
             const int buf = jj & 1;
@@ -638,8 +678,7 @@ __global__ void __launch_bounds__(NT) k_panel_reg(LuBatch<T> B, int64_t k, const
             }
         }
     });
-    if constexpr (CLUSTER)
-        if (!fast) cg::this_cluster().sync();  // no CTA leaves while its rows may still be read
+    if constexpr (CLUSTER) cg::this_cluster().sync();  // no CTA leaves while its rows may still be read
     // panels of a system run in order, so the first zero pivot recorded is the first of the factorisation
     if (zero_col >= 0) atomicCAS(&B.info[sid], 0, (int32_t)(k + zero_col + 1));
     if (B.mv) {  // the panel's row moves, for the other columns of the outer block
@@ -856,7 +895,7 @@ __global__ void __launch_bounds__(Fast<float>::DT) k_lu_diag(LuBatch<float> B, i
         __syncthreads();
     }
     if (s_bad) {
-        if (tid == 0) B.fail[sid] = 1;
+        if (tid == 0) B.fail[sid] = LU_LEFT;
         return;
     }
     float* wk = work + (int64_t)(sid - base) * F::WORK;
@@ -1001,7 +1040,7 @@ __global__ void __launch_bounds__(Fast<float>::RT) k_lu_rows(LuBatch<float> B, i
             for (int t = 0; t < GK; t++) Xs[(GK * c + t) * LDX + tid] = x[t];
     }
     if (rows) {
-        if (have && !good) B.fail[J.sid] = 1;
+        if (have && !good) B.fail[J.sid] = LU_LEFT;
         return;
     }
     __syncwarp();  // a warp's 32 columns are its own
@@ -1092,7 +1131,7 @@ __global__ void __launch_bounds__(Fast<float>::RT) k_lu_rows_split(LuBatch<float
         if (J.i0 + lane < J.n) {
             float* dst = J.A + J.i0 + lane + k0 * J.ld;
             for (int t = s; t < F::W; t += S) dst[t * J.ld] = Xs[t * LDX + lane];
-            if (!good) B.fail[J.sid] = 1;
+            if (!good) B.fail[J.sid] = LU_LEFT;
         }
         return;
     }
@@ -1102,6 +1141,60 @@ __global__ void __launch_bounds__(Fast<float>::RT) k_lu_rows_split(LuBatch<float
 #pragma unroll
         for (int c = 0; c < NB; c++) col[GK * c + lane] = Xs[(GK * c + lane) * LDX + q];
     }
+}
+
+// Whether a matrix can be factored without interchanges shows before the
+// elimination: the AICs of regular wings have no entry below the diagonal above
+// 0.6 of it (60 wings, 27 to 1900 unknowns), those that need interchanges,
+// with slivers at a tip, have entries many times it.  So a matrix is looked
+// over first, and one with an entry below the diagonal larger than it is not
+// attempted.  A matrix that passes may still turn out to need interchanges.
+// Measured (pivoting launches alone; attempt in vain, then those; with the look):
+// random matrix of 256 in float 464, 546, 485 us, of 4096 12.4, 13.5, 12.4 ms, of
+// 256 in double 1200, 1369, 1224 us; the steady solve of an elliptic 64 x 64 wing,
+// whose panels off the tip need none, 10.2, 11.6, 8.7 ms.  Without interchanges
+// nothing is lost: the copy is made anyway.
+//
+// k_lu_keep copies the matrix on the way (a warp per column), for that case, up to
+// the first such entry; copying bounds it.  found[0] becomes LU_SEEN, and so does
+// *told, in host memory, for a host that is still issuing the attempt's launches;
+// or *told becomes LU_PASSED (found[1] counts the blocks that are done, zero
+// before).  hint[p] becomes 1 for a panel p of 32 columns with such an entry.
+template <class T>
+__global__ void __launch_bounds__(256) k_lu_keep(const T* A, int64_t n, int64_t ld, T* copy, int32_t* found,
+                                                 int32_t* hint, volatile int32_t* told) {
+    const int lane = threadIdx.x & 31;
+    for (int64_t j = blockIdx.x * 8 + (threadIdx.x >> 5); j < n; j += gridDim.x * 8) {
+        const bool keep = *(volatile int32_t*)found == 0;
+        const T* a = A + j * ld;
+        T* c = copy + j * n;
+        const T d = a[j];
+        bool good = true;
+#pragma unroll 1
+        for (int64_t r0 = keep ? lane : (j & ~(int64_t)31) + lane; r0 < n; r0 += 32 * 8) {
+            T v[8];
+#pragma unroll
+            for (int u = 0; u < 8; u++) v[u] = r0 + 32 * u < n ? a[r0 + 32 * u] : (T)0;
+#pragma unroll
+            for (int u = 0; u < 8; u++) {
+                const int64_t r = r0 + 32 * u;
+                if (keep && r < n) c[r] = v[u];
+                good = good && (r <= j || r >= n || not_above(v[u], d));
+            }
+            if (!keep && !__all_sync(0xffffffffu, good)) break;
+        }
+        if (!__all_sync(0xffffffffu, good) && lane == 0) {
+            hint[j / GK] = 1;
+            if (*(volatile int32_t*)found == 0) {
+                *(volatile int32_t*)found = LU_SEEN;
+                *told = LU_SEEN;
+            }
+        }
+    }
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0 && atomicAdd(found + 1, 1) == (int)gridDim.x - 1 && *(volatile int32_t*)found == 0)
+        *told = LU_PASSED;
 }
 
 // Double: 32-column blocks.  A warp's fp64 instruction takes a sub-partition
@@ -1164,7 +1257,7 @@ __global__ void __launch_bounds__(Fast<double>::DT) k_lu_diag64(LuBatch<double> 
     });
     const bool bad = __syncthreads_or(!good);
     if (bad) {
-        if (tid == 0) B.fail[sid] = 1;
+        if (tid == 0) B.fail[sid] = LU_LEFT;
         return;
     }
     double* wk = work + (int64_t)(sid - base) * Fast<double>::WORK;
@@ -1243,7 +1336,7 @@ __global__ void __launch_bounds__(Fast<double>::DT) k_lu_rows64(LuBatch<double> 
         if (have) {
 #pragma unroll
             for (int q = 0; q < 8; q++) A[i0 + lane + (k0 + 4 * q + s) * ld] = x[q];
-            if (!good) B.fail[sid] = 1;
+            if (!good) B.fail[sid] = LU_LEFT;
         }
         return;
     }
@@ -1716,9 +1809,12 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_update_tc(LuBatch<float> B, 
     const int a = find_block(pfx, cnt, blockIdx.x);
     const int32_t sid = act[a];
     if (B.skips(sid)) return;
-    // without interchanges: nothing to do for a system that needs them (the next
-    // diagonal block may set it meanwhile: one thread's reading for all)
-    if (part != 1 && B.fail && __syncthreads_or(threadIdx.x == 0 && *(volatile int32_t*)&B.fail[sid])) return;
+    // without interchanges: nothing to do for a system that needs them (beside
+    // parts 0 and 2 the next diagonal block may find that out: one thread's
+    // reading for all)
+    if (B.fail && (part == 1 ? B.fail[sid] != 0
+                             : __syncthreads_or(threadIdx.x == 0 && *(volatile int32_t*)&B.fail[sid]) != 0))
+        return;
     const int64_t n = B.n[sid], ld = B.ld[sid];
     float* A = B.A[sid];
     const int64_t lo = k0 + w;  // systems here have n > k0 + w
@@ -3043,7 +3139,8 @@ int lu_batch_factor(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t st, bo
 }
 
 template <class T>
-int lu_batch_factor_fast(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t st, bool lookahead) {
+int lu_batch_factor_fast(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t st, bool lookahead,
+                         const volatile int32_t* told) {
     using F = Fast<T>;
     constexpr int E = sizeof(T) == 4 ? 0 : 1;
     GB_REQUIRE(B.fail && plan.d_minv, "factorisation without interchanges: no workspace");
@@ -3059,6 +3156,14 @@ int lu_batch_factor_fast(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t s
         else
             k_lu_diag64<<<(unsigned)S.n_panel, F::DT, 0, st>>>(B, S.k, act, work, plan.base);
         GB_LAUNCH_CHECK();
+        // the first diagonal block keeps the device busy (15 us and more) while the host waits to be told
+        // (not for long: other work may lie before this on the stream)
+        if (told && S.k == 0) {
+            const auto t0 = std::chrono::steady_clock::now();
+            while (*told == 0 && std::chrono::steady_clock::now() - t0 < std::chrono::microseconds(15)) {
+            }
+        }
+        if (told && *told == LU_SEEN) break;
         if (S.fr_blocks[E] == 0) continue;
         if (pending) {  // the columns that k_lu_rows solves are those the lookahead update is still working on
             GB_CUDA(cudaStreamWaitEvent(st, plan.la_join, 0));
@@ -3146,8 +3251,10 @@ int lu_batch_solve(const LuBatch<T>& B, int32_t nsys, int32_t max_nrhs, int64_t 
 
 template int lu_batch_factor<float>(const LuBatch<float>&, const LuPlan&, cudaStream_t, bool);
 template int lu_batch_factor<double>(const LuBatch<double>&, const LuPlan&, cudaStream_t, bool);
-template int lu_batch_factor_fast<float>(const LuBatch<float>&, const LuPlan&, cudaStream_t, bool);
-template int lu_batch_factor_fast<double>(const LuBatch<double>&, const LuPlan&, cudaStream_t, bool);
+template int lu_batch_factor_fast<float>(const LuBatch<float>&, const LuPlan&, cudaStream_t, bool,
+                                         const volatile int32_t*);
+template int lu_batch_factor_fast<double>(const LuBatch<double>&, const LuPlan&, cudaStream_t, bool,
+                                          const volatile int32_t*);
 template int lu_batch_solve<float>(const LuBatch<float>&, int32_t, int32_t, int64_t, cudaStream_t, int*);
 template int lu_batch_solve<double>(const LuBatch<double>&, int32_t, int32_t, int64_t, cudaStream_t, int*);
 
@@ -3882,7 +3989,7 @@ static int lu_ensure(gbvlm_lu h, int64_t n, cudaStream_t st) {
     h->d_perm = nullptr;
     GB_CUDA(cudaMalloc(&h->d_ipiv, sizeof(int32_t) * (n > 0 ? n : 1)));
     GB_CUDA(cudaMalloc(&h->d_perm, sizeof(int32_t) * (n > 0 ? n : 1)));
-    GB_CUDA(cudaMalloc(&h->d_info, 2 * sizeof(int32_t)));  // info, and that interchanges are needed
+    GB_CUDA(cudaMalloc(&h->d_info, sizeof(int32_t) * (3 + cdiv(n, GK))));  // info, k_lu_keep's found and hint
     std::vector<int64_t> ns(1, n);
     int rc = lu_plan_build(h->plan, ns, st);
     if (rc) return rc;
@@ -3891,24 +3998,32 @@ static int lu_ensure(gbvlm_lu h, int64_t n, cudaStream_t st) {
     return GBVLM_OK;
 }
 
-// a copy of the matrix; false if there is no memory for one
-template <class T>
-static bool lu_backup(gbvlm_lu h, const T* A, int64_t n, int64_t ld, cudaStream_t st) {
-    const size_t need = sizeof(T) * (size_t)n * (size_t)n;
-    if (h->backup_bytes < need) {
-        if (h->backup) cudaFree(h->backup);
-        h->backup = nullptr;
-        h->backup_bytes = 0;
-        if (cudaMalloc(&h->backup, need) != cudaSuccess) {
-            cudaGetLastError();
-            return false;
-        }
-        h->backup_bytes = need;
+// room for a copy of the matrix; false if there is no memory for one
+static bool lu_backup(gbvlm_lu h, size_t need) {
+    if (h->backup_bytes >= need) return true;
+    if (h->backup) cudaFree(h->backup);
+    h->backup = nullptr;
+    h->backup_bytes = 0;
+    if (cudaMalloc(&h->backup, need) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
     }
-    const cudaError_t e =
-        cudaMemcpy2DAsync(h->backup, sizeof(T) * n, A, sizeof(T) * ld, sizeof(T) * n, n, cudaMemcpyDeviceToDevice, st);
-    if (e != cudaSuccess) cudaGetLastError();
-    return e == cudaSuccess;
+    h->backup_bytes = need;
+    return true;
+}
+
+// The stream's work done, or the host told that the matrix needs interchanges.
+// Told at once, the host issues the pivoting launches behind the attempt's empty
+// ones; waiting for the stream first leaves the device idle for 15 us.
+static int lu_wait_told(cudaStream_t st, const volatile int32_t* told) {
+    for (int k = 0; k < 64 && *told != LU_PASSED; k++) {  // some 100 us, then a wait
+        if (*told == LU_SEEN) return GBVLM_OK;
+        const cudaError_t e = cudaStreamQuery(st);
+        if (e == cudaSuccess) return GBVLM_OK;
+        if (e != cudaErrorNotReady) GB_CUDA(e);
+    }
+    GB_CUDA(cudaStreamSynchronize(st));
+    return GBVLM_OK;
 }
 
 template <class T>
@@ -3921,36 +4036,44 @@ static int lu_factor_one(gbvlm_lu h, T* A, int64_t n, int64_t ld, cudaStream_t s
     LuBatch<T> B;
     rc = make_single_batch<T>(B, n, ld, A, h->d_ipiv, h->d_perm, h->d_info, nullptr, 0, 0, &h->work, &h->work_bytes, st);
     if (rc) return rc;
-    int32_t* hi = (int32_t*)host_scratch(5 * sizeof(int32_t));  // info, needs interchanges, solve words, tile word
+    // info, needs interchanges, solve words, tile word, told by k_lu_keep
+    int32_t* hi = (int32_t*)host_scratch(6 * sizeof(int32_t));
     GB_REQUIRE(hi != nullptr, "pinned host allocation failed");
-    auto read = [&](int words) -> int {
-        hi[4] = 0;
+    auto fetch = [&](int words) -> int {
         GB_CUDA(cudaMemcpyAsync(hi, h->d_info, words * sizeof(int32_t), cudaMemcpyDeviceToHost, st));
         const int r = lu_solve_words(h, hi + 2, st);
         if (r) return r;
         if (h->plan.d_err) GB_CUDA(cudaMemcpyAsync(hi + 4, h->plan.d_err, sizeof(int), cudaMemcpyDeviceToHost, st));
-        GB_CUDA(cudaStreamSynchronize(st));
         return GBVLM_OK;
     };
     bool done = false;
     // without interchanges first; single-block systems' panel tries that itself
-    const bool fast =
-        !pivot && (sizeof(T) == 4 ? h->plan.fast : h->plan.fast_any) && n > GK && lu_backup<T>(h, A, n, ld, st);
+    const bool fast = !pivot && (sizeof(T) == 4 ? h->plan.fast : h->plan.fast_any) && n > GK &&
+                      lu_backup(h, sizeof(T) * (size_t)n * (size_t)n);
+    hi[4] = 0;
     if (fast) {
-        GB_CUDA(cudaMemsetAsync(h->d_info + 1, 0, sizeof(int32_t), st));
+        volatile int32_t* told = hi + 5;
+        *told = 0;
+        GB_CUDA(cudaMemsetAsync(h->d_info + 1, 0, sizeof(int32_t) * (2 + cdiv(n, GK)), st));
+        k_lu_keep<T><<<(unsigned)std::min<int64_t>(cdiv(n, 8), 16 * tc_num_sms()), 256, 0, st>>>(
+            A, n, ld, (T*)h->backup, h->d_info + 1, h->d_info + 3, hi + 5);
+        GB_LAUNCH_CHECK();
         B.fail = h->d_info + 1;
-        rc = lu_batch_factor_fast<T>(B, h->plan, st, true);
+        rc = lu_batch_factor_fast<T>(B, h->plan, st, true, told);
         B.fail = nullptr;
-        if (rc) return rc;
-        if ((rc = read(2))) return rc;
-        done = hi[1] == 0;
-        if (!done)
+        // the host usually has been told by now; the words' copies then would only delay the pivoting launches
+        if (rc || (*told != LU_SEEN && ((rc = fetch(2)) || (rc = lu_wait_told(st, told))))) return rc;
+        const bool seen = *told == LU_SEEN;
+        done = !seen && hi[1] == 0;
+        if (!seen && hi[1] != 0)  // found on the way: the matrix has been worked on
             GB_CUDA(cudaMemcpy2DAsync(A, sizeof(T) * ld, h->backup, sizeof(T) * n, sizeof(T) * n, n,
                                       cudaMemcpyDeviceToDevice, st));
     }
     if (!done) {
+        if (fast) B.hint = h->d_info + 3;
         rc = lu_batch_factor<T>(B, h->plan, st, true);
-        if (rc || (rc = read(1))) return rc;
+        if (rc || (rc = fetch(1))) return rc;
+        GB_CUDA(cudaStreamSynchronize(st));
     }
     if (*hi != 0) {
         set_error("LU: exactly zero pivot at column %d", *hi);

@@ -10,6 +10,12 @@ namespace gbvlm {
 constexpr int LU_NB = 32;      // panel width
 constexpr int LU_OUTER = 128;  // outer block width with tensor-core updates
 
+// values of LuBatch::fail
+constexpr int32_t LU_SEEN = 1;  // seen in the matrix before the factorisation: nothing has been done to it
+constexpr int32_t LU_LEFT = 2;  // found on the way: the matrix is partly factored
+// what the host is told while it issues launches: LU_SEEN, or that the matrix passed
+constexpr int32_t LU_PASSED = -1;
+
 // Device tables, one entry per system (systems sorted by n descending).
 template <class T>
 struct LuBatch {
@@ -27,13 +33,17 @@ struct LuBatch {
     // ends at position k + t, [32 + r] = final offset of the row that started
     // at k + r (null: not recorded)
     int32_t* mv = nullptr;
-    // factorisation without interchanges: set to 1 for a system that needs
+    // factorisation without interchanges: not zero for a system that needs
     // them, which the later launches then pass over (zeroed by the caller; null
     // for the pivoting launches)
     int32_t* fail = nullptr;
     // pivoting launches: the systems to work on, the marked ones (null: all).
     // Every block of another system leaves at entry.
     const int32_t* only = nullptr;
+    // pivoting launches: per system (hint_ld apart) and panel of 32 columns, not
+    // zero where the matrix has an entry below the diagonal larger than it (null: not looked)
+    const int32_t* hint = nullptr;
+    int64_t hint_ld = 0;
 
     __device__ __forceinline__ bool skips(int32_t sid) const { return only && !only[sid]; }
 };
@@ -138,9 +148,11 @@ int64_t lu_plan_launches(const LuPlan& plan, int es);
 // inner steps (float, tensor-core plans; ignored while timing launches)
 template <class T>
 int lu_batch_factor(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t st, bool lookahead);
-// the same without interchanges; B.fail marks the systems that need them
+// the same without interchanges; B.fail marks the systems that need them.
+// told: host memory that the device sets once no system is left to factor (or null): no further launch is issued
 template <class T>
-int lu_batch_factor_fast(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t st, bool lookahead);
+int lu_batch_factor_fast(const LuBatch<T>& B, const LuPlan& plan, cudaStream_t st, bool lookahead,
+                         const volatile int32_t* told = nullptr);
 // number of kernel launches that makes for element size es (4 or 8)
 int64_t lu_plan_launches_fast(const LuPlan& plan, int es);
 // err: the tensor-core error word of a plan with tensor cores (a single large
