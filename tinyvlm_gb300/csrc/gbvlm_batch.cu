@@ -80,11 +80,13 @@ struct BatchArgs {
     const int64_t* goff;
     const int32_t* uidx;    // batch solve -> the caller's solve index
     int32_t* bad;           // per system: 1 if its case's vertices hold a non-finite coordinate
-    int32_t* fail;          // per system: 1 if its factorisation needs row interchanges (LuBatch::fail)
+    int32_t* fail;          // per system: whether its factorisation needs row interchanges (LuBatch::fail)
+    int32_t* hint;          // per system, hint_ld apart: LuBatch::hint
+    int64_t hint_ld;
     int32_t* info;          // per system: first zero pivot's column + 1 (LuBatch::info)
-    int32_t only_failed;    // the launches factor those systems again, with interchanges, and pass over the others
+    int32_t only_left;      // the launches restore the AICs of systems whose factorisation was given up (LU_LEFT)
 
-    __device__ __forceinline__ bool skips(int si) const { return only_failed && !fail[si]; }
+    __device__ __forceinline__ bool skips(int si) const { return only_left && fail[si] != LU_LEFT; }
 };
 
 __device__ __forceinline__ void split_hl(double x, float& h, float& l) {
@@ -105,6 +107,8 @@ __global__ void __launch_bounds__(256) k_batch_geom(BatchArgs a) {
         a.fail[blockIdx.x] = 0;
         a.info[blockIdx.x] = 0;
     }
+    if (blockIdx.y == 0)
+        for (int64_t e = threadIdx.x; e < a.hint_ld; e += blockDim.x) a.hint[blockIdx.x * a.hint_ld + e] = 0;
     int bad = 0;
     const int64_t t0 = threadIdx.x + blockIdx.y * (int64_t)blockDim.x, stride = gridDim.y * (int64_t)blockDim.x;
     if (blockIdx.y == 0)
@@ -1035,6 +1039,9 @@ struct gbvlm_batch_s {
     int32_t* d_uidx = nullptr;   // batch solve -> the caller's solve
     int32_t* d_bad = nullptr;    // per system: non-finite input vertices
     int32_t* d_fail = nullptr;   // per system: its factorisation needs row interchanges
+    int32_t* d_hint = nullptr;   // per system and 32 columns: seen to need them there
+    int64_t hint_ld = 0;
+    int32_t gsys[5] = {};             // first system of each size group
     void* status = nullptr;      // pinned: error words and pivot flags read back with the results
     SysDesc* d_sys = nullptr;
     int32_t* d_solve_sys = nullptr;
@@ -1169,17 +1176,25 @@ static bool batch_fast(gbvlm_batch h) {
     return false;
 }
 
-// one size group's factorisation: without interchanges, d_fail marking the
-// systems that need them, or (pivot) with them, those systems only
-static int batch_factor(gbvlm_batch h, int g, cudaStream_t st, bool lookahead, bool pivot) {
-    LuBatch<float> B = h->lub;
-    if (!h->plans[g].fast) return pivot ? GBVLM_OK : lu_batch_factor<float>(B, h->plans[g], st, lookahead);
-    if (pivot) {
-        B.only = h->d_fail;
-        return lu_batch_factor<float>(B, h->plans[g], st, lookahead);
+// Looks a group's AICs (systems i0 ..) over before their factorisation (k_lu_keep's
+// look, a warp per column): the rings of the next two rows, where a column that
+// needs an interchange shows it (16 wings of 36 to 2304 unknowns that do: in 70 %
+// of their columns with a larger entry anywhere, in every wing).  A system that
+// does is not attempted.
+__global__ void __launch_bounds__(256) k_batch_look(BatchArgs a, int32_t i0) {
+    const int32_t si = i0 + blockIdx.y;
+    const SysDesc& S = a.sys[si];
+    const int64_t n = S.n, j = blockIdx.x * 8 + (threadIdx.x >> 5);
+    if (j >= n) return;
+    const float* c = S.A + j * n;
+    const float d = fabsf(c[j]);
+    const int64_t end = min(n, j + 2 + 2 * S.ns);
+    bool good = true;
+    for (int64_t r = j + 1 + (threadIdx.x & 31); r < end; r += 32) good = good && fabsf(c[r]) <= d;  // (not for a NaN)
+    if (!__all_sync(0xffffffffu, good) && (threadIdx.x & 31) == 0) {
+        a.hint[si * a.hint_ld + j / LU_NB] = 1;
+        a.fail[si] = LU_SEEN;
     }
-    B.fail = h->d_fail;
-    return lu_batch_factor_fast<float>(B, h->plans[g], st, lookahead);
 }
 
 __global__ void k_batch_restore(BatchArgs a) {
@@ -1189,172 +1204,174 @@ __global__ void k_batch_restore(BatchArgs a) {
     for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += stride) S.A[e] = S.A2[e];
 }
 
-// A run's phases: FACTOR, up to the factorisation without interchanges; REPEAT,
-// the systems that need them once more (their unfactored AICs copied back where
-// they are kept, else assembled again; every other system's blocks leave at
-// entry); SOLVE, from the solves on, all systems.
-enum { BATCH_FACTOR = 1, BATCH_REPEAT = 2, BATCH_SOLVE = 4 };
-
-static int batch_enqueue(gbvlm_batch h, cudaStream_t st, int phases, cudaEvent_t* ev = nullptr,
-                         bool serial_lu = false) {
-    auto mark = [&](int k) { if (ev) cudaEventRecord(ev[k], st); };
-    int64_t nlaunch = 0;
-    for (int g = 0; g < h->ngroups; g++)
-        nlaunch += h->plans[g].fast ? lu_plan_launches_fast(h->plans[g], 4) : lu_plan_launches(h->plans[g], 4);
-    int32_t mr = 0;
-    for (auto& s : h->sys) mr = std::max(mr, s.nrhs);
-    const int64_t solves = h->use_flow ? trs_flow_launches(mr, h->flow.groups) : (mr + 7) / 8;
-    // geometry, Trefftz, the groups' assemblies, RHS, the factorisations, the
-    // solves and accumulations, the refinement sweeps, the loads
-    h->launches = 3 + h->ngroups * (h->fp64_residual ? 2 : 1) + nlaunch + solves + 1 +
-                  (int64_t)h->refine * (1 + solves + 1) + 1 + (batch_fast(h) ? 1 : 0);
+// The launches of a run
+struct BatchRun {
+    gbvlm_batch h;
     BatchArgs a;
-    a.sys = h->d_sys;
-    a.nsys = h->nsys;
-    a.u_inf = h->u_inf;
-    a.beta = h->beta;
-    a.rho = h->rho;
-    for (int k = 0; k < 3; k++) a.ref[k] = h->ref[k];
-    a.alphas = h->d_alpha;
-    a.out = h->d_out;
-    a.gamma_out = h->d_gamma;
-    a.goff = h->d_goff;
-    a.uidx = h->d_uidx;
-    a.bad = h->d_bad;
-    a.fail = h->d_fail;
-    a.info = h->lub.info;
-    a.only_failed = 0;
-    // staged: every phase after the previous one on `st` (stage timing, or
-    // kernel timing without the groups' launches overlapping); otherwise each
-    // size group's assembly and factorisation run on its own branch, group 0
-    // (the longest chain) on a high-priority stream
-    const bool staged = ev != nullptr || serial_lu;
-    // the Trefftz influence matrices need only the geometry: launched where
-    // they run beside the assembly and the factorisation
-    auto trefftz = [&]() {
-        int64_t maxns = 1;
-        for (auto& s : h->sys) maxns = std::max(maxns, s.ns);
-        const dim3 gk((unsigned)cdiv(maxns * maxns, 128), (unsigned)h->nsys);
-        k_batch_trefftz_k<<<gk, 128, 0, st>>>(a);
-        return cudaGetLastError();
-    };
-    auto assemble_all = [&]() {
-        return launch_assemble(h, (unsigned)(h->asm_rows > 1 ? h->assembly_tiles_rows : h->assembly_tiles), 0, a, st);
-    };
-    const dim3 gp((unsigned)cdiv(h->maxn, 256), (unsigned)h->nsys);  // one thread per row of every system
-    // the size groups' factorisations: one after another on `st`, or each on its branch, joined on `st`
-    auto factor = [&](bool pivot, auto&& before, auto&& beside) -> int {
-        if (staged) {
-            for (int g = 0; g < h->ngroups; g++) {
-                const int rc = batch_factor(h, g, st, !serial_lu, pivot);
-                if (rc) return rc;
-            }
-            return GBVLM_OK;
-        }
-        GB_CUDA(cudaEventRecord(h->fork, st));
-        for (int g = 0; g < h->ngroups; g++) {
-            GB_CUDA(cudaStreamWaitEvent(h->side[g], h->fork, 0));
-            int rc = before(g);
-            if (rc == GBVLM_OK) rc = batch_factor(h, g, h->side[g], true, pivot);
-            if (rc) return rc;
-            GB_CUDA(cudaEventRecord(h->join[g], h->side[g]));
-        }
-        const int rc = beside();
-        if (rc) return rc;
-        for (int g = 0; g < h->ngroups; g++) GB_CUDA(cudaStreamWaitEvent(st, h->join[g], 0));
-        return GBVLM_OK;
-    };
-    int rc = GBVLM_OK;
-    if (phases & BATCH_FACTOR) {
-        mark(0);
+    int32_t maxrhs = 0;
+
+    explicit BatchRun(gbvlm_batch h_) : h(h_) {
+        a.sys = h->d_sys;
+        a.nsys = h->nsys;
+        a.u_inf = h->u_inf;
+        a.beta = h->beta;
+        a.rho = h->rho;
+        for (int k = 0; k < 3; k++) a.ref[k] = h->ref[k];
+        a.alphas = h->d_alpha;
+        a.out = h->d_out;
+        a.gamma_out = h->d_gamma;
+        a.goff = h->d_goff;
+        a.uidx = h->d_uidx;
+        a.bad = h->d_bad;
+        a.fail = h->d_fail;
+        a.hint = h->d_hint;
+        a.hint_ld = h->hint_ld;
+        a.info = h->lub.info;
+        a.only_left = 0;
+        for (auto& s : h->sys) maxrhs = std::max(maxrhs, s.nrhs);
+    }
+
+    bool fast(int g) const { return h->plans[g].fast; }
+    // (a system of one 128-column block: the attempt is one launch, no longer than the look and its condition)
+    bool looks(int g) const { return fast(g) && h->plans[g].maxn > LU_OUTER; }
+
+    int geometry(cudaStream_t st) const {
         const int64_t fill = 2 * tc_num_sms() / std::max<int64_t>(1, h->nsys);
         const dim3 gg((unsigned)h->nsys, (unsigned)std::max<int64_t>(1, std::min(cdiv(h->maxn, 256), fill)));
         k_batch_geom<<<gg, 256, 0, st>>>(a);
         GB_LAUNCH_CHECK();
-        if (staged) GB_CUDA(trefftz());
-        mark(1);
-        if (staged) {
-            GB_CUDA(assemble_all());
-            if (h->fp64_residual)
-                GB_CUDA(launch_assemble_lo(h, (unsigned)(lo_rows(h) ? h->assembly_tiles_rows : h->assembly_tiles), 0, a, st));
-        }
-        mark(2);
-        if (staged) {
-            k_batch_rhs<<<gp, 256, 0, st>>>(a);
-            GB_LAUNCH_CHECK();
-        }
-        mark(3);
-        rc = factor(
-            false,
-            [&](int g) -> int {
-                if (h->gtile[g][1] == 0) return GBVLM_OK;
-                const int64_t(&gt)[2] = h->asm_rows > 1 ? h->gtile_rows[g] : h->gtile[g];
-                GB_CUDA(launch_assemble(h, (unsigned)gt[1], gt[0], a, h->side[g]));
-                if (h->fp64_residual) {
-                    GB_CUDA(cudaEventRecord(h->asm_done[g], h->side[g]));
-                    GB_CUDA(cudaStreamWaitEvent(h->lo_side, h->asm_done[g], 0));
-                    const int64_t(&lt)[2] = lo_rows(h) ? h->gtile_rows[g] : h->gtile[g];
-                    GB_CUDA(launch_assemble_lo(h, (unsigned)lt[1], lt[0], a, h->lo_side));
-                }
-                return GBVLM_OK;
-            },
-            [&]() -> int {
-                GB_CUDA(trefftz());
-                k_batch_rhs<<<gp, 256, 0, st>>>(a);
-                GB_LAUNCH_CHECK();
-                return GBVLM_OK;
-            });
-        if (rc) return rc;
-        if (h->fp64_residual && !staged) {
-            GB_CUDA(cudaEventRecord(h->lo_join, h->lo_side));
-            if (!(phases & BATCH_SOLVE)) GB_CUDA(cudaStreamWaitEvent(st, h->lo_join, 0));
-        }
+        return GBVLM_OK;
     }
-    if (phases & BATCH_REPEAT) {
-        a.only_failed = 1;
+    // the Trefftz influence matrices and the right-hand sides need only the
+    // geometry: launched where they run beside the assembly and the factorisation
+    int trefftz(cudaStream_t st) const {
+        int64_t maxns = 1;
+        for (auto& s : h->sys) maxns = std::max(maxns, s.ns);
+        const dim3 gk((unsigned)cdiv(maxns * maxns, 128), (unsigned)h->nsys);
+        k_batch_trefftz_k<<<gk, 128, 0, st>>>(a);
+        GB_LAUNCH_CHECK();
+        return GBVLM_OK;
+    }
+    dim3 rows() const { return dim3((unsigned)cdiv(h->maxn, 256), (unsigned)h->nsys); }  // a thread per row of every system
+    int rhs(cudaStream_t st) const {
+        k_batch_rhs<<<rows(), 256, 0, st>>>(a);
+        GB_LAUNCH_CHECK();
+        return GBVLM_OK;
+    }
+    // the float AICs of group g, of all with g < 0
+    int assemble(int g, cudaStream_t st) const {
+        const bool rw = h->asm_rows > 1;
+        const int64_t t0 = g < 0 ? 0 : (rw ? h->gtile_rows : h->gtile)[g][0];
+        const int64_t cnt = g < 0 ? (rw ? h->assembly_tiles_rows : h->assembly_tiles) : (rw ? h->gtile_rows : h->gtile)[g][1];
+        if (cnt > 0) GB_CUDA(launch_assemble(h, (unsigned)cnt, t0, a, st));
+        return GBVLM_OK;
+    }
+    // their corrections (FP64 residual plans)
+    int assemble_lo(int g, cudaStream_t st) const {
+        const bool rw = lo_rows(h);
+        const int64_t t0 = g < 0 ? 0 : (rw ? h->gtile_rows : h->gtile)[g][0];
+        const int64_t cnt = g < 0 ? (rw ? h->assembly_tiles_rows : h->assembly_tiles) : (rw ? h->gtile_rows : h->gtile)[g][1];
+        if (h->fp64_residual && cnt > 0) GB_CUDA(launch_assemble_lo(h, (unsigned)cnt, t0, a, st));
+        return GBVLM_OK;
+    }
+    int look(int g, cudaStream_t st) const {
+        if (!looks(g)) return GBVLM_OK;
+        const dim3 gl((unsigned)cdiv(h->plans[g].maxn, 8), (unsigned)(h->gsys[g + 1] - h->gsys[g]));
+        k_batch_look<<<gl, 256, 0, st>>>(a, h->gsys[g]);
+        GB_LAUNCH_CHECK();
+        return GBVLM_OK;
+    }
+    // without interchanges, a.fail marking the systems that need them
+    int factor(int g, cudaStream_t st, bool lookahead) const {
+        if (!fast(g)) return lu_batch_factor<float>(h->lub, h->plans[g], st, lookahead);
+        LuBatch<float> B = h->lub;
+        B.fail = h->d_fail;
+        return lu_batch_factor_fast<float>(B, h->plans[g], st, lookahead);
+    }
+    // with interchanges, the systems whose mark is in `mask`
+    int factor_again(int g, cudaStream_t st, bool lookahead, int32_t mask) const {
+        if (!fast(g)) return GBVLM_OK;
+        LuBatch<float> B = h->lub;
+        B.only = h->d_fail;
+        B.only_mask = mask;
+        B.hint = h->d_hint;
+        B.hint_ld = h->hint_ld;
+        return lu_batch_factor<float>(B, h->plans[g], st, lookahead);
+    }
+    // the AICs of systems whose factorisation was given up: copied back where they are kept, else assembled again
+    int restore(cudaStream_t st) {
+        a.only_left = 1;
+        int rc = GBVLM_OK;
         if (h->refine > 0) {
-            const dim3 g((unsigned)std::min<int64_t>(cdiv(h->maxn * h->maxn, 1024), 1024), (unsigned)h->nsys);
-            k_batch_restore<<<g, 256, 0, st>>>(a);
-            GB_LAUNCH_CHECK();
+            const dim3 gr((unsigned)std::min<int64_t>(cdiv(h->maxn * h->maxn, 1024), 1024), (unsigned)h->nsys);
+            k_batch_restore<<<gr, 256, 0, st>>>(a);
+            const cudaError_t e = cudaGetLastError();
+            if (e != cudaSuccess) rc = cuda_fail(e, "k_batch_restore", __FILE__, __LINE__);
         } else {
-            GB_CUDA(assemble_all());
+            rc = assemble(-1, st);
         }
-        rc = factor(true, [](int) { return GBVLM_OK; }, []() { return GBVLM_OK; });
-        if (rc) return rc;
-        a.only_failed = 0;
+        a.only_left = 0;
+        return rc;
     }
-    if (!(phases & BATCH_SOLVE)) return GBVLM_OK;
-    mark(4);
-    int32_t maxrhs = 0;
-    for (auto& s : h->sys) maxrhs = std::max(maxrhs, s.nrhs);
-    auto solve = [&]() {
+    // one(g, stream) for every group: one after another on `st` (serial), or each
+    // on its branch (group 0, the longest chain, on a high-priority stream),
+    // beside(st) next to them, joined on `st`
+    template <class One, class Beside>
+    int groups(cudaStream_t st, bool serial, One&& one, Beside&& beside) const {
+        if (serial) {
+            for (int g = 0; g < h->ngroups; g++) {
+                const int rc = one(g, st);
+                if (rc) return rc;
+            }
+            return beside(st);
+        }
+        GB_CUDA(cudaEventRecord(h->fork, st));
+        for (int g = 0; g < h->ngroups; g++) {
+            GB_CUDA(cudaStreamWaitEvent(h->side[g], h->fork, 0));
+            const int rc = one(g, h->side[g]);
+            if (rc) return rc;
+            GB_CUDA(cudaEventRecord(h->join[g], h->side[g]));
+        }
+        const int rc = beside(st);
+        if (rc) return rc;
+        for (int g = 0; g < h->ngroups; g++) GB_CUDA(cudaStreamWaitEvent(st, h->join[g], 0));
+        return GBVLM_OK;
+    }
+    // every marked system again, after the factorisations
+    int repeat(cudaStream_t st, bool serial, bool lookahead, int32_t mask) {
+        int rc = restore(st);
+        if (rc) return rc;
+        return groups(
+            st, serial, [&](int g, cudaStream_t s) { return factor_again(g, s, lookahead, mask); },
+            [](cudaStream_t) { return GBVLM_OK; });
+    }
+    int solve(cudaStream_t st) const {
         return h->use_flow ? trs_flow_solve(h->lub, h->flow, maxrhs, st)
                            : lu_batch_solve<float>(h->lub, h->nsys, maxrhs, h->maxn, st,
                                                    h->plans[0].tc_passes ? h->plans[0].d_err : nullptr);
-    };
-    rc = solve();
-    if (rc) return rc;
-    k_batch_accum<<<gp, 256, 0, st>>>(a);
-    GB_LAUNCH_CHECK();
-    if (h->fp64_residual && !staged && (phases & BATCH_FACTOR))
-        GB_CUDA(cudaStreamWaitEvent(st, h->lo_join, 0));
-    for (int it = 0; it < h->refine; it++) {
-        const dim3 rg((unsigned)h->residual_tiles, (unsigned)cdiv(maxrhs, RS_MAXRHS));
-        if (h->fp64_residual) {
-            if (it == 0) k_batch_residual<true, false><<<rg, RS_THREADS, 0, st>>>(a, h->d_rpfx);
-            else k_batch_residual<true, true><<<rg, RS_THREADS, 0, st>>>(a, h->d_rpfx);
-        } else {
-            if (it == 0) k_batch_residual<false, false><<<rg, RS_THREADS, 0, st>>>(a, h->d_rpfx);
-            else k_batch_residual<false, true><<<rg, RS_THREADS, 0, st>>>(a, h->d_rpfx);
-        }
-        GB_LAUNCH_CHECK();
-        rc = solve();
-        if (rc) return rc;
-        k_batch_accum<<<gp, 256, 0, st>>>(a);
-        GB_LAUNCH_CHECK();
     }
-    mark(5);
-    {
+    int accumulate(cudaStream_t st) const {
+        k_batch_accum<<<rows(), 256, 0, st>>>(a);
+        GB_LAUNCH_CHECK();
+        return GBVLM_OK;
+    }
+    int refine(cudaStream_t st) const {
+        for (int it = 0; it < h->refine; it++) {
+            const dim3 rg((unsigned)h->residual_tiles, (unsigned)cdiv(maxrhs, RS_MAXRHS));
+            if (h->fp64_residual) {
+                if (it == 0) k_batch_residual<true, false><<<rg, RS_THREADS, 0, st>>>(a, h->d_rpfx);
+                else k_batch_residual<true, true><<<rg, RS_THREADS, 0, st>>>(a, h->d_rpfx);
+            } else {
+                if (it == 0) k_batch_residual<false, false><<<rg, RS_THREADS, 0, st>>>(a, h->d_rpfx);
+                else k_batch_residual<false, true><<<rg, RS_THREADS, 0, st>>>(a, h->d_rpfx);
+            }
+            GB_LAUNCH_CHECK();
+            int rc = solve(st);
+            if (rc || (rc = accumulate(st))) return rc;
+        }
+        return GBVLM_OK;
+    }
+    int loads(cudaStream_t st) const {
         // the loads block: by the largest system, or the tuned width
         const int64_t lt = h->tp.batch_loads_threads ? h->tp.batch_loads_threads
                                                      : (h->maxn > 4096 ? LD_THREADS_LARGE : LD_THREADS_SMALL);
@@ -1367,73 +1384,209 @@ static int batch_enqueue(gbvlm_batch h, cudaStream_t st, int phases, cudaEvent_t
         else
             k_batch_loads<256><<<h->nsolve, 256, 0, st>>>(a, h->d_solve_sys, h->want_gamma);
         GB_LAUNCH_CHECK();
+        return GBVLM_OK;
     }
+    // launches of a run in which no system needs interchanges
+    void count() const {
+        int64_t n = 0, looked = 0;
+        for (int g = 0; g < h->ngroups; g++) {
+            n += fast(g) ? lu_plan_launches_fast(h->plans[g], 4) : lu_plan_launches(h->plans[g], 4);
+            looked += looks(g);
+        }
+        const int64_t solves = h->use_flow ? trs_flow_launches(maxrhs, h->flow.groups) : (maxrhs + 7) / 8;
+        // geometry, Trefftz, the groups' assemblies and looks, RHS, the factorisations, the
+        // solves and accumulations, the refinement sweeps, the loads, the conditions
+        h->launches = 3 + h->ngroups * (h->fp64_residual ? 2 : 1) + n + solves + 1 +
+                      (int64_t)h->refine * (1 + solves + 1) + 1 + 2 * looked + (batch_fast(h) ? 1 : 0);
+    }
+};
+
+// A run launch by launch.  No host wait: the launches for systems that need
+// interchanges are always there, and leave at entry where there is none.
+static int batch_run_launches(gbvlm_batch h, cudaStream_t st) {
+    BatchRun R(h);
+    R.count();
+    int rc = R.geometry(st);
+    if (rc) return rc;
+    rc = R.groups(
+        st, false,
+        [&](int g, cudaStream_t s) -> int {
+            int r = R.assemble(g, s);
+            if (r) return r;
+            if (h->fp64_residual) {
+                GB_CUDA(cudaEventRecord(h->asm_done[g], s));
+                GB_CUDA(cudaStreamWaitEvent(h->lo_side, h->asm_done[g], 0));
+                if ((r = R.assemble_lo(g, h->lo_side))) return r;
+            }
+            if ((r = R.look(g, s))) return r;
+            return R.factor(g, s, true);
+        },
+        [&](cudaStream_t s) {
+            const int r = R.trefftz(s);
+            return r ? r : R.rhs(s);
+        });
+    if (rc) return rc;
+    if (h->fp64_residual) GB_CUDA(cudaEventRecord(h->lo_join, h->lo_side));
+    if (batch_fast(h) && (rc = R.repeat(st, false, true, LU_SEEN | LU_LEFT))) return rc;
+    if ((rc = R.solve(st)) || (rc = R.accumulate(st))) return rc;
+    if (h->fp64_residual) GB_CUDA(cudaStreamWaitEvent(st, h->lo_join, 0));
+    if ((rc = R.refine(st))) return rc;
+    return R.loads(st);
+}
+
+// A run for the profiles, every stage after the one before; they wait anyway,
+// so the host looks whether a system needs interchanges.
+static int batch_run_staged(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev, bool lookahead) {
+    auto mark = [&](int k) { if (ev) cudaEventRecord(ev[k], st); };
+    BatchRun R(h);
+    R.count();
+    int rc;
+    mark(0);
+    if ((rc = R.geometry(st)) || (rc = R.trefftz(st))) return rc;
+    mark(1);
+    if ((rc = R.assemble(-1, st)) || (rc = R.assemble_lo(-1, st))) return rc;
+    mark(2);
+    if ((rc = R.rhs(st))) return rc;
+    mark(3);
+    rc = R.groups(
+        st, true,
+        [&](int g, cudaStream_t s) {
+            const int r = R.look(g, s);
+            return r ? r : R.factor(g, s, lookahead);
+        },
+        [](cudaStream_t) { return GBVLM_OK; });
+    if (rc) return rc;
+    if (batch_fast(h)) {
+        std::vector<int32_t> f(h->nsys, 0);
+        GB_CUDA(cudaMemcpyAsync(f.data(), h->d_fail, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
+        GB_CUDA(cudaStreamSynchronize(st));
+        if (std::any_of(f.begin(), f.end(), [](int32_t x) { return x != 0; }) &&
+            (rc = R.repeat(st, true, lookahead, LU_SEEN | LU_LEFT)))
+            return rc;
+    }
+    mark(4);
+    if ((rc = R.solve(st)) || (rc = R.accumulate(st)) || (rc = R.refine(st))) return rc;
+    mark(5);
+    if ((rc = R.loads(st))) return rc;
     mark(6);
     return GBVLM_OK;
 }
 
-// the graph's condition: a system needs interchanges
-__global__ void k_batch_condition(const int32_t* fail, int32_t n, cudaGraphConditionalHandle left) {
-    int bad = 0;
-    for (int32_t k = threadIdx.x; k < n; k += blockDim.x) bad |= fail[k] != 0;
-    bad = __syncthreads_or(bad);
-    if (threadIdx.x == 0) cudaGraphSetConditional(left, bad ? 1u : 0u);
+// a condition of the graph: one of n systems has a mark in `mask`
+__global__ void k_batch_condition(const int32_t* fail, int32_t n, int32_t mask, cudaGraphConditionalHandle cond) {
+    int any = 0;
+    for (int32_t k = threadIdx.x; k < n; k += blockDim.x) any |= (fail[k] & mask) != 0;
+    any = __syncthreads_or(any);
+    if (threadIdx.x == 0) cudaGraphSetConditional(cond, any ? 1u : 0u);
 }
 
-// The run as a graph.  Where the factorisation may leave systems that need
-// interchanges, their factorisation lies between it and the solves, under the
-// condition that there is one.  Measured, 512 wings x 8 angles: none 10.0 ms,
-// one of middle size 12.1 (13.5 with interchanges for all from the start).
+// The run as a graph.  A group's systems that are seen to need interchanges are
+// factored beside its others, under the condition that there is one; one that
+// turns out to need them, after all groups, likewise; then the solves, all
+// systems.  Measured, 512 wings x 8 angles (interchanges for all from the start,
+// these conditions): no such wing 13.4, 10.1 ms, one of middle size 13.5, 10.9, half
+// of them 22.3, 20.8; one elliptic 64 x 64 wing x 64 angles 10.8, 8.8.
 static int batch_capture(gbvlm_batch h) {
+    using Nodes = std::vector<cudaGraphNode_t>;
     cudaGraph_t g = nullptr;
     GB_CUDA(cudaGraphCreate(&g, 0));
     auto fail = [&](int rc) {
         cudaGraphDestroy(g);
         return rc;
     };
-    cudaGraphConditionalHandle left = 0;
-    // launches on h->cap into graph `into`, after its node `dep`
-    auto capture = [&](cudaGraph_t into, const cudaGraphNode_t* dep, int phases, bool condition) -> int {
-        GB_CUDA(cudaStreamBeginCaptureToGraph(h->cap, into, dep, nullptr, dep ? 1 : 0,
+    BatchRun R(h);
+    R.count();
+    // body(stream)'s launches into graph `into` after the nodes `after`; the last of them to *last
+    auto capture = [&](cudaGraph_t into, cudaStream_t s, const Nodes& after, Nodes* last, auto&& body) -> int {
+        GB_CUDA(cudaStreamBeginCaptureToGraph(s, into, after.data(), nullptr, after.size(),
                                               cudaStreamCaptureModeThreadLocal));
-        int rc = batch_enqueue(h, h->cap, phases);
-        if (rc == GBVLM_OK && condition) {
-            k_batch_condition<<<1, 256, 0, h->cap>>>(h->d_fail, h->nsys, left);
-            const cudaError_t e = cudaGetLastError();
-            if (e != cudaSuccess) rc = cuda_fail(e, "k_batch_condition", __FILE__, __LINE__);
+        int rc = body(s);
+        if (rc == GBVLM_OK && last) {
+            cudaStreamCaptureStatus status;
+            const cudaGraphNode_t* deps = nullptr;
+            const cudaGraphEdgeData* edges = nullptr;
+            size_t nd = 0;
+            const cudaError_t e = cudaStreamGetCaptureInfo(s, &status, nullptr, nullptr, &deps, &edges, &nd);
+            if (e == cudaSuccess) last->assign(deps, deps + nd);
+            else rc = cuda_fail(e, "cudaStreamGetCaptureInfo", __FILE__, __LINE__);
         }
         cudaGraph_t got = nullptr;
-        const cudaError_t e = cudaStreamEndCapture(h->cap, &got);
+        const cudaError_t e = cudaStreamEndCapture(s, &got);
         if (rc) return rc;
         GB_CUDA(e);
         return GBVLM_OK;
     };
-    auto build = [&]() -> int {
-        if (!batch_fast(h)) return capture(g, nullptr, BATCH_FACTOR | BATCH_SOLVE, false);
-        GB_CUDA(cudaGraphConditionalHandleCreate(&left, g, 0, cudaGraphCondAssignDefault));
-        int rc = capture(g, nullptr, BATCH_FACTOR, true);
+    // `body` under the condition that one of cnt systems from i0 has a mark in `mask`
+    auto conditional = [&](cudaStream_t s, const Nodes& after, int32_t i0, int32_t cnt, int32_t mask, Nodes* last,
+                           auto&& body) -> int {
+        cudaGraphConditionalHandle cond;
+        GB_CUDA(cudaGraphConditionalHandleCreate(&cond, g, 0, cudaGraphCondAssignDefault));
+        Nodes set;
+        int rc = capture(g, s, after, &set, [&](cudaStream_t c) -> int {
+            k_batch_condition<<<1, 256, 0, c>>>(h->d_fail + i0, cnt, mask, cond);
+            GB_LAUNCH_CHECK();
+            return GBVLM_OK;
+        });
         if (rc) return rc;
-        // the captured launches' last one, which every branch has joined
-        size_t nn = 0, ne = 0;
-        GB_CUDA(cudaGraphGetNodes(g, nullptr, &nn));
-        std::vector<cudaGraphNode_t> nodes(nn);
-        GB_CUDA(cudaGraphGetNodes(g, nodes.data(), &nn));
-        GB_CUDA(cudaGraphGetEdges(g, nullptr, nullptr, nullptr, &ne));
-        std::vector<cudaGraphNode_t> from(ne), to(ne), last;
-        std::vector<cudaGraphEdgeData> data(ne);
-        GB_CUDA(cudaGraphGetEdges(g, from.data(), to.data(), data.data(), &ne));
-        std::sort(from.begin(), from.end());
-        for (auto x : nodes)
-            if (!std::binary_search(from.begin(), from.end(), x)) last.push_back(x);
-        cudaGraphNode_t nif;
+        cudaGraphNode_t node;
         cudaGraphNodeParams np = {};
         np.type = cudaGraphNodeTypeConditional;
-        np.conditional.handle = left;
+        np.conditional.handle = cond;
         np.conditional.type = cudaGraphCondTypeIf;
         np.conditional.size = 1;
-        GB_CUDA(cudaGraphAddNode(&nif, g, last.data(), nullptr, last.size(), &np));
-        if ((rc = capture(np.conditional.phGraph_out[0], nullptr, BATCH_REPEAT, false))) return rc;
-        return capture(g, &nif, BATCH_SOLVE, false);
+        GB_CUDA(cudaGraphAddNode(&node, g, set.data(), nullptr, set.size(), &np));
+        last->assign(1, node);
+        return capture(np.conditional.phGraph_out[0], s, {}, nullptr, body);
+    };
+    auto build = [&]() -> int {
+        Nodes geo, side, lo, done;
+        auto join = [](Nodes& to, const Nodes& from) { to.insert(to.end(), from.begin(), from.end()); };
+        int rc = capture(g, h->cap, {}, &geo, [&](cudaStream_t s) { return R.geometry(s); });
+        if (rc) return rc;
+        for (int k = 0; k < h->ngroups; k++) {
+            Nodes ready, factored, again;
+            rc = capture(g, h->side[k], geo, &ready, [&](cudaStream_t s) {
+                const int r = R.assemble(k, s);
+                return r ? r : R.look(k, s);
+            });
+            if (rc) return rc;
+            if (h->fp64_residual) {
+                join(lo, ready);
+                Nodes after = lo;
+                if ((rc = capture(g, h->lo_side, after, &lo, [&](cudaStream_t s) { return R.assemble_lo(k, s); }))) return rc;
+            }
+            if ((rc = capture(g, h->side[k], ready, &factored, [&](cudaStream_t s) { return R.factor(k, s, true); })))
+                return rc;
+            join(done, factored);
+            if (!R.looks(k)) continue;
+            rc = conditional(h->side[k], ready, h->gsys[k], h->gsys[k + 1] - h->gsys[k], LU_SEEN, &again,
+                             [&](cudaStream_t s) { return R.factor_again(k, s, true, LU_SEEN); });
+            if (rc) return rc;
+            join(done, again);
+        }
+        rc = capture(g, h->cap, geo, &side, [&](cudaStream_t s) {
+            const int r = R.trefftz(s);
+            return r ? r : R.rhs(s);
+        });
+        if (rc) return rc;
+        if (batch_fast(h)) {
+            Nodes after = done;
+            rc = conditional(h->cap, after, 0, h->nsys, LU_LEFT, &done,
+                             [&](cudaStream_t s) { return R.repeat(s, false, true, LU_LEFT); });
+            if (rc) return rc;
+        }
+        join(done, side);
+        Nodes solved;
+        rc = capture(g, h->cap, done, &solved, [&](cudaStream_t s) {
+            const int r = R.solve(s);
+            return r ? r : R.accumulate(s);
+        });
+        if (rc) return rc;
+        join(solved, lo);
+        return capture(g, h->cap, solved, nullptr, [&](cudaStream_t s) {
+            const int r = R.refine(s);
+            return r ? r : R.loads(s);
+        });
     };
     const int rc = build();
     if (rc) return fail(rc);
@@ -1444,21 +1597,6 @@ static int batch_capture(gbvlm_batch h) {
     }
     h->graph = g;
     return GBVLM_OK;
-}
-
-// A run launch by launch for the profiles, which wait anyway: the host looks
-// whether a system needs interchanges.
-static int batch_enqueue_checked(gbvlm_batch h, cudaStream_t st, cudaEvent_t* ev, bool serial_lu) {
-    int rc = batch_enqueue(h, st, BATCH_FACTOR, ev, serial_lu);
-    if (rc) return rc;
-    std::vector<int32_t> f(h->nsys, 0);
-    if (batch_fast(h)) {
-        GB_CUDA(cudaMemcpyAsync(f.data(), h->d_fail, sizeof(int32_t) * h->nsys, cudaMemcpyDeviceToHost, st));
-        GB_CUDA(cudaStreamSynchronize(st));
-    }
-    const bool left = std::any_of(f.begin(), f.end(), [](int32_t x) { return x != 0; });
-    if (left && (rc = batch_enqueue(h, st, BATCH_REPEAT, ev, serial_lu))) return rc;
-    return batch_enqueue(h, st, BATCH_SOLVE, ev, serial_lu);
 }
 
 extern "C" {
@@ -1582,6 +1720,8 @@ int gbvlm_batch_create_ex(gbvlm_batch* out, int32_t ncases, const gbvlm_dims* di
     const size_t o_uidx = reserve(sizeof(int32_t) * solve_sys.size());
     const size_t o_bad = reserve(sizeof(int32_t) * h->nsys);
     const size_t o_fail = reserve(sizeof(int32_t) * h->nsys);
+    h->hint_ld = cdiv(h->nsys ? protos[order[0]].n : 1, (int64_t)LU_NB);  // (the largest system)
+    const size_t o_hint = reserve(sizeof(int32_t) * h->hint_ld * h->nsys);
     // tile prefix tables
     // ring rows per float assembly tile: at most 4, at most 2 with 256-ring span chunks (shared memory)
     h->asm_rows = (int)std::min<int64_t>(h->tp.batch_assembly_rows, h->tp.batch_assembly_span > 128 ? 2 : 4);
@@ -1630,6 +1770,7 @@ int gbvlm_batch_create_ex(gbvlm_batch* out, int32_t ncases, const gbvlm_dims* di
     h->d_uidx = (int32_t*)(base + o_uidx);
     h->d_bad = (int32_t*)(base + o_bad);
     h->d_fail = (int32_t*)(base + o_fail);
+    h->d_hint = (int32_t*)(base + o_hint);
     h->d_tpfx = (int64_t*)(base + o_tpfx);
     h->d_tpfx_rows = (int64_t*)(base + o_tpfx_rows);
     h->d_rpfx = (int64_t*)(base + o_rpfx);
@@ -1754,6 +1895,8 @@ int gbvlm_batch_create_ex(gbvlm_batch* out, int32_t ncases, const gbvlm_dims* di
             while (i1 < h->nsys && (g == nb || lun[i1] > bounds[g])) i1++;
             if (i1 == i0) continue;
             const int gi = h->ngroups++;
+            h->gsys[gi] = i0;
+            h->gsys[gi + 1] = i1;
             h->gtile[gi][0] = h->tpfx_host[i0];
             h->gtile[gi][1] = h->tpfx_host[i1] - h->tpfx_host[i0];
             h->gtile_rows[gi][0] = h->tpfx_rows_host[i0];
@@ -1869,8 +2012,7 @@ int gbvlm_batch_run_eager(gbvlm_batch h, int32_t want_gamma, gbvlm_stream stream
         cudaGraphExecDestroy(h->exec);
         h->exec = nullptr;
     }
-    // (no host wait: the launches for systems that need interchanges are always there, and leave where there is none)
-    int rc = batch_enqueue(h, to_cuda(stream), BATCH_FACTOR | BATCH_SOLVE | (batch_fast(h) ? BATCH_REPEAT : 0));
+    int rc = batch_run_launches(h, to_cuda(stream));
     if (rc == GBVLM_OK) GB_CUDA(cudaEventRecord(h->done, to_cuda(stream)));
     return rc;
 }
@@ -1902,7 +2044,7 @@ int gbvlm_batch_profile(gbvlm_batch h, float* stage_ms, gbvlm_stream stream) {
     cudaStream_t st = to_cuda(stream);
     cudaEvent_t ev[7];
     for (int k = 0; k < 7; k++) GB_CUDA(cudaEventCreate(&ev[k]));
-    int rc = batch_enqueue_checked(h, st, ev, false);
+    int rc = batch_run_staged(h, st, ev, true);
     if (rc == GBVLM_OK) {
         cudaEventRecord(h->done, st);
         cudaError_t e = cudaEventSynchronize(ev[6]);
@@ -1921,7 +2063,7 @@ int gbvlm_batch_update_profile(gbvlm_batch h, double* out, gbvlm_stream stream) 
     cudaStream_t st = to_cuda(stream);
     std::vector<cudaEvent_t> ev;
     for (int g = 0; g < h->ngroups; g++) h->plans[g].tc_events = &ev;
-    int rc = batch_enqueue_checked(h, st, nullptr, true);
+    int rc = batch_run_staged(h, st, nullptr, false);
     for (int g = 0; g < h->ngroups; g++) h->plans[g].tc_events = nullptr;
     double ms = 0;
     if (rc == GBVLM_OK) {

@@ -805,13 +805,11 @@ __global__ void __launch_bounds__(Fast<float>::DT) k_lu_diag(LuBatch<float> B, i
     float* A = B.A[sid] + k0 + k0 * ld;
     const int w = (int)min((int64_t)W, n - k0);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    // the identity permutation, for a system that fails too: a batch's solves
-    // run on its factors, whatever they hold, before it is factored again
+    if (B.fail[sid]) return;
     for (int e = tid; e < w; e += DT) {
         B.ipiv[sid][k0 + e] = (int32_t)(k0 + e);
         B.perm[sid][k0 + e] = (int32_t)(k0 + e);
     }
-    if (B.fail[sid]) return;
     if (tid == 0) s_bad = 0;
     // a thread takes a row's entries in four columns (coalesced down the
     // columns) and stores them as one vector; past the system's end an
@@ -1215,11 +1213,11 @@ __global__ void __launch_bounds__(Fast<double>::DT) k_lu_diag64(LuBatch<double> 
     double* A = B.A[sid] + k0 + k0 * ld;
     const int w = (int)min((int64_t)GK, n - k0);
     const int tid = threadIdx.x, lane = tid & 31, s = tid >> 5;
+    if (B.fail[sid]) return;
     if (tid < w) {
         B.ipiv[sid][k0 + tid] = (int32_t)(k0 + tid);
         B.perm[sid][k0 + tid] = (int32_t)(k0 + tid);
     }
-    if (B.fail[sid]) return;
     double x[8];  // row `lane`, columns s, s + 4, ..; past the system's end an identity
 #pragma unroll
     for (int q = 0; q < 8; q++) {
@@ -1478,7 +1476,7 @@ constexpr int TC_TRSM_MIN_SYSTEMS = 1;
 
 // INV: the same solve on the identity, two CTAs per system (64 columns
 // each): writes M = I - L11^-1 (strictly lower, column-major, ld WW) to
-// minv + (sid - base) * WW * WW, for U12 = A12 - M A12 on the tensor cores
+// minv + (sid - base) * Fast<float>::WORK, for U12 = A12 - M A12 on the tensor cores
 template <int WW, bool INV = false, int COLS = TW_COLS>
 __global__ void __launch_bounds__(256, 2) k_trsm_wide(LuBatch<float> B, int64_t k0, const int32_t* act,
                                                      const int64_t* pfx, int cnt, float* minv, int32_t base) {
@@ -1570,7 +1568,7 @@ __global__ void __launch_bounds__(256, 2) k_trsm_wide(LuBatch<float> B, int64_t 
         __syncthreads();
     }
     if constexpr (INV) {
-        float* Mo = minv + (int64_t)(sid - base) * WW * WW + c0 * WW;
+        float* Mo = minv + (int64_t)(sid - base) * Fast<float>::WORK + c0 * WW;
         for (int e = tid; e < WW * COLS; e += 256) {
             const int r = e & (WW - 1), j = e >> 7;
             Mo[r + j * WW] = r > (int)c0 + j ? -X[r * TW_XS + j] : 0.f;
@@ -1625,7 +1623,7 @@ __global__ void __launch_bounds__(tc::THREADS, 2) k_trsm_tc12(LuBatch<float> B, 
     const int64_t n = B.n[sid], ld = B.ld[sid];
     float* A = B.A[sid];
     const int64_t c0 = k0 + LU_OUTER + (int64_t)(blockIdx.x - pfx[a]) * TBN;
-    const float* M = minv + (int64_t)(sid - base) * LU_OUTER * LU_OUTER;
+    const float* M = minv + (int64_t)(sid - base) * Fast<float>::WORK;
     float* X = A + k0 + c0 * ld;
     tc::update_tile<PASSES, false, TBN>(M, LU_OUTER, X, ld, X, ld, LU_OUTER, (int)min((int64_t)TBN, n - c0), LU_OUTER,
                                         tc_smem, bar, &tslot, err);

@@ -37,15 +37,16 @@ struct LuBatch {
     // them, which the later launches then pass over (zeroed by the caller; null
     // for the pivoting launches)
     int32_t* fail = nullptr;
-    // pivoting launches: the systems to work on, the marked ones (null: all).
-    // Every block of another system leaves at entry.
+    // pivoting launches: the systems to work on, those whose value has a bit of
+    // only_mask (null: all).  Every block of another system leaves at entry.
     const int32_t* only = nullptr;
+    int32_t only_mask = 0;
     // pivoting launches: per system (hint_ld apart) and panel of 32 columns, not
     // zero where the matrix has an entry below the diagonal larger than it (null: not looked)
     const int32_t* hint = nullptr;
     int64_t hint_ld = 0;
 
-    __device__ __forceinline__ bool skips(int32_t sid) const { return only && !only[sid]; }
+    __device__ __forceinline__ bool skips(int32_t sid) const { return only && !(only[sid] & only_mask); }
 };
 
 // One panel launch: active systems [first, first + count) of a step, each
@@ -110,7 +111,8 @@ struct LuPlan {
     bool tc_trsm = false;
     int32_t tc_trsm_min = 1;  // ... for steps with at least this many systems
     // per system 2 x 128 x 128 + 128 floats: I - L11^-1 of the current outer block, or the factored
-    // diagonal block by rows and by columns and its reciprocal pivots (without interchanges)
+    // diagonal block by rows and by columns and its reciprocal pivots (without interchanges).  A
+    // system's place is the same for both, which may run side by side for different systems
     float* d_minv = nullptr;
     // systems may be factored without interchanges (GBVLM_LU_FAST=0: not): in double, and in float
     bool fast_any = false, fast = false;
