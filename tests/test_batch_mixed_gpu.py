@@ -90,3 +90,21 @@ def test_a_long_chain_is_not_paid_twice(cuda, kind):
     finally:
         os.environ.pop("GBVLM_LU_FAST") if old is None else os.environ.update(GBVLM_LU_FAST=old)
     assert t["1"] <= t["0"], t
+
+
+def test_small_systems_keep_their_one_launch(cuda):
+    """Systems of a single panel gain nothing from a factorisation without interchanges of its own, with its
+    conditions: a batch of them takes what it takes a plan that pivots (1.2 times as long with them)."""
+    cases = [M.Case(M.trapezoid(4, 6, 4.0 + 0.01 * k, 0.5, 10.0).astype(np.float32), np.radians(np.arange(8.0)), {})
+             for k in range(512)]
+    t = {}
+    old = os.environ.get("GBVLM_LU_FAST")
+    try:
+        for fast in ("1", "0"):
+            os.environ["GBVLM_LU_FAST"] = fast
+            bs = BatchSolver(cases)
+            bs.set_inputs(pack_verts(cases), pack_alphas(cases))
+            t[fast] = _best(bs, 20)
+    finally:
+        os.environ.pop("GBVLM_LU_FAST") if old is None else os.environ.update(GBVLM_LU_FAST=old)
+    assert t["1"] <= 1.06 * t["0"], t

@@ -3333,6 +3333,9 @@ int lu_plan_build(LuPlan& plan, const std::vector<int64_t>& n_sorted, cudaStream
             const char* f = getenv("GBVLM_LU_FAST");
             plan.fast_any = !(f && f[0] == '0');
             plan.fast = plan.fast_any && plan.tc_passes == 3 && !tc_persistent();
+            // systems of one panel: the panel tries that itself, in the launch that pivots (512 such systems
+            // in a batch 423 us without this, 348 with it)
+            if (plan.maxn <= GK) plan.fast_any = plan.fast = false;
             GB_CUDA(cudaFuncSetAttribute(k_lu_diag, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)Fast<float>::diag_smem));
             GB_CUDA(cudaFuncSetAttribute(k_lu_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
