@@ -539,6 +539,8 @@ int gbvlm_uvlm_loop_wait(gbvlm_uvlm_loop l, int64_t ticket, double timeout_s, in
 /* requests submitted and completed so far, and graph launches they took */
 int gbvlm_uvlm_loop_stats(gbvlm_uvlm_loop l, int64_t* submitted, int64_t* completed, int64_t* launches);
 int gbvlm_uvlm_loop_destroy(gbvlm_uvlm_loop l);
+/* gbvlm_test_lu_withhold for the handle's solver (float runs, begun before). */
+int gbvlm_test_uvlm_withhold(gbvlm_uvlm h, gbvlm_stream stream);
 /* cl: t_steps doubles, cm: 3*t_steps, gamma_last: n doubles of the last step (each may be NULL). Synchronous. */
 int gbvlm_uvlm_results(gbvlm_uvlm h, double* cl, double* cm, double* gamma_last, gbvlm_stream stream);
 
@@ -587,6 +589,8 @@ int gbvlm_aero2dof_destroy(gbvlm_aero2dof h);
  * all; each Newton loop stops when |du_prev - du| <= FLT_EPSILON or after
  * max_iter + 1 iterations (the reference uses 50).  Synchronous. */
 int gbvlm_aero2dof_run(gbvlm_aero2dof h, int64_t steps, int32_t max_iter, gbvlm_stream stream);
+/* gbvlm_test_lu_withhold for the handle's solver. */
+int gbvlm_test_aero2dof_withhold(gbvlm_aero2dof h, gbvlm_stream stream);
 /* HOST outputs for steps 0..steps_done: u, v, a, F ((steps_done+1) x 2 each,
  * row-major: h, alpha), iters (steps_done Newton counts); each may be NULL. */
 int gbvlm_aero2dof_results(gbvlm_aero2dof h, int64_t* steps_done, double* u, double* v, double* a, double* F,
@@ -677,6 +681,14 @@ int gbvlm_test_flow_wait_timeout(int32_t n, gbvlm_stream stream);
  * GBVLM_ERR_CUDA with the timeout message when the bounded wait works; the
  * CUDA context stays usable. */
 int gbvlm_test_tc_wait_timeout(gbvlm_stream stream);
+/* Test hooks with no counterpart in the reference: the next single-column solve
+ * with the factors of the handle (more than 64 unknowns, factored before) never
+ * hands out its first block, so the wait of the blocks after it must run out
+ * (after 2 s).  The error word stays set, and no solve is done, until it is read:
+ * by gbvlm_test_lu_solve_check, by the next factorisation, or by the call that
+ * returns the results of the driver whose solver it is. */
+int gbvlm_test_lu_withhold(gbvlm_lu h, gbvlm_stream stream);
+int gbvlm_test_lu_solve_check(gbvlm_lu h, gbvlm_stream stream);
 
 /* ---------------------------------------------------------------------------
  * Nonlinear VLM: NLVLM::run (vlm/include/vlm.hpp:87-115, vlm/src/vlm.cpp:
@@ -697,6 +709,8 @@ int gbvlm_nlvlm_destroy(gbvlm_nlvlm h);
 int gbvlm_nlvlm_run(gbvlm_nlvlm h, double alpha, double beta, double u_inf, double rho, const float* db_alpha,
                     const float* db_cl, int32_t n_db, double tol, int32_t max_iter, double* cl, int32_t* iters,
                     double* err, float* strip_alpha, gbvlm_stream stream);
+/* gbvlm_test_lu_withhold for the handle's solver (run before). */
+int gbvlm_test_nlvlm_withhold(gbvlm_nlvlm h, gbvlm_stream stream);
 
 #ifdef __cplusplus
 }

@@ -510,11 +510,13 @@ struct NlvlmBase {
     virtual int run(double alpha, double beta, double u_inf, double rho, const float* db_alpha, const float* db_cl,
                     int32_t ndb, double tol, int32_t max_iter, double* cl, int32_t* iters, double* err,
                     float* strip_out, cudaStream_t st) = 0;
+    virtual gbvlm_lu solver() = 0;
 };
 
 template <class T>
 struct NlvlmState : NlvlmBase {
     VlmState<T> w;  // wing, wake, AIC and per-panel buffers of the steady simulation
+    gbvlm_lu solver() override { return w.lu; }
     void* mem = nullptr;
     T* strip = nullptr;  // angles, all surfaces' strips
     int64_t strips = 0;
@@ -578,7 +580,8 @@ struct NlvlmState : NlvlmBase {
         if ((rc = w.assemble(alpha, u, tr, s, st))) return rc;
         k_fill<T><<<(unsigned)cdiv(strips, 128), 128, 0, st>>>(strip, strips, alpha);
         GB_LAUNCH_CHECK();
-        double* herr = (double*)host_scratch(sizeof(double) * (1 + 7 * nsurf) + sizeof(T) * strips);
+        // the corrections' sum, the load sums, the solves' error words, the strips
+        double* herr = (double*)host_scratch(sizeof(double) * (2 + 7 * nsurf) + sizeof(T) * strips);
         GB_REQUIRE(herr != nullptr, "pinned host allocation failed");
         double err = 1.0;
         int32_t it = 0;
@@ -594,7 +597,8 @@ struct NlvlmState : NlvlmBase {
             err = *herr;
             err /= (double)w.n;  // per panel, as the reference normalises
         }
-        T* hs = (T*)(herr + 1 + 7 * nsurf);
+        int* words = (int*)(herr + 1 + 7 * nsurf);
+        T* hs = (T*)(herr + 2 + 7 * nsurf);
         if (strip_out) GB_CUDA(cudaMemcpyAsync(hs, strip, sizeof(T) * strips, cudaMemcpyDeviceToHost, st));
         // final loads with the strips back at alpha (vlm.cpp:281-291)
         T fs[3] = {u * (T)cos(alpha) * (T)cos(beta), -(u * (T)cos(alpha) * (T)sin(beta)), u * (T)sin(alpha)};
@@ -606,6 +610,7 @@ struct NlvlmState : NlvlmBase {
         k_vlm_loads<T><<<(unsigned)w.lift_blocks, LOAD_THREADS, 0, st>>>(w.sa, false, true, u, alpha);
         GB_LAUNCH_CHECK();
         GB_CUDA(cudaMemcpyAsync(herr + 1, w.sa.out, sizeof(double) * 7 * nsurf, cudaMemcpyDeviceToHost, st));
+        if ((rc = lu_solve_words(w.lu, words, st))) return rc;
         GB_CUDA(cudaStreamSynchronize(st));
         if (strip_out)
             for (int64_t i = 0; i < strips; i++) strip_out[i] = (float)hs[i];
@@ -620,7 +625,7 @@ struct NlvlmState : NlvlmBase {
         *cl_out = (double)(cl / ta);
         if (iters_out) *iters_out = it;
         if (err_out) *err_out = err;
-        return GBVLM_OK;
+        return lu_solve_verdict(w.lu, words, st);  // the solves finished their bounded waits
     }
 };
 
@@ -731,6 +736,11 @@ int gbvlm_nlvlm_run(gbvlm_nlvlm h, double alpha, double beta, double u_inf, doub
     GB_REQUIRE(max_iter >= 0, "NLVLM: max_iter must be non-negative");
     return h->impl->run(alpha, beta, u_inf, rho, db_alpha, db_cl, n_db, tol, max_iter, cl, iters, err, strip_alpha,
                         to_cuda(stream));
+}
+
+int gbvlm_test_nlvlm_withhold(gbvlm_nlvlm h, gbvlm_stream stream) {
+    GB_REQUIRE(h && h->impl, "null argument");
+    return gbvlm_test_lu_withhold(h->impl->solver(), stream);
 }
 
 int gbvlm_read_plot3d(const char* path, int32_t quarter_chord, gbvlm_dims* dims, float* verts) {

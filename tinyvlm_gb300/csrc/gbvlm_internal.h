@@ -97,6 +97,8 @@ int lu_solve_check(gbvlm_lu h, cudaStream_t st);
 // way to `words` (2, pinned), and once they are there the verdict on them
 int lu_solve_words(gbvlm_lu h, int* words, cudaStream_t st);
 int lu_solve_verdict(gbvlm_lu h, const int* words, cudaStream_t st);
+// the two words on the device, for a kernel that reports them (null: none)
+void lu_solve_word_addresses(gbvlm_lu h, const int** words);
 // rhs -= wake influence with *it_dev active ring rows per lifting wake
 // (it_dev <= it_max); scratch of WAKE_DEV_MAX_SLICES x (total panels) floats
 constexpr int64_t WAKE_DEV_MAX_SLICES = 608;

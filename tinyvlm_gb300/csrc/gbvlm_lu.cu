@@ -3947,6 +3947,11 @@ int lu_solve_words(gbvlm_lu h, int* words, cudaStream_t st) {
     return GBVLM_OK;
 }
 
+void lu_solve_word_addresses(gbvlm_lu h, const int** words) {
+    words[0] = (const int*)h->one;
+    words[1] = h->flow_n >= 0 && h->flow.d_ctl ? h->flow.d_ctl + 1 : nullptr;
+}
+
 int lu_solve_verdict(gbvlm_lu h, const int* words, cudaStream_t st) {
     if (words[0] != 0) GB_CUDA(cudaMemsetAsync(h->one, 0, ONE_Y, st));  // the counters of the solve that gave up
     if (words[0] == 0 && words[1] == 0) return GBVLM_OK;
@@ -4254,6 +4259,15 @@ int gbvlm_test_flow_wait_timeout(int32_t n, gbvlm_stream stream) {
         if (p) cudaFree(p);
     return rc;
 }
+
+int gbvlm_test_lu_withhold(gbvlm_lu h, gbvlm_stream stream) {
+    GB_REQUIRE(h && h->one, "the handle has no single-column solve (factor more than %d unknowns first)", (int)ONE_MIN);
+    const int one = 1;  // the dispatch counter: the first item is never handed out
+    GB_CUDA(cudaMemcpyAsync((int*)h->one + 1, &one, sizeof(int), cudaMemcpyHostToDevice, to_cuda(stream)));
+    return GBVLM_OK;
+}
+
+int gbvlm_test_lu_solve_check(gbvlm_lu h, gbvlm_stream stream) { return lu_solve_check(h, to_cuda(stream)); }
 
 int gbvlm_lu_create(gbvlm_lu* out) {
     GB_REQUIRE(out != nullptr, "out is null");

@@ -1201,11 +1201,14 @@ struct Aero2Dof {
         GB_LAUNCH_CHECK();
         for (int64_t k = 0; k < steps; k++) GB_CUDA(cudaGraphLaunch(exec, st));
         std::vector<int32_t> h(steps);
+        int* words = (int*)host_scratch(2 * sizeof(int));
+        GB_REQUIRE(words != nullptr, "pinned host allocation failed");
         GB_CUDA(cudaMemcpyAsync(h.data(), iters_dev + done, sizeof(int32_t) * steps, cudaMemcpyDeviceToHost, st));
+        if ((rc = lu_solve_words(lu, words, st))) return rc;
         GB_CUDA(cudaStreamSynchronize(st));
         iters.insert(iters.end(), h.begin(), h.end());
         done += steps;
-        return GBVLM_OK;
+        return lu_solve_verdict(lu, words, st);  // the steps' solves finished their bounded waits
     }
 };
 
@@ -1239,7 +1242,8 @@ struct LoopCtl {
 };
 struct LoopRec {
     int64_t step;
-    double c[4];  // CL, CM x, y, z
+    double c[4];     // CL, CM x, y, z
+    int64_t failed;  // a solve's bounded wait ran out
 };
 
 __device__ __forceinline__ uint64_t loop_ns() {
@@ -1248,15 +1252,16 @@ __device__ __forceinline__ uint64_t loop_ns() {
     return t;
 }
 
-// last_idx: the largest step index the wake holds
+// last_idx: the largest step index the wake holds; err0, err1: the error words of the solves (or null)
 __global__ void k_uvlm_loop_next(LoopCtl* ctl, LoopRec* rec, const int64_t* idx, const double* res, int64_t last_idx,
-                                 uint64_t poll_ns, cudaGraphConditionalHandle loop) {
+                                 const int* err0, const int* err1, uint64_t poll_ns, cudaGraphConditionalHandle loop) {
     if (threadIdx.x != 0) return;
     volatile LoopCtl* vc = ctl;
     const int64_t i = idx[0] - 1;  // the step this iteration took
     const int64_t t = vc->done;
     rec[t].step = i;
     for (int k = 0; k < 4; k++) rec[t].c[k] = res[4 * i + k];
+    rec[t].failed = (err0 && *err0) || (err1 && *err1);
     __threadfence_system();
     vc->done = t + 1;
     __threadfence_system();
@@ -1445,7 +1450,10 @@ int gbvlm_uvlm_loop_create(gbvlm_uvlm_loop* out, gbvlm_uvlm h, double poll_s) {
     rc = u->enqueue_dev_step(l->st);
     if (rc == GBVLM_OK) {
         const uint64_t poll_ns = (uint64_t)(poll_s * 1e9);
-        k_uvlm_loop_next<<<1, 32, 0, l->st>>>(l->ctl_d, l->rec_d, u->d_idx, u->res, u->t_steps - 2, poll_ns, cond);
+        const int* words[2];
+        lu_solve_word_addresses(u->lu, words);
+        k_uvlm_loop_next<<<1, 32, 0, l->st>>>(l->ctl_d, l->rec_d, u->d_idx, u->res, u->t_steps - 2, words[0], words[1],
+                                              poll_ns, cond);
         const cudaError_t le = cudaGetLastError();
         if (le != cudaSuccess) rc = cuda_fail(le, "k_uvlm_loop_next", __FILE__, __LINE__);
     }
@@ -1500,6 +1508,11 @@ int gbvlm_uvlm_loop_wait(gbvlm_uvlm_loop l, int64_t ticket, double timeout_s, in
     if (cl) *cl = r.c[0];
     if (cm)
         for (int k = 0; k < 3; k++) cm[k] = r.c[1 + k];
+    if (r.failed) {
+        set_error("UVLM request loop: step %lld: a triangular solve's block timed out waiting for the blocks it depends on",
+                  (long long)r.step);
+        return GBVLM_ERR_CUDA;
+    }
     return GBVLM_OK;
 }
 
@@ -1564,6 +1577,18 @@ int gbvlm_aero2dof_destroy(gbvlm_aero2dof h) {
 int gbvlm_aero2dof_run(gbvlm_aero2dof h, int64_t steps, int32_t max_iter, gbvlm_stream stream) {
     GB_REQUIRE(h && steps >= 0 && max_iter >= 1, "bad arguments");
     return ((Aero2Dof*)h)->run(steps, max_iter, to_cuda(stream));
+}
+
+int gbvlm_test_aero2dof_withhold(gbvlm_aero2dof h, gbvlm_stream stream) {
+    GB_REQUIRE(h, "null argument");
+    return gbvlm_test_lu_withhold(((Aero2Dof*)h)->lu, stream);
+}
+
+int gbvlm_test_uvlm_withhold(gbvlm_uvlm h, gbvlm_stream stream) {
+    GB_REQUIRE(h && h->impl, "null argument");
+    auto* u = dynamic_cast<UvlmState<float>*>(h->impl);
+    GB_REQUIRE(u, "float runs only");
+    return gbvlm_test_lu_withhold(u->lu, stream);
 }
 
 int gbvlm_aero2dof_results(gbvlm_aero2dof h, int64_t* steps_done, double* u, double* v, double* a, double* F,
