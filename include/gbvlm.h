@@ -451,6 +451,11 @@ int gbvlm_batch_create(gbvlm_batch* out, int32_t ncases, const gbvlm_dims* dims,
 int gbvlm_batch_create_ex(gbvlm_batch* out, int32_t ncases, const gbvlm_dims* dims, const int32_t* nalpha,
                           int32_t mode, int32_t refine_iters, int32_t flags);
 int gbvlm_batch_destroy(gbvlm_batch h);
+/* Test hook with no counterpart in the reference: the refinement residual
+ * R = B - (A + Alo) X of one system, column-major device arrays (Alo may be
+ * null; x_lo = 0: X holds float values). */
+int gbvlm_test_batch_residual(int64_t n, int32_t nrhs, const float* A, const float* Alo, const double* X,
+                              const double* B, double* R, int32_t x_lo, gbvlm_stream stream);
 /* Sizes of the plan: solves (= sum nalpha), systems, gamma floats, Biot-Savart
  * ring-point interactions and LU flops per run, device bytes held. */
 int gbvlm_batch_info(gbvlm_batch h, int64_t* nsolve, int64_t* nsys, int64_t* gamma_floats, double* interactions,

@@ -697,78 +697,59 @@ __global__ void k_batch_accum(BatchArgs a) {
 }
 
 // R = B - A2 Xd (B - (A2 + Alo) Xd in FP64 residual plans); X = (float)R.
-// One thread per row, tiles (system, row
-// block).
-// The products of the float matrix A2 with the double solution Xd
-// (split as hi + lo floats) are accumulated in double-float arithmetic on the
-// fp32 units, about 2^-44 relative per term, where the fp64 units of this part
-// run at a small fraction of the fp32 rate.
-//
-// Bound: the fp32 pipe.  RS_CB columns at a time are added to a bias that is 32
-// times the largest product they can form, so that the running sum stays
-// within a factor two of it and a term costs four operations instead of a
-// product, its error and a branch-free two-sum (nine): with t = s + a x rounded
-// once, t - s is exact (Sterbenz), and a x - (t - s), one FMA, is the rounding
-// error.  The bias is subtracted again (exact), and the chunk's sum joins
-// (sh, sl) by a two-sum.  16384 panels, 64 right-hand sides: 8.5 -> 6.8 ms (with the
-// columns and X fetched ahead; the arithmetic alone 8.7, waiting for them).
+// One thread per row, tiles (system, row block).  The products of the float
+// matrix A2 with the double solution Xd are accumulated in double-float
+// arithmetic on the fp32 units (Xd split as hi + lo floats, each product a*hi
+// exact through an FMA, running sums (sh, sl) kept with a compensated addition):
+// about 2^-48 of the running sum per term, where the fp64 units of this part run
+// at a small fraction of the fp32 rate.
+// Bound: the fp32 pipe (ten operations a term): 16384 panels, 64 right-hand sides
+// 8.5 ms.  Not kept: the sums of eight columns on a bias of 32 times their largest
+// product, four operations a term and 6.8 ms, but six times the error (median of
+// random rows of 512 terms 2.0e-14 of the sum of |a x|, 3.4e-15 here); columns
+// and X fetched ahead, asynchronously (the run 60.6 -> 61.0 ms).
 constexpr int RS_THREADS = 64;
 constexpr int RS_MAXRHS = 8;  // (the inner loop reads them as two float4)
-constexpr int RS_CB = 8;  // columns of Xd staged per step (the bias allows for 8 of them)
-static_assert(RS_CB * RS_MAXRHS == RS_THREADS, "a thread stages one value");
+constexpr int RS_CB = 8;  // columns of Xd staged per step
 constexpr int RS_ROWS = 2;  // rows per thread
+
+// (sh, sl) += a * (xh + xl); XL = false: xl is zero
+template <bool XL>
+__device__ __forceinline__ void df_mac(float& sh, float& sl, float a, float xh, float xl) {
+    const float p = __fmul_rn(a, xh);
+    const float pe = __fmaf_rn(a, xh, -p);  // a*xh - p exactly
+    const float s = __fadd_rn(sh, p);
+    const float bb = __fsub_rn(s, sh);
+    const float e = __fadd_rn(__fsub_rn(sh, __fsub_rn(s, bb)), __fsub_rn(p, bb));  // sh + p - s exactly
+    sh = s;
+    sl = XL ? __fmaf_rn(a, xl, __fadd_rn(sl, __fadd_rn(e, pe))) : __fadd_rn(sl, __fadd_rn(e, pe));
+}
 
 // LO: the plan keeps the correction Alo of the stored AIC; its products with
 // the hi part of Xd join the low-order sums (Alo is about 2^-24 of A, so
 // the float product is exact to far below the residual's accuracy).
 // XL = false: Xd holds float values (the first sweep: Xd = 0 + the float
 // solve), so its lo part is zero and its products are left out.
-constexpr int RS_STAGES = 3;
-constexpr int RS_MIN_BLOCKS = 6;
-
-// 4 bytes to shared memory, asynchronously; zero where !valid (src is still an address of the matrix)
-__device__ __forceinline__ void copy4_async(float* dst, const float* src, bool valid) {
-    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst), bytes = valid ? 4u : 0u;
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
-}
-
 template <bool LO, bool XL>
-__global__ void __launch_bounds__(RS_THREADS, RS_MIN_BLOCKS) k_batch_residual(BatchArgs a, const int64_t* rpfx) {
-    constexpr int ROWS = RS_THREADS * RS_ROWS;
-    __shared__ __align__(16) float xh[2][RS_CB][RS_MAXRHS];
-    __shared__ __align__(16) float xl[XL ? 2 : 1][RS_CB][RS_MAXRHS];
-    __shared__ __align__(16) float xm[2][2][RS_MAXRHS];  // largest |hi| of a warp's columns
-    __shared__ float sa[RS_STAGES][RS_CB][ROWS];         // a thread reads what it copied itself
-    __shared__ float sl_[LO ? RS_STAGES : 1][LO ? RS_CB : 1][LO ? ROWS : 1];
+__global__ void __launch_bounds__(RS_THREADS) k_batch_residual(BatchArgs a, const int64_t* rpfx) {
+    __shared__ __align__(16) float xh[RS_CB][RS_MAXRHS];
+    __shared__ __align__(16) float xl[RS_CB][RS_MAXRHS];
     const int si = find_sys(rpfx, a.nsys, blockIdx.x);
     const SysDesc& S = a.sys[si];
     // RS_ROWS rows per thread, RS_THREADS apart: each staged value of X is
     // read once from shared memory for all of them
-    const int64_t r0 = (blockIdx.x - rpfx[si]) * ROWS + threadIdx.x;
+    const int64_t r0 = (blockIdx.x - rpfx[si]) * (RS_THREADS * RS_ROWS) + threadIdx.x;
     const int64_t n = S.n;
     bool rv[RS_ROWS];
+    const float* arow[RS_ROWS];
+    const float* lrow[RS_ROWS];
 #pragma unroll
-    for (int k = 0; k < RS_ROWS; k++) rv[k] = r0 + k * RS_THREADS < n;
-    const int64_t nchunk = (n + RS_CB - 1) / RS_CB;
-    // chunk c's columns of this thread's rows, one group of asynchronous copies (empty past the last chunk)
-    auto fetch = [&](int64_t c) {
-        if (c < nchunk) {
-            const int st = (int)(c % RS_STAGES);
-#pragma unroll
-            for (int cc = 0; cc < RS_CB; cc++) {
-                const int64_t col = c * RS_CB + cc;
-#pragma unroll
-                for (int k = 0; k < RS_ROWS; k++) {
-                    const bool ok = col < n && rv[k];
-                    const int64_t off = ok ? r0 + k * RS_THREADS + col * n : 0;
-                    copy4_async(&sa[st][cc][threadIdx.x + k * RS_THREADS], S.A2 + off, ok);
-                    if constexpr (LO)
-                        copy4_async(&sl_[st][cc][threadIdx.x + k * RS_THREADS], S.Alo + off, ok);
-                }
-            }
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
+    for (int k = 0; k < RS_ROWS; k++) {
+        const int64_t r = r0 + k * RS_THREADS;
+        rv[k] = r < n;
+        arow[k] = S.A2 + (rv[k] ? r : 0);
+        lrow[k] = LO ? S.Alo + (rv[k] ? r : 0) : nullptr;
+    }
     // grid.y: blocks of RS_MAXRHS right-hand sides
     for (int q0 = blockIdx.y * RS_MAXRHS; q0 < S.nrhs; q0 += RS_MAXRHS * gridDim.y) {
         const int nq = min(RS_MAXRHS, S.nrhs - q0);
@@ -777,85 +758,49 @@ __global__ void __launch_bounds__(RS_THREADS, RS_MIN_BLOCKS) k_batch_residual(Ba
         for (int k = 0; k < RS_ROWS; k++)
 #pragma unroll
             for (int q = 0; q < RS_MAXRHS; q++) sh[k][q] = sl[k][q] = 0.f;
-        const int xc = threadIdx.x / RS_MAXRHS, xq = threadIdx.x % RS_MAXRHS;  // the value of X this thread stages
-        auto xval = [&](int64_t c) {
-            const int64_t col = c * RS_CB + xc;
-            return (col < n && xq < nq) ? S.Xd[col + (q0 + xq) * n] : 0.0;
-        };
-        double xnext = xval(0);
-#pragma unroll
-        for (int c = 0; c < RS_STAGES - 1; c++) fetch(c);
-        __syncthreads();  // the last sweep's readers of xh are done
-        for (int64_t c = 0; c < nchunk; c++) {
-            const int b = (int)(c & 1), st = (int)(c % RS_STAGES);
-            {
-                const float h = (float)xnext;
-                xh[b][xc][xq] = h;
-                if (XL) xl[b][xc][xq] = (float)(xnext - (double)h);
-                float big = fabsf(h);  // over the warp's four columns
-                big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 8));
-                big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, 16));
-                if ((threadIdx.x & 31) < RS_MAXRHS) xm[b][threadIdx.x >> 5][xq] = big;
-            }
-            xnext = xval(c + 1);
-            fetch(c + RS_STAGES - 1);
-            asm volatile("cp.async.wait_group %0;" ::"n"(RS_STAGES - 1) : "memory");  // chunk c is there
+        for (int64_t c0 = 0; c0 < n; c0 += RS_CB) {
             __syncthreads();
-            float s[RS_ROWS][RS_MAXRHS], lo[RS_ROWS][RS_MAXRHS], bias[RS_ROWS][RS_MAXRHS];
-#pragma unroll
-            for (int k = 0; k < RS_ROWS; k++) {
-                float big = 0.f;
-#pragma unroll
-                for (int cc = 0; cc < RS_CB; cc++)
-                    big = fmaxf(big, fabsf(sa[st][cc][threadIdx.x + k * RS_THREADS]));
-#pragma unroll
-                for (int q = 0; q < RS_MAXRHS; q++) {
-                    bias[k][q] = s[k][q] = __fmul_rn(32.f * big, fmaxf(xm[b][0][q], xm[b][1][q]));
-                    lo[k][q] = 0.f;
-                }
+            for (int e = threadIdx.x; e < RS_CB * RS_MAXRHS; e += RS_THREADS) {
+                const int cc = e / RS_MAXRHS, q = e % RS_MAXRHS;
+                const double v = (c0 + cc < n && q < nq) ? S.Xd[(c0 + cc) + (q0 + q) * n] : 0.0;
+                const float h = (float)v;
+                xh[cc][q] = h;
+                if (XL) xl[cc][q] = (float)(v - (double)h);
             }
+            __syncthreads();
+            if (rv[0]) {
+                const int cn = (int)min((int64_t)RS_CB, n - c0);
+                float av[RS_ROWS][RS_CB], lv[RS_ROWS][RS_CB];
 #pragma unroll
-            for (int cc = 0; cc < RS_CB; cc++) {
-                // the 8 hi and 8 lo values of column cc as four 16-byte broadcasts
-                const float4 h0 = *reinterpret_cast<const float4*>(&xh[b][cc][0]);
-                const float4 h1 = *reinterpret_cast<const float4*>(&xh[b][cc][4]);
-                const float hh[RS_MAXRHS] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-                float ll[RS_MAXRHS] = {};
-                if (XL) {
-                    const float4 l0 = *reinterpret_cast<const float4*>(&xl[XL ? b : 0][cc][0]);
-                    const float4 l1 = *reinterpret_cast<const float4*>(&xl[XL ? b : 0][cc][4]);
-                    ll[0] = l0.x, ll[1] = l0.y, ll[2] = l0.z, ll[3] = l0.w;
-                    ll[4] = l1.x, ll[5] = l1.y, ll[6] = l1.z, ll[7] = l1.w;
-                }
+                for (int k = 0; k < RS_ROWS; k++)
 #pragma unroll
-                for (int k = 0; k < RS_ROWS; k++) {
-                    const float av = sa[st][cc][threadIdx.x + k * RS_THREADS];
-                    float lv = 0.f;
-                    if constexpr (LO) lv = sl_[st][cc][threadIdx.x + k * RS_THREADS];
-#pragma unroll
-                    for (int q = 0; q < RS_MAXRHS; q++) {
-                        const float t = __fmaf_rn(av, hh[q], s[k][q]);
-                        const float d = __fsub_rn(t, s[k][q]);
-                        lo[k][q] = __fadd_rn(lo[k][q], __fmaf_rn(av, hh[q], -d));
-                        s[k][q] = t;
-                        if (XL) lo[k][q] = __fmaf_rn(av, ll[q], lo[k][q]);
-                        if (LO) lo[k][q] = __fmaf_rn(lv, hh[q], lo[k][q]);
+                    for (int cc = 0; cc < RS_CB; cc++) {
+                        av[k][cc] = (cc < cn && rv[k]) ? arow[k][(c0 + cc) * n] : 0.f;
+                        if (LO) lv[k][cc] = (cc < cn && rv[k]) ? lrow[k][(c0 + cc) * n] : 0.f;
                     }
+#pragma unroll
+                for (int cc = 0; cc < RS_CB; cc++) {
+                    // the 8 hi and 8 lo values of column cc as four 16-byte broadcasts
+                    const float4 h0 = *reinterpret_cast<const float4*>(&xh[cc][0]);
+                    const float4 h1 = *reinterpret_cast<const float4*>(&xh[cc][4]);
+                    const float hh[RS_MAXRHS] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                    float ll[RS_MAXRHS] = {};
+                    if (XL) {
+                        const float4 l0 = *reinterpret_cast<const float4*>(&xl[cc][0]);
+                        const float4 l1 = *reinterpret_cast<const float4*>(&xl[cc][4]);
+                        ll[0] = l0.x, ll[1] = l0.y, ll[2] = l0.z, ll[3] = l0.w;
+                        ll[4] = l1.x, ll[5] = l1.y, ll[6] = l1.z, ll[7] = l1.w;
+                    }
+#pragma unroll
+                    for (int k = 0; k < RS_ROWS; k++)
+#pragma unroll
+                        for (int q = 0; q < RS_MAXRHS; q++) {
+                            df_mac<XL>(sh[k][q], sl[k][q], av[k][cc], hh[q], ll[q]);
+                            if (LO) sl[k][q] = __fmaf_rn(lv[k][cc], hh[q], sl[k][q]);
+                        }
                 }
             }
-#pragma unroll
-            for (int k = 0; k < RS_ROWS; k++)
-#pragma unroll
-                for (int q = 0; q < RS_MAXRHS; q++) {
-                    const float p = __fsub_rn(s[k][q], bias[k][q]);
-                    const float h = __fadd_rn(sh[k][q], p);
-                    const float bb = __fsub_rn(h, sh[k][q]);
-                    const float e = __fadd_rn(__fsub_rn(sh[k][q], __fsub_rn(h, bb)), __fsub_rn(p, bb));  // sh + p - h
-                    sh[k][q] = h;
-                    sl[k][q] = __fadd_rn(sl[k][q], __fadd_rn(e, lo[k][q]));
-                }
         }
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
         for (int k = 0; k < RS_ROWS; k++) {
             if (!rv[k]) continue;
@@ -1940,6 +1885,44 @@ int gbvlm_batch_create_ex(gbvlm_batch* out, int32_t ncases, const gbvlm_dims* di
     }
     *out = h;
     return GBVLM_OK;
+}
+
+int gbvlm_test_batch_residual(int64_t n, int32_t nrhs, const float* A, const float* Alo, const double* X,
+                              const double* B, double* Rout, int32_t x_lo, gbvlm_stream stream) {
+    GB_REQUIRE(n >= 1 && nrhs >= 1 && A && X && B && Rout, "bad arguments");
+    cudaStream_t st = to_cuda(stream);
+    SysDesc S = {};
+    S.n = n;
+    S.nrhs = nrhs;
+    S.A2 = const_cast<float*>(A);
+    S.Alo = const_cast<float*>(Alo);
+    S.Xd = const_cast<double*>(X);
+    S.B = const_cast<double*>(B);
+    S.R = Rout;
+    const int64_t tiles = cdiv(n, (int64_t)RS_THREADS * RS_ROWS), pfx[2] = {0, tiles};
+    char* d = nullptr;
+    const size_t o = (sizeof(SysDesc) + 255) / 256 * 256, px = o + 256;
+    auto run = [&]() -> int {
+        GB_CUDA(cudaMalloc(&d, px + sizeof(float) * n * nrhs));
+        S.X = (float*)(d + px);
+        GB_CUDA(cudaMemcpyAsync(d, &S, sizeof(S), cudaMemcpyHostToDevice, st));
+        GB_CUDA(cudaMemcpyAsync(d + o, pfx, sizeof(pfx), cudaMemcpyHostToDevice, st));
+        BatchArgs a = {};
+        a.sys = (SysDesc*)d;
+        a.nsys = 1;
+        const dim3 g((unsigned)tiles, (unsigned)cdiv((int64_t)nrhs, (int64_t)RS_MAXRHS));
+        const int64_t* p = (const int64_t*)(d + o);
+        if (Alo && x_lo) k_batch_residual<true, true><<<g, RS_THREADS, 0, st>>>(a, p);
+        else if (Alo) k_batch_residual<true, false><<<g, RS_THREADS, 0, st>>>(a, p);
+        else if (x_lo) k_batch_residual<false, true><<<g, RS_THREADS, 0, st>>>(a, p);
+        else k_batch_residual<false, false><<<g, RS_THREADS, 0, st>>>(a, p);
+        GB_LAUNCH_CHECK();
+        GB_CUDA(cudaStreamSynchronize(st));
+        return GBVLM_OK;
+    };
+    const int rc = run();
+    if (d) cudaFree(d);
+    return rc;
 }
 
 int gbvlm_batch_destroy(gbvlm_batch h) {
