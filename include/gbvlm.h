@@ -699,6 +699,12 @@ int gbvlm_test_tc_wait_timeout(gbvlm_stream stream);
  * returns the results of the driver whose solver it is. */
 int gbvlm_test_lu_withhold(gbvlm_lu h, gbvlm_stream stream);
 int gbvlm_test_lu_solve_check(gbvlm_lu h, gbvlm_stream stream);
+/* Test hooks with no counterpart in the reference: the square root (kind 0), the
+ * reciprocal (1) and the pair of quotients a / b (2: n pairs) of the double
+ * segment law, and the reciprocals of the LU's pivots, on device arrays. */
+int gbvlm_test_walk_math(int32_t kind, int64_t n, const double* a, const double* b, double* out, gbvlm_stream stream);
+int gbvlm_test_pivot_rcp(int64_t n, const float* a32, float* out32, const double* a64, double* out64,
+                         gbvlm_stream stream);
 
 /* ---------------------------------------------------------------------------
  * Nonlinear VLM: NLVLM::run (vlm/include/vlm.hpp:87-115, vlm/src/vlm.cpp:

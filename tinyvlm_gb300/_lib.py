@@ -102,6 +102,8 @@ def _protos():
     t["gbvlm_test_lu_solve_check"] = [P, P]
     for sfx in ("f32", "f64"):
         t["gbvlm_test_inverse_solve_" + sfx] = [P, I64, P, P, P]
+    t["gbvlm_test_walk_math"] = [I32, I64, P, P, P, P]
+    t["gbvlm_test_pivot_rcp"] = [I64, P, P, P, P, P]
     t["gbvlm_test_batch_residual"] = [I64, I32, P, P, P, P, P, I32, P]
     t["gbvlm_nlvlm_create"] = [P, I32, P, PP, I32]
     t["gbvlm_nlvlm_destroy"] = [P]

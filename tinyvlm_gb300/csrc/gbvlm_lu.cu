@@ -360,6 +360,12 @@ __device__ __forceinline__ bool pivot_fits(double d) {
     const uint32_t e = (uint32_t)__double2hiint(d) & 0x7fffffffu;
     return e >= 0x00100000u && e < 0x7fd00000u;
 }
+__global__ void k_test_pivot_rcp(int64_t n, const float* a32, float* o32, const double* a64, double* o64) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    o32[i] = pivot_rcp(a32[i]);
+    o64[i] = pivot_rcp(a64[i]);
+}
 // |x| <= |d| (false for a NaN x or d); in double by the bits, off the fp64 pipe
 __device__ __forceinline__ bool not_above(float x, float d) { return fabsf(x) <= fabsf(d); }
 __device__ __forceinline__ bool not_above(double x, double d) {
@@ -4258,6 +4264,14 @@ int gbvlm_test_flow_wait_timeout(int32_t n, gbvlm_stream stream) {
     for (void* p : {(void*)A, (void*)X, (void*)ipiv, (void*)perm, (void*)info, work})
         if (p) cudaFree(p);
     return rc;
+}
+
+int gbvlm_test_pivot_rcp(int64_t n, const float* a32, float* out32, const double* a64, double* out64,
+                         gbvlm_stream stream) {
+    GB_REQUIRE(n >= 1 && a32 && out32 && a64 && out64, "bad arguments");
+    k_test_pivot_rcp<<<(unsigned)cdiv(n, 256), 256, 0, to_cuda(stream)>>>(n, a32, out32, a64, out64);
+    GB_LAUNCH_CHECK();
+    return GBVLM_OK;
 }
 
 int gbvlm_test_lu_withhold(gbvlm_lu h, gbvlm_stream stream) {

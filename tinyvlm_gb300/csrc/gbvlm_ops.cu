@@ -993,7 +993,26 @@ using namespace gbvlm;
 // ===========================================================================
 // C ABI
 // ===========================================================================
+namespace gbvlm {
+// out[i] = length_of(a[i]) (kind 0), reciprocal(a[i]) (1); kind 2: out[2 i], out[2 i + 1] = the two quotients of
+// a[2 i] / b[2 i] and a[2 i + 1] / b[2 i + 1]
+__global__ void k_test_walk_math(int kind, int64_t n, const double* a, const double* b, double* out) {
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    if (kind == 0) out[i] = length_of(a[i]);
+    else if (kind == 1) out[i] = reciprocal(a[i]);
+    else two_quotients(a[2 * i], b[2 * i], false, a[2 * i + 1], b[2 * i + 1], false, out[2 * i], out[2 * i + 1]);
+}
+}  // namespace gbvlm
+
 extern "C" {
+int gbvlm_test_walk_math(int32_t kind, int64_t n, const double* a, const double* b, double* out, gbvlm_stream stream) {
+    GB_REQUIRE(kind >= 0 && kind <= 2 && n >= 1 && a && out && (kind != 2 || b), "bad arguments");
+    k_test_walk_math<<<(unsigned)cdiv(n, 256), 256, 0, to_cuda(stream)>>>(kind, n, a, b, out);
+    GB_LAUNCH_CHECK();
+    return GBVLM_OK;
+}
+
 
 const char* gbvlm_last_error(void) { return g_err; }
 int gbvlm_version(void) { return 10000; }
