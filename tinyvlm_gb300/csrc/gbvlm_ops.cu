@@ -56,7 +56,10 @@ void* host_scratch(size_t bytes) {
 
 // Scratch for partial sums and small reductions, one buffer per (thread,
 // device): calls from different host threads (each with its own stream) never
-// share one, and a grow only has to wait for the calling thread's stream.
+// share one, and a grow only has to wait for the calling thread's stream.  It
+// starts at the partial sums' limit (LT_SCRATCH doubles), so that only sums over
+// more points than that let it grow: a captured call that follows any other call
+// of the thread, with fewer wake rows, finds it large enough.
 int device_scratch(size_t bytes, void** out, cudaStream_t s) {
     static thread_local std::vector<std::pair<void*, size_t>> per_dev(64, {nullptr, 0});
     int dev = 0;
@@ -68,7 +71,8 @@ int device_scratch(size_t bytes, void** out, cudaStream_t s) {
             GB_CUDA(cudaStreamSynchronize(s));
             GB_CUDA(cudaFree(slot.first));
         }
-        size_t cap = bytes < (1 << 20) ? (1 << 20) : bytes;
+        constexpr size_t least = sizeof(double) * (1 << 20);
+        const size_t cap = bytes < least ? least : bytes;
         GB_CUDA(cudaMalloc(&slot.first, cap));
         slot.second = cap;
     }
@@ -747,7 +751,9 @@ static int wake_rollup(int32_t nsurf, const gbvlm_dims* dims, T* const* verts_wa
     w.sigma2 = sigma * sigma;
     const int64_t slices = lattice_slices(pieces, w.npts, 3, LT_SCRATCH);
     void* scratch = nullptr;
-    rc = device_scratch(sizeof(T) * 3 * slices * w.npts, &scratch, st);
+    int64_t whole = 0;  // the wakes' vertices: the size does not depend on the iteration
+    for (int m = 0; m < nsurf; m++) whole += dims[m].nwv * (dims[m].ns + 1);
+    rc = device_scratch(sizeof(T) * std::max(3 * slices * w.npts, 3 * whole), &scratch, st);
     if (rc) return rc;
     w.partial = (T*)scratch;
     dim3 grid((unsigned)cdiv(w.npts, LT_THREADS), (unsigned)slices);
