@@ -1121,26 +1121,46 @@ static bool batch_fast(gbvlm_batch h) {
     return false;
 }
 
-// Looks a group's AICs (systems i0 ..) over before their factorisation (k_lu_keep's
-// look, a warp per column): the rings of the next two rows, where a column that
-// needs an interchange shows it (16 wings of 36 to 2304 unknowns that do: in 70 %
-// of their columns with a larger entry anywhere, in every wing).  A system that
-// does is not attempted.
+// Looks a group's AICs (systems i0 ..) over before their factorisation, as
+// k_lu_keep does, but in each column only the rings of the next two rows, where a
+// column that needs an interchange shows it (16 wings of 36 to 2304 unknowns that
+// do: in 70 % of their columns with a larger entry anywhere, in every wing).  A
+// system that does is not attempted.  Bound: latency; a warp takes LOOK_COLS
+// columns at once (512 wings: LOOK_OLD us a column each, LOOK_NEW us).
+constexpr int LOOK_COLS = 8;
+
 __global__ void __launch_bounds__(256) k_batch_look(BatchArgs a, int32_t i0) {
     const int32_t si = i0 + blockIdx.y;
     const SysDesc& S = a.sys[si];
-    const int64_t n = S.n, j = blockIdx.x * 8 + (threadIdx.x >> 5);
-    if (j >= n) return;
-    const float* c = S.A + j * n;
-    const float d = fabsf(c[j]);
-    const int64_t end = min(n, j + 2 + 2 * S.ns);
-    bool good = true;
-    for (int64_t r = j + 1 + (threadIdx.x & 31); r < end; r += 32) good = good && fabsf(c[r]) <= d;  // (not for a NaN)
-    if (!__all_sync(0xffffffffu, good) && (threadIdx.x & 31) == 0) {
-        a.hint[si * a.hint_ld + j / LU_NB] = 1;
+    const int64_t n = S.n, j0 = (blockIdx.x * 8 + (threadIdx.x >> 5)) * (int64_t)LOOK_COLS;
+    if (j0 >= n) return;
+    const int lane = threadIdx.x & 31;
+    const float* c[LOOK_COLS];  // column j0 + u from its diagonal down
+    float d[LOOK_COLS];
+    bool good[LOOK_COLS];
+#pragma unroll
+    for (int u = 0; u < LOOK_COLS; u++) {
+        const int64_t j = min(j0 + u, n - 1);
+        c[u] = S.A + j * (n + 1);
+        d[u] = fabsf(*c[u]);
+        good[u] = true;
+    }
+    for (int64_t r = 1 + lane; r <= 2 * S.ns + 1; r += 32) {
+        float v[LOOK_COLS];
+#pragma unroll
+        for (int u = 0; u < LOOK_COLS; u++) v[u] = j0 + u + r < n ? fabsf(c[u][r]) : 0.f;
+#pragma unroll
+        for (int u = 0; u < LOOK_COLS; u++) good[u] = good[u] && v[u] <= d[u];  // (not for a NaN)
+    }
+    int bad = 0;
+#pragma unroll
+    for (int u = 0; u < LOOK_COLS; u++) bad |= __all_sync(0xffffffffu, good[u]) ? 0 : 1;
+    if (bad && lane == 0) {
+        a.hint[si * a.hint_ld + j0 / LU_NB] = 1;
         a.fail[si] = LU_SEEN;
     }
 }
+static_assert(LU_NB % LOOK_COLS == 0, "a warp's columns lie in one panel");
 
 __global__ void k_batch_restore(BatchArgs a) {
     if (a.skips(blockIdx.y)) return;
@@ -1221,7 +1241,7 @@ struct BatchRun {
     }
     int look(int g, cudaStream_t st) const {
         if (!looks(g)) return GBVLM_OK;
-        const dim3 gl((unsigned)cdiv(h->plans[g].maxn, 8), (unsigned)(h->gsys[g + 1] - h->gsys[g]));
+        const dim3 gl((unsigned)cdiv(h->plans[g].maxn, 8 * LOOK_COLS), (unsigned)(h->gsys[g + 1] - h->gsys[g]));
         k_batch_look<<<gl, 256, 0, st>>>(a, h->gsys[g]);
         GB_LAUNCH_CHECK();
         return GBVLM_OK;
