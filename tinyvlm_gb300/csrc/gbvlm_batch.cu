@@ -703,14 +703,17 @@ __global__ void k_batch_accum(BatchArgs a) {
 // exact through an FMA, running sums (sh, sl) kept with a compensated addition):
 // about 2^-48 of the running sum per term, where the fp64 units of this part run
 // at a small fraction of the fp32 rate.
-// Bound: the fp32 pipe (ten operations a term): 16384 panels, 64 right-hand sides
-// 8.5 ms.  Not kept: the sums of eight columns on a bias of 32 times their largest
-// product, four operations a term and 6.8 ms, but six times the error (median of
-// random rows of 512 terms 2.0e-14 of the sum of |a x|, 3.4e-15 here); columns
-// and X fetched ahead, asynchronously (the run 60.6 -> 61.0 ms).
+// Bound: the fp32 pipe (ten operations a term), in a small batch the latency of
+// its loads, so the columns and X are fetched ahead, asynchronously (loads where
+// they are used -> ahead: whole run of a 32 x 32 wing x 8 angles 2.12 -> 2.08 ms,
+// 64 wings x 4 exact 5.66 -> 5.58 ms, 512 x 8 11.46 -> 11.48 ms, 16384 panels x 64 60.9 -> 61.3
+// ms).  Not kept: the sums of eight columns on a bias of 32 times their largest
+// product, four operations a term, but six times the error (median of random rows
+// of 512 terms 2.0e-14 of the sum of |a x|, 3.4e-15 here).
 constexpr int RS_THREADS = 64;
 constexpr int RS_MAXRHS = 8;  // (the inner loop reads them as two float4)
 constexpr int RS_CB = 8;  // columns of Xd staged per step
+static_assert(RS_CB * RS_MAXRHS == RS_THREADS, "a thread stages one value");
 constexpr int RS_ROWS = 2;  // rows per thread
 
 // (sh, sl) += a * (xh + xl); XL = false: xl is zero
@@ -730,26 +733,51 @@ __device__ __forceinline__ void df_mac(float& sh, float& sl, float a, float xh, 
 // the float product is exact to far below the residual's accuracy).
 // XL = false: Xd holds float values (the first sweep: Xd = 0 + the float
 // solve), so its lo part is zero and its products are left out.
+constexpr int RS_STAGES = 3;
+constexpr int RS_MIN_BLOCKS = 6;
+
+// 4 bytes to shared memory, asynchronously; zero where !valid (src is still an address of the matrix)
+__device__ __forceinline__ void copy4_async(float* dst, const float* src, bool valid) {
+    const uint32_t d = (uint32_t)__cvta_generic_to_shared(dst), bytes = valid ? 4u : 0u;
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(d), "l"(src), "r"(bytes) : "memory");
+}
+
 template <bool LO, bool XL>
-__global__ void __launch_bounds__(RS_THREADS) k_batch_residual(BatchArgs a, const int64_t* rpfx) {
-    __shared__ __align__(16) float xh[RS_CB][RS_MAXRHS];
-    __shared__ __align__(16) float xl[RS_CB][RS_MAXRHS];
+__global__ void __launch_bounds__(RS_THREADS, RS_MIN_BLOCKS) k_batch_residual(BatchArgs a, const int64_t* rpfx) {
+    constexpr int ROWS = RS_THREADS * RS_ROWS;
+    __shared__ __align__(16) float xh[2][RS_CB][RS_MAXRHS];
+    __shared__ __align__(16) float xl[XL ? 2 : 1][RS_CB][RS_MAXRHS];
+    __shared__ float sa[RS_STAGES][RS_CB][ROWS];         // a thread reads what it copied itself
+    __shared__ float sl_[LO ? RS_STAGES : 1][LO ? RS_CB : 1][LO ? ROWS : 1];
     const int si = find_sys(rpfx, a.nsys, blockIdx.x);
     const SysDesc& S = a.sys[si];
     // RS_ROWS rows per thread, RS_THREADS apart: each staged value of X is
     // read once from shared memory for all of them
-    const int64_t r0 = (blockIdx.x - rpfx[si]) * (RS_THREADS * RS_ROWS) + threadIdx.x;
+    const int64_t r0 = (blockIdx.x - rpfx[si]) * ROWS + threadIdx.x;
     const int64_t n = S.n;
     bool rv[RS_ROWS];
-    const float* arow[RS_ROWS];
-    const float* lrow[RS_ROWS];
 #pragma unroll
-    for (int k = 0; k < RS_ROWS; k++) {
-        const int64_t r = r0 + k * RS_THREADS;
-        rv[k] = r < n;
-        arow[k] = S.A2 + (rv[k] ? r : 0);
-        lrow[k] = LO ? S.Alo + (rv[k] ? r : 0) : nullptr;
-    }
+    for (int k = 0; k < RS_ROWS; k++) rv[k] = r0 + k * RS_THREADS < n;
+    const int64_t nchunk = (n + RS_CB - 1) / RS_CB;
+    // chunk c's columns of this thread's rows, one group of asynchronous copies (empty past the last chunk)
+    auto fetch = [&](int64_t c) {
+        if (c < nchunk) {
+            const int st = (int)(c % RS_STAGES);
+#pragma unroll
+            for (int cc = 0; cc < RS_CB; cc++) {
+                const int64_t col = c * RS_CB + cc;
+#pragma unroll
+                for (int k = 0; k < RS_ROWS; k++) {
+                    const bool ok = col < n && rv[k];
+                    const int64_t off = ok ? r0 + k * RS_THREADS + col * n : 0;
+                    copy4_async(&sa[st][cc][threadIdx.x + k * RS_THREADS], S.A2 + off, ok);
+                    if constexpr (LO)
+                        copy4_async(&sl_[st][cc][threadIdx.x + k * RS_THREADS], S.Alo + off, ok);
+                }
+            }
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
     // grid.y: blocks of RS_MAXRHS right-hand sides
     for (int q0 = blockIdx.y * RS_MAXRHS; q0 < S.nrhs; q0 += RS_MAXRHS * gridDim.y) {
         const int nq = min(RS_MAXRHS, S.nrhs - q0);
@@ -758,49 +786,53 @@ __global__ void __launch_bounds__(RS_THREADS) k_batch_residual(BatchArgs a, cons
         for (int k = 0; k < RS_ROWS; k++)
 #pragma unroll
             for (int q = 0; q < RS_MAXRHS; q++) sh[k][q] = sl[k][q] = 0.f;
-        for (int64_t c0 = 0; c0 < n; c0 += RS_CB) {
-            __syncthreads();
-            for (int e = threadIdx.x; e < RS_CB * RS_MAXRHS; e += RS_THREADS) {
-                const int cc = e / RS_MAXRHS, q = e % RS_MAXRHS;
-                const double v = (c0 + cc < n && q < nq) ? S.Xd[(c0 + cc) + (q0 + q) * n] : 0.0;
-                const float h = (float)v;
-                xh[cc][q] = h;
-                if (XL) xl[cc][q] = (float)(v - (double)h);
+        const int xc = threadIdx.x / RS_MAXRHS, xq = threadIdx.x % RS_MAXRHS;  // the value of X this thread stages
+        auto xval = [&](int64_t c) {
+            const int64_t col = c * RS_CB + xc;
+            return (col < n && xq < nq) ? S.Xd[col + (q0 + xq) * n] : 0.0;
+        };
+        double xnext = xval(0);
+#pragma unroll
+        for (int c = 0; c < RS_STAGES - 1; c++) fetch(c);
+        __syncthreads();  // the last sweep's readers of xh are done
+        for (int64_t c = 0; c < nchunk; c++) {
+            const int b = (int)(c & 1), st = (int)(c % RS_STAGES);
+            {
+                const float h = (float)xnext;
+                xh[b][xc][xq] = h;
+                if (XL) xl[b][xc][xq] = (float)(xnext - (double)h);
             }
+            xnext = xval(c + 1);
+            fetch(c + RS_STAGES - 1);
+            asm volatile("cp.async.wait_group %0;" ::"n"(RS_STAGES - 1) : "memory");  // chunk c is there
             __syncthreads();
-            if (rv[0]) {
-                const int cn = (int)min((int64_t)RS_CB, n - c0);
-                float av[RS_ROWS][RS_CB], lv[RS_ROWS][RS_CB];
 #pragma unroll
-                for (int k = 0; k < RS_ROWS; k++)
+            for (int cc = 0; cc < RS_CB; cc++) {
+                // the 8 hi and 8 lo values of column cc as four 16-byte broadcasts
+                const float4 h0 = *reinterpret_cast<const float4*>(&xh[b][cc][0]);
+                const float4 h1 = *reinterpret_cast<const float4*>(&xh[b][cc][4]);
+                const float hh[RS_MAXRHS] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
+                float ll[RS_MAXRHS] = {};
+                if (XL) {
+                    const float4 l0 = *reinterpret_cast<const float4*>(&xl[XL ? b : 0][cc][0]);
+                    const float4 l1 = *reinterpret_cast<const float4*>(&xl[XL ? b : 0][cc][4]);
+                    ll[0] = l0.x, ll[1] = l0.y, ll[2] = l0.z, ll[3] = l0.w;
+                    ll[4] = l1.x, ll[5] = l1.y, ll[6] = l1.z, ll[7] = l1.w;
+                }
 #pragma unroll
-                    for (int cc = 0; cc < RS_CB; cc++) {
-                        av[k][cc] = (cc < cn && rv[k]) ? arow[k][(c0 + cc) * n] : 0.f;
-                        if (LO) lv[k][cc] = (cc < cn && rv[k]) ? lrow[k][(c0 + cc) * n] : 0.f;
+                for (int k = 0; k < RS_ROWS; k++) {
+                    const float av = sa[st][cc][threadIdx.x + k * RS_THREADS];
+                    float lv = 0.f;
+                    if constexpr (LO) lv = sl_[st][cc][threadIdx.x + k * RS_THREADS];
+#pragma unroll
+                    for (int q = 0; q < RS_MAXRHS; q++) {
+                        df_mac<XL>(sh[k][q], sl[k][q], av, hh[q], ll[q]);
+                        if (LO) sl[k][q] = __fmaf_rn(lv, hh[q], sl[k][q]);
                     }
-#pragma unroll
-                for (int cc = 0; cc < RS_CB; cc++) {
-                    // the 8 hi and 8 lo values of column cc as four 16-byte broadcasts
-                    const float4 h0 = *reinterpret_cast<const float4*>(&xh[cc][0]);
-                    const float4 h1 = *reinterpret_cast<const float4*>(&xh[cc][4]);
-                    const float hh[RS_MAXRHS] = {h0.x, h0.y, h0.z, h0.w, h1.x, h1.y, h1.z, h1.w};
-                    float ll[RS_MAXRHS] = {};
-                    if (XL) {
-                        const float4 l0 = *reinterpret_cast<const float4*>(&xl[cc][0]);
-                        const float4 l1 = *reinterpret_cast<const float4*>(&xl[cc][4]);
-                        ll[0] = l0.x, ll[1] = l0.y, ll[2] = l0.z, ll[3] = l0.w;
-                        ll[4] = l1.x, ll[5] = l1.y, ll[6] = l1.z, ll[7] = l1.w;
-                    }
-#pragma unroll
-                    for (int k = 0; k < RS_ROWS; k++)
-#pragma unroll
-                        for (int q = 0; q < RS_MAXRHS; q++) {
-                            df_mac<XL>(sh[k][q], sl[k][q], av[k][cc], hh[q], ll[q]);
-                            if (LO) sl[k][q] = __fmaf_rn(lv[k][cc], hh[q], sl[k][q]);
-                        }
                 }
             }
         }
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
         for (int k = 0; k < RS_ROWS; k++) {
             if (!rv[k]) continue;
@@ -1449,8 +1481,8 @@ __global__ void k_batch_condition(const int32_t* fail, int32_t n, int32_t mask, 
 // factored beside its others, under the condition that there is one; one that
 // turns out to need them, after all groups, likewise; then the solves, all
 // systems.  Measured, 512 wings x 8 angles (interchanges for all from the start,
-// these conditions): no such wing 13.4, 10.1 ms, one of middle size 13.5, 10.9, half
-// of them 22.3, 20.8; one elliptic 64 x 64 wing x 64 angles 10.8, 8.8.
+// these conditions): no such wing 13.4, 10.4 ms, one of middle size 13.5, 11.2, half
+// of them 22.3, 21.3; one elliptic 64 x 64 wing x 64 angles 10.8, 9.1.
 static int batch_capture(gbvlm_batch h) {
     using Nodes = std::vector<cudaGraphNode_t>;
     cudaGraph_t g = nullptr;
