@@ -1159,7 +1159,7 @@ static bool batch_fast(gbvlm_batch h) {
 // do: in 70 % of their columns with a larger entry anywhere, in every wing).  A
 // system that does is not attempted.  Bound: latency; a warp takes LOOK_COLS
 // columns at once (512 wings: LOOK_OLD us a column each, LOOK_NEW us).
-constexpr int LOOK_COLS = 8;
+constexpr int LOOK_COLS = 2, LOOK_ROWS = 8;
 
 __global__ void __launch_bounds__(256) k_batch_look(BatchArgs a, int32_t i0) {
     const int32_t si = i0 + blockIdx.y;
@@ -1177,12 +1177,20 @@ __global__ void __launch_bounds__(256) k_batch_look(BatchArgs a, int32_t i0) {
         d[u] = fabsf(*c[u]);
         good[u] = true;
     }
-    for (int64_t r = 1 + lane; r <= 2 * S.ns + 1; r += 32) {
-        float v[LOOK_COLS];
+    const int64_t end = 2 * S.ns + 2;
+    for (int64_t r0 = 1 + lane; r0 < end; r0 += 32 * LOOK_ROWS) {
+        float v[LOOK_COLS][LOOK_ROWS];
 #pragma unroll
-        for (int u = 0; u < LOOK_COLS; u++) v[u] = j0 + u + r < n ? fabsf(c[u][r]) : 0.f;
+        for (int u = 0; u < LOOK_COLS; u++)
 #pragma unroll
-        for (int u = 0; u < LOOK_COLS; u++) good[u] = good[u] && v[u] <= d[u];  // (not for a NaN)
+            for (int t = 0; t < LOOK_ROWS; t++) {
+                const int64_t r = r0 + 32 * t;
+                v[u][t] = r < end && j0 + u + r < n ? fabsf(c[u][r]) : 0.f;
+            }
+#pragma unroll
+        for (int u = 0; u < LOOK_COLS; u++)
+#pragma unroll
+            for (int t = 0; t < LOOK_ROWS; t++) good[u] = good[u] && v[u][t] <= d[u];  // (not for a NaN)
     }
     int bad = 0;
 #pragma unroll
