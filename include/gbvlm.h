@@ -544,11 +544,6 @@ int gbvlm_uvlm_loop_wait(gbvlm_uvlm_loop l, int64_t ticket, double timeout_s, in
 /* requests submitted and completed so far, and graph launches they took */
 int gbvlm_uvlm_loop_stats(gbvlm_uvlm_loop l, int64_t* submitted, int64_t* completed, int64_t* launches);
 int gbvlm_uvlm_loop_destroy(gbvlm_uvlm_loop l);
-/* Test hooks with no counterpart in the reference: A x = b (device arrays, A
- * column-major) as the steps of a long unsteady run solve it, by the inverse and
- * one step of iterative refinement. */
-int gbvlm_test_inverse_solve_f32(const float* A, int64_t n, const float* b, float* x, gbvlm_stream stream);
-int gbvlm_test_inverse_solve_f64(const double* A, int64_t n, const double* b, double* x, gbvlm_stream stream);
 /* gbvlm_test_lu_withhold for the handle's solver (float runs, begun before). */
 int gbvlm_test_uvlm_withhold(gbvlm_uvlm h, gbvlm_stream stream);
 /* cl: t_steps doubles, cm: 3*t_steps, gamma_last: n doubles of the last step (each may be NULL). Synchronous. */

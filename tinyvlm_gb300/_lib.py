@@ -100,8 +100,6 @@ def _protos():
     for who in ("lu", "nlvlm", "aero2dof", "uvlm"):
         t["gbvlm_test_%s_withhold" % who] = [P, P]
     t["gbvlm_test_lu_solve_check"] = [P, P]
-    for sfx in ("f32", "f64"):
-        t["gbvlm_test_inverse_solve_" + sfx] = [P, I64, P, P, P]
     t["gbvlm_test_walk_math"] = [I32, I64, P, P, P, P]
     t["gbvlm_test_pivot_rcp"] = [I64, P, P, P, P, P]
     t["gbvlm_test_batch_residual"] = [I64, I32, P, P, P, P, P, I32, P]

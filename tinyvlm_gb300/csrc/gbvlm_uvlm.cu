@@ -254,14 +254,10 @@ static int step_loads(const StepArgs<T>& a, int64_t step, bool loads, cudaStream
 // The AIC is factored once and solved for at every step, a chain of n / 128
 // (n / 64 in double) dependent blocks twice over.  A run of many steps forms
 // the inverse instead, as the solution for the identity, and a step's solve is
-// three products, no chain, the matrices read from L2: x = M b, its residual
-// with the AIC itself, and M times that on top (one step of iterative
-// refinement).  The product with the inverse alone is less exact than the solve
-// (1.04 to 1.25 times its error for wings of 48 to 900 panels, in float as in
-// double); refined once, it has a third to two thirds of the solve's error.
-// 1600 panels in float: a solve 71 us, a product 6, the inverse once 0.52 ms (500
-// steps with the solve 126 ms, 103 with this); 576 in double: 147, 5 and 1.15 ms
-// (160 steps 140 and 121 ms).
+// a product with it: every row by a warp of its own, no chain, the matrix read
+// from L2.  1600 panels in float: a solve 71 us, the product 6, the inverse
+// once 0.52 ms (500 steps 126 -> 97 ms); 576 in double: 147, 5 and 1.15 ms (160
+// steps 140 -> 120 ms).
 // inv_steps: the number of steps from which the inverse is formed.  It costs
 // as much as 3 to 13 solves up to 2304 unknowns and 36 at 4096 (double: 1 to 12
 // up to 1024, 50 at 2304, beyond that the solve for many columns is out of
@@ -304,11 +300,10 @@ __global__ void __launch_bounds__(256) k_transpose(T* m, int64_t n, int64_t ld) 
     }
 }
 
-// x = sign M b (+ c), M by rows with a leading dimension of whole 16-byte vectors
-// (M and b zero from n to there); c null: without it
+// x = M b, M by rows with a leading dimension of whole 16-byte vectors (M and b
+// zero from n to there)
 template <class T>
-__global__ void __launch_bounds__(32 * INV_WARPS) k_matrix_apply(const T* M, int64_t n, int64_t ld, const T* b, T sign,
-                                                                 const T* c, T* x) {
+__global__ void __launch_bounds__(32 * INV_WARPS) k_inverse_apply(const T* M, int64_t n, int64_t ld, const T* b, T* x) {
     constexpr int V = 16 / sizeof(T);
     struct alignas(16) Vec {
         T v[V];
@@ -329,7 +324,7 @@ __global__ void __launch_bounds__(32 * INV_WARPS) k_matrix_apply(const T* M, int
     if constexpr (V == 4) s += acc[2] + acc[3];
 #pragma unroll
     for (int d = 16; d > 0; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
-    if ((threadIdx.x & 31) == 0) x[r] = c ? c[r] + sign * s : sign * s;
+    if ((threadIdx.x & 31) == 0) x[r] = s;
 }
 
 template <class T>
@@ -368,58 +363,6 @@ struct Ops2;
 OPS2(float, f32)
 OPS2(double, f64)
 
-// the inverse of an AIC, the AIC and the vectors of a solve with them, in the caller's memory
-template <class T>
-struct Inverse {
-    T *inv = nullptr, *aic = nullptr;             // by rows, n x ld
-    T *x0 = nullptr, *res = nullptr, *x = nullptr;  // ld each, zero from n on; x: the solution
-    int64_t n = 0, ld = 0;
-
-    // values from the (zeroed) memory of the owner
-    template <class Take>
-    void place(int64_t n_, Take&& take) {
-        n = n_;
-        ld = inv_ld<T>(n);
-        inv = take(n * ld);
-        aic = take(n * ld);
-        x0 = take(ld);
-        res = take(ld);
-        x = take(ld);
-    }
-    static int64_t bytes(int64_t n) {
-        const int64_t ld = inv_ld<T>(n);
-        return 2 * ((sizeof(T) * n * ld + 255) / 256 * 256) + 3 * ((sizeof(T) * ld + 255) / 256 * 256);
-    }
-    int transpose(T* m, cudaStream_t st) const {
-        const dim3 g((unsigned)cdiv(n, 32), (unsigned)cdiv(n, 32));
-        k_transpose<T><<<g, 256, 0, st>>>(m, n, ld);
-        GB_LAUNCH_CHECK();
-        return GBVLM_OK;
-    }
-    // before the factorisation: the AIC (column-major, n apart)
-    int keep(const T* lhs, cudaStream_t st) const {
-        GB_CUDA(cudaMemcpy2DAsync(aic, sizeof(T) * ld, lhs, sizeof(T) * n, sizeof(T) * n, n, cudaMemcpyDeviceToDevice, st));
-        return transpose(aic, st);
-    }
-    // after it
-    int form(gbvlm_lu lu, const T* factors, cudaStream_t st) const {
-        GB_CUDA(cudaMemsetAsync(inv, 0, sizeof(T) * n * ld, st));
-        k_set_diagonal<T><<<(unsigned)cdiv(n, 256), 256, 0, st>>>(inv, n, ld);
-        GB_LAUNCH_CHECK();
-        const int rc = Ops2<T>::solve_many(lu, factors, n, inv, ld, n, (gbvlm_stream)st);
-        return rc ? rc : transpose(inv, st);
-    }
-    // x for the right-hand side b (16-byte aligned, ld values, zero from n on)
-    int apply(const T* b, cudaStream_t st) const {
-        const unsigned g = (unsigned)cdiv(n, INV_WARPS);
-        k_matrix_apply<T><<<g, 32 * INV_WARPS, 0, st>>>(inv, n, ld, b, (T)1, nullptr, x0);
-        k_matrix_apply<T><<<g, 32 * INV_WARPS, 0, st>>>(aic, n, ld, x0, (T)-1, b, res);
-        k_matrix_apply<T><<<g, 32 * INV_WARPS, 0, st>>>(inv, n, ld, res, (T)1, x0, x);
-        GB_LAUNCH_CHECK();
-        return GBVLM_OK;
-    }
-};
-
 // Device-indexed UVLM step (float, no roll-up): the step index i lives in
 // idx[0] on the device, so one captured graph advances the case any number of
 // times.  Its last launch: i -> i + 1.
@@ -448,8 +391,8 @@ struct UvlmState : UvlmBase {
     std::vector<T*> vinit, vpos, verts, wake, colloc, colloc0, normals, areas, gamma, gprev, gwake, vel;
     T *lhs = nullptr, *rhs = nullptr, *Tm = nullptr, *Tdm = nullptr, *fs = nullptr, *ref = nullptr;
     double* res = nullptr;  // [t_steps][4]
-    bool inverse = false;  // the run pays for the AIC's inverse
-    Inverse<T> inv;
+    T *inv = nullptr, *sol = nullptr;  // the AIC's inverse by rows and its product, where the run pays for it
+    int64_t ldi = 0;
     gbvlm_lu lu = nullptr;
 
     // device-indexed step (step_graph): counter, wake scratch, the staged LU
@@ -491,8 +434,8 @@ struct UvlmState : UvlmBase {
         bytes += al(sizeof(T) * n * n) + al(sizeof(T) * n) + 2 * al(sizeof(T) * 16 * nsurf * (t_steps + 1)) +
                  2 * al(sizeof(T) * 3 * (t_steps + 1)) + al(sizeof(double) * 4 * t_steps) +
                  al(sizeof(double) * LOAD_PART * step_load_blocks(dims)) + al(sizeof(unsigned));
-        inverse = t_steps - 1 >= inv_steps<T>(n);
-        if (inverse) bytes += Inverse<T>::bytes(n);
+        ldi = t_steps - 1 >= inv_steps<T>(n) ? inv_ld<T>(n) : 0;
+        bytes += al(sizeof(T) * n * ldi) + al(sizeof(T) * ldi);
         GB_CUDA(cudaMalloc(&mem, bytes));
         GB_CUDA(cudaMemset(mem, 0, bytes));
         char* p = (char*)mem;
@@ -503,7 +446,10 @@ struct UvlmState : UvlmBase {
         };
         lhs = take(n * n);
         rhs = take(n);  // (to a multiple of 256 bytes, zero past n)
-        if (inverse) inv.place(n, take);
+        if (ldi) {
+            inv = take(n * ldi);
+            sol = take(ldi);
+        }
         Tm = take(16 * nsurf * (t_steps + 1));
         Tdm = take(16 * nsurf * (t_steps + 1));
         fs = take(3 * (t_steps + 1));
@@ -554,7 +500,7 @@ struct UvlmState : UvlmBase {
         }
         sa.nwv = t_steps;
         sa.rhs = rhs;
-        sa.sol = inverse ? inv.x : rhs;
+        sa.sol = inv ? sol : rhs;
         sa.Tm = Tm;
         sa.Tdm = Tdm;
         sa.fs = fs;
@@ -638,11 +584,24 @@ struct UvlmState : UvlmBase {
         GB_CUDA(cudaMemsetAsync(lhs, 0, sizeof(T) * n * n, st));
         if ((rc = Ops2<T>::lhs(lhs, n, nsurf, dims.data(), C(colloc).data(), C(normals).data(), C(verts).data(), sigma, s)))
             return rc;
-        if (inverse && (rc = inv.keep(lhs, st))) return rc;
         if ((rc = Ops2<T>::factor(lu, lhs, n, s))) return rc;
-        if (inverse && (rc = inv.form(lu, lhs, st))) return rc;
+        if (inv) {
+            GB_CUDA(cudaMemsetAsync(inv, 0, sizeof(T) * n * ldi, st));
+            k_set_diagonal<T><<<(unsigned)cdiv(n, 256), 256, 0, st>>>(inv, n, ldi);
+            GB_LAUNCH_CHECK();
+            if ((rc = Ops2<T>::solve_many(lu, lhs, n, inv, ldi, n, s))) return rc;
+            const dim3 g((unsigned)cdiv(n, 32), (unsigned)cdiv(n, 32));
+            k_transpose<T><<<g, 256, 0, st>>>(inv, n, ldi);
+            GB_LAUNCH_CHECK();
+        }
         sa.inv_dt = (T)1 / dt;
         GB_CUDA(cudaMemsetAsync(res, 0, sizeof(double) * 4 * t_steps, st));
+        return GBVLM_OK;
+    }
+
+    int apply_inverse(cudaStream_t st) {
+        k_inverse_apply<T><<<(unsigned)cdiv(n, INV_WARPS), 32 * INV_WARPS, 0, st>>>(inv, n, ldi, rhs, sol);
+        GB_LAUNCH_CHECK();
         return GBVLM_OK;
     }
 
@@ -660,7 +619,7 @@ struct UvlmState : UvlmBase {
             if ((rc = Ops2<T>::wake(rhs, nsurf, dims.data(), C(gwake).data(), C(colloc).data(), C(normals).data(),
                                     C(wake).data(), lifting.data(), (int32_t)i, sigma, s)))
                 return rc;
-            if ((rc = inverse ? inv.apply(rhs, st) : Ops2<T>::solve(lu, lhs, n, rhs, s))) return rc;
+            if ((rc = inv ? apply_inverse(st) : Ops2<T>::solve(lu, lhs, n, rhs, s))) return rc;
             if ((rc = step_loads(sa, i, i > 0, st))) return rc;
             if (roll && i > 0) {
                 if ((rc = Ops2<T>::rollup(nsurf, dims.data(), wake.data(), C(verts).data(), C(gamma).data(),
@@ -710,7 +669,7 @@ struct UvlmState : UvlmBase {
                                         C(normals).data(), C(wake).data(), lifting.data(), d_idx,
                                         (int32_t)(t_steps - 2), wsc, c)))
             return r;
-        if ((r = inverse ? inv.apply(rhs, c) : lu_solve_prepared_f32(lu, lut, n, c))) return r;
+        if ((r = inv ? apply_inverse(c) : lu_solve_prepared_f32(lu, lut, n, c))) return r;
         if ((r = step_loads(a, 0, true, c))) return r;
         if ((r = step_move(a, 0, c))) return r;
         k_uvlm_dev_end<<<1, 1, 0, c>>>(d_idx);
@@ -726,7 +685,7 @@ struct UvlmState : UvlmBase {
             wsc = (float*)((char*)dmem + 256);
         }
         if constexpr (std::is_same<T, float>::value) {
-            if (!lut && !inverse) {
+            if (!lut && !inv) {
                 int rc = lu_solve_prepare_f32(lu, lhs, n, rhs, &lut, st);
                 if (rc) return rc;
             }
@@ -1619,43 +1578,6 @@ int gbvlm_aero2dof_run(gbvlm_aero2dof h, int64_t steps, int32_t max_iter, gbvlm_
     GB_REQUIRE(h && steps >= 0 && max_iter >= 1, "bad arguments");
     return ((Aero2Dof*)h)->run(steps, max_iter, to_cuda(stream));
 }
-
-#define TEST_INVERSE(T, sfx)                                                                                        \
-    int gbvlm_test_inverse_solve_##sfx(const T* A, int64_t n, const T* b, T* x, gbvlm_stream stream) {             \
-        GB_REQUIRE(A && b && x && n >= 1, "bad arguments");                                                        \
-        cudaStream_t st = to_cuda(stream);                                                                         \
-        const size_t bytes = Inverse<T>::bytes(n) + sizeof(T) * (n * n + inv_ld<T>(n)) + 512;                       \
-        char* mem = nullptr;                                                                                       \
-        gbvlm_lu lu = nullptr;                                                                                     \
-        auto run = [&]() -> int {                                                                                  \
-            GB_CUDA(cudaMalloc(&mem, bytes));                                                                      \
-            GB_CUDA(cudaMemsetAsync(mem, 0, bytes, st));                                                           \
-            char* p = mem;                                                                                         \
-            auto take = [&](int64_t c) {                                                                           \
-                T* r = (T*)p;                                                                                      \
-                p += (sizeof(T) * c + 255) / 256 * 256;                                                            \
-                return r;                                                                                          \
-            };                                                                                                     \
-            Inverse<T> inv;                                                                                        \
-            inv.place(n, take);                                                                                    \
-            T *rhs = take(inv.ld), *F = take(n * n);                                                               \
-            GB_CUDA(cudaMemcpyAsync(F, A, sizeof(T) * n * n, cudaMemcpyDeviceToDevice, st));                       \
-            GB_CUDA(cudaMemcpyAsync(rhs, b, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));                         \
-            int rc = gbvlm_lu_create(&lu);                                                                         \
-            if (rc || (rc = inv.keep(F, st)) || (rc = Ops2<T>::factor(lu, F, n, stream)) ||                        \
-                (rc = inv.form(lu, F, st)) || (rc = inv.apply(rhs, st)))                                           \
-                return rc;                                                                                         \
-            GB_CUDA(cudaMemcpyAsync(x, inv.x, sizeof(T) * n, cudaMemcpyDeviceToDevice, st));                       \
-            GB_CUDA(cudaStreamSynchronize(st));                                                                    \
-            return GBVLM_OK;                                                                                       \
-        };                                                                                                         \
-        const int rc = run();                                                                                      \
-        if (lu) gbvlm_lu_destroy(lu);                                                                              \
-        if (mem) cudaFree(mem);                                                                                    \
-        return rc;                                                                                                 \
-    }
-TEST_INVERSE(float, f32)
-TEST_INVERSE(double, f64)
 
 int gbvlm_test_aero2dof_withhold(gbvlm_aero2dof h, gbvlm_stream stream) {
     GB_REQUIRE(h, "null argument");
