@@ -258,6 +258,9 @@ static int step_loads(const StepArgs<T>& a, int64_t step, bool loads, cudaStream
 // from L2.  1600 panels in float: a solve 71 us, the product 6, the inverse
 // once 0.52 ms (500 steps 126 -> 97 ms); 576 in double: 147, 5 and 1.15 ms (160
 // steps 140 -> 120 ms).
+// Its error beside the solve's: float circulations after 500 steps of 1600 panels
+// 0.92 to 1.26 times, 1.05 on average over ten motions; double ones against
+// quadruple precision the same (1.22e-15 and 1.21e-15, 1.43e-15 and 1.46e-15).
 // inv_steps: the number of steps from which the inverse is formed.  It costs
 // as much as 3 to 13 solves up to 2304 unknowns and 36 at 4096 (double: 1 to 12
 // up to 1024, 50 at 2304, beyond that the solve for many columns is out of
